@@ -21,47 +21,11 @@ int fp_auto_groups(int64_t ray_blocks, int n_slabs) {
     return s;
 }
 
-// True if any ray of the view is x-driven (|x21| > |y21|, cu_projection.cu:39),
-// evaluated with the float arithmetic of the kernel's ray setup.
-bool view_has_xdrive(float angle, const Geom &g) {
-    const float cphi = cosf(angle), sphi = sinf(angle);
-    const float x1 = -g.SO * cphi, y1 = -g.SO * sphi;
-    const float x20 = g.SD - g.SO;
-    for (int ia = 0; ia < g.na; ia++) {
-        const float y20 = (ia + g.ai) * g.da;
-        const float x21 = (x20 * cphi - y20 * sphi) - x1;
-        const float y21 = (x20 * sphi + y20 * cphi) - y1;
-        // host and device cos/sin may differ in the last bit: be conservative
-        if (fabsf(x21) >= 0.999f * fabsf(y21)) return true;
-    }
-    return false;
-}
-
-// Which volume copies a view's projector reads: x-driven rays read the
-// y-fastest copy, y-driven rays the x-fastest one.  Evaluated with the float
-// arithmetic of the kernel's ray set-up and a margin for the last bit of the
-// host's and the device's sine and cosine, so a column near the switch
-// counts for both.
-void view_drive_axes(float angle, const Geom &g, bool *any_x, bool *any_y) {
-    const float cphi = cosf(angle), sphi = sinf(angle);
-    const float x1 = -g.SO * cphi, y1 = -g.SO * sphi;
-    const float x20 = g.SD - g.SO;
-    *any_x = *any_y = false;
-    for (int ia = 0; ia < g.na; ia++) {
-        const float y20 = (ia + g.ai) * g.da;
-        const float x21 = (x20 * cphi - y20 * sphi) - x1;
-        const float y21 = (x20 * sphi + y20 * cphi) - y1;
-        if (fabsf(x21) >= 0.999f * fabsf(y21)) *any_x = true;
-        if (fabsf(y21) >= 0.999f * fabsf(x21)) *any_y = true;
-    }
-}
-
 template <int K>
-int launch_fp_plain(mcsart_ctx *ctx, float *d_proj, const float *d_img, const float *d_imgT,
-                    float angle, const float *d_angles, int n_views, const Geom &g) {
+int launch_fp_plain(mcsart_ctx *ctx, float *d_proj, const float *d_imgZ, float angle,
+                    const float *d_angles, int n_views, const Geom &g) {
     FPArgs<float, K> a{};
-    a.vol.std[0] = d_img;
-    a.vol.tr[0] = d_imgT;
+    a.vol.zf[0] = d_imgZ;
     a.g = g;
     a.angle = angle;
     a.angles = d_angles;
@@ -70,16 +34,18 @@ int launch_fp_plain(mcsart_ctx *ctx, float *d_proj, const float *d_img, const fl
     // the reference's summation order: bitwise the reference kernel's output
     const dim3 grid(div_up(g.na, FPC_COLS), div_up(g.nb, FPC_ROWS), n_views);
     // several views (mcsart_projection_views): the multi-view instantiation
-    if (n_views > 1)
-        MC_LAUNCH(ctx, (fp_ref_kernel<K, false, float, float, true>), grid, dim3(FPC_THREADS), 0, a);
-    else
-        MC_LAUNCH(ctx, (fp_ref_kernel<K, false, float>), grid, dim3(FPC_THREADS), 0, a);
-    return MCSART_OK;
+    if (n_views > 1) return launch_fp_ref<K, false, float, float, true>(ctx, grid, a);
+    return launch_fp_ref<K, false, float>(ctx, grid, a);
 }
 
-int transpose_f32(mcsart_ctx *ctx, float *dstT, const float *src, int nx, int ny, int nz) {
-    const dim3 grid(div_up(nx, 32), div_up(ny, 32), nz), block(32, 8);
-    MC_LAUNCH(ctx, (transpose_kernel<float, float>), grid, block, 0, dstT, src, nx, ny);
+// The z-fastest copy of a volume the projector reads, in a workspace.
+template <typename VT>
+int zfast_copy(mcsart_ctx *ctx, const char *name, const VT *src, const Geom &g, const VT **out) {
+    void *ws;
+    MC_TRY(workspace(ctx, name, nvox(g.nx, g.ny, g.nz) * sizeof(VT), &ws));
+    MC_LAUNCH(ctx, (zfast_kernel<VT, VT>), zfast_grid(g.nx, g.ny, g.nz), dim3(32, 8), 0, (VT *)ws,
+              src, g.nx, g.ny, g.nz);
+    *out = (const VT *)ws;
     return MCSART_OK;
 }
 
@@ -108,14 +74,9 @@ MC_EXPORT int mcsart_projection(mcsart_ctx *ctx, float *d_proj, const float *d_i
     MC_REQUIRE(d_proj && d_img, "d_proj and d_img must be non-NULL");
     const Geom g = make_geom(SO, SD, da, na, ai, db, nb, bi, nx, ny, nz);
     MC_TRY(validate_geom(g));
-    const float *imgT = nullptr;
-    if (view_has_xdrive(angle, g)) {
-        void *ws;
-        MC_TRY(workspace(ctx, "fp_volT", nvox(nx, ny, nz) * sizeof(float), &ws));
-        MC_TRY(transpose_f32(ctx, (float *)ws, d_img, nx, ny, nz));
-        imgT = (const float *)ws;
-    }
-    MC_TRY(launch_fp_plain<1>(ctx, d_proj, d_img, imgT, angle, nullptr, 1, g));
+    const float *imgZ;
+    MC_TRY(zfast_copy(ctx, "fp_volZ", d_img, g, &imgZ));
+    MC_TRY(launch_fp_plain<1>(ctx, d_proj, imgZ, angle, nullptr, 1, g));
     return finish(ctx, "mcsart_projection");
 }
 
@@ -129,14 +90,13 @@ MC_EXPORT int mcsart_projection_views(mcsart_ctx *ctx, float *d_proj, const floa
     MC_REQUIRE(n_views > 0 && n_views <= 65535, "n_views must be in [1, 65535]");
     const Geom g = make_geom(SO, SD, da, na, ai, db, nb, bi, nx, ny, nz);
     MC_TRY(validate_geom(g));
-    void *wsT, *wsA;
-    MC_TRY(workspace(ctx, "fp_volT", nvox(nx, ny, nz) * sizeof(float), &wsT));
+    void *wsA;
+    const float *imgZ;
     MC_TRY(workspace(ctx, "fp_angles", (size_t)n_views * sizeof(float), &wsA));
     MC_CHECK_CUDA(cudaMemcpyAsync(wsA, h_angles, (size_t)n_views * sizeof(float),
                                   cudaMemcpyHostToDevice, ctx->stream));
-    MC_TRY(transpose_f32(ctx, (float *)wsT, d_img, nx, ny, nz));
-    MC_TRY(launch_fp_plain<1>(ctx, d_proj, d_img, (const float *)wsT, 0.0f, (const float *)wsA,
-                              n_views, g));
+    MC_TRY(zfast_copy(ctx, "fp_volZ", d_img, g, &imgZ));
+    MC_TRY(launch_fp_plain<1>(ctx, d_proj, imgZ, 0.0f, (const float *)wsA, n_views, g));
     // the angle staging buffer must outlive the launch before the host array is reused
     MC_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
     return finish(ctx, "mcsart_projection_views");
@@ -155,7 +115,7 @@ MC_EXPORT int mcsart_backprojection(mcsart_ctx *ctx, float *d_img, const float *
     a.g = g;
     a.angle = angle;
     a.out = d_img;
-    const dim3 grid(div_up(nx, 32), div_up(ny, BP_ROWS), div_up(nz, BP_NZ)), block(32, BP_ROWS);
+    const dim3 grid = bp_grid<BP_NZ, BP_ROWS>(g), block(32, BP_ROWS);
     if (bp_geom_proven(g))
         MC_LAUNCH(ctx, (bp_kernel<1, BP_PLAIN, false, true>), grid, block, 0, a);
     else
@@ -396,27 +356,17 @@ namespace {
 template <typename VT>
 int projection_ex_typed(mcsart_ctx *ctx, float *d_proj, const VT *d_img, int fp_sum, int geom64,
                         float angle, const Geom &g) {
-    const int64_t V = nvox(g.nx, g.ny, g.nz);
-    void *ws;
-    MC_TRY(workspace(ctx, "fp_volT_ex", V * sizeof(VT), &ws));
-    VT *imgT = (VT *)ws;
-    MC_LAUNCH(ctx, (transpose_kernel<VT, VT>), dim3(div_up(g.nx, 32), div_up(g.ny, 32), g.nz),
-              dim3(32, 8), 0, imgT, d_img, g.nx, g.ny);
     FPArgs<VT, 1, VT> a{};
-    a.vol.std[0] = d_img;
-    a.vol.tr[0] = imgT;
+    MC_TRY(zfast_copy(ctx, "fp_volZ_ex", d_img, g, &a.vol.zf[0]));
     a.g = g;
     a.angle = angle;
     a.mode = FP_PLAIN;
     a.out = d_proj;
-    if (fp_sum == SUM_REF) {
-        MC_LAUNCH(ctx, (fp_ref_kernel<1, false, VT, VT>),
-                  dim3(div_up(g.na, FPC_COLS), div_up(g.nb, FPC_ROWS), 1), dim3(FPC_THREADS), 0,
-                  a);
-        return MCSART_OK;
-    }
-    const int groups = fp_auto_groups((int64_t)div_up(g.na, 32) * g.nb, std::max(g.nx, g.ny));
-    const dim3 grid(div_up(g.na, 32), g.nb, 1), block(32, groups);
+    if (fp_sum == SUM_REF)
+        return launch_fp_ref<1, false, VT>(
+            ctx, dim3(div_up(g.na, FPC_COLS), div_up(g.nb, FPC_ROWS), 1), a);
+    const int groups = fp_auto_groups((int64_t)g.na * div_up(g.nb, 32), std::max(g.nx, g.ny));
+    const dim3 grid(g.na, div_up(g.nb, 32), 1), block(32, groups);
     const size_t smem = (size_t)groups * 2 * 32 * sizeof(float);
     if (fp_sum == SUM_PLAIN && geom64)
         MC_LAUNCH(ctx, (fp_kernel<1, false, SUM_PLAIN, VT, VT, true>), grid, block, smem, a);
@@ -494,7 +444,7 @@ MC_EXPORT int mcsart_backprojection_ex(mcsart_ctx *ctx, float *d_img, const floa
     a.g = g;
     a.angle = angle;
     a.out = d_img;
-    const dim3 grid(div_up(nx, 32), div_up(ny, BP_ROWS), div_up(nz, BP_NZ)), block(32, BP_ROWS);
+    const dim3 grid = bp_grid<BP_NZ, BP_ROWS>(g), block(32, BP_ROWS);
     MC_LAUNCH(ctx, (bp_kernel<1, BP_PLAIN, false, false, true>), grid, block, 0, a);
     return finish(ctx, "mcsart_backprojection_ex");
 }

@@ -123,7 +123,7 @@ struct BPArgs {
     float lambda;
     float *out;           // BP_PLAIN / BP_DIV: output (nullable in BP_DIV); BP_DIV_ADD:
                           // volume updated in place
-    float *outT;          // BP_DIV_ADD: y-fastest copy refreshed alongside (nullable)
+    float *outZ;          // BP_DIV_ADD: z-fastest copy refreshed alongside (nullable)
     cudaSurfaceObject_t outSurf;  // BP_DIV: 3D array receiving the ratio (0 = none)
     // Several views per launch (K == 2): n_views views of an ordered subset,
     // angles[v] (device) and pair + v*na*nb.  BP_DIV writes view v's ratio to
@@ -307,25 +307,25 @@ __device__ __forceinline__ void bp_gather_view64(const BPArgs &p, float angle, c
     }
 }
 
-// blockDim = (32, BP_ROWS); each thread backprojects the BP_NZ voxels
-// (ix, iy, z0 .. z0 + BP_NZ - 1), z0 = blockIdx.z * BP_NZ, for every view of
-// the launch.
+// blockDim = (32, ROWS); a block is 32 voxel columns of one row iy and
+// ROWS * NZ slices, each thread backprojects the NZ voxels (ix, iy, z0 ..
+// z0 + NZ - 1) for every view of the launch; grid bp_grid.
 // MULTI = false: one view (the reference's loop); the view loop and the
 // per-view outputs exist only in the ordered-subset instantiation, so that
 // the single-view kernel keeps its registers (and resident blocks).
 // GEO64: FP64 geometry and normaliser (bp_gather_view64; one view).
-// NZ (voxels per thread along z) and ROWS (voxel rows per block) are the
+// NZ (voxels per thread along z) and ROWS (threads along z) are the
 // launch shape the driver's tuning may choose; every shape gives the same
 // bits (each voxel's terms and their order do not depend on it).
 template <int K, int MODE, bool MULTI = false, bool PROVEN = false, bool GEO64 = false,
           int NZ = BP_NZ, int ROWS = BP_ROWS>
 __global__ void __launch_bounds__(256, (bp_min_blocks<GEO64, MULTI, NZ>())) bp_kernel(const BPArgs p) {
-    __shared__ float tile[NZ][ROWS][33];
     const Geom &g = p.g;
     const int tx = threadIdx.x, ty = threadIdx.y;
-    const int x0 = blockIdx.x * 32, y0 = blockIdx.y * ROWS, z0 = blockIdx.z * NZ;
-    const int ix = x0 + tx, iy = y0 + ty;
-    const bool active = ix < g.nx && iy < g.ny;
+    const unsigned gx = (g.nx + 31) / 32, by = blockIdx.x / gx;
+    const int x0 = (int)(blockIdx.x - by * gx) * 32, zb = blockIdx.y * (ROWS * NZ);
+    const int z0 = zb + ty * NZ, ix = x0 + tx, iy = (int)by;
+    const bool active = ix < g.nx;
     const int64_t plane = (int64_t)g.nx * g.ny, V = plane * g.nz, NP = (int64_t)g.na * g.nb;
     const int nv = MULTI ? p.n_views : 1;
 
@@ -369,6 +369,7 @@ __global__ void __launch_bounds__(256, (bp_min_blocks<GEO64, MULTI, NZ>())) bp_k
         }
     }
     if (MODE != BP_DIV_ADD) return;
+    __shared__ float tile[NZ * ROWS][33];
 #pragma unroll
     for (int k = 0; k < NZ; k++) {
         const int iz = z0 + k;
@@ -378,22 +379,24 @@ __global__ void __launch_bounds__(256, (bp_min_blocks<GEO64, MULTI, NZ>())) bp_k
             val = __fmaf_rn(qsum[k], p.lambda, p.out[id]);  // cu_add.cu:17
             p.out[id] = val;
         }
-        tile[k][ty][tx] = val;
+        tile[ty * NZ + k][tx] = val;
     }
-    if (p.outT != nullptr) {
+    if (p.outZ != nullptr) {
         __syncthreads();
-        // transposed store outT[iy + ix*ny + iz*nx*ny]: ROWS consecutive iy per ix
+        // z-fastest store: ROWS * NZ consecutive slices of each column
+        constexpr int TZ = ROWS * NZ;
         const int t = ty * 32 + tx;
-        const int lx = t / ROWS, ly = t % ROWS;
-        const int ixT = x0 + lx, iyT = y0 + ly;
-        if (ixT < g.nx && iyT < g.ny) {
 #pragma unroll
-            for (int k = 0; k < NZ; k++) {
-                const int iz = z0 + k;
-                if (iz < g.nz) p.outT[iyT + (int64_t)ixT * g.ny + iz * plane] = tile[k][ly][lx];
-            }
+        for (int k = 0; k < NZ; k++) {
+            const int e = t + 32 * ROWS * k, lx = e / TZ, lz = e % TZ;
+            if (x0 + lx < g.nx && zb + lz < g.nz)
+                p.outZ[zb + lz + ((int64_t)iy * g.nx + x0 + lx) * g.nz] = tile[lz][lx];
         }
     }
+}
+// The launch grid of bp_kernel<..., NZ, ROWS>.
+template <int NZ, int ROWS> inline dim3 bp_grid(const Geom &g) {
+    return dim3(div_up(g.nx, 32) * (unsigned)g.ny, div_up(g.nz, NZ * ROWS));
 }
 
 }  // namespace mcsart

@@ -147,27 +147,31 @@ template <typename DT> __global__ void cast_kernel(DT *dst, const float *src, in
     MC_GRID_STRIDE(n) { dst[id] = cvt<DT>(src[id]); }
 }
 
-// y-fastest copy of an x-fastest volume: dstT[iy + ix*ny] = src[ix + iy*nx].
-// blockDim (32, 8), 32x32 tiles of slice blockIdx.z.
+// z-fastest copy of an x-fastest volume: dst[iz + (ix + iy*nx)*nz] =
+// src[ix + iy*nx + iz*nx*ny].  blockDim (32, 8); a block turns a 32 x 32
+// (x, z) tile of row iy; gridDim (ceil(nx/32) * ny, ceil(nz/32)).
 template <typename ST, typename DT>
-static __global__ void __launch_bounds__(256) transpose_kernel(DT *dstT, const ST *src, int nx, int ny) {
+static __global__ void __launch_bounds__(256) zfast_kernel(DT *dst, const ST *src, int nx, int ny,
+                                                           int nz) {
     __shared__ float tile[32][33];
     const int tx = threadIdx.x, ty = threadIdx.y;
-    const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
-    const int64_t slice = (int64_t)blockIdx.z * nx * ny;
+    const unsigned gx = (nx + 31) / 32, iy = blockIdx.x / gx;
+    const int x0 = (int)(blockIdx.x - iy * gx) * 32, z0 = blockIdx.y * 32;
+    const int64_t plane = (int64_t)nx * ny, row = (int64_t)iy * nx;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        const int ly = ty + 8 * k;
-        const int ix = x0 + tx, iy = y0 + ly;
-        tile[ly][tx] = (ix < nx && iy < ny) ? ldv(src, ix + (int64_t)iy * nx + slice) : 0.0f;
+        const int lz = ty + 8 * k, ix = x0 + tx, iz = z0 + lz;
+        tile[lz][tx] = (ix < nx && iz < nz) ? ldv(src, ix + row + iz * plane) : 0.0f;
     }
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        const int lx = ty + 8 * k;
-        const int ix = x0 + lx, iy = y0 + tx;
-        if (ix < nx && iy < ny) dstT[iy + (int64_t)ix * ny + slice] = cvt<DT>(tile[tx][lx]);
+        const int lx = ty + 8 * k, ix = x0 + lx, iz = z0 + tx;
+        if (ix < nx && iz < nz) dst[iz + (row + ix) * nz] = cvt<DT>(tile[tx][lx]);
     }
+}
+inline dim3 zfast_grid(int nx, int ny, int nz) {
+    return dim3(div_up(nx, 32) * (unsigned)ny, div_up(nz, 32));
 }
 
 // Loads the 32x32 tile of a field read at the transposed index
@@ -183,78 +187,130 @@ __device__ __forceinline__ void load_tile_T(float (*tile)[33], const T *src, int
     }
 }
 
-// Motion pass, AUMISART.cu:252-258 and :267 fused: for the current view
-//   img0 = sum over the six (field, gradient) pairs of F[t]*w*d img
-//   ones = (dx + dy + dz img) * (-vd + -fd)
-// each written x-fastest (img0, ones) and as a y-fastest copy (img0T,
-// onesT) for the projector; either pair may be nullptr when the view's
-// projector reads only the other.  PAIR: img0 and ones interleaved in img0
-// (img0[2i], img0[2i + 1]) and img0T, for the projector's paired load; ones
-// and onesT unused.
-template <typename FT, typename VT, bool PAIR = false>
-static __global__ void __launch_bounds__(256) motion_prep_kernel(VT *img0, VT *img0T, VT *ones,
-                                                          VT *onesT, const float *img,
-                                                          Fields<FT> f, int nx, int ny, int nz,
-                                                          float vd, float fd) {
-    __shared__ float ft[6][32][33];
-    __shared__ float o0[32][33], o1[32][33];
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32, iz = blockIdx.z;
-    const int64_t slice = (int64_t)iz * nx * ny;
-    load_tile_T(ft[0], f.ay, x0, y0, nx, ny, slice);
-    load_tile_T(ft[1], f.ax, x0, y0, nx, ny, slice);
-    load_tile_T(ft[2], f.az, x0, y0, nx, ny, slice);
-    load_tile_T(ft[3], f.by, x0, y0, nx, ny, slice);
-    load_tile_T(ft[4], f.bx, x0, y0, nx, ny, slice);
-    load_tile_T(ft[5], f.bz, x0, y0, nx, ny, slice);
-    __syncthreads();
-    const int ix = x0 + tx;
+// The DVF pass's per-view kernels work on tiles of MP_T x MP_T (x, y) columns
+// and MP_Z slices, one column per thread, so that a thread ends with MP_Z
+// consecutive slices of its column, a 32-byte piece of the z-fastest img0 and
+// initial2 volumes the projector reads.  16 x 16 columns keep the x-fastest
+// rows of the fields in whole 64-byte pieces.
+constexpr int MP_T = 16, MP_Z = 4;
+inline dim3 motion_grid(int nx, int ny, int nz) {
+    return dim3(div_up(nx, MP_T), div_up(ny, MP_T), div_up(nz, MP_Z));
+}
+
+// Eight consecutive floats as one 32-byte store (p 32-byte aligned), and
+// eight consecutive 16-bit values as one 16-byte store (p 16-byte aligned).
+__device__ __forceinline__ void st8(float *p, const float *v) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]),
+                 "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+                 : "memory");
+}
+template <typename T> __device__ __forceinline__ void st8(T *p, const float *v) {
+    union {
+        T h[8];
+        uint4 u;
+    } w;
+#pragma unroll
+    for (int i = 0; i < 8; i++) w.h[i] = cvt<T>(v[i]);
+    *reinterpret_cast<uint4 *>(p) = w.u;
+}
+
+// Stores slices z0 .. z0 + MP_Z - 1 (those below nz) of column c: PAIR, img0
+// and ones interleaved in img0; otherwise apart.  Interleaved pairs of a depth
+// that is a multiple of 4 go out as one store: lanes are different columns,
+// so every store of a warp touches 32 lines, and one whole-sector store in
+// place of four 8-byte ones takes a quarter of the write transactions.
+template <typename VT, bool PAIR>
+__device__ __forceinline__ void store_column(VT *img0, VT *ones, int64_t c, int z0, int nz,
+                                             const float *a, const float *b) {
+    const int64_t i = c * nz + z0;
+    if (PAIR && nz % MP_Z == 0) {
+        const float v[8] = {a[0], b[0], a[1], b[1], a[2], b[2], a[3], b[3]};
+        st8(img0 + 2 * i, v);
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < MP_Z; k++) {
+        if (z0 + k >= nz) break;
+        if (PAIR) {
+            stv2(img0, i + k, a[k], b[k]);
+        } else {
+            img0[i + k] = cvt<VT>(a[k]);
+            ones[i + k] = cvt<VT>(b[k]);
+        }
+    }
+}
+
+// AUMISART.cu:252-258 and :267 for slices z0 .. of column (ix, iy): img0 =
+// the sum over the six (field, gradient) pairs of F*w*d img in the
+// reference's order (host_initial(img0, 0), then six host_add2) and ones =
+// (dx + dy + dz img) * (-vd + -fd) (cu_initial.cu:48).  ft[c][k]: the six
+// fields' values for slice z0 + k of this column, read at the reference's
+// transposed index.
+__device__ __forceinline__ void motion_column(const float *img, int ix, int iy, int z0, int nx,
+                                              int ny, int nz, float vd, float fd,
+                                              const float (*ft)[MP_Z], float *a, float *b) {
     const float s_ones = (-vd) + (-fd);
+    const int64_t plane = (int64_t)nx * ny, id = ix + (int64_t)iy * nx + z0 * plane;
+    float cur = ldv(img, id);
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const int ly = ty + 8 * k, iy = y0 + ly;
-        float a = 0.0f, b = 0.0f;
-        if (ix < nx && iy < ny) {
-            const int64_t id = ix + (int64_t)iy * nx + slice;
-            const Vox v{ix, iy, iz};
-            const float dfx = fwd_diff(img, id, v, nx, ny, nz, 1);
-            const float dfy = fwd_diff(img, id, v, nx, ny, nz, 2);
-            const float dfz = fwd_diff(img, id, v, nx, ny, nz, 3);
-            // host_initial(img0, 0) then six host_add2 in the reference's order
-            a = __fmaf_rn(ft[0][tx][ly] * vd, dfx, a);
-            a = __fmaf_rn(ft[1][tx][ly] * vd, dfy, a);
-            a = __fmaf_rn(ft[2][tx][ly] * vd, dfz, a);
-            a = __fmaf_rn(ft[3][tx][ly] * fd, dfx, a);
-            a = __fmaf_rn(ft[4][tx][ly] * fd, dfy, a);
-            a = __fmaf_rn(ft[5][tx][ly] * fd, dfz, a);
-            b = (dfx + dfy + dfz) * s_ones;  // cu_initial.cu:48
-            if (img0) {
-                if (PAIR) {
-                    stv2(img0, id, a, b);
-                } else {
-                    img0[id] = cvt<VT>(a);
-                    ones[id] = cvt<VT>(b);
-                }
-            }
-        }
-        o0[ly][tx] = a;
-        o1[ly][tx] = b;
+    for (int k = 0; k < MP_Z; k++) {
+        if (z0 + k >= nz) break;
+        const int64_t i = id + k * plane;
+        const float up = z0 + k == nz - 1 ? 0.0f : ldv(img, i + plane);
+        // fwd_diff along x, y and z
+        const float dfx = ix == nx - 1 ? 0.0f : ldv(img, i + 1) - cur;
+        const float dfy = iy == ny - 1 ? 0.0f : ldv(img, i + nx) - cur;
+        const float dfz = z0 + k == nz - 1 ? 0.0f : up - cur;
+        float s = 0.0f;
+        s = __fmaf_rn(ft[0][k] * vd, dfx, s);
+        s = __fmaf_rn(ft[1][k] * vd, dfy, s);
+        s = __fmaf_rn(ft[2][k] * vd, dfz, s);
+        s = __fmaf_rn(ft[3][k] * fd, dfx, s);
+        s = __fmaf_rn(ft[4][k] * fd, dfy, s);
+        s = __fmaf_rn(ft[5][k] * fd, dfz, s);
+        a[k] = s;
+        b[k] = (dfx + dfy + dfz) * s_ones;
+        cur = up;
     }
-    if (img0T == nullptr) return;  // uniform over the block
+}
+
+// Motion pass, AUMISART.cu:252-258 and :267 fused: for the current view the
+// img0 and initial2 volumes (motion_column), z-fastest for the projector.
+// PAIR: interleaved in img0 (img0[2i], img0[2i + 1]) for the projector's
+// paired load, ones unused.  blockDim (MP_T, MP_T), motion_grid.
+template <typename FT, typename VT, bool PAIR = false>
+static __global__ void __launch_bounds__(256) motion_prep_kernel(VT *img0, VT *ones,
+                                                                 const float *img, Fields<FT> f,
+                                                                 int nx, int ny, int nz, float vd,
+                                                                 float fd) {
+    __shared__ float sm[6][MP_Z][MP_T][MP_T + 1];
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int x0 = blockIdx.x * MP_T, y0 = blockIdx.y * MP_T, z0 = blockIdx.z * MP_Z;
+    const int64_t plane = (int64_t)nx * ny;
+    // the fields at the transposed index iy + ix*ny, lanes along iy
+    const bool in_t = x0 + ty < nx && y0 + tx < ny;
+    const int64_t it = (y0 + tx) + (int64_t)(x0 + ty) * ny + z0 * plane;
+#pragma unroll
+    for (int k = 0; k < MP_Z; k++) {
+        const bool in = in_t && z0 + k < nz;
+        const int64_t i = it + k * plane;
+        sm[0][k][ty][tx] = in ? ldv(f.ay, i) : 0.0f;
+        sm[1][k][ty][tx] = in ? ldv(f.ax, i) : 0.0f;
+        sm[2][k][ty][tx] = in ? ldv(f.az, i) : 0.0f;
+        sm[3][k][ty][tx] = in ? ldv(f.by, i) : 0.0f;
+        sm[4][k][ty][tx] = in ? ldv(f.bx, i) : 0.0f;
+        sm[5][k][ty][tx] = in ? ldv(f.bz, i) : 0.0f;
+    }
     __syncthreads();
+    const int ix = x0 + tx, iy = y0 + ty;
+    if (ix >= nx || iy >= ny) return;
+    float ft[6][MP_Z], a[MP_Z], b[MP_Z];
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const int lx = ty + 8 * k, ixT = x0 + lx, iyT = y0 + tx;
-        if (ixT < nx && iyT < ny) {
-            const int64_t t = iyT + (int64_t)ixT * ny + slice;
-            if (PAIR) {
-                stv2(img0T, t, o0[tx][lx], o1[tx][lx]);
-            } else {
-                img0T[t] = cvt<VT>(o0[tx][lx]);
-                onesT[t] = cvt<VT>(o1[tx][lx]);
-            }
-        }
-    }
+    for (int c = 0; c < 6; c++)
+#pragma unroll
+        for (int k = 0; k < MP_Z; k++) ft[c][k] = sm[c][k][tx][ty];
+    motion_column(img, ix, iy, z0, nx, ny, nz, vd, fd, ft, a, b);
+    store_column<VT, PAIR>(img0, ones, ix + (int64_t)iy * nx, z0, nz, a, b);
 }
 
 // Motion pass field update, AUMISART.cu:272-277 fused: with q = img_temp read
@@ -300,42 +356,43 @@ static __global__ void __launch_bounds__(256) field_update_kernel(FT *ax, FT *ay
 // next view.  Every field voxel is updated by exactly one block, and the
 // arithmetic is that of the two kernels, so the results are bitwise theirs.
 // EARLY (a launch shape the driver's tuning may choose): every thread loads
-// its 4 x 6 field values first, before the ratio tile and its barrier, so
+// its MP_Z x 6 field values first, before the ratio tile and its barrier, so
 // that 24 loads per thread are in flight at once (more registers, fewer
 // resident blocks); otherwise the fields are loaded voxel by voxel.
 // PAIR: img0 and ones interleaved, as in motion_prep_kernel.
 // BP: the view's backprojection ratio of tile A (the DVF pass's
 // host_backprojection and host_division, src/AUMISART.cu:95-100 / :265-270) is
 // computed here from `bp` (its (residual, initial2-projection) pairs and
-// column data, one slice) with the backprojector's own per-voxel code,
-// instead of being read from img_temp: the field update of a tile needs the
-// ratio of that tile only, so the ratio never goes to memory, and blocks
-// gathering from the detector (bound by instruction issue) share the SMs
-// with blocks streaming the fields (bound by memory latency).  PROVEN: as in
-// bp_kernel.  The ratio's bits are the backprojector kernel's.
+// column data) with the backprojector's own per-voxel code, instead of being
+// read from img_temp: the field update of a tile needs the ratio of that tile
+// only, so the ratio never goes to memory, and blocks gathering from the
+// detector (bound by instruction issue) share the SMs with blocks streaming
+// the fields (bound by memory latency).  PROVEN: as in bp_kernel.  The
+// ratio's bits are the backprojector kernel's.  blockDim (MP_T, MP_T),
+// motion_grid.
 template <typename FT, typename VT, bool EARLY = false, bool PAIR = false, bool BP = false,
           bool PROVEN = false>
 static __global__ void __launch_bounds__(256) field_update_prep_kernel(
     FT *ax, FT *ay, FT *az, FT *bx, FT *by, FT *bz, const float *img_temp, const float *img,
-    int nx, int ny, int nz, float nvd, float nfd, VT *img0, VT *img0T, VT *ones, VT *onesT,
-    float vd, float fd, const BPArgs bp) {
-    __shared__ float ft[6][32][33];
-    __shared__ float rt[32][33];
-    __shared__ float o0[32][33], o1[32][33];
+    int nx, int ny, int nz, float nvd, float nfd, VT *img0, VT *ones, float vd, float fd,
+    const BPArgs bp) {
+    __shared__ float sm[6][MP_Z][MP_T][MP_T + 1];
+    __shared__ float rt[MP_Z][MP_T][MP_T + 1];
     const int tx = threadIdx.x, ty = threadIdx.y;
-    const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32, iz = blockIdx.z;
-    const int64_t slice = (int64_t)iz * nx * ny;
+    const int x0 = blockIdx.x * MP_T, y0 = blockIdx.y * MP_T, z0 = blockIdx.z * MP_Z;
+    const int64_t plane = (int64_t)nx * ny;
     if (BP) {
         // The block's own field rows (tile A^T) and volume rows (A^T and A)
         // are prefetched into L2 before the backprojection gather, which
-        // then covers their memory latency: one 32-voxel row per thread
-        // (6 x 32 field rows, 2 x 32 volume rows).  Measured at 256x256x160:
-        // 151.4 to 141.9 ms per step (fields alone 145.3).
-        const int t = ty * 32 + tx, r = t % 32, w = t / 32;
-        const void *p = nullptr;
-        if (w < 7) {  // rows of A^T: memory rows x0 + r, columns from y0
-            if (x0 + r < ny && y0 < nx) {
-                const int64_t i = y0 + (int64_t)(x0 + r) * nx + slice;
+        // then covers their memory latency: rows of MP_T voxels, two per
+        // thread (7 x MP_T x MP_Z rows of A^T and MP_T x MP_Z of A).
+        const int t = ty * MP_T + tx;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int e = t + 256 * h, w = e / (MP_T * MP_Z), r = e % MP_T, z = z0 + e / MP_T % MP_Z;
+            const void *p = nullptr;
+            if (z < nz && w < 7 && x0 + r < ny && y0 < nx) {
+                const int64_t i = y0 + (int64_t)(x0 + r) * nx + z * plane;
                 switch (w) {
                     case 0: p = ax + i; break;
                     case 1: p = ay + i; break;
@@ -345,20 +402,22 @@ static __global__ void __launch_bounds__(256) field_update_prep_kernel(
                     case 5: p = bz + i; break;
                     default: p = img + i;
                 }
+            } else if (z < nz && w == 7 && y0 + r < ny && x0 < nx) {
+                p = img + x0 + (int64_t)(y0 + r) * nx + z * plane;
             }
-        } else if (y0 + r < ny && x0 < nx) {  // volume rows of A
-            p = img + x0 + (int64_t)(y0 + r) * nx + slice;
+            if (p) asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
         }
-        if (p) asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
     }
-    // the field values at this thread's 4 voxels of A^T (EARLY)
-    float fe[EARLY ? 4 : 1][6];
+    // this thread's column of A^T: (xp, yp) = (y0 + tx, x0 + ty)
+    const int xp = y0 + tx, yp = x0 + ty;
+    const bool in_t = xp < nx && yp < ny;
+    const int64_t it = xp + (int64_t)yp * nx + z0 * plane;
+    float fe[EARLY ? MP_Z : 1][6];  // its field values (EARLY)
     if (EARLY) {
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const int lx = ty + 8 * k, xp = y0 + tx, yp = x0 + lx;
-            const bool in = xp < nx && yp < ny;
-            const int64_t id = in ? xp + (int64_t)yp * nx + slice : 0;
+        for (int k = 0; k < MP_Z; k++) {
+            const bool in = in_t && z0 + k < nz;
+            const int64_t id = in ? it + k * plane : 0;
             fe[k][0] = in ? ldv(ay, id) : 0.0f;
             fe[k][1] = in ? ldv(ax, id) : 0.0f;
             fe[k][2] = in ? ldv(az, id) : 0.0f;
@@ -367,44 +426,53 @@ static __global__ void __launch_bounds__(256) field_update_prep_kernel(
             fe[k][5] = in ? ldv(bz, id) : 0.0f;
         }
     }
-    // ratio on tile A, x-fastest: rt[y - y0][x - x0]
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const int ly = ty + 8 * k, xx = x0 + tx, yy = y0 + ly;
-        float q = 0.0f;
-        if (xx < nx && yy < ny) {
+    // ratio on tile A: this thread's column (ix, iy), two slices at a time
+    const int ix = x0 + tx, iy = y0 + ty;
+    const bool in_a = ix < nx && iy < ny;
+#pragma unroll 1
+    for (int k = 0; k < MP_Z; k += 2) {
+        float q[2] = {0.0f, 0.0f};
+        if (in_a) {
             if (BP) {
-                float a0 = 0.0f, a1 = 0.0f;
-                bp_gather_view<2, PROVEN, 1>(bp, bp.angle, nullptr, bp.pair, xx, yy, iz, &a0,
-                                             &a1);
-                q = a0 / a1;                           // cu_division.cu:20
-                if (isnan(q) || isinf(q)) q = 0.0f;    // :21-24
+                float a0[2] = {0.0f, 0.0f}, a1[2] = {0.0f, 0.0f};
+                if (z0 + k < nz)
+                    bp_gather_view<2, PROVEN, 2>(bp, bp.angle, nullptr, bp.pair, ix, iy, z0 + k,
+                                                 a0, a1);
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    q[h] = a0[h] / a1[h];                           // cu_division.cu:20
+                    if (isnan(q[h]) || isinf(q[h])) q[h] = 0.0f;    // :21-24
+                }
             } else {
-                q = img_temp[xx + (int64_t)yy * nx + slice];
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+                    if (z0 + k + h < nz) q[h] = img_temp[ix + (int64_t)iy * nx + (z0 + k + h) * plane];
             }
         }
-        rt[ly][tx] = q;
+        rt[k][ty][tx] = q[0];
+        rt[k + 1][ty][tx] = q[1];
     }
     __syncthreads();
-    // field update on A^T: voxel (x', y') = (y0 + tx, x0 + lx); its q is the
-    // ratio at the transposed index, i.e. at (x0 + lx, y0 + tx) of tile A
+    // field update on A^T: voxel (xp, yp)'s q is the ratio at the transposed
+    // index, i.e. at (x0 + ty, y0 + tx) of tile A
+    if (in_t) {
+        float cur = ldv(img, it);
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const int lx = ty + 8 * k, xp = y0 + tx, yp = x0 + lx;
-        float n[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-        if (xp < nx && yp < ny) {
-            const int64_t id = xp + (int64_t)yp * nx + slice;
-            const Vox v{xp, yp, iz};
-            const float dfx = fwd_diff(img, id, v, nx, ny, nz, 1);
-            const float dfy = fwd_diff(img, id, v, nx, ny, nz, 2);
-            const float dfz = fwd_diff(img, id, v, nx, ny, nz, 3);
-            const float q = rt[tx][lx];
-            const float fay = EARLY ? fe[k % (EARLY ? 4 : 1)][0] : ldv(ay, id);
-            const float fax = EARLY ? fe[k % (EARLY ? 4 : 1)][1] : ldv(ax, id);
-            const float faz = EARLY ? fe[k % (EARLY ? 4 : 1)][2] : ldv(az, id);
-            const float fby = EARLY ? fe[k % (EARLY ? 4 : 1)][3] : ldv(by, id);
-            const float fbx = EARLY ? fe[k % (EARLY ? 4 : 1)][4] : ldv(bx, id);
-            const float fbz = EARLY ? fe[k % (EARLY ? 4 : 1)][5] : ldv(bz, id);
+        for (int k = 0; k < MP_Z; k++) {
+            if (z0 + k >= nz) break;
+            const int64_t id = it + k * plane;
+            const float up = z0 + k == nz - 1 ? 0.0f : ldv(img, id + plane);
+            const float dfx = xp == nx - 1 ? 0.0f : ldv(img, id + 1) - cur;
+            const float dfy = yp == ny - 1 ? 0.0f : ldv(img, id + nx) - cur;
+            const float dfz = z0 + k == nz - 1 ? 0.0f : up - cur;
+            cur = up;
+            const float q = rt[k][tx][ty];
+            const float fay = EARLY ? fe[k % (EARLY ? MP_Z : 1)][0] : ldv(ay, id);
+            const float fax = EARLY ? fe[k % (EARLY ? MP_Z : 1)][1] : ldv(ax, id);
+            const float faz = EARLY ? fe[k % (EARLY ? MP_Z : 1)][2] : ldv(az, id);
+            const float fby = EARLY ? fe[k % (EARLY ? MP_Z : 1)][3] : ldv(by, id);
+            const float fbx = EARLY ? fe[k % (EARLY ? MP_Z : 1)][4] : ldv(bx, id);
+            const float fbz = EARLY ? fe[k % (EARLY ? MP_Z : 1)][5] : ldv(bz, id);
             const FT nay = cvt<FT>(__fmaf_rn(q * nvd, dfx, fay));
             const FT nax = cvt<FT>(__fmaf_rn(q * nvd, dfy, fax));
             const FT naz = cvt<FT>(__fmaf_rn(q * nvd, dfz, faz));
@@ -413,60 +481,24 @@ static __global__ void __launch_bounds__(256) field_update_prep_kernel(
             const FT nbz = cvt<FT>(__fmaf_rn(q * nfd, dfz, fbz));
             ay[id] = nay; ax[id] = nax; az[id] = naz;
             by[id] = nby; bx[id] = nbx; bz[id] = nbz;
-            n[0] = tof(nay); n[1] = tof(nax); n[2] = tof(naz);
-            n[3] = tof(nby); n[4] = tof(nbx); n[5] = tof(nbz);
+            sm[0][k][ty][tx] = tof(nay);
+            sm[1][k][ty][tx] = tof(nax);
+            sm[2][k][ty][tx] = tof(naz);
+            sm[3][k][ty][tx] = tof(nby);
+            sm[4][k][ty][tx] = tof(nbx);
+            sm[5][k][ty][tx] = tof(nbz);
         }
-#pragma unroll
-        for (int c = 0; c < 6; c++) ft[c][lx][tx] = n[c];
     }
     __syncthreads();
     // motion_prep_kernel for tile A with the next view's weights
-    const int ix = x0 + tx;
-    const float s_ones = (-vd) + (-fd);
+    if (!in_a) return;
+    float ft[6][MP_Z], a[MP_Z], b[MP_Z];
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const int ly = ty + 8 * k, iy = y0 + ly;
-        float a = 0.0f, b = 0.0f;
-        if (ix < nx && iy < ny) {
-            const int64_t id = ix + (int64_t)iy * nx + slice;
-            const Vox v{ix, iy, iz};
-            const float dfx = fwd_diff(img, id, v, nx, ny, nz, 1);
-            const float dfy = fwd_diff(img, id, v, nx, ny, nz, 2);
-            const float dfz = fwd_diff(img, id, v, nx, ny, nz, 3);
-            a = __fmaf_rn(ft[0][tx][ly] * vd, dfx, a);
-            a = __fmaf_rn(ft[1][tx][ly] * vd, dfy, a);
-            a = __fmaf_rn(ft[2][tx][ly] * vd, dfz, a);
-            a = __fmaf_rn(ft[3][tx][ly] * fd, dfx, a);
-            a = __fmaf_rn(ft[4][tx][ly] * fd, dfy, a);
-            a = __fmaf_rn(ft[5][tx][ly] * fd, dfz, a);
-            b = (dfx + dfy + dfz) * s_ones;  // cu_initial.cu:48
-            if (img0) {
-                if (PAIR) {
-                    stv2(img0, id, a, b);
-                } else {
-                    img0[id] = cvt<VT>(a);
-                    ones[id] = cvt<VT>(b);
-                }
-            }
-        }
-        o0[ly][tx] = a;
-        o1[ly][tx] = b;
-    }
-    if (img0T == nullptr) return;  // uniform over the block
-    __syncthreads();
+    for (int c = 0; c < 6; c++)
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const int lx = ty + 8 * k, ixT = x0 + lx, iyT = y0 + tx;
-        if (ixT < nx && iyT < ny) {
-            const int64_t t = iyT + (int64_t)ixT * ny + slice;
-            if (PAIR) {
-                stv2(img0T, t, o0[tx][lx], o1[tx][lx]);
-            } else {
-                img0T[t] = cvt<VT>(o0[tx][lx]);
-                onesT[t] = cvt<VT>(o1[tx][lx]);
-            }
-        }
-    }
+        for (int k = 0; k < MP_Z; k++) ft[c][k] = sm[c][k][tx][ty];
+    motion_column(img, ix, iy, z0, nx, ny, nz, vd, fd, ft, a, b);
+    store_column<VT, PAIR>(img0, ones, ix + (int64_t)iy * nx, z0, nz, a, b);
 }
 
 // Norm ratios ||r_v|| / ||b_v|| from per-block partials (fixed order); one

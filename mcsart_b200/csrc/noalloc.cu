@@ -1,6 +1,6 @@
 // mcsart_projection_noalloc: the projector of mcsart_projection (the
 // reference's host_projection, src/cu_projection.cu:7-12) with its one scratch
-// buffer, the y-fastest copy of the volume that x-driven rays read, held in a
+// buffer, the z-fastest copy of the volume that the projector reads, held in a
 // fixed file-scope device array instead of a context workspace.  It allocates
 // nothing and needs no context.  The kernels and their launch shapes are those
 // of mcsart_projection, so the results are bitwise the same.
@@ -14,14 +14,10 @@
 
 #define MC_EXPORT extern "C" __attribute__((visibility("default")))
 
-namespace mcsart {
-bool view_has_xdrive(float angle, const Geom &g);  // abi_kernels.cu
-}  // namespace mcsart
-
 using namespace mcsart;
 
-// The scratch: one y-fastest FP32 volume copy per device (16 MiB).
-static __device__ __align__(256) float g_noalloc_volT[MCSART_NOALLOC_MAX_VOXELS];
+// The scratch: one z-fastest FP32 volume copy per device (16 MiB).
+static __device__ __align__(256) float g_noalloc_volZ[MCSART_NOALLOC_MAX_VOXELS];
 
 namespace {
 
@@ -39,7 +35,7 @@ std::mutex g_setup_mu;
 // thread's current context is another one.
 struct Setup {
     unsigned long long ctx_id = 0;  // 0: not set up
-    float *scratch = nullptr;       // device address of g_noalloc_volT in that context
+    float *scratch = nullptr;       // device address of g_noalloc_volZ in that context
 };
 Setup g_setup[kMaxDevices];
 
@@ -101,9 +97,9 @@ int scratch_of_current_device(float **out) {
         }
     }
     void *p = nullptr;
-    MC_CHECK_CUDA(cudaGetSymbolAddress(&p, g_noalloc_volT));
+    MC_CHECK_CUDA(cudaGetSymbolAddress(&p, g_noalloc_volZ));
     cudaFuncAttributes fa;
-    MC_CHECK_CUDA(cudaFuncGetAttributes(&fa, transpose_kernel<float, float>));
+    MC_CHECK_CUDA(cudaFuncGetAttributes(&fa, zfast_kernel<float, float>));
     MC_CHECK_CUDA(cudaFuncGetAttributes(&fa, fp_ref_kernel<1, false, float>));
     unsigned long long id = 0;
     MC_TRY(current_context_id(&id));
@@ -134,23 +130,19 @@ MC_EXPORT int mcsart_projection_noalloc(void *stream, float *d_proj, const float
     MC_TRY(scratch_of_current_device(&scratch));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
 
-    const float *imgT = nullptr;
-    if (view_has_xdrive(angle, g)) {
-        const dim3 grid(div_up(nx, 32), div_up(ny, 32), nz), block(32, 8);
-        transpose_kernel<float, float><<<grid, block, 0, s>>>(scratch, d_img, nx, ny);
-        MC_CHECK_CUDA(cudaGetLastError());
-        imgT = scratch;
-    }
+    zfast_kernel<float, float><<<zfast_grid(nx, ny, nz), dim3(32, 8), 0, s>>>(scratch, d_img, nx,
+                                                                              ny, nz);
+    MC_CHECK_CUDA(cudaGetLastError());
     FPArgs<float, 1> a{};
-    a.vol.std[0] = d_img;
-    a.vol.tr[0] = imgT;
+    a.vol.zf[0] = scratch;
     a.g = g;
     a.angle = angle;
     a.angles = nullptr;
     a.mode = FP_PLAIN;
     a.out = d_proj;
     const dim3 grid(div_up(na, FPC_COLS), div_up(nb, FPC_ROWS), 1);
-    fp_ref_kernel<1, false, float><<<grid, dim3(FPC_THREADS), 0, s>>>(a);
+    constexpr size_t smem = fp_ref_smem<float, false, fp_stage<1>(), 2>();
+    fp_ref_kernel<1, false, float><<<grid, dim3(FPC_THREADS), smem, s>>>(a);
     MC_CHECK_CUDA(cudaGetLastError());
     return MCSART_OK;
 }

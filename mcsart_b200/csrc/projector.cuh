@@ -9,16 +9,22 @@
 //
 // Restructured for the hardware:
 //   * one thread per ray (the reference runs 4 redundant threads per ray that
-//     race on a non-atomic +=);
-//   * the slabs of a ray are split across `groups` warps of a block and
-//     recombined in a fixed order through shared memory (deterministic);
+//     race on a non-atomic +=), the 32 lanes of a warp being 32 consecutive
+//     detector rows of one detector column;
+//   * every volume is read through a z-fastest copy
+//     zf[iz + (ix + iy*nx)*nz]: a warp's rays meet each slab in the same one
+//     or two in-plane voxel columns and in neighbouring slices, so one copy
+//     serves both driving axes, a ray's two axial voxels are neighbours in
+//     memory, and everything in-plane (weights, which columns are visited,
+//     their addresses) is the same for the whole warp;
 //   * the loop-invariant ratios are hoisted out of the slab loop;
-//   * x-driven rays read a y-fastest copy of the volume so that the 32 lanes
-//     of a warp (adjacent detector columns) gather adjacent addresses;
 //   * up to three volumes are projected with one set of weights, the
 //     projection of a ones-volume (sum of weights) comes for free, and the
 //     SART residual, its norm partial sums and the packing for the
-//     backprojector are done in the epilogue.
+//     backprojector are done in the epilogue;
+//   * in the split summation modes the slabs of a ray are split across
+//     `groups` warps of a block and recombined in a fixed order through shared
+//     memory (deterministic).
 #pragma once
 
 #include "backprojector.cuh"
@@ -82,10 +88,18 @@ __device__ __forceinline__ RayGeom ray_geom(float cphi, float sphi, int ia, int 
     return r;
 }
 
+// z-fastest volumes: zf[k][iz + (ix + iy*nx)*nz]
 template <typename VT, int K> struct FPVolumes {
-    const VT *std[K];  // x-fastest volumes
-    const VT *tr[K];   // y-fastest copies (tr[k][iy + ix*ny + iz*nx*ny]) or nullptr
+    const VT *zf[K];
 };
+
+// Distance in a z-fastest volume between in-plane neighbours along the
+// in-plane axis (su) and along the driving axis (sd) of a ray.
+__device__ __forceinline__ void zf_strides(bool xdrive, const Geom &g, int &su, int &sd) {
+    const int row = g.nx * g.nz;  // fits: volumes hold fewer than 2^31 voxels
+    su = xdrive ? row : g.nz;
+    sd = xdrive ? g.nz : row;
+}
 
 // The K volumes' values at voxel offset a into t[0..K-1]: one load per
 // volume, or (PAIR, three volumes) the second and third interleaved in one
@@ -103,7 +117,6 @@ __device__ __forceinline__ void fp_voxel(const VT *const *base, int64_t a, float
         for (int k = 0; k < K; k++) t[k] = ldv(base[k], a);
     }
 }
-
 // Ray-sum order.  SUM_REF accumulates every voxel term straight into the ray
 // sum in the reference's order (slabs, then in-plane, then axial index,
 // acc = fma(v*w_u, w_z, acc), cu_projection.cu:81-88), so that results are
@@ -114,28 +127,14 @@ __device__ __forceinline__ void fp_voxel(const VT *const *base, int64_t a, float
 enum SumMode { SUM_REF = 0, SUM_PLAIN = 1, SUM_KAHAN = 2 };
 
 // Accumulates the footprint of slabs [d0, d1) of one ray into s[0..K-1]
-// (volume sums) and sw (sum of weights = projection of a ones-volume).
+// (volume sums) and sw (sum of weights = projection of a ones-volume), in the
+// split summation modes.
 template <int K, bool ONES, int SUM, typename VT>
 __device__ __forceinline__ void ray_slabs(const RayGeom &r, const FPVolumes<VT, K> &v,
                                           const Geom &g, int d0, int d1, float *s, float &sw) {
-    const VT *base[K];
-    int64_t su, sd;
-    const int64_t sz = (int64_t)g.nx * g.ny;
-    if (r.xdrive) {
-        if (v.tr[0] != nullptr) {
-#pragma unroll
-            for (int k = 0; k < K; k++) base[k] = v.tr[k];
-            su = 1; sd = g.ny;
-        } else {
-#pragma unroll
-            for (int k = 0; k < K; k++) base[k] = v.std[k];
-            su = g.nx; sd = 1;
-        }
-    } else {
-#pragma unroll
-        for (int k = 0; k < K; k++) base[k] = v.std[k];
-        su = 1; sd = g.nx;
-    }
+    static_assert(SUM != SUM_REF, "the reference order is fp_ref_kernel's");
+    int su, sd;
+    zf_strides(r.xdrive, g, su, sd);
     const float z_half = (float)(g.nz / 2);
     float acc[K], cmp[K], accw = 0.0f, cmpw = 0.0f;
 #pragma unroll
@@ -158,43 +157,6 @@ __device__ __forceinline__ void ray_slabs(const RayGeom &r, const FPVolumes<VT, 
         const int U1 = (int)floorf(ui1), U2 = (int)floorf(ui2);
         const int Z1 = (int)floorf(zi1), Z2 = (int)floorf(zi2);
         const float du = __fsub_rn(ui2, ui1), dz = __fsub_rn(zi2, zi1);
-        if (SUM == SUM_REF && U2 - U1 <= 1 && Z2 - Z1 <= 1) {
-            // The footprint fits a 2x2 voxel window (U1, U1+1) x (Z1, Z1+1): the
-            // reference's loops visit its in-volume members in this order, so
-            // evaluating the four candidates with predication gives the same
-            // sequence of fma's, without data-dependent trip counts.
-            const bool u0 = U1 >= 0 && U1 <= r.nu - 1;
-            const bool u1 = U1 + 1 <= U2 && U1 + 1 >= 0 && U1 + 1 <= r.nu - 1;
-            const bool z0 = Z1 >= 0 && Z1 <= g.nz - 1;
-            const bool z1 = Z1 + 1 <= Z2 && Z1 + 1 >= 0 && Z1 + 1 <= g.nz - 1;
-            const float fu0 = (float)U1, fu1 = (float)(U1 + 1);
-            const float fz0 = (float)Z1, fz1 = (float)(Z1 + 1);
-            const float wu0 = __fdiv_rn(__fsub_rn(fminf(__fadd_rn(fu0, 1.0f), ui2), fmaxf(fu0, ui1)), du);
-            const float wu1 = __fdiv_rn(__fsub_rn(fminf(__fadd_rn(fu1, 1.0f), ui2), fmaxf(fu1, ui1)), du);
-            const float wz0 = __fdiv_rn(__fsub_rn(fminf(__fadd_rn(fz0, 1.0f), zi2), fmaxf(fz0, zi1)), dz);
-            const float wz1 = __fdiv_rn(__fsub_rn(fminf(__fadd_rn(fz1, 1.0f), zi2), fmaxf(fz1, zi1)), dz);
-            // in-bounds addresses for every candidate (unused ones are not read)
-            const int cu0 = min(max(U1, 0), r.nu - 1), cu1 = min(max(U1 + 1, 0), r.nu - 1);
-            const int cz0 = min(max(Z1, 0), g.nz - 1), cz1 = min(max(Z1 + 1, 0), g.nz - 1);
-            const int64_t r0 = (int64_t)cu0 * su + (int64_t)d * sd;
-            const int64_t r1 = (int64_t)cu1 * su + (int64_t)d * sd;
-            const int64_t a00 = r0 + (int64_t)cz0 * sz, a01 = r0 + (int64_t)cz1 * sz;
-            const int64_t a10 = r1 + (int64_t)cz0 * sz, a11 = r1 + (int64_t)cz1 * sz;
-#pragma unroll
-            for (int k = 0; k < K; k++) {
-                if (u0 && z0) acc[k] = __fmaf_rn(__fmul_rn(ldv(base[k], a00), wu0), wz0, acc[k]);
-                if (u0 && z1) acc[k] = __fmaf_rn(__fmul_rn(ldv(base[k], a01), wu0), wz1, acc[k]);
-                if (u1 && z0) acc[k] = __fmaf_rn(__fmul_rn(ldv(base[k], a10), wu1), wz0, acc[k]);
-                if (u1 && z1) acc[k] = __fmaf_rn(__fmul_rn(ldv(base[k], a11), wu1), wz1, acc[k]);
-            }
-            if (ONES) {
-                if (u0 && z0) accw = __fmaf_rn(wu0, wz0, accw);
-                if (u0 && z1) accw = __fmaf_rn(wu0, wz1, accw);
-                if (u1 && z0) accw = __fmaf_rn(wu1, wz0, accw);
-                if (u1 && z1) accw = __fmaf_rn(wu1, wz1, accw);
-            }
-            continue;
-        }
         const int u_lo = max(0, U1), u_hi = min(r.nu - 1, U2);
         const int z_lo = max(0, Z1), z_hi = min(g.nz - 1, Z2);
         if (u_lo > u_hi || z_lo > z_hi) continue;
@@ -204,24 +166,16 @@ __device__ __forceinline__ void ray_slabs(const RayGeom &r, const FPVolumes<VT, 
         for (int u = u_lo; u <= u_hi; u++) {
             // :83 / :136
             const float wu = __fdiv_rn(__fsub_rn(fminf(__fadd_rn((float)u, 1.0f), ui2), fmaxf((float)u, ui1)), du);
-            const int64_t row = (int64_t)u * su + (int64_t)d * sd;
+            const int row = u * su + d * sd;
             for (int z = z_lo; z <= z_hi; z++) {
                 // :86 / :139
                 const float wz = __fdiv_rn(__fsub_rn(fminf(__fadd_rn((float)z, 1.0f), zi2), fmaxf((float)z, zi1)), dz);
-                const int64_t a = row + (int64_t)z * sz;
-                if (SUM == SUM_REF) {
+                const int a = row + z;
 #pragma unroll
-                    for (int k = 0; k < K; k++)
-                        acc[k] = __fmaf_rn(__fmul_rn(ldv(base[k], a), wu), wz, acc[k]);  // :87 / :140
-                    if (ONES) accw = __fmaf_rn(wu, wz, accw);
-                } else {
-#pragma unroll
-                    for (int k = 0; k < K; k++) ss[k] = __fmaf_rn(__fmul_rn(ldv(base[k], a), wu), wz, ss[k]);
-                    if (ONES) ssw = __fmaf_rn(wu, wz, ssw);
-                }
+                for (int k = 0; k < K; k++) ss[k] = __fmaf_rn(__fmul_rn(ldv(v.zf[k], a), wu), wz, ss[k]);
+                if (ONES) ssw = __fmaf_rn(wu, wz, ssw);
             }
         }
-        if (SUM == SUM_REF) continue;
 #pragma unroll
         for (int k = 0; k < K; k++) {
             if (SUM == SUM_KAHAN) {
@@ -297,18 +251,8 @@ __device__ __forceinline__ RayGeom64 ray_geom64(double cphi, double sphi, int ia
 template <int K, bool ONES, int SUM, typename VT>
 __device__ __forceinline__ void ray_slabs64(const RayGeom64 &r, const FPVolumes<VT, K> &v,
                                             const Geom &g, int d0, int d1, float *s, double &sw) {
-    const VT *base[K];
-    int64_t su, sd;
-    const int64_t sz = (int64_t)g.nx * g.ny;
-    if (r.xdrive && v.tr[0] != nullptr) {
-#pragma unroll
-        for (int k = 0; k < K; k++) base[k] = v.tr[k];
-        su = 1; sd = g.ny;
-    } else {
-#pragma unroll
-        for (int k = 0; k < K; k++) base[k] = v.std[k];
-        if (r.xdrive) { su = g.nx; sd = 1; } else { su = 1; sd = g.nx; }
-    }
+    int su, sd;
+    zf_strides(r.xdrive, g, su, sd);
     const double z_half = (double)(g.nz / 2);
     float acc[K], cmp[K];
 #pragma unroll
@@ -334,14 +278,14 @@ __device__ __forceinline__ void ray_slabs64(const RayGeom64 &r, const FPVolumes<
         for (int k = 0; k < K; k++) ss[k] = 0.0f;
         for (int u = u_lo; u <= u_hi; u++) {
             const double wu = (fmin(u + 1.0, ui2) - fmax((double)u, ui1)) / du;  // :83 / :136
-            const int64_t row = (int64_t)u * su + (int64_t)d * sd;
+            const int row = u * su + d * sd;
             for (int z = z_lo; z <= z_hi; z++) {
                 const double wz = (fmin(z + 1.0, zi2) - fmax((double)z, zi1)) / dz;  // :86 / :139
                 const double w = wu * wz;
                 const float wf = (float)w;
-                const int64_t a = row + (int64_t)z * sz;
+                const int a = row + z;
 #pragma unroll
-                for (int k = 0; k < K; k++) ss[k] = __fmaf_rn(ldv(base[k], a), wf, ss[k]);
+                for (int k = 0; k < K; k++) ss[k] = __fmaf_rn(ldv(v.zf[k], a), wf, ss[k]);
                 if (ONES) accw += w;
             }
         }
@@ -388,35 +332,76 @@ template <typename VT, int K, typename MT = VT> struct FPArgs {
 };
 
 // ------------------------------------------------------------------------
-// Column-shared projector for the reference summation order (SUM_REF).
+// Row-lane projector for the reference summation order (SUM_REF).
 //
-// Every ray of one detector column ia has the same in-plane geometry: the
-// driving axis, the four edge ratios and so, per slab, the in-plane voxel
-// range U1..U2 and weights w_u (only the axial part depends on the row ib,
-// through z2).  A block of FPC_COLS columns x FPC_ROWS rows computes the
-// in-plane part once per (column, slab) into shared memory (SlabC: weights,
-// slab distance, clamped voxel-row offsets, visit flags), FPC_CHUNK slabs at
-// a time, and every ray then adds its axial part and its terms in the
-// reference's order.  The per-ray arithmetic is unchanged, so the sums are
-// bitwise those of the per-ray form (and of the reference kernel).
-#ifndef MCSART_FP_COLS
-#define MCSART_FP_COLS 16
-#endif
-#ifndef MCSART_FP_ROWS
-#define MCSART_FP_ROWS 8
-#endif
-constexpr int FPC_COLS = MCSART_FP_COLS, FPC_ROWS = MCSART_FP_ROWS;
-constexpr int FPC_THREADS = FPC_COLS * FPC_ROWS;
-// at least 512 threads per SM: lets the compiler use up to 128 registers
-constexpr int FPC_MIN_BLOCKS = 512 / FPC_THREADS;
-// Slabs per table fill (a 32 KB table per block; 64 measured 1 % faster than
-// 32 at both benchmark sizes).
-constexpr int FPC_CHUNK = 64;
-// Slabs per group in the 2x2 fast path: with three volumes 4 (more loads in
-// flight within the 128-register budget: the DVF pass's projector 6 % faster
-// than with 2), with one volume 2 (4 spills inside the 80 registers that keep
-// 6 blocks per SM).
-template <int K> constexpr int fp_group() { return K >= 3 ? 4 : 2; }
+// A warp is 32 consecutive detector rows of one detector column.  Every ray
+// of a column has the same in-plane geometry (driving axis, edge ratios and
+// so, per slab, the in-plane voxels and weights w_u); only the axial part
+// depends on the row, through z2.  So the warp's lanes compute the in-plane
+// part of 32 slabs at a time, one slab each, into a table of the warp's own in
+// shared memory, and then walk the slabs together: the in-plane weights, the
+// addresses of the voxel columns and whether there are one or two of them are
+// the same for all lanes, and each lane adds its ray's axial part and terms in
+// the reference's order.  The axial weights of two slabs are computed at once
+// with packed FP32 instructions (each half rounds as the scalar one).
+//
+// The rays of a warp meet a slab within some 20 neighbouring slices of one or
+// two voxel columns (32 rows of less than a voxel each), so the lanes copy
+// both windows, two slices each, into shared memory with one cp.async, S slabs
+// at a time and a stage ahead: no ray waits on the L2, and every voxel is
+// requested once per warp instead of once per ray.  Warps share nothing; the
+// slab loop has no block barrier.
+//
+// What bounds it: instruction issue (66-72 % of the slots at 256x256x160 with
+// a 512x384 detector) and, with three volumes, shared-memory bandwidth (80 %).
+// Two thirds of a slab's instructions are the axial footprint's correctly
+// rounded weights and the terms, which the reference's bits require of every
+// ray and slab.  Measured there, one view: 107 us with one volume and the
+// weights' sum (77 M warp instructions), 160 us with three; with 16 columns x
+// 2 rows per warp reading x- or y-fastest copies straight from L2 they took
+// 199 us (126 M) and 229 us.  128x128x96, 256x192: 25 and 34 us (43 and 50).
+// Also measured, same bits: direct loads instead of the windows 128 / 197 us
+// (L2 latency), two rows per lane with the packed operations across the rows
+// 117 / 180 us (half the warps), 1 or 2 columns per block no difference.
+constexpr int FPC_COLS = 4;                    // detector columns (warps) per block
+constexpr int FPC_ROWS = 32;                   // detector rows per block: a warp's lanes
+constexpr int FPC_THREADS = FPC_COLS * 32;
+
+// Two FP32 values in one 64-bit register pair and the packed operations on
+// them (PTX f32x2), each half rounded as the scalar operation.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 f2_pack(float lo, float hi) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ void f2_unpack(f32x2 v, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 f2_add_rd(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+// a - b, as fma(b, -1, a): one rounding of the exact difference
+__device__ __forceinline__ f32x2 f2_sub(f32x2 a, f32x2 b) {
+    return f2_fma(b, f2_pack(-1.0f, -1.0f), a);
+}
 
 // In-plane footprint of one slab.  U2 - U1 <= 1: (a, b) = weights of voxels
 // U1 and U1 + 1; otherwise (a, b) = (ui1, ui2), the footprint edges.
@@ -470,125 +455,23 @@ __device__ __forceinline__ SlabU slab_u(const RayGeom &r, int d) {
     return e;
 }
 
-// What every ray of one detector column shares for slab d, kept in shared
-// memory: slab_u's footprint, the slab distance dc, the clamped offsets of
-// the window's two in-plane voxel rows (cu * su + d * sd) and which of the two
-// the reference's loops visit (:80-82 / :133-135).
-struct __align__(16) SlabC {
-    int r0, r1;
-    float a, b;  // SlabU's
-    float dc;
-    int U1, U2;
-    int flags;   // SC_U0 | SC_U1 | SC_NARROW (U2 - U1 <= 1) | SC_UANY
-};
-// SC_UANY: the reference's in-plane loop over max(0, U1) .. min(nu-1, U2) is
-// not empty (:80-81 / :133-134)
-constexpr int SC_U0 = 1, SC_U1 = 2, SC_NARROW = 4, SC_UANY = 8;
-
-__device__ __forceinline__ SlabC slab_c(const RayGeom &r, int d, int su, int sd) {
-    const SlabU e = slab_u(r, d);
-    SlabC c;
-    c.a = e.a;
-    c.b = e.b;
-    c.U1 = e.U1;
-    c.U2 = e.U2;
-    c.dc = slab_dc(r, d);
-    const int U1 = e.U1, U2 = e.U2;
-    const bool u0 = U1 >= 0 && U1 <= r.nu - 1;
-    const bool u1 = U1 + 1 <= U2 && U1 + 1 >= 0 && U1 + 1 <= r.nu - 1;
-    c.flags = (u0 ? SC_U0 : 0) | (u1 ? SC_U1 : 0) | (U2 - U1 <= 1 ? SC_NARROW : 0) |
-              (U2 >= 0 && U1 <= r.nu - 1 ? SC_UANY : 0);
-    const int cu0 = min(max(U1, 0), r.nu - 1), cu1 = min(max(U1 + 1, 0), r.nu - 1);
-    c.r0 = cu0 * su + d * sd;
-    c.r1 = cu1 * su + d * sd;
-    return c;
-}
-
-// A 2x2 footprint window (U1, U1+1) x (Z1, Z1+1) of one slab: weights,
-// clamped (always in-bounds) addresses and which of the four voxels the
-// reference's loops visit (:80-88 / :133-141).
-struct SlabZ {
-    float wu0, wu1, wz0, wz1;
-    int a00, a01, a10, a11;
-    bool p00, p01, p10, p11;
-};
-
-// Axial part of slab d for this ray; true (and w filled) if the footprint is
-// a 2x2 window whose weights the branch-free division computed exactly.
-// zsafe: the ray's axial coordinates stay inside the range of the
-// magic-number floor (otherwise the caller takes the general path).  CHECK:
-// test the division's operand range here; without it the caller has shown it
-// for every slab of the ray (ray_axial).  CLAMP: the four candidates'
-// addresses are clamped to the volume, so that they can be loaded before the
-// predicates are known; otherwise they are exact only where their predicate
-// holds, and the caller loads under the predicate.  Voxel indices are
-// 32-bit: volumes are validated to hold fewer than 2^31 voxels (the
-// reference indexes with int as well).
-template <bool CHECK, bool CLAMP = true>
-__device__ __forceinline__ bool slab_window(const RayGeom &r, const Geom &g, const SlabC &c, int sz,
-                                            float z_half, bool zsafe, SlabZ &w) {
-    // :71-77 / :124-130 ("ratio * xc + z1 + nz / 2", z1 = 0)
-    const float cz0 = __fadd_rn(__fmul_rn(r.rz0, c.dc), z_half);
-    const float cz1 = __fadd_rn(__fmul_rn(r.rz1, c.dc), z_half);
-    const float zi1 = fminf(cz0, cz1), zi2 = fmaxf(cz0, cz1);
-    float fz0;
-    const int Z1 = mk_floor(zi1, fz0);
-    const float fz1 = __fadd_rn(fz0, 1.0f), fz2 = __fadd_rn(fz1, 1.0f);
-    const float dz = __fsub_rn(zi2, zi1);
-    // Z2 = floor(zi2) is Z1 (zi2 < Z1 + 1) or Z1 + 1 (zi2 < Z1 + 2) for a
-    // window of at most two slices: compared against the exact floats
-    // Z1 + 1, Z1 + 2 (zsafe: |zi| < 2^19)
-    const bool two = zi2 >= fz1, narrow = zi2 < fz2;
-    const unsigned nz = (unsigned)g.nz;
-    // the reference's axial loop visits Z1 and (when Z2 = Z1 + 1) Z1 + 1,
-    // clamped to the volume (:80-82 / :133-135)
-    const bool u0 = c.flags & SC_U0, u1 = c.flags & SC_U1;
-    const bool z0 = (unsigned)Z1 < nz;
-    const bool z1 = two && (unsigned)Z1 + 1u < nz;
-    w.p00 = u0 && z0;
-    w.p01 = u0 && z1;
-    w.p10 = u1 && z0;
-    w.p11 = u1 && z1;
-    w.wu0 = c.a;
-    w.wu1 = c.b;
-    const float n0 = __fsub_rn(fminf(fz1, zi2), fmaxf(fz0, zi1));
-    const float n1 = __fsub_rn(fminf(fz2, zi2), fmaxf(fz1, zi1));
-    const float y = mk_recip(dz);
-    w.wz0 = mk_div(n0, dz, y);
-    w.wz1 = mk_div(n1, dz, y);
-    const bool exact = CHECK ? (mk_den_ok(dz) && mk_num_ok(n0) && mk_num_ok(n1)) : true;
-    if (CLAMP) {
-        const int cz0i = min(max(Z1, 0), g.nz - 1), cz1i = min(max(Z1 + 1, 0), g.nz - 1);
-        w.a00 = c.r0 + cz0i * sz;
-        w.a01 = c.r0 + cz1i * sz;
-        w.a10 = c.r1 + cz0i * sz;
-        w.a11 = c.r1 + cz1i * sz;
-    } else {  // (unsigned: wraps instead of overflowing where Z1 is out of range)
-        const unsigned zo = (unsigned)Z1 * (unsigned)sz;
-        w.a00 = (int)((unsigned)c.r0 + zo);
-        w.a01 = (int)((unsigned)w.a00 + (unsigned)sz);
-        w.a10 = (int)((unsigned)c.r1 + zo);
-        w.a11 = (int)((unsigned)w.a10 + (unsigned)sz);
-    }
-    // outside the division's checked range the caller takes the general path
-    return (c.flags & SC_NARROW) && narrow && exact && zsafe;
-}
-
 // Per-ray facts about the axial footprint over all the ray's slabs, bounded
 // from the ray's constants with rounding margins: the slab distance dc runs
 // monotonically over [dc(0), dc(nd - 1)] and cz = rz * dc + nz/2 is linear in
 // it, computed with an error below 2^-23 * max|cz|.
-//  zsafe: |cz| < 2^19, inside the magic-number floor's range, so that also
-//         dz = zi2 - zi1 < 2^20;
-//  exact: additionally dc keeps one sign, dz >= 2^-19 (|rz1 - rz0| * |dc|
-//         less the rounding) and no cz comes within 2^-50 of zero.  Then
-//         every slab's division operands are in mk_div's checked range: dz is
-//         in [2^-20, 2^20); n0 is either dz or (Z1 + 1) - zi1, a positive
-//         multiple of ulp(zi1) >= 2^-73; n1, used only when Z2 = Z1 + 1, is
-//         zi2 - (Z1 + 1), zero or a positive multiple of ulp(zi2); cz is
-//         never -0, so neither is -0.  (n1 when Z2 = Z1 is never used.)
+//  zsafe:  |cz| < 2^19, inside the magic-number floor's range, so that also
+//          dz = zi2 - zi1 < 2^20;
+//  narrow: additionally dc keeps one sign, x21 or y21 the same one, so that
+//          cz0 and cz1 grow with the detector row (products, quotients and
+//          sums round monotonically) and cz0 <= cz1 are the minimum and the
+//          maximum themselves; and dz is in [2^-19, 0.99], so the footprint
+//          spans at most the two slices Z1 and Z1 + 1.
+// On a narrow ray's slabs with 0 <= Z1 every division's operands are in
+// mk_div's checked range: dz is; n0 is dz or (Z1 + 1) - zi1 with
+// 0 <= zi1 < Z1 + 1, at least 2^-24 and positive; n1, used only when
+// Z2 = Z1 + 1, is zi2 - (Z1 + 1), +0 or at least an ulp of 1.
 struct RayAxial {
-    bool zsafe, exact;
+    bool zsafe, narrow;
 };
 __device__ __forceinline__ RayAxial ray_axial(const RayGeom &r, float z_half) {
     const float dc_lo = __fsub_rn(__fsub_rn(0.5f, r.d_half), r.src_d) - 1.0f;
@@ -599,17 +482,13 @@ __device__ __forceinline__ RayAxial ray_axial(const RayGeom &r, float z_half) {
     const float err = zmax * 0x1p-21f;  // >= 4 ulp of any cz, covers these bounds' rounding
     RayAxial a;
     a.zsafe = zmax + err < 0x1p19f;
-    const bool one_sign = dc_lo > 0.0f || dc_hi < 0.0f;
+    // rz = (z2 -+ db/2) / x21: rz0 < rz1 exactly when x21 > 0
+    const bool ordered = (dc_lo > 0.0f && r.rz0 < r.rz1) || (dc_hi < 0.0f && r.rz0 > r.rz1);
     const float dmin = fminf(fabsf(dc_lo), fabsf(dc_hi));
     const float drz = fabsf(r.rz1 - r.rz0);
     const float dz_min = (drz * dmin - 2.0f * err) * (1.0f - 0x1p-20f);
-    // the range of each cz over the ray, from its ends
-    const float e0a = fmaf(r.rz0, dc_lo, z_half), e0b = fmaf(r.rz0, dc_hi, z_half);
-    const float e1a = fmaf(r.rz1, dc_lo, z_half), e1b = fmaf(r.rz1, dc_hi, z_half);
-    const float tiny = 0x1p-50f + err;
-    const bool off0 = fminf(e0a, e0b) > tiny || fmaxf(e0a, e0b) < -tiny;
-    const bool off1 = fminf(e1a, e1b) > tiny || fmaxf(e1a, e1b) < -tiny;
-    a.exact = a.zsafe && one_sign && dz_min >= 0x1p-19f && off0 && off1;
+    const float dz_max = (drz * dmax + 2.0f * err) * (1.0f + 0x1p-20f);
+    a.narrow = a.zsafe && ordered && dz_min >= 0x1p-19f && dz_max <= 0.99f;
     return a;
 }
 
@@ -618,110 +497,152 @@ __device__ __forceinline__ RayAxial ray_axial(const RayGeom &r, float z_half) {
 // reference's axial loop over max(0, Z1) .. min(nz-1, Z2) is empty
 // (:80-82 / :133-135) and the slab adds nothing.  Worked from the exact lines
 // c_k(dc) = rz_k * dc + nz/2 of the ray's own (float) constants with a
-// tolerance of 1/64 voxel, far above the difference of their float
-// evaluation (a few ulp of values below 2^20); each condition's set of dc is
-// a union of half-lines whose hull is taken, and the intersection of the
-// hulls is mapped to slab indices with one slab of margin on either side.
-// Returns lo > hi when no slab can contribute.
-__device__ __forceinline__ void ray_zrange(const RayGeom &r, float z_half, int nz, int &lo,
-                                           int &hi) {
-    const double tol = 1.0 / 64.0, zh = z_half, rz[2] = {r.rz0, r.rz1};
-    const double inf = 1e300;
-    // hull of F1 = U_k {rz_k dc >= -tol - zh}: [lo1, hi1]
-    double lo1 = inf, hi1 = -inf;
-    // hull of F2 = U_k {rz_k dc < nz + tol - zh}: [lo2, hi2]
-    double lo2 = inf, hi2 = -inf;
+// tolerance of 1/16 voxel, far above the difference of their float evaluation
+// (a few ulp of values below 2^16 at the faces); each condition's set of dc is
+// a union of half-lines whose hull is taken, and the intersection of the hulls
+// is mapped to slab indices with a margin of one slab plus the rounding of
+// these float expressions (2^-19 of the largest magnitude, four times the sum
+// of their relative errors).  Returns lo > hi when no slab can contribute.
+__device__ __forceinline__ void ray_zrange(const RayGeom &r, float zh, int nz, int &lo, int &hi) {
+    const float tol = 1.0f / 16.0f, inf = __int_as_float(0x7f800000);
+    const float rz[2] = {r.rz0, r.rz1};
+    // hulls of U_k {rz_k dc >= -tol - zh} and U_k {rz_k dc < nz + tol - zh}
+    float lo1 = inf, hi1 = -inf, lo2 = inf, hi2 = -inf;
+    const float t1 = -tol - zh, t2 = (float)nz + tol - zh;
 #pragma unroll
     for (int k = 0; k < 2; k++) {
-        const double a = rz[k];
-        const double t1 = (-tol - zh) / a, t2 = ((double)nz + tol - zh) / a;
-        if (a > 0.0) {
-            lo1 = fmin(lo1, t1); hi1 = inf;    // [t1, inf)
-            lo2 = -inf; hi2 = fmax(hi2, t2);   // (-inf, t2)
-        } else if (a < 0.0) {
-            lo1 = -inf; hi1 = fmax(hi1, t1);   // (-inf, t1]
-            lo2 = fmin(lo2, t2); hi2 = inf;    // (t2, inf)
+        const float a = rz[k];
+        float y;  // 1 / a to 2^-22
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(a));
+        if (a > 0.0f) {
+            lo1 = fminf(lo1, t1 * y); hi1 = inf;    // [t1, inf)
+            lo2 = -inf; hi2 = fmaxf(hi2, t2 * y);   // (-inf, t2)
+        } else if (a < 0.0f) {
+            lo1 = -inf; hi1 = fmaxf(hi1, t1 * y);   // (-inf, t1]
+            lo2 = fminf(lo2, t2 * y); hi2 = inf;    // (t2, inf)
         } else {  // constant zh: inside [0, nz)
             lo1 = -inf; hi1 = inf;
             lo2 = -inf; hi2 = inf;
         }
     }
-    const double dlo = fmax(lo1, lo2), dhi = fmin(hi1, hi2);
-    // slab d has dc = d + 0.5 - d_half - src_d (up to the rounding of
-    // those floats)
-    const double off = (double)r.d_half + (double)r.src_d - 0.5;
-    const double a = fmax(dlo + off, -2.0), b = fmin(dhi + off, (double)r.nd + 1.0);
-    if (!(a <= b)) {  // also NaN
-        lo = 1;
-        hi = 0;
-        return;
+    // slab d has dc = d + 0.5 - d_half - src_d (up to the rounding of those floats)
+    const float off = r.d_half + r.src_d - 0.5f, fn = (float)r.nd;
+    const float m = 1.0f + 0x1p-19f * (fn + fabsf(off) + 2.0f);
+    const float a = fmaxf(fmaxf(lo1, lo2) + off - m, -1.0f);
+    const float b = fminf(fminf(hi1, hi2) + off + m, fn);
+    if (a <= b) {
+        lo = max(0, (int)floorf(a));
+        hi = min(r.nd - 1, (int)ceilf(b));
+    } else {  // also NaN
+        lo = INT_MAX;
+        hi = INT_MIN;
     }
-    lo = max(0, (int)floor(a) - 1);
-    hi = min(r.nd - 1, (int)ceil(b) + 1);
 }
 
-// One slab of one ray, any footprint: the 2x2 window with predication or the
-// reference's loops (:80-88 / :133-141).
-template <int K, bool ONES, typename VT, bool CHECK, bool PAIR = false>
-__device__ __forceinline__ void fp_slab(const RayGeom &r, const Geom &g, const SlabC &e, int d,
-                                        const VT *const *base, int su, int sd, int sz,
-                                        float z_half, bool zsafe, float *acc, float &accw) {
-    SlabZ w;
-    // (every load below is under its voxel's predicate)
-    if (slab_window<CHECK, false>(r, g, e, sz, z_half, zsafe, w)) {
-        // each volume's terms in the window's order (the volumes' sums are
-        // independent, so visiting the voxels outermost keeps every order)
-        float t[K];
-        if (w.p00) {
-            fp_voxel<K, PAIR>(base, w.a00, t);
-#pragma unroll
-            for (int k = 0; k < K; k++) acc[k] = __fmaf_rn(__fmul_rn(t[k], w.wu0), w.wz0, acc[k]);
+// A slab of a warp's table: what its rays share.  In-plane, for a footprint
+// of at most two voxels, the voxels the reference's loop visits (:80-82 /
+// :133-135), in its order, a single one always first: the offset o of the
+// warp's window in the first one's column of the z-fastest volume (the second
+// one's is su further) and the weights a, b (zero for a voxel not visited).
+// The window begins at slice zlo, the even one at or below the first ray's Z1;
+// slices lo .. hi of it (range = lo | hi << 8) are needed and in the volume.
+// pairs (for an even nz): bit l is set where slices 2l, 2l + 1 are, bit 16 + l
+// where they are and the second voxel is visited.
+struct __align__(8) SlabCopy {
+    int o;
+    unsigned pairs;
+};
+struct SlabRest {
+    int range;
+    int flags;  // SC_*
+};
+// The rest of two neighbouring slabs, side by side for the packed operations.
+struct __align__(16) SlabPair {
+    float a[2], b[2];
+    float dc[2];  // the slabs' distances (slab_dc)
+    int zb[2];    // MK_MAGIC_BITS + zlo: a ray's place in the window is (bits
+                  // of its magic-number sum) - zb
+};
+// SC_ANY: some ray can meet the volume in the slab; SC_FAST: the in-plane
+// footprint is at most two voxels wide, and o, a, b are valid; SC_TWO: it
+// visits two voxels; SC_STAGE: additionally all rays are narrow and the window
+// holds every slice they need; SC_IN: additionally every ray's slices Z1 and
+// Z1 + 1 are in the volume.
+constexpr int SC_ANY = 1, SC_FAST = 2, SC_TWO = 4, SC_STAGE = 8, SC_IN = 16;
+constexpr int FPW = 32;  // slices per window
+
+// The table entry of slab d; rz_first, rz_last: rz0 of the warp's first and
+// last row; narrow: every ray of the warp is (ray_axial).
+__device__ __forceinline__ void slab_entry(const RayGeom &r, int d, int su, int sd, float rz_first,
+                                           float rz_last, bool narrow, float z_half, int nz,
+                                           SlabCopy &c, SlabRest &t, float &a, float &b, float &dc,
+                                           int &zb) {
+    const SlabU e = slab_u(r, d);
+    const bool two_wide = e.U2 - e.U1 <= 1;
+    const bool u0 = e.U1 >= 0 && e.U1 <= r.nu - 1;
+    const bool u1 = e.U1 + 1 <= e.U2 && e.U1 + 1 >= 0 && e.U1 + 1 <= r.nu - 1;
+    const bool any = e.U2 >= 0 && e.U1 <= r.nu - 1;
+    int f = (any ? SC_ANY : 0) | (two_wide && (u0 || u1) ? SC_FAST : 0) |
+            (two_wide && u0 && u1 ? SC_TWO : 0);
+    dc = slab_dc(r, d);
+    c.pairs = 0;
+    t.range = 1;  // none (lo > hi)
+    int zlo = 0;
+    if (narrow) {
+        // cz0 as every ray computes it (:71 / :124); rows in order, so these
+        // are the warp's smallest and largest Z1
+        const int zf = mk_floor_i(__fadd_rn(__fmul_rn(rz_first, dc), z_half));
+        const int zl = mk_floor_i(__fadd_rn(__fmul_rn(rz_last, dc), z_half)) + 1;
+        zlo = zf & ~1;
+        const int lo = max(0, -zlo), hi = min(zl, nz - 1) - zlo;
+        if (lo > hi) f = 0;  // no ray meets a slice of the volume here
+        if ((f & SC_FAST) && zl - zlo < FPW) {
+            f |= SC_STAGE | (zf >= 0 && zl <= nz - 1 ? SC_IN : 0);
+            t.range = lo | hi << 8;
+            c.pairs = (0xffffu >> (15 - (hi >> 1))) & (0xffffu << (lo >> 1));
+            if (f & SC_TWO) c.pairs |= c.pairs << 16;
         }
-        if (w.p01) {
-            fp_voxel<K, PAIR>(base, w.a01, t);
-#pragma unroll
-            for (int k = 0; k < K; k++) acc[k] = __fmaf_rn(__fmul_rn(t[k], w.wu0), w.wz1, acc[k]);
-        }
-        if (w.p10) {
-            fp_voxel<K, PAIR>(base, w.a10, t);
-#pragma unroll
-            for (int k = 0; k < K; k++) acc[k] = __fmaf_rn(__fmul_rn(t[k], w.wu1), w.wz0, acc[k]);
-        }
-        if (w.p11) {
-            fp_voxel<K, PAIR>(base, w.a11, t);
-#pragma unroll
-            for (int k = 0; k < K; k++) acc[k] = __fmaf_rn(__fmul_rn(t[k], w.wu1), w.wz1, acc[k]);
-        }
-        if (ONES) {
-            if (w.p00) accw = __fmaf_rn(w.wu0, w.wz0, accw);
-            if (w.p01) accw = __fmaf_rn(w.wu0, w.wz1, accw);
-            if (w.p10) accw = __fmaf_rn(w.wu1, w.wz0, accw);
-            if (w.p11) accw = __fmaf_rn(w.wu1, w.wz1, accw);
-        }
-        return;
     }
-    const float cz0 = __fadd_rn(__fmul_rn(r.rz0, e.dc), z_half);
-    const float cz1 = __fadd_rn(__fmul_rn(r.rz1, e.dc), z_half);
+    t.flags = f;
+    const int U = u0 ? e.U1 : u1 ? e.U1 + 1 : 0;  // the first visited voxel
+    c.o = U * su + d * sd + zlo;
+    a = f & SC_FAST ? (u0 ? e.a : e.b) : 0.0f;
+    b = f & SC_TWO ? e.b : 0.0f;
+    zb = MK_MAGIC_BITS + zlo;
+}
+
+// One slab of one ray by the reference's loops, any footprint (:80-88 /
+// :133-141).
+template <int K, bool ONES, typename VT, bool PAIR>
+__device__ __forceinline__ void fp_slab_general(const RayGeom &r, const Geom &g, int d,
+                                                const VT *const *base, float z_half, float *acc,
+                                                float &accw) {
+    int su, sd;
+    zf_strides(r.xdrive, g, su, sd);
+    const SlabU e = slab_u(r, d);
+    const float dc = slab_dc(r, d);
+    // :71-77 / :124-130 ("ratio * xc + z1 + nz / 2", z1 = 0)
+    const float cz0 = __fadd_rn(__fmul_rn(r.rz0, dc), z_half);
+    const float cz1 = __fadd_rn(__fmul_rn(r.rz1, dc), z_half);
     const float zi1 = fminf(cz0, cz1), zi2 = fmaxf(cz0, cz1);
     const int Z1 = (int)floorf(zi1), Z2 = (int)floorf(zi2);
     const float dz = __fsub_rn(zi2, zi1);
     const int U1 = e.U1, U2 = e.U2;
-    const bool fast_u = U2 - U1 <= 1;
+    const bool narrow = U2 - U1 <= 1;
     const int u_lo = max(0, U1), u_hi = min(r.nu - 1, U2);
     const int z_lo = max(0, Z1), z_hi = min(g.nz - 1, Z2);
     const float ui1 = e.a, ui2 = e.b;
-    const float du = fast_u ? 0.0f : __fsub_rn(ui2, ui1);
+    const float du = narrow ? 0.0f : __fsub_rn(ui2, ui1);
     for (int u = u_lo; u <= u_hi; u++) {
-        const float wu = fast_u ? (u == U1 ? e.a : e.b)
+        const float wu = narrow ? (u == U1 ? e.a : e.b)
                                 : __fdiv_rn(__fsub_rn(fminf(__fadd_rn((float)u, 1.0f), ui2),
                                                       fmaxf((float)u, ui1)), du);
-        const int rowa = u * su + d * sd;
+        const int row = u * su + d * sd;
         for (int z = z_lo; z <= z_hi; z++) {
             const float wz = __fdiv_rn(__fsub_rn(fminf(__fadd_rn((float)z, 1.0f), zi2),
                                                  fmaxf((float)z, zi1)), dz);
-            const int a = rowa + z * sz;
             float t[K];
-            fp_voxel<K, PAIR>(base, a, t);
+            fp_voxel<K, PAIR>(base, row + z, t);
 #pragma unroll
             for (int k = 0; k < K; k++) acc[k] = __fmaf_rn(__fmul_rn(t[k], wu), wz, acc[k]);
             if (ONES) accw = __fmaf_rn(wu, wz, accw);
@@ -729,121 +650,261 @@ __device__ __forceinline__ void fp_slab(const RayGeom &r, const Geom &g, const S
     }
 }
 
-// The windows of slabs d0+j .. d0+j+G-1 of a ray and the 4*K voxel
-// values of each (addresses are clamped, so every load is in bounds and can
-// be issued before the predicates are known; loading under the predicates
-// from unclamped addresses measured 2-3 % slower at 256x256x160); true if
-// all of them are exact 2x2 windows.
-template <int K, int G, bool CHECK, typename VT, bool PAIR = false>
-__device__ __forceinline__ bool fp_group_load(const RayGeom &r, const Geom &g,
-                                              const SlabC (*sm_c)[FPC_COLS], int col, int j, int sz,
-                                              const VT *const *base, float z_half, bool zsafe,
-                                              SlabZ *w,
-                                              float (*v)[K][4]) {
-    bool all_fast = true;
-#pragma unroll
-    for (int q = 0; q < G; q++)
-        all_fast &= slab_window<CHECK>(r, g, sm_c[j + q][col], sz, z_half, zsafe, w[q]);
-#pragma unroll
-    for (int q = 0; q < G; q++) {
-        const int a[4] = {w[q].a00, w[q].a01, w[q].a10, w[q].a11};
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            float t[K];
-            fp_voxel<K, PAIR>(base, a[i], t);
-#pragma unroll
-            for (int k = 0; k < K; k++) v[q][k][i] = t[k];
-        }
-    }
-    return all_fast;
-}
-
-// The terms of one group in the reference's order: from the loaded windows
-// when all are 2x2 (fast), else slab by slab on the general path.
-template <int K, int G, bool ONES, typename VT, bool CHECK, bool PAIR = false>
-__device__ __forceinline__ void fp_group_sum(const RayGeom &r, const Geom &g,
-                                             const SlabC (*sm_c)[FPC_COLS], int col, int j, int d0,
-                                             const VT *const *base, int su, int sd, int sz,
-                                             float z_half, bool zsafe, bool fast, const SlabZ *w,
-                                             const float (*v)[K][4], float *acc, float &accw) {
-    if (!fast) {
-#pragma unroll 1
-        for (int q = 0; q < G; q++)
-            fp_slab<K, ONES, VT, CHECK, PAIR>(r, g, sm_c[j + q][col], d0 + j + q, base, su, sd, sz,
-                                              z_half, zsafe, acc, accw);
-        return;
-    }
-#pragma unroll
-    for (int q = 0; q < G; q++) {
-        const SlabZ &x = w[q];
-        if (K == 1 && ONES) {
-            // one volume and the weight sum: the two chains interleaved term
-            // by term (measured faster here; the per-volume order below is
-            // faster with three volumes)
-            if (x.p00) {
-                acc[0] = __fmaf_rn(__fmul_rn(v[q][0][0], x.wu0), x.wz0, acc[0]);
-                accw = __fmaf_rn(x.wu0, x.wz0, accw);
-            }
-            if (x.p01) {
-                acc[0] = __fmaf_rn(__fmul_rn(v[q][0][1], x.wu0), x.wz1, acc[0]);
-                accw = __fmaf_rn(x.wu0, x.wz1, accw);
-            }
-            if (x.p10) {
-                acc[0] = __fmaf_rn(__fmul_rn(v[q][0][2], x.wu1), x.wz0, acc[0]);
-                accw = __fmaf_rn(x.wu1, x.wz0, accw);
-            }
-            if (x.p11) {
-                acc[0] = __fmaf_rn(__fmul_rn(v[q][0][3], x.wu1), x.wz1, acc[0]);
-                accw = __fmaf_rn(x.wu1, x.wz1, accw);
-            }
-            continue;
-        }
+// One slab of one ray straight from memory, for warps whose rays are not
+// narrow: at most two slices Z1, Z1 + 1, with the operand ranges tested; false,
+// with nothing added, where a lane's footprint does not fit.
+template <int K, bool ONES, typename VT, bool PAIR>
+__device__ __forceinline__ bool fp_slab_direct(float rz0, float rz1, float dc, float a, float b,
+                                               int o, int su, bool two_u, const VT *const *base,
+                                               int nz, float z_half, float *acc, float &accw) {
+    // :71-77 / :124-130 ("ratio * xc + z1 + nz / 2", z1 = 0)
+    const float cz0 = __fadd_rn(__fmul_rn(rz0, dc), z_half);
+    const float cz1 = __fadd_rn(__fmul_rn(rz1, dc), z_half);
+    const float zi1 = fminf(cz0, cz1), zi2 = fmaxf(cz0, cz1);
+    float fz0;
+    const int Z1 = mk_floor(zi1, fz0);
+    const float fz1 = __fadd_rn(fz0, 1.0f), dz = __fsub_rn(zi2, zi1);
+    // Z2 = floor(zi2) is Z1 (zi2 < Z1 + 1) or Z1 + 1 (zi2 < Z1 + 2): compared
+    // against the exact floats
+    const bool two = zi2 >= fz1, narrow = zi2 < __fadd_rn(fz1, 1.0f);
+    // :86 / :139: min(Z1 + 1, zi2) - max(Z1, zi1), where Z1 <= zi1; and, when
+    // Z2 = Z1 + 1, min(Z1 + 2, zi2) - max(Z1 + 1, zi1) = zi2 - (Z1 + 1)
+    const float n0 = __fsub_rn(fminf(fz1, zi2), zi1);
+    const float n1 = __fsub_rn(zi2, fz1);
+    const bool outside = zi2 < 0.0f || zi1 >= (float)nz;
+    const bool ok = outside || (narrow && mk_den_ok(dz) && mk_num_ok(n0) && mk_num_ok(n1));
+    if (!__all_sync(0xffffffffu, ok)) return false;
+    const float y = mk_recip(dz);
+    const float wz0 = mk_div(n0, dz, y), wz1 = mk_div(n1, dz, y);
+    const bool p0 = (unsigned)Z1 < (unsigned)nz, p1 = two && (unsigned)(Z1 + 1) < (unsigned)nz;
+    const int z0 = min(max(Z1, 0), nz - 1), z1 = min(max(Z1 + 1, 0), nz - 1);
+    for (int u = 0; u < (two_u ? 2 : 1); u++) {
+        const float wu = u ? b : a;
+        float v0[K], v1[K];
+        fp_voxel<K, PAIR>(base, o + u * su + z0, v0);
+        fp_voxel<K, PAIR>(base, o + u * su + z1, v1);
 #pragma unroll
         for (int k = 0; k < K; k++) {
-            if (x.p00) acc[k] = __fmaf_rn(__fmul_rn(v[q][k][0], x.wu0), x.wz0, acc[k]);
-            if (x.p01) acc[k] = __fmaf_rn(__fmul_rn(v[q][k][1], x.wu0), x.wz1, acc[k]);
-            if (x.p10) acc[k] = __fmaf_rn(__fmul_rn(v[q][k][2], x.wu1), x.wz0, acc[k]);
-            if (x.p11) acc[k] = __fmaf_rn(__fmul_rn(v[q][k][3], x.wu1), x.wz1, acc[k]);
+            if (p0) acc[k] = __fmaf_rn(__fmul_rn(v0[k], wu), wz0, acc[k]);
+            if (p1) acc[k] = __fmaf_rn(__fmul_rn(v1[k], wu), wz1, acc[k]);
         }
         if (ONES) {
-            if (x.p00) accw = __fmaf_rn(x.wu0, x.wz0, accw);
-            if (x.p01) accw = __fmaf_rn(x.wu0, x.wz1, accw);
-            if (x.p10) accw = __fmaf_rn(x.wu1, x.wz0, accw);
-            if (x.p11) accw = __fmaf_rn(x.wu1, x.wz1, accw);
+            if (p0) accw = __fmaf_rn(wu, wz0, accw);
+            if (p1) accw = __fmaf_rn(wu, wz1, accw);
+        }
+    }
+    return true;
+}
+
+// ---- the warp's windows in shared memory
+// One window: FPW slices of one voxel column and of the paired volumes' (PAIR),
+// zeros in the place of slices outside the volume, and behind each a zero.
+template <typename VT, bool PAIR> struct FPWindow {
+    static constexpr unsigned ES = sizeof(VT);              // bytes per slice
+    static constexpr unsigned PAIRS = FPW * ES + 16;        // offset of the paired volumes
+    static constexpr unsigned BYTES = PAIRS + (PAIR ? 2 * FPW * ES + 16 : 0);
+};
+
+// An N-byte asynchronous copy, or N zeros where !in (nothing is read then).
+template <int N> __device__ __forceinline__ void cp_async(unsigned dst, const void *src, bool in) {
+    const int n = in ? N : 0;
+    if (N == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n)
+                     : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %3, %2;" ::"r"(dst), "l"(src), "r"(n),
+                     "n"(N)
+                     : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() {
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int N> __device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void sts_zero4(unsigned a) {
+    asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(0) : "memory");
+}
+
+// This lane's part of a slab's two windows at dst (shared memory), the second
+// one all zeros where the slab visits one in-plane voxel.  EVEN (an even nz, so
+// windows begin on even elements): slices 2j and 2j + 1 of window h as one
+// copy, lane = 16 h + j, lane_off and lane_dst that place in the volume and
+// the windows; otherwise slice `lane` of both.
+template <bool EVEN, typename VT, bool PAIR>
+__device__ __forceinline__ void window_copy(unsigned dst, const VT *const *base, const int2 c,
+                                            const SlabRest &t, int su, int lane, int bit,
+                                            int64_t lane_off, unsigned lane_dst) {
+    using W = FPWindow<VT, PAIR>;
+    constexpr int ES = sizeof(VT);
+    if (EVEN) {
+        const bool in = c.y & bit;
+        cp_async<2 * ES>(dst + lane_dst, base[0] + lane_off + c.x, in);
+        if constexpr (PAIR)
+            cp_async<4 * ES>(dst + lane_dst + W::PAIRS + 2 * ES * (lane & 15),
+                             base[1] + 2 * (lane_off + c.x), in);
+        return;
+    }
+    const int lo = t.range & 255, hi = t.range >> 8;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int64_t i = (int64_t)c.x + h * (int64_t)su + lane;
+        const unsigned w = dst + h * W::BYTES;
+        const bool in = lane >= lo && lane <= hi && (h == 0 || (t.flags & SC_TWO));
+        if constexpr (ES == 4) {
+            cp_async<4>(w + 4 * lane, base[0] + i, in);
+            if constexpr (PAIR) cp_async<8>(w + W::PAIRS + 8 * lane, base[1] + 2 * i, in);
+        } else {  // (2-byte elements: no such asynchronous copy)
+            const unsigned short v =
+                in ? *reinterpret_cast<const unsigned short *>(base[0] + i) : (unsigned short)0;
+            asm volatile("st.shared.b16 [%0], %1;" ::"r"(w + 2 * lane), "h"(v) : "memory");
+            if constexpr (PAIR) cp_async<4>(w + W::PAIRS + 4 * lane, base[1] + 2 * i, in);
         }
     }
 }
 
-// Slabs d0 + j0 .. d0 + jend - 1 of a ray from the shared table (j0 is the
-// same for the whole warp).  Groups of G slabs: the windows and loads of a
-// whole group are issued together before its terms enter the sums in the
-// reference's order, so that a warp waits for memory once per group instead
-// of per slab.  A group whose footprints are not all 2x2 windows takes the
-// general per-slab path.
-template <int K, int G, bool ONES, typename VT, bool CHECK, bool PAIR = false>
-__device__ __forceinline__ void fp_chunk(const RayGeom &r, const Geom &g,
-                                         const SlabC (*sm_c)[FPC_COLS], int col, int j0, int jend,
-                                         int d0, const VT *const *base, int su, int sd, int sz,
-                                         float z_half, bool zsafe, float *acc, float &accw) {
-    int j = j0;
-    for (; j + G <= jend; j += G) {
-        SlabZ w[G];
-        float v[G][K][4];
-        const bool fast = fp_group_load<K, G, CHECK, VT, PAIR>(r, g, sm_c, col, j, sz, base,
-                                                            z_half, zsafe, w, v);
-        fp_group_sum<K, G, ONES, VT, CHECK, PAIR>(r, g, sm_c, col, j, d0, base, su, sd, sz,
-                                               z_half, zsafe, fast, w, v, acc, accw);
+// The K volumes' values of slice z of both windows of the slab at w.
+template <int K, typename VT, bool PAIR>
+__device__ __forceinline__ void window_read(const unsigned char *w, int z, float (*v)[K]) {
+    using W = FPWindow<VT, PAIR>;
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        v[i][0] = tof(reinterpret_cast<const VT *>(w + i * W::BYTES)[z]);
+        if constexpr (PAIR) {
+            const unsigned char *q = w + i * W::BYTES + W::PAIRS;
+            if constexpr (sizeof(VT) == 4) {
+                const float2 a = reinterpret_cast<const float2 *>(q)[z];
+                v[i][1] = a.x;
+                v[i][2] = a.y;
+            } else {
+                union {
+                    unsigned u;
+                    VT h[2];
+                } a;
+                a.u = reinterpret_cast<const unsigned *>(q)[z];
+                v[i][1] = tof(a.h[0]);
+                v[i][2] = tof(a.h[1]);
+            }
+        }
     }
-    for (; j < jend; j++)
-        fp_slab<K, ONES, VT, CHECK, PAIR>(r, g, sm_c[j][col], d0 + j, base, su, sd, sz, z_half,
-                                          zsafe, acc, accw);
 }
 
-// blockDim = FPC_THREADS: thread t is column t % FPC_COLS, row t / FPC_COLS;
-// gridDim = (ceil(na/FPC_COLS), ceil(nb/FPC_ROWS), views).
-// MULTI = true: several views per launch (ordered subsets, kernel-level
-// multi-view projection), view = blockIdx.z with the per-view offsets of
-// FPArgs; false: one view per launch without them.
+// Two neighbouring staged slabs (narrow rays, nz >= 2).  The branch-free
+// division is exact wherever its quotient is used (ray_axial; with Z1 = -1, n1
+// is cz1 itself, a sum with nz/2 >= 1, so +0 or at least 2^-24).
+// What the reference's loops do not visit is read as zero, so its terms add a
+// zero to the sums: slices outside the volume and a second in-plane voxel that
+// is not visited are zeros in the window, and slice Z1 + 1 of a ray whose Z2 is
+// Z1 is read behind it; for the weights' sum their weights are set to zero.
+// Without branches the slabs of a stage are one straight line of code, whose
+// long chains (reciprocal, divisions, sums) overlap.
+// IN: every ray's slices Z1 and Z1 + 1 are in the volume; otherwise on tells
+// whether a slab is a staged one at all (its weights a, b are zero if not).
+// w: the first slab's windows.
+template <int K, bool ONES, bool IN, typename VT, bool PAIR>
+__device__ __forceinline__ void fp_pair_staged(float rz0, float rz1, const SlabPair &y, bool on_a,
+                                               bool on_b, const unsigned char *w, int nz,
+                                               float z_half, float *acc, float &accw) {
+    using W = FPWindow<VT, PAIR>;
+    const ulonglong2 ab = *reinterpret_cast<const ulonglong2 *>(&y.a);
+    const ulonglong2 dcz = *reinterpret_cast<const ulonglong2 *>(&y.dc);
+    const f32x2 dc = dcz.x;
+    const int zb[2] = {(int)(unsigned)dcz.y, (int)(unsigned)(dcz.y >> 32)};
+    const f32x2 zh = f2_pack(z_half, z_half);
+    // :71-77 / :124-130 ("ratio * xc + z1 + nz / 2", z1 = 0)
+    // (scalar products: ptxas contracts a packed product and sum, both .rn,
+    // into one fma, whose single rounding is not the reference's)
+    float d[2];
+    f2_unpack(dc, d[0], d[1]);
+    const f32x2 zi1 = f2_add(f2_pack(__fmul_rn(rz0, d[0]), __fmul_rn(rz0, d[1])), zh);
+    const f32x2 zi2 = f2_add(f2_pack(__fmul_rn(rz1, d[0]), __fmul_rn(rz1, d[1])), zh);
+    // floor(zi1) and floor(zi1) + 1 as a float from one magic-number sum (exact)
+    const f32x2 tm = f2_add_rd(zi1, f2_pack(MK_MAGIC, MK_MAGIC));
+    const f32x2 fz1 = f2_add(tm, f2_pack(1.0f - MK_MAGIC, 1.0f - MK_MAGIC));
+    const f32x2 ndz = f2_sub(zi1, zi2);  // -dz, exactly negated
+    float t[2], e2[2], f1[2], nd[2], wu[2][2];
+    f2_unpack(tm, t[0], t[1]);
+    f2_unpack(zi2, e2[0], e2[1]);
+    f2_unpack(fz1, f1[0], f1[1]);
+    f2_unpack(ndz, nd[0], nd[1]);
+    f2_unpack(ab.x, wu[0][0], wu[0][1]);
+    f2_unpack(ab.y, wu[1][0], wu[1][1]);
+    // :86 / :139: min(Z1 + 1, zi2) - max(Z1, zi1), where Z1 <= zi1; and, when
+    // Z2 = Z1 + 1, min(Z1 + 2, zi2) - max(Z1 + 1, zi1) = zi2 - (Z1 + 1)
+    const f32x2 n0 = f2_sub(f2_pack(fminf(f1[0], e2[0]), fminf(f1[1], e2[1])), zi1);
+    const f32x2 n1 = f2_sub(zi2, fz1);
+    // mk_recip and mk_div, packed
+    float y0[2];
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0[0]) : "f"(-nd[0]));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0[1]) : "f"(-nd[1]));
+    const f32x2 ys = f2_pack(y0[0], y0[1]);
+    const f32x2 yr = f2_fma(ys, f2_fma(ndz, ys, f2_pack(1.0f, 1.0f)), ys);
+    const f32x2 q0 = f2_mul(n0, yr), q1 = f2_mul(n1, yr);
+    float wz[2][2];  // [slice][slab]
+    f2_unpack(f2_fma(f2_fma(ndz, q0, n0), yr, q0), wz[0][0], wz[0][1]);
+    f2_unpack(f2_fma(f2_fma(ndz, q1, n1), yr, q1), wz[1][0], wz[1][1]);
+    float v[2][2][2][K];  // [slab][slice][in-plane voxel][volume]
+    float ow[2][2];       // weights of the weights' sum
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const unsigned char *const wh = w + h * 2 * W::BYTES;
+        // Z2 = floor(zi2) is Z1 (zi2 < Z1 + 1) or Z1 + 1: a narrow footprint,
+        // compared against the exact float
+        const bool two = e2[h] >= f1[h];
+        int z = (int)(__float_as_uint(t[h]) - (unsigned)zb[h]);  // place in the window
+        if (!IN) z = (h ? on_b : on_a) ? z : 0;
+        const int z1 = two ? z : FPW - 1;  // slice Z1 + 1, or the zero behind the window
+        window_read<K, VT, PAIR>(wh, z, v[h][0]);
+        window_read<K, VT, PAIR>(wh, z1 + 1, v[h][1]);
+        if (ONES) {
+            bool p0 = true, p2 = two;
+            if (!IN) {
+                const int Z1 = (int)(__float_as_uint(t[h]) - (unsigned)MK_MAGIC_BITS);
+                p0 = (unsigned)Z1 < (unsigned)nz;
+                p2 = two && (unsigned)(Z1 + 1) < (unsigned)nz;
+            }
+            ow[0][h] = p0 ? wz[0][h] : 0.0f;
+            ow[1][h] = p2 ? wz[1][h] : 0.0f;
+        }
+    }
+    // v * w_u of both slabs, then the terms in the reference's order: slab,
+    // in-plane voxel, slice
+    float m[2][2][2][K];
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            f2_unpack(f2_mul(f2_pack(v[0][j][i][0], v[1][j][i][0]), i ? ab.y : ab.x), m[0][j][i][0],
+                      m[1][j][i][0]);
+#pragma unroll
+            for (int k = 1; k < K; k++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) m[h][j][i][k] = __fmul_rn(v[h][j][i][k], wu[i][h]);
+        }
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+#pragma unroll
+                for (int k = 0; k < K; k++) acc[k] = __fmaf_rn(m[h][j][i][k], wz[j][h], acc[k]);
+                if (ONES) accw = __fmaf_rn(wu[i][h], ow[j][h], accw);
+            }
+}
+
+// Shared memory of a warp of fp_ref_kernel: NST * S slabs of two windows, two
+// tables of 32 slabs, their masks and the column's constants.
+template <typename VT, bool PAIR, int S, int NST> struct FPShared {
+    SlabPair pairs[32];
+    SlabCopy copy[64];
+    SlabRest rest[64];
+    uint4 mask[2];  // bit i: slab i of a table is SC_IN, SC_STAGE, neither staged nor empty
+    RayGeom ray;
+    float rz_last;
+    __align__(16) unsigned char win[NST * S][2][FPWindow<VT, PAIR>::BYTES];
+};
+
 // Row block i of n in dispatch order, from the middle of the detector
 // outwards (m, m+1, m-1, m+2, ...): central rays cross the whole volume,
 // outer ones fewer slabs (ray_zrange), so the longest blocks start first and
@@ -853,140 +914,201 @@ __device__ __forceinline__ int middle_out(int i, int n) {
     return (i & 1) ? m + (i + 1) / 2 : m - i / 2;
 }
 
-// Whether a launch of bx x by projector blocks is resident at once with
-// FPC_MIN_BLOCKS blocks per SM (so that the larger register budget of deeper
-// slab groups costs no occupancy).
-inline bool fp_one_wave(const mcsart_ctx *ctx, unsigned bx, unsigned by) {
-    return ctx->sms > 0 && (int64_t)bx * by <= (int64_t)FPC_MIN_BLOCKS * ctx->sms;
-}
-
-// Resident blocks per SM the register budget must allow: one volume, 6 (at
-// most 80 registers, which the kernel fits without spilling); three volumes,
-// FPC_MIN_BLOCKS.  Large detectors fill every SM, and there the one-volume
-// projector runs 6 blocks per SM instead of 5 (4.6 % less projector time at
-// 512x384 rays per view; unchanged at 256x192, where fewer blocks exist).
-// G = 4 slab groups keep more loads in flight and need the 128-register
-// budget; the one-volume projector takes them when every block of the launch
-// is resident at once (fp_one_wave), where the register budget costs no
-// occupancy.
-constexpr int FPC_MIN_BLOCKS_K1 = 6;
-// MINB: resident blocks per SM the register budget must allow (the launch
-// shape the driver's tuning may choose, with G; every choice gives the same
-// bits).
+// blockDim = FPC_THREADS: warp w is detector column blockIdx.x*FPC_COLS + w,
+// lane l row 32*(row block) + l; gridDim = (ceil(na/FPC_COLS),
+// ceil(nb/FPC_ROWS), views); dynamic shared memory fp_ref_smem.
+// MULTI = true: several views per launch (ordered subsets, kernel-level
+// multi-view projection), view = blockIdx.z with the per-view offsets of
+// FPArgs; false: one view per launch without them.
+// S: slabs per stage; NST: stages, NST - 1 of them in flight; MINB: resident
+// blocks per SM the register budget must allow (the launch shape the driver's
+// tuning may choose; every choice gives the same bits).
 // PAIR (three volumes): the second and third volumes interleaved in one
-// array, vol.std[1] / vol.tr[1] (fp_voxel).
+// array, vol.zf[1] (fp_voxel).
+template <int K> constexpr int fp_stage() { return K >= 3 ? 4 : 8; }
+template <int K> constexpr int fp_min_blocks() { return K >= 3 ? 5 : 6; }
 template <int K, bool ONES, typename VT, typename MT = VT, bool MULTI = false,
-          int G = fp_group<K>(), int MINB = (K == 1 && G == 2) ? FPC_MIN_BLOCKS_K1 : FPC_MIN_BLOCKS,
-          bool PAIR = false>
+          int S = fp_stage<K>(), int NST = 2, int MINB = fp_min_blocks<K>(), bool PAIR = false>
 __global__ void __launch_bounds__(FPC_THREADS, MINB) fp_ref_kernel(const FPArgs<VT, K, MT> p) {
-    __shared__ SlabC sm_c[FPC_CHUNK][FPC_COLS];
+    static_assert(K == 1 || PAIR, "one volume, or three with the last two paired");
+    static_assert(32 % S == 0 && S % 2 == 0 && (NST - 1) * S <= 32, "a table holds whole stages");
+    using W = FPWindow<VT, PAIR>;
+    using Shared = FPShared<VT, PAIR, S, NST>;
+    extern __shared__ __align__(16) unsigned char sm_warps[];
+    __shared__ float sm_s[K + (ONES ? 1 : 0)][FPC_ROWS][FPC_COLS + 1];
     __shared__ double2 sm_norm[FPC_THREADS / 32];
-    __shared__ int sm_wr[FPC_THREADS / 32][2];  // each warp's slab range
-    __shared__ int sm_ur[2];                    // the chunk's in-plane slab range
     const Geom &g = p.g;
-    const int t = threadIdx.x, col = t % FPC_COLS, row = t / FPC_COLS;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int by = middle_out(blockIdx.y, gridDim.y);  // this block's row block
-    const int ia = blockIdx.x * FPC_COLS + col, ib = by * FPC_ROWS + row;
-    const bool col_ok = ia < g.na;
-    const bool active = col_ok && ib < g.nb;
     const float angle = p.angles ? p.angles[blockIdx.z] : p.angle;
-    const float cphi = cosf(angle), sphi = sinf(angle);  // :23-24
-    // rows past the detector still compute their column's in-plane part
-    const RayGeom r = ray_geom(cphi, sphi, col_ok ? ia : 0, min(ib, g.nb - 1), g);
-
-    const VT *base[K];
-    int su, sd;
-    const int sz = g.nx * g.ny;
-    const int64_t voff = MULTI ? (int64_t)blockIdx.z * p.vol_stride : 0;
-    if (r.xdrive) {
-        if (p.vol.tr[0] != nullptr) {
+    {
+        const int ia = blockIdx.x * FPC_COLS + warp, ib = by * FPC_ROWS + lane;
+        float acc[K], accw = 0.0f;
 #pragma unroll
-            for (int k = 0; k < K; k++) base[k] = p.vol.tr[k] + voff;
-            su = 1; sd = g.ny;
-        } else {
+        for (int k = 0; k < K; k++) acc[k] = 0.0f;
+        if (ia < g.na) {  // the same for the whole warp
+            Shared &sm = reinterpret_cast<Shared *>(sm_warps)[warp];
+            const VT *base[K];
+            const int64_t voff = MULTI ? (int64_t)blockIdx.z * p.vol_stride : 0;
 #pragma unroll
-            for (int k = 0; k < K; k++) base[k] = p.vol.std[k] + voff;
-            su = g.nx; sd = 1;
-        }
-    } else {
-#pragma unroll
-        for (int k = 0; k < K; k++) base[k] = p.vol.std[k] + voff;
-        su = 1; sd = g.nx;
-    }
-    const float z_half = (float)(g.nz / 2);
-    float acc[K], accw = 0.0f;
-#pragma unroll
-    for (int k = 0; k < K; k++) acc[k] = 0.0f;
-
-    // warps whose rays all have proven division operands skip the per-slab
-    // range checks (warp-uniform, so neither form diverges)
-    const RayAxial ax = ray_axial(r, z_half);
-    const bool warp_exact = __all_sync(0xffffffffu, !active || ax.exact);
-    // Slabs that can add to some ray of the warp: the union of the rays'
-    // axial ranges (ray_zrange); the block visits the union of its warps'.
-    // Outside them, and outside the slabs where some column of the block
-    // meets the volume in-plane (SC_UANY), the reference's loops are empty.
-    int zlo = 1, zhi = 0;
-    if (active) ray_zrange(r, z_half, g.nz, zlo, zhi);
-    if (zlo > zhi) {
-        zlo = INT_MAX;
-        zhi = INT_MIN;
-    }
-    const int wlo = __reduce_min_sync(0xffffffffu, zlo), whi = __reduce_max_sync(0xffffffffu, zhi);
-    if ((t & 31) == 0) {
-        sm_wr[t >> 5][0] = wlo;
-        sm_wr[t >> 5][1] = whi;
-    }
-    __syncthreads();
-    int blo = INT_MAX, bhi = INT_MIN;
-#pragma unroll
-    for (int w = 0; w < FPC_THREADS / 32; w++) {
-        blo = min(blo, sm_wr[w][0]);
-        bhi = max(bhi, sm_wr[w][1]);
-    }
-    const int first = blo <= bhi ? blo - blo % FPC_CHUNK : 0;
-    for (int d0 = first; d0 <= bhi; d0 += FPC_CHUNK) {
-        for (int j = row; j < FPC_CHUNK; j += FPC_ROWS) {
-            const int d = d0 + j;
-            SlabC e;
-            e.r0 = 0; e.r1 = 0; e.a = 0.0f; e.b = 0.0f; e.dc = 0.0f;
-            e.U1 = 0; e.U2 = -1; e.flags = 0;
-            if (col_ok && d < r.nd) e = slab_c(r, d, su, sd);
-            sm_c[j][col] = e;
-        }
-        __syncthreads();
-        if (t < 32) {  // the chunk's slabs where some column meets the volume in-plane
-            unsigned m[FPC_CHUNK / 32];
-#pragma unroll
-            for (int h = 0; h < FPC_CHUNK / 32; h++) {
-                bool any = false;
-#pragma unroll
-                for (int c = 0; c < FPC_COLS; c++) any |= (sm_c[h * 32 + t][c].flags & SC_UANY) != 0;
-                m[h] = __ballot_sync(0xffffffffu, any);
+            for (int k = 0; k < K; k++)
+                base[k] = PAIR && k == 2 ? nullptr : p.vol.zf[k] + (PAIR && k == 1 ? 2 : 1) * voff;
+            const float z_half = (float)(g.nz / 2);
+            const int nz = g.nz;
+            float rz0, rz1;
+            int wlo, whi;
+            bool w_safe, w_narrow;
+            {
+                const float cphi = cosf(angle), sphi = sinf(angle);  // :23-24
+                // lanes past the last row repeat its ray; nothing of them is stored
+                const RayGeom r = ray_geom(cphi, sphi, ia, min(ib, g.nb - 1), g);
+                const RayAxial ax = ray_axial(r, z_half);
+                w_safe = __all_sync(0xffffffffu, ax.zsafe);
+                w_narrow = __all_sync(0xffffffffu, ax.narrow) && nz >= 2;
+                // the warp's slabs: those where some ray meets the volume
+                int lo, hi;
+                ray_zrange(r, z_half, nz, lo, hi);
+                wlo = __reduce_min_sync(0xffffffffu, lo);
+                whi = __reduce_max_sync(0xffffffffu, hi);
+                // the column's constants live in shared memory, read again
+                // per table, so that the slab loop's registers hold the ray's own
+                if (lane == 0) sm.ray = r;
+                if (lane == 31) sm.rz_last = r.rz0;
+                rz0 = r.rz0;
+                rz1 = r.rz1;
             }
-            if (t == 0) {
-                int lo = FPC_CHUNK, hi = -1;
+            const unsigned win0 = (unsigned)__cvta_generic_to_shared(&sm.win[0][0][0]);
+            // the zeros behind the windows
+            for (int i = lane; i < NST * S * 2; i += 32) {
+                sts_zero4(win0 + i * W::BYTES + FPW * W::ES);
+                if (PAIR) {
+                    sts_zero4(win0 + i * W::BYTES + W::PAIRS + 2 * FPW * W::ES);
+                    sts_zero4(win0 + i * W::BYTES + W::PAIRS + 2 * FPW * W::ES + 4);
+                }
+            }
+            __syncwarp();
+            const bool even = nz % 2 == 0;
+            const int bit = 1 << lane;
+            int su_;
+            {
+                int sd;
+                zf_strides(sm.ray.xdrive, g, su_, sd);
+            }
+            const int su = su_;
+            const int64_t lane_off = (lane >> 4) * (int64_t)su + 2 * (lane & 15);
+            const unsigned lane_dst = (lane >> 4) * W::BYTES + 2 * W::ES * (lane & 15);
+            const int n = wlo <= whi ? whi - wlo + 1 : 0;  // slab i of the warp is wlo + i
+            const int stages = (n + S - 1) / S;
+
+            // Copies the windows of stage s (slabs s*S ..), filling the table
+            // of 32 slabs first where the stage begins one.
+            auto issue = [&](int s) {
+                if (s < stages) {
+                    const int i0 = s * S;
+                    if (i0 % 32 == 0) {
+                        const int i = i0 + lane;
+                        const RayGeom rc = sm.ray;
+                        int su, sd;
+                        zf_strides(rc.xdrive, g, su, sd);
+                        SlabCopy c;
+                        SlabRest e;
+                        float a, b, dc;
+                        int zb;
+                        slab_entry(rc, wlo + min(i, n - 1), su, sd, rc.rz0, sm.rz_last, w_narrow,
+                                   z_half, nz, c, e, a, b, dc, zb);
+                        if (i >= n) {
+                            e.flags = 0;
+                            c.pairs = 0;
+                            e.range = 1;
+                            a = b = 0.0f;
+                        }
+                        const unsigned in = __ballot_sync(0xffffffffu, (e.flags & SC_IN) != 0);
+                        const unsigned st = __ballot_sync(0xffffffffu, (e.flags & SC_STAGE) != 0);
+                        const unsigned slow = __ballot_sync(
+                            0xffffffffu, (e.flags & (SC_ANY | SC_STAGE)) == SC_ANY);
+                        sm.copy[i & 63] = c;
+                        sm.rest[i & 63] = e;
+                        SlabPair &y = sm.pairs[(i & 63) >> 1];
+                        y.a[i & 1] = a;
+                        y.b[i & 1] = b;
+                        y.dc[i & 1] = dc;
+                        y.zb[i & 1] = zb;
+                        if (lane == 0) sm.mask[(i0 >> 5) & 1] = make_uint4(in, st, slow, 0);
+                        __syncwarp();
+                    }
+                    const SlabCopy *const c = sm.copy + (i0 & 63);
+                    const SlabRest *const e = sm.rest + (i0 & 63);
+                    const unsigned dst = win0 + s % NST * (S * 2 * W::BYTES);
+                    if (even) {
 #pragma unroll
-                for (int h = FPC_CHUNK / 32 - 1; h >= 0; h--)
-                    if (m[h]) lo = h * 32 + __ffs(m[h]) - 1;
+                        for (int q = 0; q < S; q++)
+                            window_copy<true, VT, PAIR>(
+                                dst + q * 2 * W::BYTES, base, *reinterpret_cast<const int2 *>(c + q),
+                                e[q], su, lane, bit, lane_off, lane_dst);
+                    } else {
+#pragma unroll 1
+                        for (int q = 0; q < S; q++)
+                            window_copy<false, VT, PAIR>(
+                                dst + q * 2 * W::BYTES, base, *reinterpret_cast<const int2 *>(c + q),
+                                e[q], su, lane, bit, lane_off, lane_dst);
+                    }
+                }
+                cp_async_commit();
+            };
+
+#pragma unroll 1
+            for (int s = 0; s < NST - 1; s++) issue(s);
+#pragma unroll 1
+            for (int s = 0; s < stages; s++) {
+                issue(s + NST - 1);
+                cp_async_wait<NST - 1>();
+                __syncwarp();
+                const int i0 = s * S;
+                const unsigned char(*const w)[2][W::BYTES] = sm.win + s % NST * S;
+                const SlabPair *const y = sm.pairs + ((i0 & 63) >> 1);
+                // the stage's bits of the table's masks (in, staged, slow)
+                uint4 m = sm.mask[(i0 >> 5) & 1];
+                constexpr unsigned ALL = (1u << S) - 1;
+                m.x = m.x >> (i0 & 31) & ALL;
+                m.y = m.y >> (i0 & 31) & ALL;
+                m.z = m.z >> (i0 & 31) & ALL;
+                if (m.x == ALL) {
 #pragma unroll
-                for (int h = 0; h < FPC_CHUNK / 32; h++)
-                    if (m[h]) hi = h * 32 + 31 - __clz(m[h]);
-                sm_ur[0] = lo;
-                sm_ur[1] = hi;
+                    for (int q = 0; q < S; q += 2)
+                        fp_pair_staged<K, ONES, true, VT, PAIR>(rz0, rz1, y[q / 2], true, true,
+                                                                w[q][0], nz, z_half, acc, accw);
+                } else if (m.z == 0) {
+                    if (m.y == 0) continue;  // no staged slab: no ray meets the volume
+#pragma unroll
+                    for (int q = 0; q < S; q += 2)
+                        fp_pair_staged<K, ONES, false, VT, PAIR>(rz0, rz1, y[q / 2], m.y >> q & 1u,
+                                                                 m.y >> (q + 1) & 1u, w[q][0], nz,
+                                                                 z_half, acc, accw);
+                } else {
+#pragma unroll 1
+                    for (int q = 0; q < S; q++) {
+                        const int o = sm.copy[(i0 + q) & 63].o, f = sm.rest[(i0 + q) & 63].flags;
+                        if (!(f & SC_ANY)) continue;
+                        const SlabPair &yq = y[q / 2];
+                        RayGeom rc = sm.ray;
+                        rc.rz0 = rz0;
+                        rc.rz1 = rz1;
+                        if (w_safe && (f & SC_FAST) &&
+                            fp_slab_direct<K, ONES, VT, PAIR>(
+                                rz0, rz1, yq.dc[q & 1], yq.a[q & 1], yq.b[q & 1],
+                                o - (yq.zb[q & 1] - MK_MAGIC_BITS), su, (f & SC_TWO) != 0,
+                                base, nz, z_half, acc, accw))
+                            continue;
+                        fp_slab_general<K, ONES, VT, PAIR>(rc, g, wlo + i0 + q, base, z_half, acc,
+                                                           accw);
+                    }
+                }
+                __syncwarp();  // the stage's windows may be overwritten now
             }
         }
-        __syncthreads();
-        // (an empty warp range is wlo = INT_MAX > whi = INT_MIN)
-        const int j0 = wlo <= whi ? max(sm_ur[0], wlo - d0) : 0;
-        const int jend = (active && wlo <= whi) ? min(min(sm_ur[1], whi - d0) + 1, r.nd - d0) : 0;
-        if (warp_exact)
-            fp_chunk<K, G, ONES, VT, false, PAIR>(r, g, sm_c, col, max(j0, 0), jend, d0, base, su,
-                                               sd, sz, z_half, ax.zsafe, acc, accw);
-        else
-            fp_chunk<K, G, ONES, VT, true, PAIR>(r, g, sm_c, col, max(j0, 0), jend, d0, base, su,
-                                              sd, sz, z_half, ax.zsafe, acc, accw);
-        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < K; k++) sm_s[k][lane][warp] = acc[k];
+        if (ONES) sm_s[K][lane][warp] = accw;
     }
 
     if (p.bpcolA != nullptr) {
@@ -1005,29 +1127,38 @@ __global__ void __launch_bounds__(FPC_THREADS, MINB) fp_ref_kernel(const FPArgs<
             p.bpcolB[coff + c] = col.r0;
         }
     }
+    __syncthreads();
 
-    const int64_t pix = ia + (int64_t)ib * g.na;
-    const int64_t vpix = MULTI ? pix + (int64_t)blockIdx.z * g.na * g.nb : pix;  // this view's cell
+    // epilogue with the block's columns along the lanes, as the detector is stored
     double nb2 = 0.0, nr2 = 0.0;
-    if (active) {
+#pragma unroll
+    for (int e = t; e < FPC_ROWS * FPC_COLS; e += FPC_THREADS) {
+        const int ecol = e % FPC_COLS, erow = e / FPC_COLS;
+        const int ia = blockIdx.x * FPC_COLS + ecol, ib = by * FPC_ROWS + erow;
+        if (ia >= g.na || ib >= g.nb) continue;
+        const int64_t pix = ia + (int64_t)ib * g.na;
+        // this view's cell
+        const int64_t vpix = MULTI ? pix + (int64_t)blockIdx.z * g.na * g.nb : pix;
+        const float s0 = sm_s[0][erow][ecol];
         if (p.mode == FP_PLAIN) {
-            p.out[vpix] = acc[0];
-        } else {
-            const float b = ldv(p.meas, vpix);
-            // AUMISART.cu:206 host_add(proj, proj_temp, -1): proj += proj_temp * -1
-            float res = __fmaf_rn(acc[0], -1.0f, b);
-            float ones = ONES ? accw : 0.0f;
-            if (p.mode == FP_MOTION) {
-                res = __fmaf_rn(acc[K > 1 ? 1 : 0], 1.0f, res);  // AUMISART.cu:260, + FP(img0)
-                if (K >= 3) ones = acc[K - 1];                   // FP(initial2(...)), :267-268
-            }
-            if (p.resid) p.resid[vpix] = res;
-            // the backprojector's operands as the reference's texture reads
-            // them; resid and the norms keep the residual itself
-            p.bp_in[vpix] = make_float2(tex_texel(res), tex_texel(ones));
-            nb2 = (double)b * (double)b;
-            nr2 = (double)res * (double)res;
+            p.out[vpix] = s0;
+            continue;
         }
+        const float b = ldv(p.meas, vpix);
+        // AUMISART.cu:206 host_add(proj, proj_temp, -1): proj += proj_temp * -1
+        float res = __fmaf_rn(s0, -1.0f, b);
+        float ones = ONES ? sm_s[ONES ? K : 0][erow][ecol] : 0.0f;
+        if (p.mode == FP_MOTION) {
+            // AUMISART.cu:260, + FP(img0)
+            res = __fmaf_rn(sm_s[K > 1 ? 1 : 0][erow][ecol], 1.0f, res);
+            if (K >= 3) ones = sm_s[K - 1][erow][ecol];  // FP(initial2(...)), :267-268
+        }
+        if (p.resid) p.resid[vpix] = res;
+        // the backprojector's operands as the reference's texture reads
+        // them; resid and the norms keep the residual itself
+        p.bp_in[vpix] = make_float2(tex_texel(res), tex_texel(ones));
+        nb2 += (double)b * (double)b;
+        nr2 += (double)res * (double)res;
     }
     if (p.mode == FP_PLAIN) return;
     // block partial of the two squared norms, fixed-order reduction
@@ -1036,7 +1167,7 @@ __global__ void __launch_bounds__(FPC_THREADS, MINB) fp_ref_kernel(const FPArgs<
         nb2 += __shfl_down_sync(0xffffffffu, nb2, off);
         nr2 += __shfl_down_sync(0xffffffffu, nr2, off);
     }
-    if ((t & 31) == 0) sm_norm[t >> 5] = make_double2(nb2, nr2);
+    if (lane == 0) sm_norm[warp] = make_double2(nb2, nr2);
     __syncthreads();
     if (t == 0) {
         double tb = 0.0, tr = 0.0;
@@ -1049,26 +1180,40 @@ __global__ void __launch_bounds__(FPC_THREADS, MINB) fp_ref_kernel(const FPArgs<
     }
 }
 
-// Per-ray projector, used for the split summation modes (the engine launches
-// fp_ref_kernel for SUM_REF).
-// Launch shapes.  SUM_REF: blockDim (32, 8), one ray per thread, 32 columns x
-// 8 rows per block, gridDim (ceil(na/32), ceil(nb/8), views).  Split modes:
-// blockDim (32, groups), threadIdx.y = slab group of the same 32 rays,
-// gridDim (ceil(na/32), nb, views).
-// GEO64: FP64 geometry and weight sum (ray_geom64 / ray_slabs64); split
-// summation modes only.
+// Launch of fp_ref_kernel, one block per FPC_COLS x FPC_ROWS detector cells and
+// view.
+template <typename VT, bool PAIR, int S, int NST> constexpr size_t fp_ref_smem() {
+    return FPC_COLS * sizeof(FPShared<VT, PAIR, S, NST>);
+}
+template <int K, bool ONES, typename VT, typename MT = VT, bool MULTI = false,
+          int S = fp_stage<K>(), int NST = 2, int MINB = fp_min_blocks<K>(), bool PAIR = false>
+int launch_fp_ref(mcsart_ctx *ctx, dim3 grid, const FPArgs<VT, K, MT> &a) {
+    constexpr size_t smem = fp_ref_smem<VT, PAIR, S, NST>();
+    const auto kernel = fp_ref_kernel<K, ONES, VT, MT, MULTI, S, NST, MINB, PAIR>;
+    // above 48 KB with the kernel's static arrays a launch needs the larger limit
+    if (smem > 44 * 1024)
+        MC_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)smem));
+    if (!ctx->label) ctx->label = "fp_ref_kernel";
+    MC_LAUNCH(ctx, kernel, grid, dim3(FPC_THREADS), smem, a);
+    return MCSART_OK;
+}
+
+// Per-ray projector of the split summation modes: blockDim (32, groups), the
+// 32 lanes 32 consecutive detector rows of one column, threadIdx.y = slab
+// group of the same 32 rays, gridDim (na, ceil(nb/32), views).
+// GEO64: FP64 geometry and weight sum (ray_geom64 / ray_slabs64).
 template <int K, bool ONES, int SUM, typename VT, typename MT = VT, bool GEO64 = false>
 __global__ void __launch_bounds__(256) fp_kernel(const FPArgs<VT, K, MT> p) {
-    static_assert(!GEO64 || SUM != SUM_REF, "FP64 geometry needs a split summation mode");
+    static_assert(SUM != SUM_REF, "the reference order is fp_ref_kernel's");
     constexpr int NS = K + (ONES ? 1 : 0);
-    extern __shared__ float sm_fp[];  // split modes: [groups][NS][32]
-    __shared__ double2 sm_norm[8];
+    extern __shared__ float sm_fp[];  // [groups][NS][32]
     __shared__ double sm_w64[GEO64 ? 8 : 1][32];  // GEO64: the groups' FP64 weight sums
     const int lane = threadIdx.x;
     const Geom &g = p.g;
-    const int ia = blockIdx.x * 32 + lane;
-    const int ib = (SUM == SUM_REF) ? blockIdx.y * 8 + threadIdx.y : blockIdx.y;
-    const bool active = ia < g.na && ib < g.nb;
+    const int ia = blockIdx.x, ib = blockIdx.y * 32 + lane;
+    const bool active = ib < g.nb;
+    const int groups = blockDim.y, grp = threadIdx.y;
     float s[K], sw = 0.0f;
     double sw64 = 0.0;
 #pragma unroll
@@ -1079,40 +1224,31 @@ __global__ void __launch_bounds__(256) fp_kernel(const FPArgs<VT, K, MT> p) {
             double sd, cd;
             sincos((double)angle, &sd, &cd);
             const RayGeom64 r = ray_geom64(cd, sd, ia, ib, g);
-            const int groups = blockDim.y, grp = threadIdx.y;
             const int per = (r.nd + groups - 1) / groups;
             const int d0 = grp * per, d1 = min(r.nd, d0 + per);
             ray_slabs64<K, ONES, SUM, VT>(r, p.vol, g, d0, d1, s, sw64);
         } else {
             const float cphi = cosf(angle), sphi = sinf(angle);  // :23-24
             const RayGeom r = ray_geom(cphi, sphi, ia, ib, g);
-            if (SUM == SUM_REF) {
-                ray_slabs<K, ONES, SUM, VT>(r, p.vol, g, 0, r.nd, s, sw);
-            } else {
-                const int groups = blockDim.y, grp = threadIdx.y;
-                const int per = (r.nd + groups - 1) / groups;
-                const int d0 = grp * per, d1 = min(r.nd, d0 + per);
-                ray_slabs<K, ONES, SUM, VT>(r, p.vol, g, d0, d1, s, sw);
-            }
+            const int per = (r.nd + groups - 1) / groups;
+            const int d0 = grp * per, d1 = min(r.nd, d0 + per);
+            ray_slabs<K, ONES, SUM, VT>(r, p.vol, g, d0, d1, s, sw);
         }
     }
-    if (SUM != SUM_REF) {
-        const int grp = threadIdx.y, groups = blockDim.y;
 #pragma unroll
-        for (int k = 0; k < K; k++) sm_fp[(grp * NS + k) * 32 + lane] = s[k];
-        if (ONES) sm_fp[(grp * NS + K) * 32 + lane] = sw;
-        if (GEO64) sm_w64[grp][lane] = sw64;
-        __syncthreads();
-        if (grp != 0) return;
-        // fixed-order combination of the slab groups
-        for (int q = 1; q < groups; q++) {
+    for (int k = 0; k < K; k++) sm_fp[(grp * NS + k) * 32 + lane] = s[k];
+    if (ONES) sm_fp[(grp * NS + K) * 32 + lane] = sw;
+    if (GEO64) sm_w64[grp][lane] = sw64;
+    __syncthreads();
+    if (grp != 0) return;
+    // fixed-order combination of the slab groups
+    for (int q = 1; q < groups; q++) {
 #pragma unroll
-            for (int k = 0; k < K; k++) s[k] += sm_fp[(q * NS + k) * 32 + lane];
-            if (ONES) sw += sm_fp[(q * NS + K) * 32 + lane];
-            if (GEO64) sw64 += sm_w64[q][lane];
-        }
-        if (GEO64) sw = (float)sw64;
+        for (int k = 0; k < K; k++) s[k] += sm_fp[(q * NS + k) * 32 + lane];
+        if (ONES) sw += sm_fp[(q * NS + K) * 32 + lane];
+        if (GEO64) sw64 += sm_w64[q][lane];
     }
+    if (GEO64) sw = (float)sw64;
     const int64_t pix = ia + (int64_t)ib * g.na;
     double nb2 = 0.0, nr2 = 0.0;
     if (active) {
@@ -1124,8 +1260,8 @@ __global__ void __launch_bounds__(256) fp_kernel(const FPArgs<VT, K, MT> p) {
             float res = __fmaf_rn(s[0], -1.0f, b);
             float ones = ONES ? sw : 0.0f;
             if (p.mode == FP_MOTION) {
-                res = __fmaf_rn(s[1], 1.0f, res);  // AUMISART.cu:260, + FP(img0)
-                if (K >= 3) ones = s[2];            // FP(initial2(...)), :267-268
+                res = __fmaf_rn(s[K > 1 ? 1 : 0], 1.0f, res);  // AUMISART.cu:260, + FP(img0)
+                if (K >= 3) ones = s[K - 1];                   // FP(initial2(...)), :267-268
             }
             if (p.resid) p.resid[pix] = res;
             p.bp_in[pix] = make_float2(tex_texel(res), tex_texel(ones));
@@ -1134,26 +1270,13 @@ __global__ void __launch_bounds__(256) fp_kernel(const FPArgs<VT, K, MT> p) {
         }
     }
     if (p.mode == FP_PLAIN) return;
-    // block partial of the two squared norms, fixed-order reduction
+    // the block's partial of the two squared norms (one warp is left)
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
         nb2 += __shfl_down_sync(0xffffffffu, nb2, off);
         nr2 += __shfl_down_sync(0xffffffffu, nr2, off);
     }
-    if (SUM != SUM_REF) {  // only warp 0 is left
-        if (lane == 0) p.norm_part[blockIdx.y * gridDim.x + blockIdx.x] = make_double2(nb2, nr2);
-        return;
-    }
-    if (lane == 0) sm_norm[threadIdx.y] = make_double2(nb2, nr2);
-    __syncthreads();
-    if (threadIdx.y == 0 && lane == 0) {
-        double tb = 0.0, tr = 0.0;
-        for (int w = 0; w < (int)blockDim.y; w++) {
-            tb += sm_norm[w].x;
-            tr += sm_norm[w].y;
-        }
-        p.norm_part[blockIdx.y * gridDim.x + blockIdx.x] = make_double2(tb, tr);
-    }
+    if (lane == 0) p.norm_part[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] = make_double2(nb2, nr2);
 }
 
 }  // namespace mcsart

@@ -8,7 +8,7 @@
 //
 //   image pass, static (overload 1, AUMISART.cu:42-63):
 //     FP(img) + FP(ones) + residual + norms  ->  BP(residual)/BP(FP(ones)),
-//     img += lambda * ratio (and its y-fastest copy)            2 kernels/view
+//     img += lambda * ratio (and its z-fastest copy)            2 kernels/view
 //   image pass, motion-compensated (overload 2, :184-233):
 //     warp(img) -> FP + FP(ones) + residual + norms -> BP ratio ->
 //     img += lambda * warp^-1(ratio)                            4 kernels/view
@@ -76,7 +76,6 @@ template <typename ST, int INTERP, int SUM> struct Runner {
     int cols_view = -1;  // first view whose backprojector column data the last projector wrote
     int cols_views = 0;  // and how many views from it
     std::vector<int> views_img, views_mot;
-    std::vector<char> reads_std, reads_tr;  // per view: the copies its projector reads
     Tuning tune;  // launch shapes (variant indices; -1 = built-in choice)
 
     Runner(mcsart_ctx *c, const Problem &p, const mcsart_options &o)
@@ -84,8 +83,8 @@ template <typename ST, int INTERP, int SUM> struct Runner {
         tune = c->tuning_override ? *c->tuning_override : tuning_for(c, p.g, o.storage);
         V = nvox(P.g.nx, P.g.ny, P.g.nz);
         NP = (int64_t)P.g.na * P.g.nb;
-        fp_bx = SUM == SUM_REF ? (int)div_up(P.g.na, FPC_COLS) : (int)div_up(P.g.na, 32);
-        fp_by = SUM == SUM_REF ? (int)div_up(P.g.nb, FPC_ROWS) : P.g.nb;
+        fp_bx = SUM == SUM_REF ? (int)div_up(P.g.na, FPC_COLS) : P.g.na;
+        fp_by = (int)div_up(P.g.nb, SUM == SUM_REF ? FPC_ROWS : 32);
         fp_blocks = fp_bx * fp_by;
         groups = SUM == SUM_REF ? 1
                  : opt.fp_groups > 0 ? std::min(opt.fp_groups, 8)
@@ -95,19 +94,7 @@ template <typename ST, int INTERP, int SUM> struct Runner {
         for (int v = 0; v < P.n_views; v++) views_img.push_back(v);
         const int step = P.motion_model ? 1 : 10;  // AUMISART.cu:242 vs :72
         for (int v = 1; v < P.n_views; v += step) views_mot.push_back(v);
-        reads_std.resize(P.n_views);
-        reads_tr.resize(P.n_views);
-        for (int v = 0; v < P.n_views; v++) {
-            bool ax, ay;
-            view_drive_axes(P.angles[v], P.g, &ax, &ay);
-            reads_tr[v] = ax;
-            reads_std[v] = ay;
-        }
     }
-
-    // A per-view copy of a volume the projector of view v reads, else nullptr.
-    ST *std_or_null(int v, const DevBuf &b) const { return reads_std[v] ? b.as<ST>() : nullptr; }
-    ST *tr_or_null(int v, const DevBuf &b) const { return reads_tr[v] ? b.as<ST>() : nullptr; }
 
     Fields<ST> fields() const {
         const ST *f = (const ST *)P.fields;
@@ -118,17 +105,13 @@ template <typename ST, int INTERP, int SUM> struct Runner {
     int alloc() {
         const size_t vs = V * sizeof(ST), vf = V * sizeof(float);
         MC_TRY(S.img1.ensure(vs * subset));
-        MC_TRY(S.img1T.ensure(vs * subset));
         MC_TRY(S.imgS.ensure(vs));
-        MC_TRY(S.imgST.ensure(vs));
         // img0 and the initial2 volume interleaved for the reference-order
         // projector (PAIR), separate for the split-sum one
         MC_TRY(S.img0.ensure(2 * vs));
-        MC_TRY(S.img0T.ensure(2 * vs));
         MC_TRY(S.ones.ensure(vs));
-        MC_TRY(S.onesT.ensure(vs));
         MC_TRY(S.ratio.ensure(vf * subset));
-        MC_TRY(S.imgT.ensure(vf));
+        MC_TRY(S.imgZ.ensure(vf));
         MC_TRY(S.pairs.ensure(NP * subset * sizeof(float2)));
         MC_TRY(S.bpcolA.ensure((size_t)P.g.nx * P.g.ny * subset * sizeof(float4)));
         MC_TRY(S.bpcolB.ensure((size_t)P.g.nx * P.g.ny * subset * sizeof(float)));
@@ -184,32 +167,21 @@ template <typename ST, int INTERP, int SUM> struct Runner {
             a.bpcolB = S.bpcolB.as<float>();
         }
         if constexpr (SUM == SUM_REF && K == 1) {
-            // built-in: deeper slab groups when every block is resident at once
-            const int var = tune.fp1 >= 0 ? tune.fp1 : fp_one_wave(ctx, fp_bx, fp_by) ? 1 : 0;
-            // (slab-group depth, resident blocks per SM)
-            switch (var) {
-                case 1: MC_LAUNCH(ctx, (fp_ref_kernel<K, ONES, VT, ST, false, 4, 4>), grid,
-                                  dim3(FPC_THREADS), 0, a); break;
-                case 2: MC_LAUNCH(ctx, (fp_ref_kernel<K, ONES, VT, ST, false, 1, 8>), grid,
-                                  dim3(FPC_THREADS), 0, a); break;
-                case 3: MC_LAUNCH(ctx, (fp_ref_kernel<K, ONES, VT, ST, false, 2, 7>), grid,
-                                  dim3(FPC_THREADS), 0, a); break;
-                case 4: MC_LAUNCH(ctx, (fp_ref_kernel<K, ONES, VT, ST, false, 4, 5>), grid,
-                                  dim3(FPC_THREADS), 0, a); break;
-                default: MC_LAUNCH(ctx, (fp_ref_kernel<K, ONES, VT, ST, false, 2, 6>), grid,
-                                   dim3(FPC_THREADS), 0, a);
+            // (slabs per stage, stages, resident blocks per SM)
+            switch (tune.fp1) {
+                case 1: MC_TRY((launch_fp_ref<K, ONES, VT, ST, false, 8, 2, 7>(ctx, grid, a))); break;
+                case 2: MC_TRY((launch_fp_ref<K, ONES, VT, ST, false, 8, 2, 5>(ctx, grid, a))); break;
+                case 3: MC_TRY((launch_fp_ref<K, ONES, VT, ST, false, 4, 2, 8>(ctx, grid, a))); break;
+                case 4: MC_TRY((launch_fp_ref<K, ONES, VT, ST, false, 8, 3, 5>(ctx, grid, a))); break;
+                default: MC_TRY((launch_fp_ref<K, ONES, VT, ST, false, 8, 2, 6>(ctx, grid, a))); break;
             }
         } else if constexpr (SUM == SUM_REF) {
             // three volumes, the second and third paired (enqueue_motion)
             switch (tune.fp3) {
-                case 1: MC_LAUNCH(ctx, (fp_ref_kernel<K, ONES, VT, ST, false, 2, 4, K == 3>), grid,
-                                  dim3(FPC_THREADS), 0, a); break;
-                case 2: MC_LAUNCH(ctx, (fp_ref_kernel<K, ONES, VT, ST, false, 2, 5, K == 3>), grid,
-                                  dim3(FPC_THREADS), 0, a); break;
-                case 3: MC_LAUNCH(ctx, (fp_ref_kernel<K, ONES, VT, ST, false, 4, 5, K == 3>), grid,
-                                  dim3(FPC_THREADS), 0, a); break;
-                default: MC_LAUNCH(ctx, (fp_ref_kernel<K, ONES, VT, ST, false, 4, 4, K == 3>), grid,
-                                   dim3(FPC_THREADS), 0, a);
+                case 1: MC_TRY((launch_fp_ref<K, ONES, VT, ST, false, 4, 2, 6, K == 3>(ctx, grid, a))); break;
+                case 2: MC_TRY((launch_fp_ref<K, ONES, VT, ST, false, 4, 2, 4, K == 3>(ctx, grid, a))); break;
+                case 3: MC_TRY((launch_fp_ref<K, ONES, VT, ST, false, 2, 2, 6, K == 3>(ctx, grid, a))); break;
+                default: MC_TRY((launch_fp_ref<K, ONES, VT, ST, false, 4, 2, 5, K == 3>(ctx, grid, a))); break;
             }
         } else if (opt.geom64) {
             const size_t smem = (size_t)groups * (K + 1) * 32 * sizeof(float);
@@ -238,7 +210,7 @@ template <typename ST, int INTERP, int SUM> struct Runner {
     }
 
     // label: the profile label (default bp_div / bp_div_add by mode)
-    int launch_bp(int v, int mode, float *out, float *outT, cudaSurfaceObject_t surf = 0,
+    int launch_bp(int v, int mode, float *out, float *outZ, cudaSurfaceObject_t surf = 0,
                   const char *label = nullptr) {
         BPArgs b{};
         b.outSurf = surf;
@@ -247,7 +219,7 @@ template <typename ST, int INTERP, int SUM> struct Runner {
         b.angle = P.angles[v];
         b.lambda = P.lambda;
         b.out = out;
-        b.outT = outT;
+        b.outZ = outZ;
         if (cols_view == v) {
             b.colA = S.bpcolA.as<float4>();
             b.colB = S.bpcolB.as<float>();
@@ -256,15 +228,14 @@ template <typename ST, int INTERP, int SUM> struct Runner {
         if (opt.geom64) {  // FP64 geometry and normaliser (no precomputed columns)
             b.colA = nullptr;
             b.colB = nullptr;
-            const dim3 grid(div_up(P.g.nx, 32), div_up(P.g.ny, BP_ROWS), div_up(P.g.nz, BP_NZ)),
-                block(32, BP_ROWS);
+            const dim3 grid = bp_grid<BP_NZ, BP_ROWS>(P.g), block(32, BP_ROWS);
             if (mode == BP_DIV)
                 MC_LAUNCH(ctx, (bp_kernel<2, BP_DIV, false, false, true>), grid, block, 0, b);
             else
                 MC_LAUNCH(ctx, (bp_kernel<2, BP_DIV_ADD, false, false, true>), grid, block, 0, b);
             return MCSART_OK;
         }
-        switch (tune.bp) {  // voxels per thread along z x voxel rows per block
+        switch (tune.bp) {  // voxels per thread along z x threads along z per block
             case 1: return launch_bp_shape<1, 4>(mode, b);
             case 2: return launch_bp_shape<2, 8>(mode, b);
             case 3: return launch_bp_shape<4, 4>(mode, b);
@@ -273,8 +244,7 @@ template <typename ST, int INTERP, int SUM> struct Runner {
     }
 
     template <int NZ, int ROWS> int launch_bp_shape(int mode, const BPArgs &b) {
-        const dim3 grid(div_up(P.g.nx, 32), div_up(P.g.ny, ROWS), div_up(P.g.nz, NZ)),
-            block(32, ROWS);
+        const dim3 grid = bp_grid<NZ, ROWS>(P.g), block(32, ROWS);
         // the proven form skips the division range checks (bp_geom_proven)
         const bool proven = bp_geom_proven(P.g);
         if (mode == BP_DIV && proven) {
@@ -314,15 +284,14 @@ template <typename ST, int INTERP, int SUM> struct Runner {
         cols_view = v0;
         cols_views = kk;
         ctx->label = mode == FP_MOTION ? "fp_motion" : "fp_image";
-        MC_LAUNCH(ctx, (fp_ref_kernel<K, ONES, VT, ST, true>), dim3(fp_bx, fp_by, kk),
-                  dim3(FPC_THREADS), 0, a);
+        MC_TRY((launch_fp_ref<K, ONES, VT, ST, true>(ctx, dim3(fp_bx, fp_by, kk), a)));
         return MCSART_OK;
     }
 
     // One backprojector launch over the subset: BP_DIV writes view j's ratio
     // to out + j*V / surfs[j]; BP_DIV_ADD adds lambda/kk times the sum of the
     // views' ratios to out.
-    int launch_bp_subset(int v0, int kk, int mode, float *out, float *outT,
+    int launch_bp_subset(int v0, int kk, int mode, float *out, float *outZ,
                          const cudaSurfaceObject_t *surfs) {
         BPArgs b{};
         b.pair = S.pairs.as<float2>();
@@ -332,14 +301,13 @@ template <typename ST, int INTERP, int SUM> struct Runner {
         b.n_views = kk;
         b.lambda = P.lambda / (float)kk;
         b.out = out;
-        b.outT = outT;
+        b.outZ = outZ;
         for (int j = 0; j < kk && surfs; j++) b.outSurfs[j] = surfs[j];
         if (cols_view == v0 && cols_views == kk) {  // written by the subset's projector launch
             b.colA = S.bpcolA.as<float4>();
             b.colB = S.bpcolB.as<float>();
         }
-        const dim3 grid(div_up(P.g.nx, 32), div_up(P.g.ny, BP_ROWS), div_up(P.g.nz, BP_NZ)),
-            block(32, BP_ROWS);
+        const dim3 grid = bp_grid<BP_NZ, BP_ROWS>(P.g), block(32, BP_ROWS);
         const bool proven = bp_geom_proven(P.g);
         ctx->label = mode == BP_DIV ? "bp_div" : "bp_div_add";
         if (mode == BP_DIV && proven) {
@@ -355,35 +323,40 @@ template <typename ST, int INTERP, int SUM> struct Runner {
     }
 
     dim3 tile_grid() const { return dim3(div_up(P.g.nx, 32), div_up(P.g.ny, 32), P.g.nz); }
-    // warp_fwd_kernel / warp_back_add_kernel: 32 x (8 * WR) tiles
+    dim3 motion_tiles() const { return motion_grid(P.g.nx, P.g.ny, P.g.nz); }
+    // warp_back_add_kernel: 32 x (8 * WR) tiles
     template <int WR = WARP_ROWS> dim3 warp_grid() const {
         return dim3(div_up(P.g.nx, 32), div_up(P.g.ny, 8 * WR), P.g.nz);
     }
 
-    // The image pass's forward warp of the volume into view v's phase, in
-    // the tuned launch shape (voxel rows per thread), writing only the
-    // copies view v's projector reads.
-    template <int WR> int warp_fwd_shape(int v, bool hw, float volume, float flow) {
+    // A z-fastest copy for the projector.
+    template <typename SRC_T, typename DST_T> int zfast(DST_T *dst, const SRC_T *src) {
+        MC_LAUNCH(ctx, (zfast_kernel<SRC_T, DST_T>), zfast_grid(P.g.nx, P.g.ny, P.g.nz),
+                  dim3(32, 8), 0, dst, src, P.g.nx, P.g.ny, P.g.nz);
+        return MCSART_OK;
+    }
+
+    // The image pass's forward warp of the volume into a view's phase, in the
+    // tuned launch shape (slices per thread).
+    template <int WR> int warp_fwd_shape(ST *d, bool hw, float volume, float flow) {
         const Geom &g = P.g;
         const Fields<ST> f = fields();
-        ST *d = reads_std[v] ? S.img1.as<ST>() : nullptr;
-        ST *dT = reads_tr[v] ? S.img1T.as<ST>() : nullptr;
+        const dim3 grid = warp_fwd_grid<WR>(g.nx, g.ny, g.nz), block(32, 8);
         ctx->label = "warp_fwd";
         if (hw) {
-            MC_LAUNCH(ctx, (warp_fwd_kernel<SrcTex, ST, ST, WR>), warp_grid<WR>(), dim3(32, 8), 0,
-                      d, dT, SrcTex{S.tv_img.tex}, f, g.nx, g.ny, g.nz, volume, flow);
+            MC_LAUNCH(ctx, (warp_fwd_kernel<SrcTex, ST, ST, WR>), grid, block, 0, d,
+                      SrcTex{S.tv_img.tex}, f, g.nx, g.ny, g.nz, volume, flow);
         } else {
-            MC_LAUNCH(ctx, (warp_fwd_kernel<SrcLinear<float>, ST, ST, WR>), warp_grid<WR>(),
-                      dim3(32, 8), 0, d, dT, SrcLinear<float>{P.img}, f, g.nx, g.ny, g.nz, volume,
-                      flow);
+            MC_LAUNCH(ctx, (warp_fwd_kernel<SrcLinear<float>, ST, ST, WR>), grid, block, 0, d,
+                      SrcLinear<float>{P.img}, f, g.nx, g.ny, g.nz, volume, flow);
         }
         return MCSART_OK;
     }
-    int warp_fwd(int v, bool hw, float volume, float flow) {
+    int warp_fwd(ST *d, bool hw, float volume, float flow) {
         switch (tune.warp) {
-            case 1: return warp_fwd_shape<1>(v, hw, volume, flow);
-            case 2: return warp_fwd_shape<4>(v, hw, volume, flow);
-            default: return warp_fwd_shape<WARP_ROWS>(v, hw, volume, flow);
+            case 1: return warp_fwd_shape<1>(d, hw, volume, flow);
+            case 2: return warp_fwd_shape<4>(d, hw, volume, flow);
+            default: return warp_fwd_shape<WARP_ROWS>(d, hw, volume, flow);
         }
     }
     // The backward warp of a view's correction and the update, tuned shape.
@@ -413,22 +386,19 @@ template <typename ST, int INTERP, int SUM> struct Runner {
 
     // AUMISART.cu:42-63
     int enqueue_image_static() {
-        const Geom &g = P.g;
         MC_CHECK_CUDA(cudaMemsetAsync(S.norm_tmp.ptr, 0, P.n_views * sizeof(float), ctx->stream));
-        MC_LAUNCH(ctx, (transpose_kernel<float, float>), tile_grid(), dim3(32, 8), 0,
-                  S.imgT.as<float>(), P.img, g.nx, g.ny);
+        MC_TRY(zfast(S.imgZ.as<float>(), (const float *)P.img));
         FPVolumes<float, 1> vol{};
-        vol.std[0] = P.img;
-        vol.tr[0] = S.imgT.as<float>();
+        vol.zf[0] = S.imgZ.as<float>();
         const int n = (int)views_img.size();
         for (int k = 0; k < n; k += subset) {
             const int kk = std::min(subset, n - k), v = views_img[k];
             if (kk == 1) {  // one view at a time: the reference's loop
                 MC_TRY((launch_fp<1, true, float>(vol, v, k, FP_IMAGE)));
-                MC_TRY(launch_bp(v, BP_DIV_ADD, P.img, S.imgT.as<float>()));
+                MC_TRY(launch_bp(v, BP_DIV_ADD, P.img, S.imgZ.as<float>()));
             } else {
                 MC_TRY((launch_fp_subset<1, true, float>(vol, v, k, kk, FP_IMAGE, 0)));
-                MC_TRY(launch_bp_subset(v, kk, BP_DIV_ADD, P.img, S.imgT.as<float>(), nullptr));
+                MC_TRY(launch_bp_subset(v, kk, BP_DIV_ADD, P.img, S.imgZ.as<float>(), nullptr));
             }
         }
         return finalize_norms(S.views_image.as<int>(), (int)views_img.size());
@@ -481,27 +451,15 @@ template <typename ST, int INTERP, int SUM> struct Runner {
     // ratio is warped back from its own phase (:222) and added with weight
     // lambda/kk, in view order.
     int image_mc_subset(int k0, int kk, bool hw) {
-        const Geom &g = P.g;
-        const Fields<ST> f = fields();
         const int v0 = views_img[k0];
         for (int j = 0; j < kk; j++) {
             const int v = v0 + j;
             const float volume = P.volumes[v] - P.volumes[0];
             const float flow = P.flows[v] - P.flows[0];
-            ST *d = S.img1.as<ST>() + j * V, *dT = S.img1T.as<ST>() + j * V;
-            ctx->label = "warp_fwd";
-            if (hw) {
-                MC_LAUNCH(ctx, (warp_fwd_kernel<SrcTex, ST, ST>), warp_grid<>(), dim3(32, 8), 0, d,
-                          dT, SrcTex{S.tv_img.tex}, f, g.nx, g.ny, g.nz, volume, flow);
-            } else {
-                MC_LAUNCH(ctx, (warp_fwd_kernel<SrcLinear<float>, ST, ST>), warp_grid<>(),
-                          dim3(32, 8), 0, d, dT, SrcLinear<float>{P.img}, f, g.nx, g.ny, g.nz,
-                          volume, flow);
-            }
+            MC_TRY(warp_fwd(S.img1.as<ST>() + j * V, hw, volume, flow));
         }
         FPVolumes<ST, 1> vol{};
-        vol.std[0] = S.img1.as<ST>();
-        vol.tr[0] = S.img1T.as<ST>();
+        vol.zf[0] = S.img1.as<ST>();
         MC_TRY((launch_fp_subset<1, true, ST>(vol, v0, k0, kk, FP_IMAGE, V)));
         cudaSurfaceObject_t surfs[BP_MAX_VIEWS] = {};
         for (int j = 0; j < kk; j++) surfs[j] = j == 0 ? S.tv_ratio.surf : S.tv_ratio_sub[j - 1].surf;
@@ -522,14 +480,11 @@ template <typename ST, int INTERP, int SUM> struct Runner {
     // backprojector and the update write them through surfaces, so the only
     // copy is the volume's upload at the start of the pass.
     int enqueue_image_mc() {
-        const Geom &g = P.g;
-        const Fields<ST> f = fields();
         MC_CHECK_CUDA(cudaMemsetAsync(S.norm_tmp.ptr, 0, P.n_views * sizeof(float), ctx->stream));
         const bool hw = INTERP == MCSART_INTERP_TEXTURE;
         if (hw) MC_TRY(S.tv_img.upload(P.img, ctx->stream));
         FPVolumes<ST, 1> vol{};
-        vol.std[0] = S.img1.as<ST>();
-        vol.tr[0] = S.img1T.as<ST>();
+        vol.zf[0] = S.img1.as<ST>();
         const int n = (int)views_img.size();
         for (int k = 0; k < n; k += subset) {
             const int kk = std::min(subset, n - k);
@@ -540,7 +495,7 @@ template <typename ST, int INTERP, int SUM> struct Runner {
             const int v = views_img[k];
             const float volume = P.volumes[v] - P.volumes[0];   // :193
             const float flow = P.flows[v] - P.flows[0];
-            MC_TRY(warp_fwd(v, hw, volume, flow));
+            MC_TRY(warp_fwd(S.img1.as<ST>(), hw, volume, flow));
             MC_TRY((launch_fp<1, true, ST>(vol, v, k, FP_IMAGE)));
             if (hw)
                 MC_TRY(launch_bp(v, BP_DIV, nullptr, nullptr, S.tv_ratio.surf));
@@ -558,25 +513,14 @@ template <typename ST, int INTERP, int SUM> struct Runner {
         ST *fw = (ST *)P.fields;
         MC_CHECK_CUDA(cudaMemsetAsync(S.norm_tmp.ptr, 0, P.n_views * sizeof(float), ctx->stream));
         FPVolumes<ST, 3> vol{};
-        if (sizeof(ST) == sizeof(float)) {
-            vol.std[0] = (const ST *)P.img;
-        } else {
-            MC_LAUNCH(ctx, (cast_kernel<ST>), stream_blocks(V), 256, 0, S.imgS.as<ST>(),
-                      (const float *)P.img, V);
-            vol.std[0] = S.imgS.as<ST>();
-        }
-        MC_LAUNCH(ctx, (transpose_kernel<float, ST>), tile_grid(), dim3(32, 8), 0,
-                  S.imgST.as<ST>(), (const float *)P.img, g.nx, g.ny);
-        vol.tr[0] = S.imgST.as<ST>();
+        MC_TRY((zfast<float, ST>(S.imgS.as<ST>(), (const float *)P.img)));
+        vol.zf[0] = S.imgS.as<ST>();
         // the reference-order projector reads img0 and the initial2 volume
         // as interleaved pairs (one load for both), the split-sum one apart
         constexpr bool pair = SUM == SUM_REF;
-        vol.std[1] = S.img0.as<ST>();
-        vol.tr[1] = S.img0T.as<ST>();
-        vol.std[2] = pair ? nullptr : S.ones.as<ST>();
-        vol.tr[2] = pair ? nullptr : S.onesT.as<ST>();
-        ST *const ones_std = pair ? nullptr : S.ones.as<ST>();
-        ST *const ones_tr = pair ? nullptr : S.onesT.as<ST>();
+        ST *const img0 = S.img0.as<ST>(), *const ones = pair ? nullptr : S.ones.as<ST>();
+        vol.zf[1] = img0;
+        vol.zf[2] = ones;
         // square slices: each view's field update and the next view's prep
         // run as one kernel (one pass over the fields)
         const bool fuse = g.nx == g.ny;
@@ -587,10 +531,9 @@ template <typename ST, int INTERP, int SUM> struct Runner {
             const float fd = P.flows[v] - P.flows[v - 1];
             if (!fuse || k == 0) {
                 ctx->label = "motion_prep";
-                MC_LAUNCH(ctx, (motion_prep_kernel<ST, ST, pair>), tile_grid(), dim3(32, 8), 0,
-                          std_or_null(v, S.img0), tr_or_null(v, S.img0T),
-                          reads_std[v] ? ones_std : nullptr, reads_tr[v] ? ones_tr : nullptr,
-                          (const float *)P.img, f, g.nx, g.ny, g.nz, vd, fd);
+                MC_LAUNCH(ctx, (motion_prep_kernel<ST, ST, pair>), motion_tiles(),
+                          dim3(MP_T, MP_T), 0, img0, ones, (const float *)P.img, f, g.nx, g.ny,
+                          g.nz, vd, fd);
             }
             MC_TRY((launch_fp<3, false, ST>(vol, v, k, FP_MOTION)));
             // square slices, FP32 geometry: the backprojection ratio is
@@ -606,33 +549,31 @@ template <typename ST, int INTERP, int SUM> struct Runner {
                 const float vdn = P.volumes[vn] - P.volumes[vn - 1];
                 const float fdn = P.flows[vn] - P.flows[vn - 1];
                 ctx->label = fused_bp ? "bp_field_update_prep" : "field_update_prep";
-                ST *const o_std = reads_std[vn] ? ones_std : nullptr;
-                ST *const o_tr = reads_tr[vn] ? ones_tr : nullptr;
                 const BPArgs b = bp_args(v);
                 if (fused_bp && bp_geom_proven(g))
                     MC_LAUNCH(ctx, (field_update_prep_kernel<ST, ST, false, pair, true, true>),
-                              tile_grid(), dim3(32, 8), 0, fw, fw + V, fw + 2 * V, fw + 3 * V,
-                              fw + 4 * V, fw + 5 * V, (const float *)nullptr, (const float *)P.img,
-                              g.nx, g.ny, g.nz, nvd, nfd, std_or_null(vn, S.img0),
-                              tr_or_null(vn, S.img0T), o_std, o_tr, vdn, fdn, b);
+                              motion_tiles(), dim3(MP_T, MP_T), 0, fw, fw + V, fw + 2 * V,
+                              fw + 3 * V, fw + 4 * V, fw + 5 * V, (const float *)nullptr,
+                              (const float *)P.img, g.nx, g.ny, g.nz, nvd, nfd, img0, ones, vdn,
+                              fdn, b);
                 else if (fused_bp)
                     MC_LAUNCH(ctx, (field_update_prep_kernel<ST, ST, false, pair, true, false>),
-                              tile_grid(), dim3(32, 8), 0, fw, fw + V, fw + 2 * V, fw + 3 * V,
-                              fw + 4 * V, fw + 5 * V, (const float *)nullptr, (const float *)P.img,
-                              g.nx, g.ny, g.nz, nvd, nfd, std_or_null(vn, S.img0),
-                              tr_or_null(vn, S.img0T), o_std, o_tr, vdn, fdn, b);
+                              motion_tiles(), dim3(MP_T, MP_T), 0, fw, fw + V, fw + 2 * V,
+                              fw + 3 * V, fw + 4 * V, fw + 5 * V, (const float *)nullptr,
+                              (const float *)P.img, g.nx, g.ny, g.nz, nvd, nfd, img0, ones, vdn,
+                              fdn, b);
                 else if (tune.fup == 1)
-                    MC_LAUNCH(ctx, (field_update_prep_kernel<ST, ST, true, pair>), tile_grid(),
-                              dim3(32, 8), 0, fw, fw + V, fw + 2 * V, fw + 3 * V, fw + 4 * V,
-                              fw + 5 * V, (const float *)S.ratio.as<float>(), (const float *)P.img,
-                              g.nx, g.ny, g.nz, nvd, nfd, std_or_null(vn, S.img0),
-                              tr_or_null(vn, S.img0T), o_std, o_tr, vdn, fdn, b);
+                    MC_LAUNCH(ctx, (field_update_prep_kernel<ST, ST, true, pair>),
+                              motion_tiles(), dim3(MP_T, MP_T), 0, fw, fw + V, fw + 2 * V,
+                              fw + 3 * V, fw + 4 * V, fw + 5 * V, (const float *)S.ratio.as<float>(),
+                              (const float *)P.img, g.nx, g.ny, g.nz, nvd, nfd, img0, ones, vdn,
+                              fdn, b);
                 else
-                    MC_LAUNCH(ctx, (field_update_prep_kernel<ST, ST, false, pair>), tile_grid(),
-                              dim3(32, 8), 0, fw, fw + V, fw + 2 * V, fw + 3 * V, fw + 4 * V,
-                              fw + 5 * V, (const float *)S.ratio.as<float>(), (const float *)P.img,
-                              g.nx, g.ny, g.nz, nvd, nfd, std_or_null(vn, S.img0),
-                              tr_or_null(vn, S.img0T), o_std, o_tr, vdn, fdn, b);
+                    MC_LAUNCH(ctx, (field_update_prep_kernel<ST, ST, false, pair>),
+                              motion_tiles(), dim3(MP_T, MP_T), 0, fw, fw + V, fw + 2 * V,
+                              fw + 3 * V, fw + 4 * V, fw + 5 * V, (const float *)S.ratio.as<float>(),
+                              (const float *)P.img, g.nx, g.ny, g.nz, nvd, nfd, img0, ones, vdn,
+                              fdn, b);
             } else {
                 ctx->label = "field_update";
                 MC_LAUNCH(ctx, (field_update_kernel<ST>), tile_grid(), dim3(32, 8), 0, fw, fw + V,
@@ -670,8 +611,7 @@ template <typename ST, int INTERP, int SUM> struct Runner {
         put(&P.lambda, sizeof(float));
         const void *ptrs[4] = {P.img, P.proj, P.fields, P.resid};
         put(ptrs, sizeof(ptrs));
-        const void *bufs[16] = {S.img1.ptr, S.img1T.ptr, S.imgS.ptr, S.imgST.ptr, S.img0.ptr,
-                                S.img0T.ptr, S.ones.ptr, S.onesT.ptr, S.ratio.ptr, S.imgT.ptr,
+        const void *bufs[12] = {S.img1.ptr, S.imgS.ptr, S.img0.ptr, S.ones.ptr, S.ratio.ptr, S.imgZ.ptr,
                                 S.pairs.ptr, S.norm_part.ptr, (const void *)S.tv_img.arr,
                                 (const void *)S.tv_ratio.arr, S.bpcolA.ptr, S.bpcolB.ptr};
         put(bufs, sizeof(bufs));

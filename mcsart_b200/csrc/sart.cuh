@@ -43,11 +43,6 @@ struct Problem {
     float *resid;                           // device FP32 or nullptr
 };
 
-// Which volume copies the projector reads for a view (abi_kernels.cu):
-// any_x: some rays are x-driven (the y-fastest copy), any_y: some are
-// y-driven (the x-fastest volume).
-void view_drive_axes(float angle, const Geom &g, bool *any_x, bool *any_y);
-
 // Runs n_iter passes of host_AUMISART's loop (sart.cu).
 int run_driver(mcsart_ctx *ctx, const Problem &P, int n_iter, const int *op_iter, float *norm_out,
                const mcsart_options &opt);
@@ -62,7 +57,8 @@ int autotune_problem(mcsart_ctx *ctx, const Problem &P, const mcsart_options &op
 
 struct DriverState {
     // working volumes of the passes
-    DevBuf img1, img1T, imgS, imgST, img0, img0T, ones, onesT, ratio, imgT;
+    // (z-fastest for the projector: img1, imgS, img0, ones, imgZ)
+    DevBuf img1, imgS, img0, ones, ratio, imgZ;
     DevBuf pairs, norm_part, norm_tmp, views_image, views_motion, zero_fields;
     DevBuf bpcolA, bpcolB;  // one view's backprojector column data (projector output)
     // staging for the host-pointer entry point

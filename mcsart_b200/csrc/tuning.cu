@@ -28,12 +28,13 @@
 namespace mcsart {
 
 // Variant counts of each kernel class (the launches are in sart.cu's Runner):
-//   fp1  one-volume projector   (slab-group depth, resident blocks per SM)
-//                               0: (2, 6)  1: (4, 4)  2: (1, 8)  3: (2, 7)  4: (4, 5)
-//   fp3  three-volume projector 0: (4, 4)  1: (2, 4)  2: (2, 5)  3: (4, 5)
-//   bp   backprojector          0: 2 voxels/thread, 4 rows      1: 1 voxel, 4 rows
-//                               2: 2 voxels, 8 rows             3: 4 voxels, 4 rows
-//   warp image-pass warps       0: 2 rows/thread  1: 1 row  2: 4 rows
+//   fp1  one-volume projector   (slabs per stage, stages, resident blocks per SM)
+//                               0: (8, 2, 6)  1: (8, 2, 7)  2: (8, 2, 5)  3: (4, 2, 8)
+//                               4: (8, 3, 5)
+//   fp3  three-volume projector 0: (4, 2, 5)  1: (4, 2, 6)  2: (4, 2, 4)  3: (2, 2, 6)
+//   bp   backprojector          0: 2 voxels/thread, 4 threads along z   1: 1 voxel, 4
+//                               2: 2 voxels, 8                          3: 4 voxels, 4
+//   warp image-pass warps       0: 2 rows (slices) per thread  1: 1  2: 4
 //   fup  DVF-pass field update  0: with the backprojection ratio computed in it
 //                               (square slices, FP32 geometry; else as 2)
 //                               1: after a backprojector launch, fields loaded first

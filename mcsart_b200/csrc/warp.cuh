@@ -171,49 +171,74 @@ __device__ __forceinline__ void prefetch_tile_rows(const Fields<FT> &f, const fl
 // there), 1 row costs 8 % at 256x256x160.
 constexpr int WARP_ROWS = 2;
 
-// SART image pass, forward warp of the current volume into the view's phase:
-// dst[id] = warp(src)[id] stored in VT, plus the y-fastest copy
-// dstT[iy + ix*ny] of the result (x-fastest reading) for the projector.
-// Either output may be nullptr when the view's projector reads only the
-// other (all its rays driven along y, or all along x).
-// blockDim (32, 8); block covers a 32 x (8 * WR) (x, y) tile of slice
-// blockIdx.z.
-// WR: rows of voxels per thread (the launch shape the driver's tuning may
-// choose; the same bits for every value).
+// The prefetch for a block of warp_fwd_kernel's grid of 32 x TZ (x, z) tiles
+// (x tiles of row 0, of row 1, ... along gridDim.x, z tiles along gridDim.y).
+template <typename FT>
+__device__ __forceinline__ void prefetch_xz_rows(const Fields<FT> &f, int TZ, int nx, int ny,
+                                                 int nz, int t) {
+    const unsigned nxy = gridDim.x;
+    unsigned b = blockIdx.x + WARP_PREFETCH_AHEAD, bz = blockIdx.y;
+    while (b >= nxy) {  // the tile WARP_PREFETCH_AHEAD blocks later may be in a later z tile row
+        b -= nxy;
+        bz++;
+    }
+    if (t >= 6 * TZ) return;
+    const unsigned gx = (nx + 31) / 32, y = b / gx;
+    const int a = t / TZ, z = (int)bz * TZ + t % TZ, x = (int)(b - y * gx) * 32;
+    if (z >= nz) return;
+    const int64_t i = x + (int64_t)y * nx + (int64_t)z * nx * ny;
+    const void *p;
+    switch (a) {
+        case 0: p = f.ax + i; break;
+        case 1: p = f.ay + i; break;
+        case 2: p = f.az + i; break;
+        case 3: p = f.bx + i; break;
+        case 4: p = f.by + i; break;
+        default: p = f.bz + i;
+    }
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
+// SART image pass, forward warp of the current volume into the view's phase,
+// z-fastest for the projector: dst[iz + (x + y*nx)*nz] = warp(src) at memory
+// position x + y*nx + iz*nx*ny, stored in VT.
+// blockDim (32, 8); a block covers a 32 x (8 * WR) (x, z) tile of row y,
+// gridDim (ceil(nx/32) * ny, ceil(nz/(8*WR))).
+// WR: slices per thread (the launch shape the driver's tuning may choose; the
+// same bits for every value).
 template <typename SRC, typename FT, typename VT, int WR = WARP_ROWS>
-static __global__ void __launch_bounds__(256) warp_fwd_kernel(VT *dst, VT *dstT, const SRC src,
-                                                              Fields<FT> f, int nx, int ny,
-                                                              int nz, float volume, float flow) {
-    constexpr int TH = 8 * WR;
-    __shared__ float tile[TH][33];
+static __global__ void __launch_bounds__(256) warp_fwd_kernel(VT *dst, const SRC src, Fields<FT> f,
+                                                              int nx, int ny, int nz, float volume,
+                                                              float flow) {
+    constexpr int TZ = 8 * WR;
+    __shared__ float tile[TZ][33];
     const int tx = threadIdx.x, ty = threadIdx.y;
-    const int x0 = blockIdx.x * 32, y0 = blockIdx.y * TH, iz = blockIdx.z;
-    const int64_t slice = (int64_t)iz * nx * ny;
+    prefetch_xz_rows(f, TZ, nx, ny, nz, ty * 32 + tx);
+    const unsigned gx = (nx + 31) / 32, ym = blockIdx.x / gx;
+    const int x0 = (int)(blockIdx.x - ym * gx) * 32, z0 = blockIdx.y * TZ;
+    const int64_t plane = (int64_t)nx * ny, row = (int64_t)ym * nx;
     const int xm = x0 + tx;
-    prefetch_tile_rows(f, nullptr, TH, nx, ny, nz, ty * 32 + tx);
+    int ix, iy;
+    warp_coords(xm, ym, nx, ny, ix, iy);
 #pragma unroll
     for (int k = 0; k < WR; k++) {
-        const int ly = ty + 8 * k, ym = y0 + ly;
-        float v = 0.0f;
-        if (xm < nx && ym < ny) {
-            const int64_t id = xm + (int64_t)ym * nx + slice;
-            int ix, iy;
-            warp_coords(xm, ym, nx, ny, ix, iy);
-            v = warp_sample_at(src, f, id, ix, iy, iz, nx, ny, nz, volume, flow);
-            if (dst) dst[id] = cvt<VT>(v);
-        }
-        tile[ly][tx] = v;
+        const int lz = ty + 8 * k, iz = z0 + lz;
+        if (xm < nx && iz < nz)
+            tile[lz][tx] = warp_sample_at(src, f, xm + row + iz * plane, ix, iy, iz, nx, ny, nz,
+                                          volume, flow);
     }
-    if (dstT == nullptr) return;  // uniform over the block
     __syncthreads();
-    // transposed store: runs of TH consecutive iy per ix
+    // turned store: runs of TZ consecutive slices per column
     const int t = ty * 32 + tx;
 #pragma unroll
     for (int k = 0; k < WR; k++) {
-        const int e = t + 256 * k, lx = e / TH, ly = e % TH;
-        const int xmT = x0 + lx, ymT = y0 + ly;
-        if (xmT < nx && ymT < ny) dstT[ymT + (int64_t)xmT * ny + slice] = cvt<VT>(tile[ly][lx]);
+        const int e = t + 256 * k, lx = e / TZ, lz = e % TZ;
+        if (x0 + lx < nx && z0 + lz < nz)
+            dst[z0 + lz + (row + x0 + lx) * nz] = cvt<VT>(tile[lz][lx]);
     }
+}
+template <int WR> inline dim3 warp_fwd_grid(int nx, int ny, int nz) {
+    return dim3(div_up(nx, 32) * (unsigned)ny, div_up(nz, 8 * WR));
 }
 
 // SART image pass, backward warp of the normalised correction and update:
