@@ -1,5 +1,6 @@
 // Kernel-level C ABI: one entry point per reference launcher (include/mcsart.h).
 #include <algorithm>
+#include <initializer_list>
 
 #include "backprojector.cuh"
 #include "common.cuh"
@@ -53,6 +54,15 @@ unsigned stream_blocks(int64_t n) {
     const int64_t b = (n + 255) / 256;
     return (unsigned)std::min<int64_t>(b, 148LL * 16);
 }
+
+// Whether every array begins on 16 bytes (four elements per load and store).
+static bool aligned16(std::initializer_list<const void *> ptrs) {
+    for (const void *p : ptrs)
+        if ((uintptr_t)p % 16 != 0) return false;
+    return true;
+}
+// Blocks of a pointwise kernel over n elements.
+static unsigned pointwise_blocks(int64_t n, bool vec) { return stream_blocks(vec ? (n + 3) / 4 : n); }
 
 }  // namespace mcsart
 
@@ -224,7 +234,9 @@ MC_EXPORT int mcsart_add(mcsart_ctx *ctx, float *img1, const float *img, int nx,
     MC_TRY(validate_dims(nx, ny, nz));
     MC_REQUIRE(img1 && img, "pointers must be non-NULL");
     const int64_t n = nvox(nx, ny, nz);
-    MC_LAUNCH(ctx, add_kernel, stream_blocks(n), 256, 0, img1, img, n, weight);
+    const bool vec = aligned16({img1, img});
+    MC_LAUNCH(ctx, (vec ? &add_kernel<true> : &add_kernel<false>), pointwise_blocks(n, vec), 256, 0,
+              img1, img, n, weight);
     return finish(ctx, "mcsart_add");
 }
 
@@ -235,7 +247,7 @@ MC_EXPORT int mcsart_add2(mcsart_ctx *ctx, float *img1, const float *img, int nx
     MC_TRY(validate_dims(nx, ny, nz));
     MC_REQUIRE(img1 && img && img0, "pointers must be non-NULL");
     MC_REQUIRE(ind >= 1 && ind <= 3, "ind must be 1, 2 or 3 (got %d)", ind);
-    MC_LAUNCH(ctx, add2_kernel, stream_blocks(nvox(nx, ny, nz)), 256, 0, img1, img, nx, ny, nz,
+    MC_LAUNCH(ctx, add2_kernel, stencil_grid(nx, ny, nz), dim3(32, 8), 0, img1, img, nx, ny, nz,
               img0, weight, ind);
     return finish(ctx, "mcsart_add2");
 }
@@ -246,7 +258,9 @@ MC_EXPORT int mcsart_initial(mcsart_ctx *ctx, float *img, int nx, int ny, int nz
     MC_TRY(validate_dims(nx, ny, nz));
     MC_REQUIRE(img, "img must be non-NULL");
     const int64_t n = nvox(nx, ny, nz);
-    MC_LAUNCH(ctx, initial_kernel, stream_blocks(n), 256, 0, img, n, value);
+    const bool vec = aligned16({img});
+    MC_LAUNCH(ctx, (vec ? &initial_kernel<true> : &initial_kernel<false>), pointwise_blocks(n, vec), 256, 0,
+              img, n, value);
     return finish(ctx, "mcsart_initial");
 }
 
@@ -256,7 +270,7 @@ MC_EXPORT int mcsart_initial2(mcsart_ctx *ctx, float *img, int nx, int ny, int n
     MC_TRY(validate_ctx(ctx));
     MC_TRY(validate_dims(nx, ny, nz));
     MC_REQUIRE(img && img0, "pointers must be non-NULL");
-    MC_LAUNCH(ctx, initial2_kernel, stream_blocks(nvox(nx, ny, nz)), 256, 0, img, nx, ny, nz, img0,
+    MC_LAUNCH(ctx, initial2_kernel, stencil_grid(nx, ny, nz), dim3(32, 8), 0, img, nx, ny, nz, img0,
               volume, flow);
     return finish(ctx, "mcsart_initial2");
 }
@@ -268,7 +282,9 @@ MC_EXPORT int mcsart_division(mcsart_ctx *ctx, float *img1, const float *img, in
     MC_TRY(validate_dims(nx, ny, nz));
     MC_REQUIRE(img1 && img, "pointers must be non-NULL");
     const int64_t n = nvox(nx, ny, nz);
-    MC_LAUNCH(ctx, division_kernel, stream_blocks(n), 256, 0, img1, img, n);
+    const bool vec = aligned16({img1, img});
+    MC_LAUNCH(ctx, (vec ? &division_kernel<true> : &division_kernel<false>), pointwise_blocks(n, vec), 256, 0,
+              img1, img, n);
     return finish(ctx, "mcsart_division");
 }
 
@@ -279,7 +295,7 @@ MC_EXPORT int mcsart_multiple(mcsart_ctx *ctx, float *img1, int nx, int ny, int 
     MC_TRY(validate_dims(nx, ny, nz));
     MC_REQUIRE(img1 && img0, "pointers must be non-NULL");
     MC_REQUIRE(ind >= 1 && ind <= 3, "ind must be 1, 2 or 3 (got %d)", ind);
-    MC_LAUNCH(ctx, multiple_kernel, stream_blocks(nvox(nx, ny, nz)), 256, 0, img1, nx, ny, nz,
+    MC_LAUNCH(ctx, multiple_kernel, stencil_grid(nx, ny, nz), dim3(32, 8), 0, img1, nx, ny, nz,
               img0, weight, ind);
     return finish(ctx, "mcsart_multiple");
 }
@@ -293,7 +309,7 @@ MC_EXPORT int mcsart_update_udvf(mcsart_ctx *ctx, float *ax, float *ay, float *a
     MC_TRY(validate_ctx(ctx));
     MC_TRY(validate_dims(nx, ny, nz));
     MC_REQUIRE(ax && ay && az && bx && by && bz && img && img0, "pointers must be non-NULL");
-    MC_LAUNCH(ctx, update_udvf_kernel, stream_blocks(nvox(nx, ny, nz)), 256, 0, ax, ay, az, bx, by,
+    MC_LAUNCH(ctx, update_udvf_kernel, stencil_grid(nx, ny, nz), dim3(32, 8), 0, ax, ay, az, bx, by,
               bz, img, img0, volume_diff, flow_diff, nx, ny, nz);
     return finish(ctx, "mcsart_update_udvf");
 }
@@ -305,7 +321,7 @@ MC_EXPORT int mcsart_diff(mcsart_ctx *ctx, float *img1, const float *img, int nx
     MC_TRY(validate_dims(nx, ny, nz));
     MC_REQUIRE(img1 && img, "pointers must be non-NULL");
     MC_REQUIRE(ind >= 1 && ind <= 3, "ind must be 1, 2 or 3 (got %d)", ind);
-    MC_LAUNCH(ctx, diff_kernel, stream_blocks(nvox(nx, ny, nz)), 256, 0, img1, img, nx, ny, nz,
+    MC_LAUNCH(ctx, diff_kernel, stencil_grid(nx, ny, nz), dim3(32, 8), 0, img1, img, nx, ny, nz,
               ind);
     return finish(ctx, "mcsart_diff");
 }

@@ -4,6 +4,8 @@
 // the engine's driver uses instead of chains of them.
 #pragma once
 
+#include <algorithm>
+
 #include "backprojector.cuh"
 #include "common.cuh"
 #include "warp.cuh"
@@ -14,18 +16,31 @@ namespace mcsart {
     for (int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; id < (n);                \
          id += (int64_t)gridDim.x * blockDim.x)
 
+// The pointwise kernels (bound by memory): VEC, four elements per load and
+// store, for arrays that all begin on 16 bytes; otherwise one.  At 512x512x256
+// host_add took 175 us with one element per load and 130 us with four (806 MB,
+// 6.2 TB/s), host_division 195 and 146 us.
+template <bool VEC, typename F> __device__ __forceinline__ void pointwise(int64_t n, F f) {
+    const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    if (VEC) {
+        for (int64_t i = t0; i < n / 4; i += step) f.four(i);
+        const int64_t id = n / 4 * 4 + t0;
+        if (id < n) f.one(id);
+    } else {
+        for (int64_t id = t0; id < n; id += step) f.one(id);
+    }
+}
+__device__ __forceinline__ float4 ld4(const float *p, int64_t i) {
+    return reinterpret_cast<const float4 *>(p)[i];
+}
+__device__ __forceinline__ void st4(float *p, int64_t i, float4 v) {
+    reinterpret_cast<float4 *>(p)[i] = v;
+}
+
 struct Vox {
     int ix, iy, iz;
 };
-__device__ __forceinline__ Vox vox_of(int64_t id, int nx, int ny) {
-    const int64_t plane = (int64_t)nx * ny;
-    Vox v;
-    v.iz = (int)(id / plane);
-    const int64_t r = id - (int64_t)v.iz * plane;
-    v.iy = (int)(r / nx);
-    v.ix = (int)(r - (int64_t)v.iy * nx);
-    return v;
-}
 
 // Forward difference along ind, 0 on the last plane (cu_add.cu:37-57).
 template <typename T>
@@ -39,114 +54,186 @@ __device__ __forceinline__ float fwd_diff(const T *img0, int64_t id, const Vox &
     }
 }
 
+// The stencil kernels (bound by memory): blockDim (32, 8), 32 x 32 (x, y)
+// tiles of one slice, four voxels per thread; the grid (stencil_grid) covers
+// the tiles of a slice and as many slices as a grid may, and a block goes on
+// through the rest.  No voxel's coordinates are divided out of its index, whose
+// 64-bit divisions took much of the time of a one-dimensional grid (at
+// 201x173x97: initial2 21 against 13 us, add2, which also read a field across
+// its rows, 25 against 18.5, event time of a few us included).
+#define MC_STENCIL_TILES(nx, ny, nz)                                                           \
+    for (int iz = blockIdx.z; iz < (nz); iz += gridDim.z)                                      \
+        for (int y0 = blockIdx.y * 32; y0 < (ny); y0 += gridDim.y * 32)
+#define MC_STENCIL_VOXELS(nx, ny)                                                              \
+    _Pragma("unroll") for (int k = 0; k < 4; k++) if (const int iy = y0 + threadIdx.y + 8 * k;  \
+                                                      ix < (nx) && iy < (ny))
+inline dim3 stencil_grid(int nx, int ny, int nz) {
+    return dim3(div_up(nx, 32), std::min(div_up(ny, 32), 65535u), std::min((unsigned)nz, 65535u));
+}
+
 // cu_add.cu:9-18
-static __global__ void add_kernel(float *img1, const float *img, int64_t n, float weight) {
-    MC_GRID_STRIDE(n) { img1[id] = __fmaf_rn(img[id], weight, img1[id]); }
+struct AddOp {
+    float *img1;
+    const float *img;
+    float weight;
+    __device__ void one(int64_t id) const { img1[id] = __fmaf_rn(img[id], weight, img1[id]); }
+    __device__ void four(int64_t i) const {
+        const float4 a = ld4(img, i), b = ld4(img1, i);
+        st4(img1, i, make_float4(__fmaf_rn(a.x, weight, b.x), __fmaf_rn(a.y, weight, b.y),
+                                 __fmaf_rn(a.z, weight, b.z), __fmaf_rn(a.w, weight, b.w)));
+    }
+};
+template <bool VEC>
+static __global__ void __launch_bounds__(256) add_kernel(float *img1, const float *img, int64_t n,
+                                                         float weight) {
+    pointwise<VEC>(n, AddOp{img1, img, weight});
 }
 
 // cu_add.cu:28-59: img1[id] += img[iy + ix*ny + iz*nx*ny] * weight * d_ind img0
-static __global__ void add2_kernel(float *img1, const float *img, int nx, int ny, int nz,
-                            const float *img0, float weight, int ind) {
-    const int64_t n = nvox(nx, ny, nz);
-    MC_GRID_STRIDE(n) {
-        const Vox v = vox_of(id, nx, ny);
-        const float df = fwd_diff(img0, id, v, nx, ny, nz, ind);
-        const int64_t t = v.iy + (int64_t)v.ix * ny + (int64_t)v.iz * nx * ny;
-        img1[id] = __fmaf_rn(img[t] * weight, df, img1[id]);
+// (img read through a tile, with its memory order along the lanes; the other
+// arrays' values are loaded before the barrier, so that a block waits on
+// memory once)
+static __global__ void __launch_bounds__(256) add2_kernel(float *img1, const float *img, int nx,
+                                                          int ny, int nz, const float *img0,
+                                                          float weight, int ind) {
+    __shared__ float tile[32][33];
+    const int x0 = blockIdx.x * 32, ix = x0 + threadIdx.x;
+    const int64_t step = ind == 1 ? 1 : ind == 2 ? nx : (int64_t)nx * ny;
+    MC_STENCIL_TILES(nx, ny, nz) {
+        const int64_t slice = (int64_t)iz * nx * ny;
+        float t[4], df[4], old[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int tx = x0 + threadIdx.y + 8 * k, ty = y0 + threadIdx.x;
+            t[k] = tx < nx && ty < ny ? img[ty + (int64_t)tx * ny + slice] : 0.0f;
+        }
+        MC_STENCIL_VOXELS(nx, ny) {
+            const int64_t id = ix + (int64_t)iy * nx + slice;
+            const bool last = ind == 1 ? ix == nx - 1 : ind == 2 ? iy == ny - 1 : iz == nz - 1;
+            df[k] = last ? 0.0f : img0[id + step] - img0[id];  // fwd_diff
+            old[k] = img1[id];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) tile[threadIdx.y + 8 * k][threadIdx.x] = t[k];
+        __syncthreads();
+        MC_STENCIL_VOXELS(nx, ny) {
+            const int64_t id = ix + (int64_t)iy * nx + slice;
+            img1[id] = __fmaf_rn(tile[threadIdx.x][iy - y0] * weight, df[k], old[k]);
+        }
+        __syncthreads();
     }
 }
 
 // cu_initial.cu:10-17
-static __global__ void initial_kernel(float *img, int64_t n, float value) {
-    MC_GRID_STRIDE(n) { img[id] = value; }
+struct InitialOp {
+    float *img;
+    float value;
+    __device__ void one(int64_t id) const { img[id] = value; }
+    __device__ void four(int64_t i) const { st4(img, i, make_float4(value, value, value, value)); }
+};
+template <bool VEC>
+static __global__ void __launch_bounds__(256) initial_kernel(float *img, int64_t n, float value) {
+    pointwise<VEC>(n, InitialOp{img, value});
 }
 
 // cu_initial.cu:27-49
-static __global__ void initial2_kernel(float *img, int nx, int ny, int nz, const float *img0,
-                                float volume, float flow) {
-    const int64_t n = nvox(nx, ny, nz);
-    MC_GRID_STRIDE(n) {
-        const Vox v = vox_of(id, nx, ny);
-        const float dfx = fwd_diff(img0, id, v, nx, ny, nz, 1);
-        const float dfy = fwd_diff(img0, id, v, nx, ny, nz, 2);
-        const float dfz = fwd_diff(img0, id, v, nx, ny, nz, 3);
-        img[id] = (dfx + dfy + dfz) * (volume + flow);
+static __global__ void __launch_bounds__(256) initial2_kernel(float *img, int nx, int ny, int nz,
+                                                              const float *img0, float volume,
+                                                              float flow) {
+    const int ix = blockIdx.x * 32 + threadIdx.x;
+    MC_STENCIL_TILES(nx, ny, nz) {
+        MC_STENCIL_VOXELS(nx, ny) {
+            const int64_t id = ix + (int64_t)iy * nx + (int64_t)iz * nx * ny;
+            const Vox v{ix, iy, iz};
+            const float dfx = fwd_diff(img0, id, v, nx, ny, nz, 1);
+            const float dfy = fwd_diff(img0, id, v, nx, ny, nz, 2);
+            const float dfz = fwd_diff(img0, id, v, nx, ny, nz, 3);
+            img[id] = (dfx + dfy + dfz) * (volume + flow);
+        }
     }
 }
 
 // cu_division.cu:11-25
-static __global__ void division_kernel(float *img1, const float *img, int64_t n) {
-    MC_GRID_STRIDE(n) {
-        float q = img1[id] / img[id];
-        if (isnan(q) || isinf(q)) q = 0.0f;
-        img1[id] = q;
+struct DivisionOp {
+    float *img1;
+    const float *img;
+    static __device__ float ratio(float a, float b) {
+        const float q = a / b;
+        return (isnan(q) || isinf(q)) ? 0.0f : q;
     }
+    __device__ void one(int64_t id) const { img1[id] = ratio(img1[id], img[id]); }
+    __device__ void four(int64_t i) const {
+        const float4 a = ld4(img1, i), b = ld4(img, i);
+        st4(img1, i, make_float4(ratio(a.x, b.x), ratio(a.y, b.y), ratio(a.z, b.z), ratio(a.w, b.w)));
+    }
+};
+template <bool VEC>
+static __global__ void __launch_bounds__(256) division_kernel(float *img1, const float *img,
+                                                              int64_t n) {
+    pointwise<VEC>(n, DivisionOp{img1, img});
 }
 
 // cu_multiple.cu:11-43
-static __global__ void multiple_kernel(float *img1, int nx, int ny, int nz, const float *img0,
-                                float weight, int ind) {
-    const int64_t n = nvox(nx, ny, nz);
-    MC_GRID_STRIDE(n) {
-        const Vox v = vox_of(id, nx, ny);
-        img1[id] *= weight * fwd_diff(img0, id, v, nx, ny, nz, ind);
+static __global__ void __launch_bounds__(256) multiple_kernel(float *img1, int nx, int ny, int nz,
+                                                              const float *img0, float weight,
+                                                              int ind) {
+    const int ix = blockIdx.x * 32 + threadIdx.x;
+    MC_STENCIL_TILES(nx, ny, nz) {
+        MC_STENCIL_VOXELS(nx, ny) {
+            const int64_t id = ix + (int64_t)iy * nx + (int64_t)iz * nx * ny;
+            img1[id] *= weight * fwd_diff(img0, id, Vox{ix, iy, iz}, nx, ny, nz, ind);
+        }
     }
 }
 
 // cu_update_udvf.cu:11-62.  b pairs alpha_y/beta_y with the x gradient and
 // alpha_x/beta_x with the y gradient (:45-50) while the update adds the x
 // component to alpha_x (:55), exactly as the reference does.
-static __global__ void update_udvf_kernel(float *ax, float *ay, float *az, float *bx, float *by,
-                                   float *bz, const float *img, const float *img0,
-                                   float volume_diff, float flow_diff, int nx, int ny, int nz) {
-    const int64_t n = nvox(nx, ny, nz);
-    MC_GRID_STRIDE(n) {
-        const Vox v = vox_of(id, nx, ny);
-        const float dfI = img0[id] - img[id];
-        const float dfx = fwd_diff(img, id, v, nx, ny, nz, 1);
-        const float dfy = fwd_diff(img, id, v, nx, ny, nz, 2);
-        const float dfz = fwd_diff(img, id, v, nx, ny, nz, 3);
-        const float cax = dfx * volume_diff, cay = dfy * volume_diff, caz = dfz * volume_diff;
-        const float cbx = dfx * flow_diff, cby = dfy * flow_diff, cbz = dfz * flow_diff;
-        const float w = cax * cax + cay * cay + caz * caz + cbx * cbx + cby * cby + cbz * cbz;
-        const float a_x = ay[id], a_y = ax[id], a_z = az[id];
-        const float b_x = by[id], b_y = bx[id], b_z = bz[id];
-        float b = dfI - cax * a_x - cay * a_y - caz * a_z - cbx * b_x - cby * b_y - cbz * b_z;
-        if (w == 0) continue;
-        b /= w;
-        ax[id] += 1.0f / 6 * b * cax;
-        ay[id] += 1.0f / 6 * b * cay;
-        az[id] += 1.0f / 6 * b * caz;
-        bx[id] += 1.0f / 6 * b * cbx;
-        by[id] += 1.0f / 6 * b * cby;
-        bz[id] += 1.0f / 6 * b * cbz;
+static __global__ void __launch_bounds__(256) update_udvf_kernel(
+    float *ax, float *ay, float *az, float *bx, float *by, float *bz, const float *img,
+    const float *img0, float volume_diff, float flow_diff, int nx, int ny, int nz) {
+    const int ix = blockIdx.x * 32 + threadIdx.x;
+    MC_STENCIL_TILES(nx, ny, nz) {
+        MC_STENCIL_VOXELS(nx, ny) {
+            const int64_t id = ix + (int64_t)iy * nx + (int64_t)iz * nx * ny;
+            const Vox v{ix, iy, iz};
+            const float dfI = img0[id] - img[id];
+            const float dfx = fwd_diff(img, id, v, nx, ny, nz, 1);
+            const float dfy = fwd_diff(img, id, v, nx, ny, nz, 2);
+            const float dfz = fwd_diff(img, id, v, nx, ny, nz, 3);
+            const float cax = dfx * volume_diff, cay = dfy * volume_diff, caz = dfz * volume_diff;
+            const float cbx = dfx * flow_diff, cby = dfy * flow_diff, cbz = dfz * flow_diff;
+            const float w = cax * cax + cay * cay + caz * caz + cbx * cbx + cby * cby + cbz * cbz;
+            const float a_x = ay[id], a_y = ax[id], a_z = az[id];
+            const float b_x = by[id], b_y = bx[id], b_z = bz[id];
+            float b = dfI - cax * a_x - cay * a_y - caz * a_z - cbx * b_x - cby * b_y - cbz * b_z;
+            if (w == 0) continue;
+            b /= w;
+            ax[id] += 1.0f / 6 * b * cax;
+            ay[id] += 1.0f / 6 * b * cay;
+            az[id] += 1.0f / 6 * b * caz;
+            bx[id] += 1.0f / 6 * b * cbx;
+            by[id] += 1.0f / 6 * b * cby;
+            bz[id] += 1.0f / 6 * b * cbz;
+        }
     }
 }
 
 // mex_diff.cu:75-113: backward difference, 0 on both faces.
-static __global__ void diff_kernel(float *img1, const float *img, int nx, int ny, int nz, int ind) {
-    const int64_t n = nvox(nx, ny, nz);
-    MC_GRID_STRIDE(n) {
-        const Vox v = vox_of(id, nx, ny);
-        float r;
-        switch (ind) {
-            case 1: r = (v.ix == nx - 1 || v.ix == 0) ? 0.0f : img[id] - img[id - 1]; break;
-            case 2: r = (v.iy == ny - 1 || v.iy == 0) ? 0.0f : img[id] - img[id - nx]; break;
-            case 3:
-                r = (v.iz == nz - 1 || v.iz == 0) ? 0.0f : img[id] - img[id - (int64_t)nx * ny];
-                break;
-            default: continue;
+static __global__ void __launch_bounds__(256) diff_kernel(float *img1, const float *img, int nx,
+                                                          int ny, int nz, int ind) {
+    const int ix = blockIdx.x * 32 + threadIdx.x;
+    MC_STENCIL_TILES(nx, ny, nz) {
+        MC_STENCIL_VOXELS(nx, ny) {
+            const int64_t id = ix + (int64_t)iy * nx + (int64_t)iz * nx * ny;
+            const int i = ind == 1 ? ix : ind == 2 ? iy : iz, m = ind == 1 ? nx : ind == 2 ? ny : nz;
+            const int64_t step = ind == 1 ? 1 : ind == 2 ? nx : (int64_t)nx * ny;
+            img1[id] = (i == m - 1 || i == 0) ? 0.0f : img[id] - img[id - step];
         }
-        img1[id] = r;
     }
 }
 
 // --------------------------------------------------------- fused kernels
-// Storage-type copy of an FP32 volume.
-template <typename DT> __global__ void cast_kernel(DT *dst, const float *src, int64_t n) {
-    MC_GRID_STRIDE(n) { dst[id] = cvt<DT>(src[id]); }
-}
-
 // z-fastest copy of an x-fastest volume: dst[iz + (ix + iy*nx)*nz] =
 // src[ix + iy*nx + iz*nx*ny].  blockDim (32, 8); a block turns a 32 x 32
 // (x, z) tile of row iy; gridDim (ceil(nx/32) * ny, ceil(nz/32)).
