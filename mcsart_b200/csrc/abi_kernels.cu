@@ -133,6 +133,21 @@ MC_EXPORT int mcsart_backprojection(mcsart_ctx *ctx, float *d_img, const float *
     return finish(ctx, "mcsart_backprojection");
 }
 
+// The warp of a volume given as a texture or in memory: four voxels per thread
+// where rows and arrays allow (warp_vec).
+template <typename SRC, typename FT>
+static int launch_deform(mcsart_ctx *ctx, FT *out, const SRC &src, const Fields<FT> &f, int nx,
+                         int ny, int nz, float volume, float flow) {
+    if (warp_vec(nx, f, sizeof(FT) == 4 ? (const void *)out : nullptr) &&
+        (uintptr_t)out % (4 * sizeof(FT)) == 0)
+        MC_LAUNCH(ctx, (deform_kernel<4, SRC, FT>), warp_grid<4>(nx, ny, nz), dim3(32, 8), 0, out, src,
+                  f, nx, ny, nz, volume, flow);
+    else
+        MC_LAUNCH(ctx, (deform_kernel<1, SRC, FT>), warp_grid<1>(nx, ny, nz), dim3(32, 8), 0, out, src,
+                  f, nx, ny, nz, volume, flow);
+    return MCSART_OK;
+}
+
 static int deform_common(mcsart_ctx *ctx, bool first_order, float *d_img1, const float *d_img,
                          int nx, int ny, int nz, float volume, float flow, const float *ax,
                          const float *ay, const float *az, const float *bx, const float *by,
@@ -143,7 +158,6 @@ static int deform_common(mcsart_ctx *ctx, bool first_order, float *d_img1, const
                "volume and field pointers must be non-NULL");
     const int64_t n = nvox(nx, ny, nz);
     const Fields<float> f{ax, ay, az, bx, by, bz};
-    const unsigned blocks = stream_blocks(n);
     if (!first_order && ctx->interp == MCSART_INTERP_TEXTURE) {
         // the reference samples a texture over a copy of the input
         // (cu_deform.cu:13-38); here the 3D array persists across calls
@@ -151,9 +165,7 @@ static int deform_common(mcsart_ctx *ctx, bool first_order, float *d_img1, const
         TexVol &tv = ctx->driver->tv_deform;
         MC_TRY(tv.ensure(nx, ny, nz));
         MC_TRY(tv.upload(d_img, ctx->stream));
-        MC_LAUNCH(ctx, deform_kernel<SrcTex>, blocks, 256, 0, d_img1, SrcTex{tv.tex}, f, nx, ny,
-                  nz, volume, flow);
-        return MCSART_OK;
+        return launch_deform(ctx, d_img1, SrcTex{tv.tex}, f, nx, ny, nz, volume, flow);
     }
     const float *src = d_img;
     if (d_img1 == d_img) {  // the reference samples a copy (cu_deform.cu:13-23)
@@ -164,12 +176,11 @@ static int deform_common(mcsart_ctx *ctx, bool first_order, float *d_img1, const
         src = (const float *)ws;
     }
     if (first_order) {
-        MC_LAUNCH(ctx, deform2_kernel, blocks, 256, 0, d_img1, src, f, nx, ny, nz, volume, flow);
-    } else {
-        MC_LAUNCH(ctx, deform_kernel<SrcLinear<float>>, blocks, 256, 0, d_img1,
-                  SrcLinear<float>{src}, f, nx, ny, nz, volume, flow);
+        MC_LAUNCH(ctx, deform2_kernel, warp_grid<1>(nx, ny, nz), dim3(32, 8), 0, d_img1, src, f, nx,
+                  ny, nz, volume, flow);
+        return MCSART_OK;
     }
-    return MCSART_OK;
+    return launch_deform(ctx, d_img1, SrcLinear<float>{src}, f, nx, ny, nz, volume, flow);
 }
 
 MC_EXPORT int mcsart_deform(mcsart_ctx *ctx, float *d_img1, const float *d_img, int nx, int ny,
@@ -200,7 +211,9 @@ MC_EXPORT int mcsart_forward_dvf(mcsart_ctx *ctx, float *mx, float *my, float *m
     MC_REQUIRE(mx && my && mz && ax && ay && az && bx && by && bz, "pointers must be non-NULL");
     const int64_t n = nvox(nx, ny, nz);
     const Fields<float> f{ax, ay, az, bx, by, bz};
-    MC_LAUNCH(ctx, forward_dvf_kernel, stream_blocks(n), 256, 0, mx, my, mz, f, n, volume, flow);
+    const bool vec = aligned16({mx, my, mz, ax, ay, az, bx, by, bz});
+    MC_LAUNCH(ctx, (vec ? &forward_dvf_kernel<true> : &forward_dvf_kernel<false>),
+              pointwise_blocks(n, vec), 256, 0, mx, my, mz, f, n, volume, flow);
     return finish(ctx, "mcsart_forward_dvf");
 }
 
@@ -217,13 +230,12 @@ MC_EXPORT int mcsart_invert_dvf(mcsart_ctx *ctx, float *inv_x, float *inv_y, flo
     MC_REQUIRE(n_iter >= 1 && n_iter <= 64, "n_iter must be in [1, 64]");
     const int64_t n = nvox(nx, ny, nz);
     void *ws;
-    MC_TRY(workspace(ctx, "inv_m", 3 * n * sizeof(float), &ws));
-    float *m = (float *)ws;
+    MC_TRY(workspace(ctx, "inv_m", n * sizeof(float4), &ws));
+    float4 *m = (float4 *)ws;
     const Fields<float> f{ax, ay, az, bx, by, bz};
-    MC_LAUNCH(ctx, forward_dvf_kernel, stream_blocks(n), 256, 0, m, m + n, m + 2 * n, f, n, volume,
-              flow);
+    MC_LAUNCH(ctx, forward_dvf4_kernel, stream_blocks(n), 256, 0, m, f, n, volume, flow);
     MC_LAUNCH(ctx, invert_dvf_kernel, dim3(div_up(nx, 32), div_up(ny, 8), nz), dim3(32, 8), 0,
-              inv_x, inv_y, inv_z, m, m + n, m + 2 * n, nx, ny, nz, n_iter);
+              inv_x, inv_y, inv_z, m, nx, ny, nz, n_iter);
     return finish(ctx, "mcsart_invert_dvf");
 }
 
@@ -401,19 +413,14 @@ int deform_ex_typed(mcsart_ctx *ctx, FT *d_img1, const float *d_img, int nx, int
     const int64_t V = nvox(nx, ny, nz);
     const Fields<FT> f{fields, fields + V, fields + 2 * V, fields + 3 * V, fields + 4 * V,
                        fields + 5 * V};
-    const unsigned blocks = stream_blocks(V);
     if (interp == MCSART_INTERP_TEXTURE) {
         if (!ctx->driver) ctx->driver.reset(new DriverState());
         TexVol &tv = ctx->driver->tv_deform;
         MC_TRY(tv.ensure(nx, ny, nz));
         MC_TRY(tv.upload(d_img, ctx->stream));
-        MC_LAUNCH(ctx, (deform_typed_kernel<SrcTex, FT>), blocks, 256, 0, d_img1, SrcTex{tv.tex},
-                  f, nx, ny, nz, volume, flow);
-    } else {
-        MC_LAUNCH(ctx, (deform_typed_kernel<SrcLinear<float>, FT>), blocks, 256, 0, d_img1,
-                  SrcLinear<float>{d_img}, f, nx, ny, nz, volume, flow);
+        return launch_deform(ctx, d_img1, SrcTex{tv.tex}, f, nx, ny, nz, volume, flow);
     }
-    return MCSART_OK;
+    return launch_deform(ctx, d_img1, SrcLinear<float>{d_img}, f, nx, ny, nz, volume, flow);
 }
 
 }  // namespace

@@ -122,7 +122,7 @@ template <typename ST, int INTERP, int SUM> struct Runner {
                 MC_TRY(S.tv_ratio_sub[j - 1].ensure(P.g.nx, P.g.ny, P.g.nz));
         }
         if (inv_iters > 0) {
-            MC_TRY(S.m3.ensure(3 * vf));
+            MC_TRY(S.m3.ensure(4 * vf));
             MC_TRY(S.inv3.ensure(3 * vf));
         }
         MC_TRY(S.angles_dev.ensure((size_t)P.n_views * sizeof(float)));
@@ -324,9 +324,9 @@ template <typename ST, int INTERP, int SUM> struct Runner {
 
     dim3 tile_grid() const { return dim3(div_up(P.g.nx, 32), div_up(P.g.ny, 32), P.g.nz); }
     dim3 motion_tiles() const { return motion_grid(P.g.nx, P.g.ny, P.g.nz); }
-    // warp_back_add_kernel: 32 x (8 * WR) tiles
-    template <int WR = WARP_ROWS> dim3 warp_grid() const {
-        return dim3(div_up(P.g.nx, 32), div_up(P.g.ny, 8 * WR), P.g.nz);
+    // warp_back_add_kernel: 32 * N x (8 * WR) tiles
+    template <int N, int WR> dim3 warp_back_grid() const {
+        return dim3(div_up(P.g.nx, 32 * N), div_up(P.g.ny, 8 * WR), P.g.nz);
     }
 
     // A z-fastest copy for the projector.
@@ -339,15 +339,20 @@ template <typename ST, int INTERP, int SUM> struct Runner {
     // The image pass's forward warp of the volume into a view's phase, in the
     // tuned launch shape (slices per thread).
     template <int WR> int warp_fwd_shape(ST *d, bool hw, float volume, float flow) {
-        const Geom &g = P.g;
         const Fields<ST> f = fields();
-        const dim3 grid = warp_fwd_grid<WR>(g.nx, g.ny, g.nz), block(32, 8);
+        if (warp_vec(P.g.nx, f)) return warp_fwd_n<4, WR>(d, hw, f, volume, flow);
+        return warp_fwd_n<1, WR>(d, hw, f, volume, flow);
+    }
+    template <int N, int WR>
+    int warp_fwd_n(ST *d, bool hw, const Fields<ST> &f, float volume, float flow) {
+        const Geom &g = P.g;
+        const dim3 grid = warp_fwd_grid<N, WR>(g.nx, g.ny, g.nz), block(32, 8);
         ctx->label = "warp_fwd";
         if (hw) {
-            MC_LAUNCH(ctx, (warp_fwd_kernel<SrcTex, ST, ST, WR>), grid, block, 0, d,
+            MC_LAUNCH(ctx, (warp_fwd_kernel<N, SrcTex, ST, ST, WR>), grid, block, 0, d,
                       SrcTex{S.tv_img.tex}, f, g.nx, g.ny, g.nz, volume, flow);
         } else {
-            MC_LAUNCH(ctx, (warp_fwd_kernel<SrcLinear<float>, ST, ST, WR>), grid, block, 0, d,
+            MC_LAUNCH(ctx, (warp_fwd_kernel<N, SrcLinear<float>, ST, ST, WR>), grid, block, 0, d,
                       SrcLinear<float>{P.img}, f, g.nx, g.ny, g.nz, volume, flow);
         }
         return MCSART_OK;
@@ -363,16 +368,24 @@ template <typename ST, int INTERP, int SUM> struct Runner {
     template <int WR>
     int warp_back_shape(bool hw, cudaTextureObject_t tex, const float *lin, float ivolume,
                         float iflow, float lam) {
-        const Geom &g = P.g;
         const Fields<ST> f = fields();
+        if (warp_vec(P.g.nx, f, P.img))
+            return warp_back_n<4, WR>(hw, tex, lin, f, ivolume, iflow, lam);
+        return warp_back_n<1, WR>(hw, tex, lin, f, ivolume, iflow, lam);
+    }
+    template <int N, int WR>
+    int warp_back_n(bool hw, cudaTextureObject_t tex, const float *lin, const Fields<ST> &f,
+                    float ivolume, float iflow, float lam) {
+        const Geom &g = P.g;
+        const dim3 grid = warp_back_grid<N, WR>(), block(32, 8);
         ctx->label = "warp_back_add";
         if (hw) {
-            MC_LAUNCH(ctx, (warp_back_add_kernel<SrcTex, ST, WR>), warp_grid<WR>(), dim3(32, 8), 0,
-                      P.img, S.tv_img.surf, SrcTex{tex}, f, g.nx, g.ny, g.nz, ivolume, iflow, lam);
+            MC_LAUNCH(ctx, (warp_back_add_kernel<N, SrcTex, ST, WR>), grid, block, 0, P.img,
+                      S.tv_img.surf, SrcTex{tex}, f, g.nx, g.ny, g.nz, ivolume, iflow, lam);
         } else {
-            MC_LAUNCH(ctx, (warp_back_add_kernel<SrcLinear<float>, ST, WR>), warp_grid<WR>(),
-                      dim3(32, 8), 0, P.img, (cudaSurfaceObject_t)0, SrcLinear<float>{lin}, f,
-                      g.nx, g.ny, g.nz, ivolume, iflow, lam);
+            MC_LAUNCH(ctx, (warp_back_add_kernel<N, SrcLinear<float>, ST, WR>), grid, block, 0, P.img,
+                      (cudaSurfaceObject_t)0, SrcLinear<float>{lin}, f, g.nx, g.ny, g.nz, ivolume,
+                      iflow, lam);
         }
         return MCSART_OK;
     }
@@ -416,14 +429,13 @@ template <typename ST, int INTERP, int SUM> struct Runner {
             const Fields<float> ff{F, F + V, F + 2 * V, F + 3 * V, F + 4 * V, F + 5 * V};
             const float volume = P.volumes[v] - P.volumes[0];
             const float flow = P.flows[v] - P.flows[0];
-            float *m = S.m3.as<float>(), *n = S.inv3.as<float>();
+            float4 *m = S.m3.as<float4>();
+            float *n = S.inv3.as<float>();
             ctx->label = "dvf_inverse";
-            MC_LAUNCH(ctx, forward_dvf_kernel, stream_blocks(V), 256, 0, m, m + V, m + 2 * V, ff,
-                      V, volume, flow);
+            MC_LAUNCH(ctx, forward_dvf4_kernel, stream_blocks(V), 256, 0, m, ff, V, volume, flow);
             ctx->label = "dvf_inverse";
             MC_LAUNCH(ctx, invert_dvf_kernel, dim3(div_up(g.nx, 32), div_up(g.ny, 8), g.nz),
-                      dim3(32, 8), 0, n, n + V, n + 2 * V, m, m + V, m + 2 * V, g.nx, g.ny, g.nz,
-                      inv_iters);
+                      dim3(32, 8), 0, n, n + V, n + 2 * V, m, g.nx, g.ny, g.nz, inv_iters);
             ctx->label = "warp_back_add";
             if (hw) {
                 MC_LAUNCH(ctx, warp_back_add_disp_kernel<SrcTex>, tile_grid(), dim3(32, 8), 0,
