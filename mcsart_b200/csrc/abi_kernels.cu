@@ -120,13 +120,29 @@ MC_EXPORT int mcsart_backprojection(mcsart_ctx *ctx, float *d_img, const float *
     MC_REQUIRE(d_proj && d_img, "d_proj and d_img must be non-NULL");
     const Geom g = make_geom(SO, SD, da, na, ai, db, nb, bi, nx, ny, nz);
     MC_TRY(validate_geom(g));
+    const bool proven = bp_geom_proven(g);
+    if (nvox(nx, ny, nz) >= BP_SLICE_LANES_MIN) {
+        void *ws;
+        MC_TRY(workspace(ctx, "bp_cells", bp_cells(na, nb) * sizeof(float), &ws));
+        float *cells = (float *)ws;
+        MC_LAUNCH(ctx, bp_cells_kernel, dim3(div_up(na, 32), div_up(nb, 32)), dim3(32, 8), 0, cells,
+                  d_proj, na, nb);
+        // 16 slices per tile where the last 32 would be at most half full
+        if ((nz - 1) % 32 < 16)
+            MC_LAUNCH(ctx, (proven ? &bp_slice_kernel<true, 16> : &bp_slice_kernel<false, 16>),
+                      bp_slice_grid<16>(g), BP_THREADS, 0, d_img, cells, angle, g);
+        else
+            MC_LAUNCH(ctx, (proven ? &bp_slice_kernel<true, 32> : &bp_slice_kernel<false, 32>),
+                      bp_slice_grid<32>(g), BP_THREADS, 0, d_img, cells, angle, g);
+        return finish(ctx, "mcsart_backprojection");
+    }
     BPArgs a{};
     a.proj = d_proj;
     a.g = g;
     a.angle = angle;
     a.out = d_img;
     const dim3 grid = bp_grid<BP_NZ, BP_ROWS>(g), block(32, BP_ROWS);
-    if (bp_geom_proven(g))
+    if (proven)
         MC_LAUNCH(ctx, (bp_kernel<1, BP_PLAIN, false, true>), grid, block, 0, a);
     else
         MC_LAUNCH(ctx, (bp_kernel<1, BP_PLAIN>), grid, block, 0, a);

@@ -399,4 +399,190 @@ template <int NZ, int ROWS> inline dim3 bp_grid(const Geom &g) {
     return dim3(div_up(g.nx, 32) * (unsigned)g.ny, div_up(g.nz, NZ * ROWS));
 }
 
+// ------------------------------------------------------------------------
+// Slice-lane backprojector of one projection (mcsart_backprojection on larger
+// volumes): the lanes of a warp are consecutive slices of one voxel column (or
+// of two), so that the detector columns it meets, their weights and the loop
+// over them are the same for all lanes, and the projection is first turned
+// into a layout whose rows lie next to each other (bp_cell).  The 32-column
+// tile is turned in shared memory for x-fastest stores.
+// Bound by instruction issue.  At 512x512x256 with a 1024x768 detector: 482 us,
+// bp_kernel 691 us; at 201x173x97, 301x211: 41 and 46 us, of which the extra
+// launch that turns the projection takes 2-3 back, so smaller volumes than
+// BP_SLICE_LANES_MIN keep bp_kernel (64x64x64: both 8.5 us, event time
+// included).  With the driver's two projections, whose 8-byte pairs take twice
+// the L1 bandwidth, it gained 9 % at 256x256x160 and nothing at 128x128x96, so
+// the driver keeps bp_kernel and its layout.
+constexpr int64_t BP_SLICE_LANES_MIN = 1 << 21;
+
+// A projection as the slice-lane backprojector reads it: detector columns
+// apart, each column's even rows first, then its odd ones.  Neighbouring slices meet
+// rows about two apart (the magnification over the pitch is near 2 voxels'
+// worth of rows), so a warp's lanes read neighbouring elements.
+__host__ __device__ __forceinline__ int bp_half_rows(int nb) { return (nb + 1) / 2; }
+__host__ __device__ __forceinline__ int64_t bp_cells(int na, int nb) {
+    return (int64_t)na * 2 * bp_half_rows(nb);
+}
+__device__ __forceinline__ int64_t bp_cell(int ia, int ib, int nb) {
+    return (2 * (int64_t)ia + (ib & 1)) * bp_half_rows(nb) + (ib >> 1);
+}
+
+// A slice's distances from the centre plane (:68,96-97).
+struct BPSlice {
+    float zc, zp, zm;
+};
+__device__ __forceinline__ BPSlice bp_slice(int iz, int nz) {
+    const float zc = (float)iz - nz / 2 + 0.5f;
+    return BPSlice{zc, zc + 0.5f, zc - 0.5f};
+}
+
+// Row box of a voxel (:68,96-97,115-122,137-138), as bp_rows, both ends in one
+// packed division where the operands are proven.
+template <bool PROVEN>
+__device__ __forceinline__ void bp_box(const BPColumn &c, const BPSlice &z, const Geom &g, float &bmin,
+                                       float &bmax) {
+    const float bl = __fmul_rn(c.rl, z.zc), br = __fmul_rn(c.rr, z.zc);
+    const float bt = __fmul_rn(c.r0, z.zp), bb = __fmul_rn(c.r0, z.zm);
+    const float hi = fmaxf(fmaxf(bl, br), fmaxf(bt, bb));
+    const float lo = fminf(fminf(bl, br), fminf(bt, bb));
+    if (PROVEN) {
+        const float y = mk_recip(g.db);
+        const f32x2 n = f2_pack(lo, hi), yy = f2_pack(y, y), nd = f2_pack(-g.db, -g.db);
+        const f32x2 q0 = f2_mul(n, yy);
+        const f32x2 q = f2_fma(f2_fma(nd, q0, n), yy, q0);
+        f2_unpack(f2_add(f2_add(q, f2_pack(-g.bi, -g.bi)), f2_pack(0.5f, 0.5f)), bmin, bmax);
+        return;
+    }
+    const float y = mk_recip(g.db);
+    float qhi = mk_div(hi, g.db, y), qlo = mk_div(lo, g.db, y);
+    if (!(mk_den_ok(g.db) && mk_num_ok(hi) && mk_num_ok(lo))) {
+        qhi = hi / g.db;
+        qlo = lo / g.db;
+    }
+    bmax = qhi - g.bi + 0.5f;
+    bmin = qlo - g.bi + 0.5f;
+}
+
+// Overlap-weighted gather of one projection for one voxel of a voxel column in
+// the reference's order (detector column outer, row inner, acc = fma(wa*wb, p,
+// acc), :150-168); the row weights wb are computed once.  cells: the
+// projection (bp_cell).  All lanes of the warp call it (on: the lane's voxel
+// exists).
+template <bool PROVEN>
+__device__ __forceinline__ float bp_gather_column(const Geom &g, const BPColumn &col, const BPSlice &z,
+                                                  bool on, const float *cells) {
+    const int h = bp_half_rows(g.nb);
+    const float fna = (float)g.na, fnb = (float)g.nb;
+    float bmn, bmx;
+    bp_box<PROVEN>(col, z, g, bmn, bmx);
+    const float blim = on ? ((fnb < bmx) ? fnb : bmx) : -1.0f;     // MIN(nb, b_max)
+    const float alim = (fna < col.amax) ? fna : col.amax;          // MIN(na, a_max)
+    // first row max(0, floor(b_min)) (at most nb, where there is none) and
+    // first column, as floats: every index is exact in float
+    const float tb = __fadd_rd(fminf(fmaxf(bmn, 0.0f), fnb), MK_MAGIC);
+    const float fb = __fsub_rn(tb, MK_MAGIC);
+    const int ib0 = (int)(__float_as_uint(tb) - (unsigned)MK_MAGIC_BITS);
+    float fa = floorf(fminf(fmaxf(col.amin, 0.0f), fna));
+    const int ia0 = (int)fa;
+    const float f1 = fb + 1.0f, f2 = fb + 2.0f, f3 = fb + 3.0f, f4 = fb + 4.0f;
+    float acc = 0.0f;
+    if (__any_sync(0xffffffffu, f4 < blim)) {
+        // a footprint of more than four rows in the warp
+        for (; fa < alim; fa += 1.0f) {
+            const float wa = fminf(fa + 1.0f, col.amax) - fmaxf(fa, col.amin);
+            int ib = ib0;
+            for (float f = fb; f < blim; f += 1.0f, ib++) {
+                const float w = __fmul_rn(wa, fminf(f + 1.0f, bmx) - fmaxf(f, bmn));
+                acc = __fmaf_rn(w, __ldg(cells + bp_cell((int)fa, ib, g.nb)), acc);
+            }
+        }
+        return acc;
+    }
+    const bool p0 = fb < blim, p1 = f1 < blim, p2 = f2 < blim, p3 = f3 < blim;
+    // max(ib, b_min) is ib itself for every row after the first
+    const float wb0 = fminf(f1, bmx) - fmaxf(fb, bmn), wb1 = fminf(f2, bmx) - f1;
+    const float wb2 = fminf(f3, bmx) - f2, wb3 = fminf(f4, bmx) - f3;
+    // rows ib0, ib0 + 2 are neighbours in their half of the detector column,
+    // ib0 + 1, ib0 + 3 in the other
+    const int odd = ib0 & 1, half = ib0 >> 1;
+    const float *pe = cells + (int64_t)ia0 * (2 * h) + ((odd ? h : 0) + half);
+    const float *po = cells + (int64_t)ia0 * (2 * h) + ((odd ? 0 : h) + half + odd);
+#pragma unroll 1
+    for (; fa < alim; pe += 2 * h, po += 2 * h) {
+        const float fn = fa + 1.0f, wa = fminf(fn, col.amax) - fmaxf(fa, col.amin);
+        fa = fn;
+        float v0, v1, v2, v3;
+        if (p0) v0 = __ldg(pe);
+        if (p1) v1 = __ldg(po);
+        if (p2) v2 = __ldg(pe + 1);
+        if (p3) v3 = __ldg(po + 1);
+        if (p0) acc = __fmaf_rn(__fmul_rn(wa, wb0), v0, acc);
+        if (p1) acc = __fmaf_rn(__fmul_rn(wa, wb1), v1, acc);
+        if (p2) acc = __fmaf_rn(__fmul_rn(wa, wb2), v2, acc);
+        if (p3) acc = __fmaf_rn(__fmul_rn(wa, wb3), v3, acc);
+    }
+    return acc;
+}
+
+// blockDim = BP_THREADS; a block backprojects a tile of BP_X voxel columns of
+// one row iy and ZL slices: the lanes of a warp are ZL slices of 32 / ZL
+// neighbouring columns, and each warp does BP_X / warps of the columns.  Grid
+// bp_slice_grid<ZL>.
+constexpr int BP_X = 32, BP_THREADS = 256;
+template <bool PROVEN, int ZL>
+__global__ void __launch_bounds__(BP_THREADS) bp_slice_kernel(float *out, const float *cells,
+                                                              float angle, const Geom g) {
+    constexpr int XL = 32 / ZL;                   // columns side by side in a warp
+    constexpr int WC = BP_X / (BP_THREADS / 32);  // columns per warp
+    __shared__ float tile[ZL][BP_X + 1];
+    __shared__ BPColumn cols[BP_X];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const unsigned gx = (g.nx + BP_X - 1) / BP_X, by = blockIdx.x / gx;
+    const int x0 = (int)(blockIdx.x - by * gx) * BP_X, z0 = blockIdx.y * ZL, iy = (int)by;
+    const int lz = lane % ZL, iz = z0 + lz;
+    const BPSlice z = bp_slice(iz, g.nz);
+    if (t < BP_X)
+        cols[t] = bp_column<PROVEN>(min(x0 + t, g.nx - 1), iy, __cosf(angle), __sinf(angle), g);
+    __syncthreads();
+#pragma unroll 1
+    for (int c = 0; c < WC; c += XL) {
+        const int lx = warp * WC + c + lane / ZL;
+        const bool on = x0 + lx < g.nx && iz < g.nz;
+        tile[lz][lx] = bp_gather_column<PROVEN>(g, cols[lx], z, on, cells);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = t; e < BP_X * ZL; e += BP_THREADS) {
+        const int ix = x0 + e % BP_X, k = z0 + e / BP_X;
+        if (ix < g.nx && k < g.nz)
+            out[ix + (int64_t)iy * g.nx + (int64_t)k * g.nx * g.ny] = tile[e / BP_X][e % BP_X];
+    }
+}
+template <int ZL> inline dim3 bp_slice_grid(const Geom &g) {
+    return dim3(div_up(g.nx, BP_X) * (unsigned)g.ny, div_up(g.nz, ZL));
+}
+
+// The backprojector's cell layout (bp_cell) of a projection stored row by row,
+// with the values its texture read gives (tex_texel).  blockDim (32, 8),
+// 32 x 32 tiles (columns, rows).
+static __global__ void __launch_bounds__(256) bp_cells_kernel(float *dst, const float *proj, int na,
+                                                              int nb) {
+    __shared__ float tile[32][33];
+    const int tx = threadIdx.x, ty = threadIdx.y, a0 = blockIdx.x * 32, b0 = blockIdx.y * 32;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int ia = a0 + tx, ib = b0 + ty + 8 * k;
+        const float v = (ia < na && ib < nb) ? __ldg(proj + ia + (int64_t)ib * na) : 0.0f;
+        tile[ty + 8 * k][tx] = tex_texel(v);
+    }
+    __syncthreads();
+    // lanes: the tile's even rows, then its odd ones
+    const int lb = tx < 16 ? 2 * tx : 2 * (tx - 16) + 1;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int la = ty + 8 * k, ia = a0 + la, ib = b0 + lb;
+        if (ia < na && ib < nb) dst[bp_cell(ia, ib, nb)] = tile[lb][la];
+    }
+}
+
 }  // namespace mcsart

@@ -367,42 +367,6 @@ constexpr int FPC_COLS = 4;                    // detector columns (warps) per b
 constexpr int FPC_ROWS = 32;                   // detector rows per block: a warp's lanes
 constexpr int FPC_THREADS = FPC_COLS * 32;
 
-// Two FP32 values in one 64-bit register pair and the packed operations on
-// them (PTX f32x2), each half rounded as the scalar operation.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 f2_pack(float lo, float hi) {
-    f32x2 d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-    return d;
-}
-__device__ __forceinline__ void f2_unpack(f32x2 v, float &lo, float &hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f32x2 f2_add_rd(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-// a - b, as fma(b, -1, a): one rounding of the exact difference
-__device__ __forceinline__ f32x2 f2_sub(f32x2 a, f32x2 b) {
-    return f2_fma(b, f2_pack(-1.0f, -1.0f), a);
-}
-
 // In-plane footprint of one slab.  U2 - U1 <= 1: (a, b) = weights of voxels
 // U1 and U1 + 1; otherwise (a, b) = (ui1, ui2), the footprint edges.
 struct SlabU {

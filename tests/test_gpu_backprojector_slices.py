@@ -1,0 +1,54 @@
+"""The slice-lane backprojector against bp_kernel and the FP64 oracle.
+
+mcsart_backprojection takes it from 2^21 voxels on; every voxel's sum has the
+same operations in the same order in both kernels, so the middle slices of a
+volume above the line equal the volume below it that they make.
+"""
+import numpy as np
+import pytest
+
+from conftest import dev, geo, host, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+MIN = 1 << 21  # BP_SLICE_LANES_MIN
+
+
+def _args(g):
+    return (g["SO"], g["SD"], g["da"], g["na"], g["ai"], g["db"], g["nb"], g["bi"], g["nx"],
+            g["ny"], g["nz"])
+
+
+def _bp(ctx, torch, proj, a, g):
+    out = torch.full((g["nz"], g["ny"], g["nx"]), 7.0, device="cuda")
+    ctx.host_backprojection(out, dev(torch, proj), a, *_args(g))
+    ctx.synchronize()
+    return host(out)
+
+
+# depths with full, half-empty and nearly empty last tiles; odd rows; wide
+# voxels (more than four rows each); a source too close for the proof
+@pytest.mark.parametrize("nx,ny,nz,na,nb,kw", [
+    (181, 173, 67, 97, 51, {}), (160, 160, 96, 64, 64, {}), (129, 131, 129, 75, 80, dict(db=0.3)),
+    (200, 180, 82, 90, 61, dict(SO=138.0, SD=207.0, da=3.0, db=2.0))])
+def test_larger_volume_equals_its_slabs_of_slices(ctx, torch_cuda, nx, ny, nz, na, nb, kw):
+    torch = torch_cuda
+    assert nx * ny * nz >= MIN
+    g = geo(nx=nx, ny=ny, nz=nz, na=na, nb=nb, **{**dict(SO=300.0, SD=450.0, da=2.9, db=2.3), **kw})
+    rng = np.random.default_rng(nx)
+    proj = rng.random((nb, na), dtype=np.float32)
+    proj[0, :3] = 1e-40  # denormal texels read as zeros
+    for a in (0.3, 0.7853982, 2.4):
+        big = _bp(ctx, torch, proj, a, g)
+        # its middle 40 slices are a volume of their own with the same centre plane
+        assert nx * ny * 40 < MIN
+        small = _bp(ctx, torch, proj, a, dict(g, nz=40))
+        np.testing.assert_array_equal(big[nz // 2 - 20: nz // 2 + 20], small)
+
+
+def test_larger_volume_matches_the_oracle(ctx, torch_cuda, oracle):
+    torch = torch_cuda
+    g = geo(nx=130, ny=128, nz=127, na=80, nb=70, SO=300.0, SD=450.0, da=2.9, db=2.9)
+    proj = np.random.default_rng(3).random((70, 80), dtype=np.float32)
+    for a in (0.3, 2.4):
+        assert rel_l2(_bp(ctx, torch, proj, a, g), oracle.backprojection(proj, a, g)) <= 1e-4
