@@ -1,5 +1,6 @@
 // Kernel-level C ABI: one entry point per reference launcher (include/mcsart.h).
 #include <algorithm>
+#include <cmath>
 #include <initializer_list>
 
 #include "backprojector.cuh"
@@ -409,6 +410,8 @@ int projection_ex_typed(mcsart_ctx *ctx, float *d_proj, const VT *d_img, int fp_
     if (fp_sum == SUM_REF)
         return launch_fp_ref<1, false, VT>(
             ctx, dim3(div_up(g.na, FPC_COLS), div_up(g.nb, FPC_ROWS), 1), a);
+    a.cos64 = cos((double)angle);
+    a.sin64 = sin((double)angle);
     const int groups = fp_auto_groups((int64_t)g.na * div_up(g.nb, 32), std::max(g.nx, g.ny));
     const dim3 grid(g.na, div_up(g.nb, 32), 1), block(32, groups);
     const size_t smem = (size_t)groups * 2 * 32 * sizeof(float);
@@ -482,6 +485,8 @@ MC_EXPORT int mcsart_backprojection_ex(mcsart_ctx *ctx, float *d_img, const floa
     a.proj = d_proj;
     a.g = g;
     a.angle = angle;
+    a.cos64 = cos((double)angle);
+    a.sin64 = sin((double)angle);
     a.out = d_img;
     const dim3 grid = bp_grid<BP_NZ, BP_ROWS>(g), block(32, BP_ROWS);
     MC_LAUNCH(ctx, (bp_kernel<1, BP_PLAIN, false, false, true>), grid, block, 0, a);

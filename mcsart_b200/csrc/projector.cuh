@@ -126,83 +126,6 @@ __device__ __forceinline__ void fp_voxel(const VT *const *base, int64_t a, float
 // split across warps.
 enum SumMode { SUM_REF = 0, SUM_PLAIN = 1, SUM_KAHAN = 2 };
 
-// Accumulates the footprint of slabs [d0, d1) of one ray into s[0..K-1]
-// (volume sums) and sw (sum of weights = projection of a ones-volume), in the
-// split summation modes.
-template <int K, bool ONES, int SUM, typename VT>
-__device__ __forceinline__ void ray_slabs(const RayGeom &r, const FPVolumes<VT, K> &v,
-                                          const Geom &g, int d0, int d1, float *s, float &sw) {
-    static_assert(SUM != SUM_REF, "the reference order is fp_ref_kernel's");
-    int su, sd;
-    zf_strides(r.xdrive, g, su, sd);
-    const float z_half = (float)(g.nz / 2);
-    float acc[K], cmp[K], accw = 0.0f, cmpw = 0.0f;
-#pragma unroll
-    for (int k = 0; k < K; k++) { acc[k] = 0.0f; cmp[k] = 0.0f; }
-
-    for (int d = d0; d < d1; d++) {
-        // :52 / :105
-        const float dc = __fsub_rn(__fsub_rn(__fadd_rn((float)d, 0.5f), r.d_half), r.src_d);
-        // :54-61 / :107-114 ("ratio * xc + y1 + ny / 2")
-        const float c0 = __fadd_rn(__fmaf_rn(r.r0, dc, r.u_off), r.u_half);
-        const float c1 = __fadd_rn(__fmaf_rn(r.r1, dc, r.u_off), r.u_half);
-        const float c2 = __fadd_rn(__fmaf_rn(r.r2, dc, r.u_off), r.u_half);
-        const float c3 = __fadd_rn(__fmaf_rn(r.r3, dc, r.u_off), r.u_half);
-        const float ui1 = fminf(fminf(c0, c1), fminf(c2, c3));
-        const float ui2 = fmaxf(fmaxf(c0, c1), fmaxf(c2, c3));
-        // :71-77 / :124-130 ("ratio * xc + z1 + nz / 2", z1 = 0)
-        const float cz0 = __fadd_rn(__fmul_rn(r.rz0, dc), z_half);
-        const float cz1 = __fadd_rn(__fmul_rn(r.rz1, dc), z_half);
-        const float zi1 = fminf(cz0, cz1), zi2 = fmaxf(cz0, cz1);
-        const int U1 = (int)floorf(ui1), U2 = (int)floorf(ui2);
-        const int Z1 = (int)floorf(zi1), Z2 = (int)floorf(zi2);
-        const float du = __fsub_rn(ui2, ui1), dz = __fsub_rn(zi2, zi1);
-        const int u_lo = max(0, U1), u_hi = min(r.nu - 1, U2);
-        const int z_lo = max(0, Z1), z_hi = min(g.nz - 1, Z2);
-        if (u_lo > u_hi || z_lo > z_hi) continue;
-        float ss[K], ssw = 0.0f;
-#pragma unroll
-        for (int k = 0; k < K; k++) ss[k] = 0.0f;
-        for (int u = u_lo; u <= u_hi; u++) {
-            // :83 / :136
-            const float wu = __fdiv_rn(__fsub_rn(fminf(__fadd_rn((float)u, 1.0f), ui2), fmaxf((float)u, ui1)), du);
-            const int row = u * su + d * sd;
-            for (int z = z_lo; z <= z_hi; z++) {
-                // :86 / :139
-                const float wz = __fdiv_rn(__fsub_rn(fminf(__fadd_rn((float)z, 1.0f), zi2), fmaxf((float)z, zi1)), dz);
-                const int a = row + z;
-#pragma unroll
-                for (int k = 0; k < K; k++) ss[k] = __fmaf_rn(__fmul_rn(ldv(v.zf[k], a), wu), wz, ss[k]);
-                if (ONES) ssw = __fmaf_rn(wu, wz, ssw);
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            if (SUM == SUM_KAHAN) {
-                const float y = ss[k] - cmp[k];
-                const float t = acc[k] + y;
-                cmp[k] = (t - acc[k]) - y;
-                acc[k] = t;
-            } else {
-                acc[k] += ss[k];
-            }
-        }
-        if (ONES) {
-            if (SUM == SUM_KAHAN) {
-                const float y = ssw - cmpw;
-                const float t = accw + y;
-                cmpw = (t - accw) - y;
-                accw = t;
-            } else {
-                accw += ssw;
-            }
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < K; k++) s[k] = acc[k];
-    sw = accw;
-}
-
 // ------------------------------------------------------------------------
 // FP64 geometry (options.geom64, with the split summation modes): the same
 // footprint formulas as ray_geom / ray_slabs (src/cu_projection.cu:23-144),
@@ -246,70 +169,11 @@ __device__ __forceinline__ RayGeom64 ray_geom64(double cphi, double sphi, int ia
     return r;
 }
 
-// Slabs [d0, d1) of one ray with FP64 geometry: s[k] (FP32 sums of the
-// volumes' terms) and sw (FP64 sum of the weights).
-template <int K, bool ONES, int SUM, typename VT>
-__device__ __forceinline__ void ray_slabs64(const RayGeom64 &r, const FPVolumes<VT, K> &v,
-                                            const Geom &g, int d0, int d1, float *s, double &sw) {
-    int su, sd;
-    zf_strides(r.xdrive, g, su, sd);
-    const double z_half = (double)(g.nz / 2);
-    float acc[K], cmp[K];
-#pragma unroll
-    for (int k = 0; k < K; k++) { acc[k] = 0.0f; cmp[k] = 0.0f; }
-    double accw = 0.0;
-    for (int d = d0; d < d1; d++) {
-        const double dc = ((double)d + 0.5) - r.d_half - r.src_d;  // :52 / :105
-        const double c0 = r.r0 * dc + r.u_off + r.u_half, c1 = r.r1 * dc + r.u_off + r.u_half;
-        const double c2 = r.r2 * dc + r.u_off + r.u_half, c3 = r.r3 * dc + r.u_off + r.u_half;
-        const double ui1 = fmin(fmin(c0, c1), fmin(c2, c3));
-        const double ui2 = fmax(fmax(c0, c1), fmax(c2, c3));
-        const double cz0 = r.rz0 * dc + z_half, cz1 = r.rz1 * dc + z_half;  // :71-77
-        const double zi1 = fmin(cz0, cz1), zi2 = fmax(cz0, cz1);
-        // loop bounds clamped to the volume before the integer conversion
-        const int u_lo = max(0, (int)floor(fmax(ui1, -1.0)));
-        const int u_hi = min(r.nu - 1, (int)floor(fmin(ui2, (double)r.nu)));
-        const int z_lo = max(0, (int)floor(fmax(zi1, -1.0)));
-        const int z_hi = min(g.nz - 1, (int)floor(fmin(zi2, (double)g.nz)));
-        if (u_lo > u_hi || z_lo > z_hi) continue;
-        const double du = ui2 - ui1, dz = zi2 - zi1;
-        float ss[K];
-#pragma unroll
-        for (int k = 0; k < K; k++) ss[k] = 0.0f;
-        for (int u = u_lo; u <= u_hi; u++) {
-            const double wu = (fmin(u + 1.0, ui2) - fmax((double)u, ui1)) / du;  // :83 / :136
-            const int row = u * su + d * sd;
-            for (int z = z_lo; z <= z_hi; z++) {
-                const double wz = (fmin(z + 1.0, zi2) - fmax((double)z, zi1)) / dz;  // :86 / :139
-                const double w = wu * wz;
-                const float wf = (float)w;
-                const int a = row + z;
-#pragma unroll
-                for (int k = 0; k < K; k++) ss[k] = __fmaf_rn(ldv(v.zf[k], a), wf, ss[k]);
-                if (ONES) accw += w;
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            if (SUM == SUM_KAHAN) {
-                const float y = ss[k] - cmp[k];
-                const float t = acc[k] + y;
-                cmp[k] = (t - acc[k]) - y;
-                acc[k] = t;
-            } else {
-                acc[k] += ss[k];
-            }
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < K; k++) s[k] = acc[k];
-    sw = accw;
-}
-
 template <typename VT, int K, typename MT = VT> struct FPArgs {
     FPVolumes<VT, K> vol;
     Geom g;
     float angle;            // used when angles == nullptr
+    double cos64, sin64;    // of the angle (single views with FP64 geometry)
     const float *angles;    // per-view angles (device), view = blockIdx.z
     int mode;
     // FP_PLAIN: out[view*na*nb + ia + ib*na] = s0
@@ -1163,16 +1027,200 @@ int launch_fp_ref(mcsart_ctx *ctx, dim3 grid, const FPArgs<VT, K, MT> &a) {
     return MCSART_OK;
 }
 
-// Per-ray projector of the split summation modes: blockDim (32, groups), the
-// 32 lanes 32 consecutive detector rows of one column, threadIdx.y = slab
-// group of the same 32 rays, gridDim (na, ceil(nb/32), views).
-// GEO64: FP64 geometry and weight sum (ray_geom64 / ray_slabs64).
+// ------------------------------------------------------------------------
+// Projector of the split summation modes: blockDim (32, groups), the 32 lanes
+// 32 consecutive detector rows of one column, threadIdx.y = slab group of the
+// same 32 rays, gridDim (na, ceil(nb/32), views).  A warp's lanes compute the
+// column's in-plane footprint of 32 slabs at a time, one slab each, into a
+// table of the warp's own, and then walk the slabs together, each lane adding
+// its ray's axial part.  Each slab's terms are summed first (in-plane voxel,
+// then slice) and the slab sums added, plainly or with Kahan compensation.
+// GEO64: FP64 geometry and weight sum (ray_geom64): every coordinate, box edge
+// and overlap weight in FP64 (an edge's overlap is divided by the footprint's
+// width by way of its reciprocal, one FP64 rounding more), volume terms in FP32.
+// Bound by instruction issue: FP64 operations, and divisions in FP32 geometry.
+// 128x128x96, 256x192 detector, Kahan, FP64 geometry: 146 us with a thread
+// computing its ray's footprints by itself, now 65; 256x256x160, 512x384, FP32
+// geometry: 387, now 338.
+
+// In-plane footprint of one slab: voxels u_lo .. u_lo + n - 1 (in the volume)
+// with the first one's column at element `row`, the edges, the reciprocal width
+// (GEO64; the width itself otherwise) and the first two weights.
+template <typename R> struct SlabSplit {
+    R lo, hi, inv, dc;
+    R w0, w1;
+    int row, u_lo, n;
+};
+__device__ __forceinline__ double overlap(double i, double lo, double hi) {
+    return fmin(i + 1.0, hi) - fmax(i, lo);
+}
+__device__ __forceinline__ float overlap(float i, float lo, float hi) {
+    return __fsub_rn(fminf(__fadd_rn(i, 1.0f), hi), fmaxf(i, lo));
+}
+__device__ __forceinline__ double split_weight(double i, double lo, double hi, double inv) {
+    return overlap(i, lo, hi) * inv;
+}
+// (FP32: the correctly rounded quotient by the width, as the reference order)
+__device__ __forceinline__ float split_weight(float i, float lo, float hi, float width) {
+    return __fdiv_rn(overlap(i, lo, hi), width);
+}
+
+__device__ __forceinline__ SlabSplit<double> slab_split(const RayGeom64 &r, int d, int su, int sd) {
+    SlabSplit<double> e;
+    e.dc = ((double)d + 0.5) - r.d_half - r.src_d;  // :52 / :105
+    const double c0 = r.r0 * e.dc + r.u_off + r.u_half, c1 = r.r1 * e.dc + r.u_off + r.u_half;
+    const double c2 = r.r2 * e.dc + r.u_off + r.u_half, c3 = r.r3 * e.dc + r.u_off + r.u_half;
+    e.lo = fmin(fmin(c0, c1), fmin(c2, c3));
+    e.hi = fmax(fmax(c0, c1), fmax(c2, c3));
+    e.inv = 1.0 / (e.hi - e.lo);
+    e.u_lo = max(0, __double2int_rd(e.lo));
+    e.n = max(0, min(r.nu - 1, __double2int_rd(e.hi)) - e.u_lo + 1);
+    e.w0 = split_weight((double)e.u_lo, e.lo, e.hi, e.inv);  // :83 / :136
+    e.w1 = split_weight(e.u_lo + 1.0, e.lo, e.hi, e.inv);
+    e.row = e.u_lo * su + d * sd;
+    return e;
+}
+__device__ __forceinline__ SlabSplit<float> slab_split(const RayGeom &r, int d, int su, int sd) {
+    SlabSplit<float> e;
+    e.dc = __fsub_rn(__fsub_rn(__fadd_rn((float)d, 0.5f), r.d_half), r.src_d);  // :52 / :105
+    // :54-63 / :107-116
+    const float c0 = __fadd_rn(__fmaf_rn(r.r0, e.dc, r.u_off), r.u_half);
+    const float c1 = __fadd_rn(__fmaf_rn(r.r1, e.dc, r.u_off), r.u_half);
+    const float c2 = __fadd_rn(__fmaf_rn(r.r2, e.dc, r.u_off), r.u_half);
+    const float c3 = __fadd_rn(__fmaf_rn(r.r3, e.dc, r.u_off), r.u_half);
+    e.lo = fminf(fminf(c0, c1), fminf(c2, c3));
+    e.hi = fmaxf(fmaxf(c0, c1), fmaxf(c2, c3));
+    e.inv = __fsub_rn(e.hi, e.lo);
+    e.u_lo = max(0, (int)floorf(e.lo));
+    e.n = max(0, min(r.nu - 1, (int)floorf(e.hi)) - e.u_lo + 1);
+    e.w0 = split_weight((float)e.u_lo, e.lo, e.hi, e.inv);  // :83 / :136
+    e.w1 = split_weight((float)(e.u_lo + 1), e.lo, e.hi, e.inv);
+    e.row = e.u_lo * su + d * sd;
+    return e;
+}
+
+// Axial edges of a slab (:71-77 / :124-130, "ratio * xc + z1 + nz / 2", z1 = 0)
+// and their slices, clamped to the volume; inv as SlabSplit's.
+template <typename R> struct SplitZ {
+    R lo, hi, inv;
+    int z0, z1;
+};
+__device__ __forceinline__ SplitZ<double> split_z(double rz0, double rz1, double dc, double z_half,
+                                                  int nz) {
+    const double a = rz0 * dc + z_half, b = rz1 * dc + z_half;
+    SplitZ<double> z;
+    z.lo = fmin(a, b);
+    z.hi = fmax(a, b);
+    z.inv = 1.0 / (z.hi - z.lo);
+    z.z0 = max(0, __double2int_rd(z.lo));
+    z.z1 = min(nz - 1, __double2int_rd(z.hi));
+    return z;
+}
+__device__ __forceinline__ SplitZ<float> split_z(float rz0, float rz1, float dc, float z_half, int nz) {
+    const float a = __fadd_rn(__fmul_rn(rz0, dc), z_half), b = __fadd_rn(__fmul_rn(rz1, dc), z_half);
+    SplitZ<float> z;
+    z.lo = fminf(a, b);
+    z.hi = fmaxf(a, b);
+    z.inv = __fsub_rn(z.hi, z.lo);
+    z.z0 = max(0, (int)floorf(z.lo));
+    z.z1 = min(nz - 1, (int)floorf(z.hi));
+    return z;
+}
+
+// One voxel's terms: FP32, or the FP64 weight rounded to FP32 and its sum in FP64.
+template <int K, bool ONES, typename VT>
+__device__ __forceinline__ void split_term(const VT *const *zf, int a, float wu, float wz, float *ss,
+                                           float &sw) {
+#pragma unroll
+    for (int k = 0; k < K; k++) ss[k] = __fmaf_rn(__fmul_rn(ldv(zf[k], a), wu), wz, ss[k]);
+    if (ONES) sw = __fmaf_rn(wu, wz, sw);
+}
+template <int K, bool ONES, typename VT>
+__device__ __forceinline__ void split_term(const VT *const *zf, int a, double wu, double wz, float *ss,
+                                           double &sw) {
+    const double w = wu * wz;
+    const float wf = (float)w;
+#pragma unroll
+    for (int k = 0; k < K; k++) ss[k] = __fmaf_rn(ldv(zf[k], a), wf, ss[k]);
+    if (ONES) sw += w;
+}
+
+// Adds slab sum x to sum s, plainly or with Kahan compensation c.
+template <int SUM> __device__ __forceinline__ void split_add(float &s, float &c, float x) {
+    if (SUM == SUM_KAHAN) {
+        const float y = x - c, t = s + y;
+        c = (t - s) - y;
+        s = t;
+    } else {
+        s += x;
+    }
+}
+
+template <bool GEO64> struct SplitReal { using R = float; using Ray = RayGeom; };
+template <> struct SplitReal<true> { using R = double; using Ray = RayGeom64; };
+
+// Slabs [d0, d1) of the warp's rays: s[k], and sw (FP32 slab sums of FP32
+// weights, FP64 sum of FP64 weights); tab: 32 entries of the warp's own.
+template <int K, bool ONES, int SUM, bool GEO64, typename VT>
+__device__ __forceinline__ void split_slabs(const typename SplitReal<GEO64>::Ray &r,
+                                            const FPVolumes<VT, K> &v, const Geom &g, int d0, int d1,
+                                            SlabSplit<typename SplitReal<GEO64>::R> *tab, float *s,
+                                            typename SplitReal<GEO64>::R &sw) {
+    using R = typename SplitReal<GEO64>::R;
+    static_assert(SUM != SUM_REF, "the reference order is fp_ref_kernel's");
+    const int lane = threadIdx.x;
+    int su, sd;
+    zf_strides(r.xdrive, g, su, sd);
+    const R z_half = (R)(g.nz / 2);
+    float acc[K], cmp[K], cmpw = 0.0f;
+    R accw = 0;
+#pragma unroll
+    for (int k = 0; k < K; k++) { acc[k] = 0.0f; cmp[k] = 0.0f; }
+    for (int c0 = d0; c0 < d1; c0 += 32) {
+        __syncwarp();
+        if (c0 + lane < d1) tab[lane] = slab_split(r, c0 + lane, su, sd);
+        __syncwarp();
+        const int m = min(32, d1 - c0);
+        for (int j = 0; j < m; j++) {
+            const SlabSplit<R> &e = tab[j];
+            if (e.n == 0) continue;  // the same for the whole warp
+            const SplitZ<R> z = split_z(r.rz0, r.rz1, e.dc, z_half, g.nz);
+            if (z.z0 > z.z1) continue;
+            const R wz0 = split_weight((R)z.z0, z.lo, z.hi, z.inv);  // :86 / :139
+            const R wz1 = z.z1 > z.z0 ? split_weight((R)(z.z0 + 1), z.lo, z.hi, z.inv) : (R)0;
+            float ss[K];
+            R ssw = 0;
+#pragma unroll
+            for (int k = 0; k < K; k++) ss[k] = 0.0f;
+            for (int i = 0; i < e.n; i++) {
+                const R wu = i == 0 ? e.w0 : i == 1 ? e.w1 : split_weight((R)(e.u_lo + i), e.lo, e.hi, e.inv);
+                const int a = e.row + i * su;
+                split_term<K, ONES>(v.zf, a + z.z0, wu, wz0, ss, ssw);
+                if (z.z1 > z.z0) split_term<K, ONES>(v.zf, a + z.z0 + 1, wu, wz1, ss, ssw);
+                for (int q = z.z0 + 2; q <= z.z1; q++)
+                    split_term<K, ONES>(v.zf, a + q, wu, split_weight((R)q, z.lo, z.hi, z.inv), ss, ssw);
+            }
+#pragma unroll
+            for (int k = 0; k < K; k++) split_add<SUM>(acc[k], cmp[k], ss[k]);
+            if constexpr (ONES) {
+                if constexpr (GEO64)
+                    accw += ssw;
+                else
+                    split_add<SUM>(accw, cmpw, ssw);
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++) s[k] = acc[k];
+    sw = accw;
+}
+
 template <int K, bool ONES, int SUM, typename VT, typename MT = VT, bool GEO64 = false>
 __global__ void __launch_bounds__(256) fp_kernel(const FPArgs<VT, K, MT> p) {
-    static_assert(SUM != SUM_REF, "the reference order is fp_ref_kernel's");
     constexpr int NS = K + (ONES ? 1 : 0);
     extern __shared__ float sm_fp[];  // [groups][NS][32]
     __shared__ double sm_w64[GEO64 ? 8 : 1][32];  // GEO64: the groups' FP64 weight sums
+    __shared__ SlabSplit<typename SplitReal<GEO64>::R> sm_tab[8][32];
     const int lane = threadIdx.x;
     const Geom &g = p.g;
     const int ia = blockIdx.x, ib = blockIdx.y * 32 + lane;
@@ -1180,23 +1228,18 @@ __global__ void __launch_bounds__(256) fp_kernel(const FPArgs<VT, K, MT> p) {
     const int groups = blockDim.y, grp = threadIdx.y;
     float s[K], sw = 0.0f;
     double sw64 = 0.0;
-#pragma unroll
-    for (int k = 0; k < K; k++) s[k] = 0.0f;
-    if (active) {
-        const float angle = p.angles ? p.angles[blockIdx.z] : p.angle;
-        if (GEO64) {
-            double sd, cd;
-            sincos((double)angle, &sd, &cd);
-            const RayGeom64 r = ray_geom64(cd, sd, ia, ib, g);
-            const int per = (r.nd + groups - 1) / groups;
-            const int d0 = grp * per, d1 = min(r.nd, d0 + per);
-            ray_slabs64<K, ONES, SUM, VT>(r, p.vol, g, d0, d1, s, sw64);
+    {
+        // lanes past the last row repeat its ray; nothing of them is stored
+        const int row = min(ib, g.nb - 1);
+        if constexpr (GEO64) {
+            const RayGeom64 r = ray_geom64(p.cos64, p.sin64, ia, row, g);
+            const int per = (r.nd + groups - 1) / groups, d0 = grp * per, d1 = min(r.nd, d0 + per);
+            split_slabs<K, ONES, SUM, true, VT>(r, p.vol, g, d0, d1, sm_tab[grp], s, sw64);
         } else {
-            const float cphi = cosf(angle), sphi = sinf(angle);  // :23-24
-            const RayGeom r = ray_geom(cphi, sphi, ia, ib, g);
-            const int per = (r.nd + groups - 1) / groups;
-            const int d0 = grp * per, d1 = min(r.nd, d0 + per);
-            ray_slabs<K, ONES, SUM, VT>(r, p.vol, g, d0, d1, s, sw);
+            const float angle = p.angles ? p.angles[blockIdx.z] : p.angle;
+            const RayGeom r = ray_geom(cosf(angle), sinf(angle), ia, row, g);  // :23-24
+            const int per = (r.nd + groups - 1) / groups, d0 = grp * per, d1 = min(r.nd, d0 + per);
+            split_slabs<K, ONES, SUM, false, VT>(r, p.vol, g, d0, d1, sm_tab[grp], s, sw);
         }
     }
 #pragma unroll

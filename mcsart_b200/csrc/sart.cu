@@ -18,6 +18,7 @@
 //
 // The sequence of a pass is captured once as a CUDA graph and replayed for
 // every outer iteration of that kind.
+#include <cmath>
 #include <cstring>
 #include <vector>
 
@@ -185,6 +186,8 @@ template <typename ST, int INTERP, int SUM> struct Runner {
             }
         } else if (opt.geom64) {
             const size_t smem = (size_t)groups * (K + 1) * 32 * sizeof(float);
+            a.cos64 = cos((double)P.angles[v]);
+            a.sin64 = sin((double)P.angles[v]);
             MC_LAUNCH(ctx, (fp_kernel<K, ONES, SUM == SUM_REF ? SUM_PLAIN : SUM, VT, ST, true>),
                       grid, dim3(32, groups), smem, a);
         } else {
@@ -228,6 +231,8 @@ template <typename ST, int INTERP, int SUM> struct Runner {
         if (opt.geom64) {  // FP64 geometry and normaliser (no precomputed columns)
             b.colA = nullptr;
             b.colB = nullptr;
+            b.cos64 = cos((double)P.angles[v]);
+            b.sin64 = sin((double)P.angles[v]);
             const dim3 grid = bp_grid<BP_NZ, BP_ROWS>(P.g), block(32, BP_ROWS);
             if (mode == BP_DIV)
                 MC_LAUNCH(ctx, (bp_kernel<2, BP_DIV, false, false, true>), grid, block, 0, b);
