@@ -142,7 +142,7 @@ MC_EXPORT int mcsart_backprojection(mcsart_ctx *ctx, float *d_img, const float *
     a.g = g;
     a.angle = angle;
     a.out = d_img;
-    const dim3 grid = bp_grid<BP_NZ, BP_ROWS>(g), block(32, BP_ROWS);
+    const dim3 grid = bp_grid<BP_NZ, BP_ROWS>(g, BP_PLAIN), block(32, BP_ROWS);
     if (proven)
         MC_LAUNCH(ctx, (bp_kernel<1, BP_PLAIN, false, true>), grid, block, 0, a);
     else
@@ -488,7 +488,7 @@ MC_EXPORT int mcsart_backprojection_ex(mcsart_ctx *ctx, float *d_img, const floa
     a.cos64 = cos((double)angle);
     a.sin64 = sin((double)angle);
     a.out = d_img;
-    const dim3 grid = bp_grid<BP_NZ, BP_ROWS>(g), block(32, BP_ROWS);
+    const dim3 grid = bp_grid<BP_NZ, BP_ROWS>(g, BP_PLAIN), block(32, BP_ROWS);
     MC_LAUNCH(ctx, (bp_kernel<1, BP_PLAIN, false, false, true>), grid, block, 0, a);
     return finish(ctx, "mcsart_backprojection_ex");
 }

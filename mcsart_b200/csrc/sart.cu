@@ -233,7 +233,7 @@ template <typename ST, int INTERP, int SUM> struct Runner {
             b.colB = nullptr;
             b.cos64 = cos((double)P.angles[v]);
             b.sin64 = sin((double)P.angles[v]);
-            const dim3 grid = bp_grid<BP_NZ, BP_ROWS>(P.g), block(32, BP_ROWS);
+            const dim3 grid = bp_grid<BP_NZ, BP_ROWS>(P.g, mode), block(32, BP_ROWS);
             if (mode == BP_DIV)
                 MC_LAUNCH(ctx, (bp_kernel<2, BP_DIV, false, false, true>), grid, block, 0, b);
             else
@@ -249,7 +249,7 @@ template <typename ST, int INTERP, int SUM> struct Runner {
     }
 
     template <int NZ, int ROWS> int launch_bp_shape(int mode, const BPArgs &b) {
-        const dim3 grid = bp_grid<NZ, ROWS>(P.g), block(32, ROWS);
+        const dim3 grid = bp_grid<NZ, ROWS>(P.g, mode), block(32, ROWS);
         // the proven form skips the division range checks (bp_geom_proven)
         const bool proven = bp_geom_proven(P.g);
         if (mode == BP_DIV && proven) {
@@ -312,7 +312,7 @@ template <typename ST, int INTERP, int SUM> struct Runner {
             b.colA = S.bpcolA.as<float4>();
             b.colB = S.bpcolB.as<float>();
         }
-        const dim3 grid = bp_grid<BP_NZ, BP_ROWS>(P.g), block(32, BP_ROWS);
+        const dim3 grid = bp_grid<BP_NZ, BP_ROWS>(P.g, mode), block(32, BP_ROWS);
         const bool proven = bp_geom_proven(P.g);
         ctx->label = mode == BP_DIV ? "bp_div" : "bp_div_add";
         if (mode == BP_DIV && proven) {
