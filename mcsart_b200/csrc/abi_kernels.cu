@@ -44,9 +44,9 @@ int launch_fp_plain(mcsart_ctx *ctx, float *d_proj, const float *d_imgZ, float a
 template <typename VT>
 int zfast_copy(mcsart_ctx *ctx, const char *name, const VT *src, const Geom &g, const VT **out) {
     void *ws;
-    MC_TRY(workspace(ctx, name, nvox(g.nx, g.ny, g.nz) * sizeof(VT), &ws));
+    MC_TRY(workspace(ctx, name, nvox(g.nx, g.ny, g.nzp) * sizeof(VT), &ws));
     MC_LAUNCH(ctx, (zfast_kernel<VT, VT>), zfast_grid(g.nx, g.ny, g.nz), dim3(32, 8), 0, (VT *)ws,
-              src, g.nx, g.ny, g.nz);
+              src, g.nx, g.ny, g.nz, g.nzp);
     *out = (const VT *)ws;
     return MCSART_OK;
 }
@@ -74,6 +74,7 @@ static Geom make_geom(float SO, float SD, float da, int na, float ai, float db, 
     Geom g;
     g.SO = SO; g.SD = SD; g.da = da; g.ai = ai; g.db = db; g.bi = bi;
     g.na = na; g.nb = nb; g.nx = nx; g.ny = ny; g.nz = nz;
+    g.nzp = zf_pitch(nx, ny, nz);
     return g;
 }
 

@@ -403,8 +403,8 @@ __global__ void __launch_bounds__(256, (bp_min_blocks<GEO64, MULTI, NZ>())) bp_k
 #pragma unroll
         for (int k = 0; k < NZ; k++) {
             const int e = t + 32 * ROWS * k, lx = e / TZ, lz = e % TZ;
-            if (x0 + lx < g.nx && zb + lz < g.nz)
-                p.outZ[zb + lz + ((int64_t)iy * g.nx + x0 + lx) * g.nz] = tile[lz][lx];
+            if (x0 + lx < g.nx && zb + lz < g.nzp)
+                p.outZ[zb + lz + ((int64_t)iy * g.nx + x0 + lx) * g.nzp] = tile[lz][lx];
         }
     }
 }

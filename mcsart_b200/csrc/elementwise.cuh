@@ -234,12 +234,12 @@ static __global__ void __launch_bounds__(256) diff_kernel(float *img1, const flo
 }
 
 // --------------------------------------------------------- fused kernels
-// z-fastest copy of an x-fastest volume: dst[iz + (ix + iy*nx)*nz] =
-// src[ix + iy*nx + iz*nx*ny].  blockDim (32, 8); a block turns a 32 x 32
+// z-fastest copy of an x-fastest volume: dst[iz + (ix + iy*nx)*nzp] =
+// src[ix + iy*nx + iz*nx*ny], zero for nz <= iz < nzp (zf_pitch).  blockDim (32, 8); a block turns a 32 x 32
 // (x, z) tile of row iy; gridDim (ceil(nx/32) * ny, ceil(nz/32)).
 template <typename ST, typename DT>
 static __global__ void __launch_bounds__(256) zfast_kernel(DT *dst, const ST *src, int nx, int ny,
-                                                           int nz) {
+                                                           int nz, int nzp) {
     __shared__ float tile[32][33];
     const int tx = threadIdx.x, ty = threadIdx.y;
     const unsigned gx = (nx + 31) / 32, iy = blockIdx.x / gx;
@@ -254,7 +254,7 @@ static __global__ void __launch_bounds__(256) zfast_kernel(DT *dst, const ST *sr
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         const int lx = ty + 8 * k, ix = x0 + lx, iz = z0 + tx;
-        if (ix < nx && iz < nz) dst[iz + (row + ix) * nz] = cvt<DT>(tile[tx][lx]);
+        if (ix < nx && iz < nzp) dst[iz + (row + ix) * nzp] = cvt<DT>(tile[tx][lx]);
     }
 }
 inline dim3 zfast_grid(int nx, int ny, int nz) {
@@ -301,23 +301,26 @@ template <typename T> __device__ __forceinline__ void st8(T *p, const float *v) 
     *reinterpret_cast<uint4 *>(p) = w.u;
 }
 
-// Stores slices z0 .. z0 + MP_Z - 1 (those below nz) of column c: PAIR, img0
-// and ones interleaved in img0; otherwise apart.  Interleaved pairs of a depth
-// that is a multiple of 4 go out as one store: lanes are different columns,
+// Stores slices z0 .. z0 + MP_Z - 1 (those below nzp, zero from nz on) of column
+// c: PAIR, img0 and ones interleaved in img0; otherwise apart.  Interleaved
+// pairs of a pitch that is a multiple of 4 go out as one store: lanes are different columns,
 // so every store of a warp touches 32 lines, and one whole-sector store in
 // place of four 8-byte ones takes a quarter of the write transactions.
 template <typename VT, bool PAIR>
 __device__ __forceinline__ void store_column(VT *img0, VT *ones, int64_t c, int z0, int nz,
-                                             const float *a, const float *b) {
-    const int64_t i = c * nz + z0;
-    if (PAIR && nz % MP_Z == 0) {
+                                             int nzp, float *a, float *b) {
+    const int64_t i = c * nzp + z0;
+#pragma unroll
+    for (int k = 0; k < MP_Z; k++)
+        if (z0 + k >= nz) a[k] = b[k] = 0.0f;
+    if (PAIR && nzp % MP_Z == 0) {
         const float v[8] = {a[0], b[0], a[1], b[1], a[2], b[2], a[3], b[3]};
         st8(img0 + 2 * i, v);
         return;
     }
 #pragma unroll
     for (int k = 0; k < MP_Z; k++) {
-        if (z0 + k >= nz) break;
+        if (z0 + k >= nzp) break;
         if (PAIR) {
             stv2(img0, i + k, a[k], b[k]);
         } else {
@@ -368,8 +371,8 @@ __device__ __forceinline__ void motion_column(const float *img, int ix, int iy, 
 template <typename FT, typename VT, bool PAIR = false>
 static __global__ void __launch_bounds__(256) motion_prep_kernel(VT *img0, VT *ones,
                                                                  const float *img, Fields<FT> f,
-                                                                 int nx, int ny, int nz, float vd,
-                                                                 float fd) {
+                                                                 int nx, int ny, int nz, int nzp,
+                                                                 float vd, float fd) {
     __shared__ float sm[6][MP_Z][MP_T][MP_T + 1];
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int x0 = blockIdx.x * MP_T, y0 = blockIdx.y * MP_T, z0 = blockIdx.z * MP_Z;
@@ -397,7 +400,7 @@ static __global__ void __launch_bounds__(256) motion_prep_kernel(VT *img0, VT *o
 #pragma unroll
         for (int k = 0; k < MP_Z; k++) ft[c][k] = sm[c][k][tx][ty];
     motion_column(img, ix, iy, z0, nx, ny, nz, vd, fd, ft, a, b);
-    store_column<VT, PAIR>(img0, ones, ix + (int64_t)iy * nx, z0, nz, a, b);
+    store_column<VT, PAIR>(img0, ones, ix + (int64_t)iy * nx, z0, nz, nzp, a, b);
 }
 
 // Motion pass field update, AUMISART.cu:272-277 fused: with q = img_temp read
@@ -461,7 +464,7 @@ template <typename FT, typename VT, bool EARLY = false, bool PAIR = false, bool 
           bool PROVEN = false>
 static __global__ void __launch_bounds__(256) field_update_prep_kernel(
     FT *ax, FT *ay, FT *az, FT *bx, FT *by, FT *bz, const float *img_temp, const float *img,
-    int nx, int ny, int nz, float nvd, float nfd, VT *img0, VT *ones, float vd, float fd,
+    int nx, int ny, int nz, int nzp, float nvd, float nfd, VT *img0, VT *ones, float vd, float fd,
     const BPArgs bp) {
     __shared__ float sm[6][MP_Z][MP_T][MP_T + 1];
     __shared__ float rt[MP_Z][MP_T][MP_T + 1];
@@ -585,7 +588,7 @@ static __global__ void __launch_bounds__(256) field_update_prep_kernel(
 #pragma unroll
         for (int k = 0; k < MP_Z; k++) ft[c][k] = sm[c][k][tx][ty];
     motion_column(img, ix, iy, z0, nx, ny, nz, vd, fd, ft, a, b);
-    store_column<VT, PAIR>(img0, ones, ix + (int64_t)iy * nx, z0, nz, a, b);
+    store_column<VT, PAIR>(img0, ones, ix + (int64_t)iy * nx, z0, nz, nzp, a, b);
 }
 
 // Norm ratios ||r_v|| / ||b_v|| from per-block partials (fixed order); one

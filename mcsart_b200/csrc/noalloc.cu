@@ -126,12 +126,13 @@ MC_EXPORT int mcsart_projection_noalloc(void *stream, float *d_proj, const float
                "mcsart_projection_noalloc: the volume has %lld voxels, more than the %d its "
                "static scratch holds (use mcsart_projection)",
                (long long)n, MCSART_NOALLOC_MAX_VOXELS);
+    g.nzp = zf_pitch(nx, ny, nz, MCSART_NOALLOC_MAX_VOXELS);
     float *scratch = nullptr;
     MC_TRY(scratch_of_current_device(&scratch));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
 
     zfast_kernel<float, float><<<zfast_grid(nx, ny, nz), dim3(32, 8), 0, s>>>(scratch, d_img, nx,
-                                                                              ny, nz);
+                                                                              ny, nz, g.nzp);
     MC_CHECK_CUDA(cudaGetLastError());
     FPArgs<float, 1> a{};
     a.vol.zf[0] = scratch;

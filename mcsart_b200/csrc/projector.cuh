@@ -12,7 +12,7 @@
 //     race on a non-atomic +=), the 32 lanes of a warp being 32 consecutive
 //     detector rows of one detector column;
 //   * every volume is read through a z-fastest copy
-//     zf[iz + (ix + iy*nx)*nz]: a warp's rays meet each slab in the same one
+//     zf[iz + (ix + iy*nx)*nzp]: a warp's rays meet each slab in the same one
 //     or two in-plane voxel columns and in neighbouring slices, so one copy
 //     serves both driving axes, a ray's two axial voxels are neighbours in
 //     memory, and everything in-plane (weights, which columns are visited,
@@ -88,7 +88,7 @@ __device__ __forceinline__ RayGeom ray_geom(float cphi, float sphi, int ia, int 
     return r;
 }
 
-// z-fastest volumes: zf[k][iz + (ix + iy*nx)*nz]
+// z-fastest volumes: zf[k][iz + (ix + iy*nx)*nzp], zero for nz <= iz < nzp (zf_pitch)
 template <typename VT, int K> struct FPVolumes {
     const VT *zf[K];
 };
@@ -96,9 +96,9 @@ template <typename VT, int K> struct FPVolumes {
 // Distance in a z-fastest volume between in-plane neighbours along the
 // in-plane axis (su) and along the driving axis (sd) of a ray.
 __device__ __forceinline__ void zf_strides(bool xdrive, const Geom &g, int &su, int &sd) {
-    const int row = g.nx * g.nz;  // fits: volumes hold fewer than 2^31 voxels
-    su = xdrive ? row : g.nz;
-    sd = xdrive ? g.nz : row;
+    const int row = g.nx * g.nzp;  // fits: the copies hold fewer than 2^31 elements
+    su = xdrive ? row : g.nzp;
+    sd = xdrive ? g.nzp : row;
 }
 
 // The K volumes' values at voxel offset a into t[0..K-1]: one load per
@@ -373,16 +373,12 @@ __device__ __forceinline__ void ray_zrange(const RayGeom &r, float zh, int nz, i
 // warp's window in the first one's column of the z-fastest volume (the second
 // one's is su further) and the weights a, b (zero for a voxel not visited).
 // The window begins at slice zlo, the even one at or below the first ray's Z1;
-// slices lo .. hi of it (range = lo | hi << 8) are needed and in the volume.
-// pairs (for an even nz): bit l is set where slices 2l, 2l + 1 are, bit 16 + l
-// where they are and the second voxel is visited.
+// pairs: bit l is set where one of its slices 2l, 2l + 1 is needed and in the
+// volume (the other is too, or is the zero behind an odd depth), bit 16 + l
+// where moreover the second voxel is visited.
 struct __align__(8) SlabCopy {
     int o;
     unsigned pairs;
-};
-struct SlabRest {
-    int range;
-    int flags;  // SC_*
 };
 // The rest of two neighbouring slabs, side by side for the packed operations.
 struct __align__(16) SlabPair {
@@ -403,7 +399,7 @@ constexpr int FPW = 32;  // slices per window
 // last row; narrow: every ray of the warp is (ray_axial).
 __device__ __forceinline__ void slab_entry(const RayGeom &r, int d, int su, int sd, float rz_first,
                                            float rz_last, bool narrow, float z_half, int nz,
-                                           SlabCopy &c, SlabRest &t, float &a, float &b, float &dc,
+                                           SlabCopy &c, int &flags, float &a, float &b, float &dc,
                                            int &zb) {
     const SlabU e = slab_u(r, d);
     const bool two_wide = e.U2 - e.U1 <= 1;
@@ -414,7 +410,6 @@ __device__ __forceinline__ void slab_entry(const RayGeom &r, int d, int su, int 
             (two_wide && u0 && u1 ? SC_TWO : 0);
     dc = slab_dc(r, d);
     c.pairs = 0;
-    t.range = 1;  // none (lo > hi)
     int zlo = 0;
     if (narrow) {
         // cz0 as every ray computes it (:71 / :124); rows in order, so these
@@ -426,12 +421,11 @@ __device__ __forceinline__ void slab_entry(const RayGeom &r, int d, int su, int 
         if (lo > hi) f = 0;  // no ray meets a slice of the volume here
         if ((f & SC_FAST) && zl - zlo < FPW) {
             f |= SC_STAGE | (zf >= 0 && zl <= nz - 1 ? SC_IN : 0);
-            t.range = lo | hi << 8;
             c.pairs = (0xffffu >> (15 - (hi >> 1))) & (0xffffu << (lo >> 1));
             if (f & SC_TWO) c.pairs |= c.pairs << 16;
         }
     }
-    t.flags = f;
+    flags = f;
     const int U = u0 ? e.U1 : u1 ? e.U1 + 1 : 0;  // the first visited voxel
     c.o = U * su + d * sd + zlo;
     a = f & SC_FAST ? (u0 ? e.a : e.b) : 0.0f;
@@ -555,40 +549,20 @@ __device__ __forceinline__ void sts_zero4(unsigned a) {
 }
 
 // This lane's part of a slab's two windows at dst (shared memory), the second
-// one all zeros where the slab visits one in-plane voxel.  EVEN (an even nz, so
-// windows begin on even elements): slices 2j and 2j + 1 of window h as one
-// copy, lane = 16 h + j, lane_off and lane_dst that place in the volume and
-// the windows; otherwise slice `lane` of both.
-template <bool EVEN, typename VT, bool PAIR>
+// one all zeros where the slab visits one in-plane voxel: slices 2j and 2j + 1
+// of window h as one copy, lane = 16 h + j, lane_off and lane_dst that place in
+// the volume and the windows (which begin on even elements: the pitch is even).
+template <typename VT, bool PAIR>
 __device__ __forceinline__ void window_copy(unsigned dst, const VT *const *base, const int2 c,
-                                            const SlabRest &t, int su, int lane, int bit,
-                                            int64_t lane_off, unsigned lane_dst) {
+                                            int lane, int bit, int64_t lane_off,
+                                            unsigned lane_dst) {
     using W = FPWindow<VT, PAIR>;
     constexpr int ES = sizeof(VT);
-    if (EVEN) {
-        const bool in = c.y & bit;
-        cp_async<2 * ES>(dst + lane_dst, base[0] + lane_off + c.x, in);
-        if constexpr (PAIR)
-            cp_async<4 * ES>(dst + lane_dst + W::PAIRS + 2 * ES * (lane & 15),
-                             base[1] + 2 * (lane_off + c.x), in);
-        return;
-    }
-    const int lo = t.range & 255, hi = t.range >> 8;
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        const int64_t i = (int64_t)c.x + h * (int64_t)su + lane;
-        const unsigned w = dst + h * W::BYTES;
-        const bool in = lane >= lo && lane <= hi && (h == 0 || (t.flags & SC_TWO));
-        if constexpr (ES == 4) {
-            cp_async<4>(w + 4 * lane, base[0] + i, in);
-            if constexpr (PAIR) cp_async<8>(w + W::PAIRS + 8 * lane, base[1] + 2 * i, in);
-        } else {  // (2-byte elements: no such asynchronous copy)
-            const unsigned short v =
-                in ? *reinterpret_cast<const unsigned short *>(base[0] + i) : (unsigned short)0;
-            asm volatile("st.shared.b16 [%0], %1;" ::"r"(w + 2 * lane), "h"(v) : "memory");
-            if constexpr (PAIR) cp_async<4>(w + W::PAIRS + 4 * lane, base[1] + 2 * i, in);
-        }
-    }
+    const bool in = c.y & bit;
+    cp_async<2 * ES>(dst + lane_dst, base[0] + lane_off + c.x, in);
+    if constexpr (PAIR)
+        cp_async<4 * ES>(dst + lane_dst + W::PAIRS + 2 * ES * (lane & 15),
+                         base[1] + 2 * (lane_off + c.x), in);
 }
 
 // The K volumes' values of slice z of both windows of the slab at w.
@@ -726,7 +700,7 @@ __device__ __forceinline__ void fp_pair_staged(float rz0, float rz1, const SlabP
 template <typename VT, bool PAIR, int S, int NST> struct FPShared {
     SlabPair pairs[32];
     SlabCopy copy[64];
-    SlabRest rest[64];
+    int flags[64];  // SC_*
     uint4 mask[2];  // bit i: slab i of a table is SC_IN, SC_STAGE, neither staged nor empty
     RayGeom ray;
     float rz_last;
@@ -792,7 +766,7 @@ __global__ void __launch_bounds__(FPC_THREADS, MINB) fp_ref_kernel(const FPArgs<
                 const RayGeom r = ray_geom(cphi, sphi, ia, min(ib, g.nb - 1), g);
                 const RayAxial ax = ray_axial(r, z_half);
                 w_safe = __all_sync(0xffffffffu, ax.zsafe);
-                w_narrow = __all_sync(0xffffffffu, ax.narrow) && nz >= 2;
+                w_narrow = __all_sync(0xffffffffu, ax.narrow) && nz >= 2 && g.nzp % 2 == 0;
                 // the warp's slabs: those where some ray meets the volume
                 int lo, hi;
                 ray_zrange(r, z_half, nz, lo, hi);
@@ -815,7 +789,6 @@ __global__ void __launch_bounds__(FPC_THREADS, MINB) fp_ref_kernel(const FPArgs<
                 }
             }
             __syncwarp();
-            const bool even = nz % 2 == 0;
             const int bit = 1 << lane;
             int su_;
             {
@@ -839,23 +812,22 @@ __global__ void __launch_bounds__(FPC_THREADS, MINB) fp_ref_kernel(const FPArgs<
                         int su, sd;
                         zf_strides(rc.xdrive, g, su, sd);
                         SlabCopy c;
-                        SlabRest e;
+                        int f;
                         float a, b, dc;
                         int zb;
                         slab_entry(rc, wlo + min(i, n - 1), su, sd, rc.rz0, sm.rz_last, w_narrow,
-                                   z_half, nz, c, e, a, b, dc, zb);
+                                   z_half, nz, c, f, a, b, dc, zb);
                         if (i >= n) {
-                            e.flags = 0;
+                            f = 0;
                             c.pairs = 0;
-                            e.range = 1;
                             a = b = 0.0f;
                         }
-                        const unsigned in = __ballot_sync(0xffffffffu, (e.flags & SC_IN) != 0);
-                        const unsigned st = __ballot_sync(0xffffffffu, (e.flags & SC_STAGE) != 0);
+                        const unsigned in = __ballot_sync(0xffffffffu, (f & SC_IN) != 0);
+                        const unsigned st = __ballot_sync(0xffffffffu, (f & SC_STAGE) != 0);
                         const unsigned slow = __ballot_sync(
-                            0xffffffffu, (e.flags & (SC_ANY | SC_STAGE)) == SC_ANY);
+                            0xffffffffu, (f & (SC_ANY | SC_STAGE)) == SC_ANY);
                         sm.copy[i & 63] = c;
-                        sm.rest[i & 63] = e;
+                        sm.flags[i & 63] = f;
                         SlabPair &y = sm.pairs[(i & 63) >> 1];
                         y.a[i & 1] = a;
                         y.b[i & 1] = b;
@@ -865,21 +837,12 @@ __global__ void __launch_bounds__(FPC_THREADS, MINB) fp_ref_kernel(const FPArgs<
                         __syncwarp();
                     }
                     const SlabCopy *const c = sm.copy + (i0 & 63);
-                    const SlabRest *const e = sm.rest + (i0 & 63);
                     const unsigned dst = win0 + s % NST * (S * 2 * W::BYTES);
-                    if (even) {
 #pragma unroll
-                        for (int q = 0; q < S; q++)
-                            window_copy<true, VT, PAIR>(
-                                dst + q * 2 * W::BYTES, base, *reinterpret_cast<const int2 *>(c + q),
-                                e[q], su, lane, bit, lane_off, lane_dst);
-                    } else {
-#pragma unroll 1
-                        for (int q = 0; q < S; q++)
-                            window_copy<false, VT, PAIR>(
-                                dst + q * 2 * W::BYTES, base, *reinterpret_cast<const int2 *>(c + q),
-                                e[q], su, lane, bit, lane_off, lane_dst);
-                    }
+                    for (int q = 0; q < S; q++)
+                        window_copy<VT, PAIR>(dst + q * 2 * W::BYTES, base,
+                                              *reinterpret_cast<const int2 *>(c + q), lane, bit,
+                                              lane_off, lane_dst);
                 }
                 cp_async_commit();
             };
@@ -915,7 +878,7 @@ __global__ void __launch_bounds__(FPC_THREADS, MINB) fp_ref_kernel(const FPArgs<
                 } else {
 #pragma unroll 1
                     for (int q = 0; q < S; q++) {
-                        const int o = sm.copy[(i0 + q) & 63].o, f = sm.rest[(i0 + q) & 63].flags;
+                        const int o = sm.copy[(i0 + q) & 63].o, f = sm.flags[(i0 + q) & 63];
                         if (!(f & SC_ANY)) continue;
                         const SlabPair &yq = y[q / 2];
                         RayGeom rc = sm.ray;
@@ -945,12 +908,13 @@ __global__ void __launch_bounds__(FPC_THREADS, MINB) fp_ref_kernel(const FPArgs<
         // device code, so the same bits as computing it there; spread over
         // all threads of the view's blocks
         const float bs = __sinf(angle), bc = __cosf(angle);
-        const int64_t ncol = (int64_t)g.nx * g.ny;
+        const int64_t ncol = (int64_t)g.nx * g.ny;  // below 2^31
         const int64_t coff = MULTI ? (int64_t)blockIdx.z * ncol : 0;
         const int64_t nthr = (int64_t)gridDim.x * gridDim.y * FPC_THREADS;
         for (int64_t c = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * FPC_THREADS + t; c < ncol;
              c += nthr) {
-            const BPColumn col = bp_column<false>((int)(c % g.nx), (int)(c / g.nx), bc, bs, g);
+            const unsigned cu = (unsigned)c, cy = cu / (unsigned)g.nx, cx = cu - cy * (unsigned)g.nx;
+            const BPColumn col = bp_column<false>((int)cx, (int)cy, bc, bs, g);
             p.bpcolA[coff + c] = make_float4(col.amin, col.amax, col.rl, col.rr);
             p.bpcolB[coff + c] = col.r0;
         }

@@ -71,6 +71,7 @@ template <typename ST, int INTERP, int SUM> struct Runner {
     const Problem &P;
     const mcsart_options &opt;
     int64_t V = 0, NP = 0;
+    int64_t VZ = 0;  // elements of a z-fastest volume (Geom::nzp)
     int fp_bx = 0, fp_by = 0, fp_blocks = 0, groups = 1;
     int subset = 1;  // views per ordered subset in image passes
     int inv_iters = 0;  // fixed-point steps of the true DVF inverse (0: negated amplitudes)
@@ -83,6 +84,7 @@ template <typename ST, int INTERP, int SUM> struct Runner {
         : ctx(c), S(*c->driver), P(p), opt(o) {
         tune = c->tuning_override ? *c->tuning_override : tuning_for(c, p.g, o.storage);
         V = nvox(P.g.nx, P.g.ny, P.g.nz);
+        VZ = nvox(P.g.nx, P.g.ny, P.g.nzp);
         NP = (int64_t)P.g.na * P.g.nb;
         fp_bx = SUM == SUM_REF ? (int)div_up(P.g.na, FPC_COLS) : P.g.na;
         fp_by = (int)div_up(P.g.nb, SUM == SUM_REF ? FPC_ROWS : 32);
@@ -104,7 +106,7 @@ template <typename ST, int INTERP, int SUM> struct Runner {
     const ST *meas(int v) const { return (const ST *)P.proj + (int64_t)v * NP; }
 
     int alloc() {
-        const size_t vs = V * sizeof(ST), vf = V * sizeof(float);
+        const size_t vs = VZ * sizeof(ST), vf = V * sizeof(float);
         MC_TRY(S.img1.ensure(vs * subset));
         MC_TRY(S.imgS.ensure(vs));
         // img0 and the initial2 volume interleaved for the reference-order
@@ -112,7 +114,7 @@ template <typename ST, int INTERP, int SUM> struct Runner {
         MC_TRY(S.img0.ensure(2 * vs));
         MC_TRY(S.ones.ensure(vs));
         MC_TRY(S.ratio.ensure(vf * subset));
-        MC_TRY(S.imgZ.ensure(vf));
+        MC_TRY(S.imgZ.ensure(VZ * sizeof(float)));
         MC_TRY(S.pairs.ensure(NP * subset * sizeof(float2)));
         MC_TRY(S.bpcolA.ensure((size_t)P.g.nx * P.g.ny * subset * sizeof(float4)));
         MC_TRY(S.bpcolB.ensure((size_t)P.g.nx * P.g.ny * subset * sizeof(float)));
@@ -337,7 +339,7 @@ template <typename ST, int INTERP, int SUM> struct Runner {
     // A z-fastest copy for the projector.
     template <typename SRC_T, typename DST_T> int zfast(DST_T *dst, const SRC_T *src) {
         MC_LAUNCH(ctx, (zfast_kernel<SRC_T, DST_T>), zfast_grid(P.g.nx, P.g.ny, P.g.nz),
-                  dim3(32, 8), 0, dst, src, P.g.nx, P.g.ny, P.g.nz);
+                  dim3(32, 8), 0, dst, src, P.g.nx, P.g.ny, P.g.nz, P.g.nzp);
         return MCSART_OK;
     }
 
@@ -355,10 +357,10 @@ template <typename ST, int INTERP, int SUM> struct Runner {
         ctx->label = "warp_fwd";
         if (hw) {
             MC_LAUNCH(ctx, (warp_fwd_kernel<N, SrcTex, ST, ST, WR>), grid, block, 0, d,
-                      SrcTex{S.tv_img.tex}, f, g.nx, g.ny, g.nz, volume, flow);
+                      SrcTex{S.tv_img.tex}, f, g.nx, g.ny, g.nz, g.nzp, volume, flow);
         } else {
             MC_LAUNCH(ctx, (warp_fwd_kernel<N, SrcLinear<float>, ST, ST, WR>), grid, block, 0, d,
-                      SrcLinear<float>{P.img}, f, g.nx, g.ny, g.nz, volume, flow);
+                      SrcLinear<float>{P.img}, f, g.nx, g.ny, g.nz, g.nzp, volume, flow);
         }
         return MCSART_OK;
     }
@@ -473,11 +475,11 @@ template <typename ST, int INTERP, int SUM> struct Runner {
             const int v = v0 + j;
             const float volume = P.volumes[v] - P.volumes[0];
             const float flow = P.flows[v] - P.flows[0];
-            MC_TRY(warp_fwd(S.img1.as<ST>() + j * V, hw, volume, flow));
+            MC_TRY(warp_fwd(S.img1.as<ST>() + j * VZ, hw, volume, flow));
         }
         FPVolumes<ST, 1> vol{};
         vol.zf[0] = S.img1.as<ST>();
-        MC_TRY((launch_fp_subset<1, true, ST>(vol, v0, k0, kk, FP_IMAGE, V)));
+        MC_TRY((launch_fp_subset<1, true, ST>(vol, v0, k0, kk, FP_IMAGE, VZ)));
         cudaSurfaceObject_t surfs[BP_MAX_VIEWS] = {};
         for (int j = 0; j < kk; j++) surfs[j] = j == 0 ? S.tv_ratio.surf : S.tv_ratio_sub[j - 1].surf;
         if (hw)
@@ -550,7 +552,7 @@ template <typename ST, int INTERP, int SUM> struct Runner {
                 ctx->label = "motion_prep";
                 MC_LAUNCH(ctx, (motion_prep_kernel<ST, ST, pair>), motion_tiles(),
                           dim3(MP_T, MP_T), 0, img0, ones, (const float *)P.img, f, g.nx, g.ny,
-                          g.nz, vd, fd);
+                          g.nz, g.nzp, vd, fd);
             }
             MC_TRY((launch_fp<3, false, ST>(vol, v, k, FP_MOTION)));
             // square slices, FP32 geometry: the backprojection ratio is
@@ -571,26 +573,26 @@ template <typename ST, int INTERP, int SUM> struct Runner {
                     MC_LAUNCH(ctx, (field_update_prep_kernel<ST, ST, false, pair, true, true>),
                               motion_tiles(), dim3(MP_T, MP_T), 0, fw, fw + V, fw + 2 * V,
                               fw + 3 * V, fw + 4 * V, fw + 5 * V, (const float *)nullptr,
-                              (const float *)P.img, g.nx, g.ny, g.nz, nvd, nfd, img0, ones, vdn,
-                              fdn, b);
+                              (const float *)P.img, g.nx, g.ny, g.nz, g.nzp, nvd, nfd, img0, ones,
+                              vdn, fdn, b);
                 else if (fused_bp)
                     MC_LAUNCH(ctx, (field_update_prep_kernel<ST, ST, false, pair, true, false>),
                               motion_tiles(), dim3(MP_T, MP_T), 0, fw, fw + V, fw + 2 * V,
                               fw + 3 * V, fw + 4 * V, fw + 5 * V, (const float *)nullptr,
-                              (const float *)P.img, g.nx, g.ny, g.nz, nvd, nfd, img0, ones, vdn,
-                              fdn, b);
+                              (const float *)P.img, g.nx, g.ny, g.nz, g.nzp, nvd, nfd, img0, ones,
+                              vdn, fdn, b);
                 else if (tune.fup == 1)
                     MC_LAUNCH(ctx, (field_update_prep_kernel<ST, ST, true, pair>),
                               motion_tiles(), dim3(MP_T, MP_T), 0, fw, fw + V, fw + 2 * V,
                               fw + 3 * V, fw + 4 * V, fw + 5 * V, (const float *)S.ratio.as<float>(),
-                              (const float *)P.img, g.nx, g.ny, g.nz, nvd, nfd, img0, ones, vdn,
-                              fdn, b);
+                              (const float *)P.img, g.nx, g.ny, g.nz, g.nzp, nvd, nfd, img0, ones,
+                              vdn, fdn, b);
                 else
                     MC_LAUNCH(ctx, (field_update_prep_kernel<ST, ST, false, pair>),
                               motion_tiles(), dim3(MP_T, MP_T), 0, fw, fw + V, fw + 2 * V,
                               fw + 3 * V, fw + 4 * V, fw + 5 * V, (const float *)S.ratio.as<float>(),
-                              (const float *)P.img, g.nx, g.ny, g.nz, nvd, nfd, img0, ones, vdn,
-                              fdn, b);
+                              (const float *)P.img, g.nx, g.ny, g.nz, g.nzp, nvd, nfd, img0, ones,
+                              vdn, fdn, b);
             } else {
                 ctx->label = "field_update";
                 MC_LAUNCH(ctx, (field_update_kernel<ST>), tile_grid(), dim3(32, 8), 0, fw, fw + V,
@@ -775,6 +777,7 @@ static int prepare_problem(mcsart_ctx *ctx, const mcsart_problem *prob, const mc
     g.SO = prob->SO; g.SD = prob->SD; g.da = prob->da; g.ai = prob->ai; g.db = prob->db;
     g.bi = prob->bi; g.na = prob->na; g.nb = prob->nb; g.nx = prob->nx; g.ny = prob->ny;
     g.nz = prob->nz;
+    g.nzp = zf_pitch(g.nx, g.ny, g.nz);
     MC_TRY(validate_geom(g));
     MC_REQUIRE(prob->n_views > 0, "n_views must be positive");
     MC_REQUIRE(prob->h_angles && prob->h_volumes && prob->h_flows,
@@ -909,6 +912,7 @@ static int aumisart_host(mcsart_ctx *ctx, float *h_outimg, float *h_outproj, flo
     Geom g;
     g.SO = SO; g.SD = SD; g.da = da; g.ai = ai; g.db = db; g.bi = bi;
     g.na = na; g.nb = nb; g.nx = nx; g.ny = ny; g.nz = nz;
+    g.nzp = zf_pitch(nx, ny, nz);
     MC_TRY(validate_geom(g));
     MC_TRY(validate_iter(n_views, n_iter, op_iter, angles, volumes, flows));
     MC_REQUIRE(h_outimg && h_outproj && h_outnorm && h_out_fields[0] && h_img && h_proj,

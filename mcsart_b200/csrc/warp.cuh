@@ -284,14 +284,14 @@ __device__ __forceinline__ void prefetch_xz_rows(const Fields<FT> &f, int TZ, in
 }
 
 // SART image pass, forward warp of the current volume into the view's phase,
-// z-fastest for the projector: dst[iz + (x + y*nx)*nz] = warp(src) at memory
+// z-fastest for the projector: dst[iz + (x + y*nx)*nzp] = warp(src) at memory
 // position x + y*nx + iz*nx*ny, stored in VT.
 // blockDim (32, 8); a block covers a 32 * N x (8 * WR) (x, z) tile of row y,
 // gridDim (ceil(nx/(32*N)) * ny, ceil(nz/(8*WR))).
 template <int N, typename SRC, typename FT, typename VT, int WR = WARP_ROWS>
 static __global__ void __launch_bounds__(256) warp_fwd_kernel(VT *dst, const SRC src, Fields<FT> f,
-                                                              int nx, int ny, int nz, float volume,
-                                                              float flow) {
+                                                              int nx, int ny, int nz, int nzp,
+                                                              float volume, float flow) {
     constexpr int TZ = 8 * WR, TX = 32 * N;
     // column c of a row at place(c): with N = 4, 33 apart, so that the lanes'
     // stores of column i, and the turned reads, fall on different banks
@@ -320,8 +320,9 @@ static __global__ void __launch_bounds__(256) warp_fwd_kernel(VT *dst, const SRC
 #pragma unroll
     for (int k = 0; k < WR * N; k++) {
         const int e = t + 256 * k, lx = e / TZ, lz = e % TZ;
-        if (x0 + lx < nx && z0 + lz < nz)
-            dst[z0 + lz + (row + x0 + lx) * nz] = cvt<VT>(tile[lz][place(lx)]);
+        if (x0 + lx < nx && z0 + lz < nzp)
+            dst[z0 + lz + (row + x0 + lx) * nzp] =
+                cvt<VT>(z0 + lz < nz ? tile[lz][place(lx)] : 0.0f);
     }
 }
 template <int N, int WR> inline dim3 warp_fwd_grid(int nx, int ny, int nz) {
