@@ -160,10 +160,10 @@ def algorithmic_bytes(p) -> dict:
         "bp_div": 8 * P + 4 * V,
         # the same in the DVF pass when it runs as its own launch
         "bp_div_motion": 8 * P + 4 * V,
-        # read volume (+ its update), write volume and its y-fastest copy
+        # read volume (+ its update), write volume and its z-fastest copy
         "bp_div_add": 8 * P + 12 * V,
-        # read img, 6 fields; write the warped volume in the layout the
-        # view's projector reads (x- or y-fastest)
+        # read img, 6 fields; write the warped volume, z-fastest for the
+        # view's projector
         "warp_fwd": 4 * V + 24 * V + 4 * V,
         # read ratio, 6 fields, img; write img and (texture model, the
         # default) its 3D-array copy
@@ -378,7 +378,7 @@ def run_kernel_case(args, ctx, torch, stream):
            g["ny"], g["nz"])
     fields = ([torch.rand(shape, device="cuda", generator=gen) * 4 - 2 for _ in range(6)]
               if args.kernel_case == "warp" else None)
-    angle = 0.3  # rays driven along x: the projector reads the volume's y-fastest copy
+    angle = 0.3  # rays driven along x
 
     def call():
         if args.kernel_case == "fp":
@@ -407,7 +407,7 @@ def run_kernel_case(args, ctx, torch, stream):
                       "ms_min": float(np.min(ms)),
                       "algorithmic_bytes": abytes[args.kernel_case],
                       "note": "each call is one C-ABI call (the projector's includes the "
-                              "y-fastest copy of the volume for x-driven rays)"}), flush=True)
+                              "z-fastest copy of the volume)"}), flush=True)
 
 
 def run_batch_config(args, ctx, torch, stream, m, rank, world):

@@ -14,9 +14,10 @@
 //
 // Restructured for the hardware: one thread per column of BP_NZ voxels (no
 // atomics, so runs are bitwise reproducible), 32-wide rows of voxels per warp
-// for coalesced stores and a shared-memory transpose when the y-fastest copy
-// of the volume must be kept current; two projections (SART residual and ones-projection, packed as
-// float2) are gathered with one set of weights and the SART division
+// for coalesced stores and a shared-memory transpose when the z-fastest copy
+// of the volume must be kept current (bp_kernel), or, for one projection of a
+// large volume, warps along z (bp_slice_kernel); two projections (SART residual
+// and ones-projection, packed as float2) are gathered with one set of weights and the SART division
 // (src/cu_division.cu:20-24) and update (src/cu_add.cu:17) run in the epilogue.
 #pragma once
 

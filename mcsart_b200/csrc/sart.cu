@@ -857,7 +857,6 @@ MC_EXPORT int mcsart_batch_run(mcsart_ctx *ctx, const mcsart_problem *problems,
     while ((int)ctx->lanes.size() < n_problems) {
         std::unique_ptr<mcsart_ctx> lane(new mcsart_ctx());
         lane->device = ctx->device;
-        lane->sms = ctx->sms;
         MC_CHECK_CUDA(cudaStreamCreateWithFlags(&lane->own_stream, cudaStreamNonBlocking));
         lane->stream = lane->own_stream;
         cudaEvent_t done;

@@ -32,8 +32,8 @@ namespace mcsart {
 //                               0: (8, 2, 6)  1: (8, 2, 7)  2: (8, 2, 5)  3: (4, 2, 8)
 //                               4: (8, 3, 5)
 //   fp3  three-volume projector 0: (4, 2, 5)  1: (4, 2, 6)  2: (4, 2, 4)  3: (2, 2, 6)
-//   bp   backprojector          0: 2 voxels/thread, 4 threads along z   1: 1 voxel, 4
-//                               2: 2 voxels, 8                          3: 4 voxels, 4
+//   bp   backprojector          0: 2 voxels per thread along z, blocks of 4 rows (static
+//                               update: 4 threads along z)   1: 1 voxel, 4   2: 2, 8   3: 4, 4
 //   warp image-pass warps       0: 2 rows (slices) per thread  1: 1  2: 4
 //   fup  DVF-pass field update  0: with the backprojection ratio computed in it
 //                               (square slices, FP32 geometry; else as 2)

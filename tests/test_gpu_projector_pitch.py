@@ -5,10 +5,12 @@ mcsart_projection_noalloc's scratch) must project to the same bits."""
 import numpy as np
 import pytest
 
-from conftest import dev, geo, host, volume
+from conftest import dev, geo, host, rel_l2, volume
 from test_gpu_sart import make_case
 
 pytestmark = pytest.mark.gpu
+
+ARGS = ("SO", "SD", "da", "na", "ai", "db", "nb", "bi", "nx", "ny", "nz")
 
 
 def _run(m, torch, ctx, case, **opt):
@@ -46,7 +48,7 @@ def test_copy_without_the_added_slice_projects_to_the_same_bits(ctx, torch_cuda)
     import mcsart_b200 as m
     torch = torch_cuda
     g = geo(nx=568, ny=567, nz=13, na=70, nb=33, SO=1700.0, SD=2550.0, da=12.0, db=0.9)
-    a = [g[k] for k in ("SO", "SD", "da", "na", "ai", "db", "nb", "bi", "nx", "ny", "nz")]
+    a = [g[k] for k in ARGS]
     n = g["nx"] * g["ny"]
     assert n * 13 <= 4194304 < n * 14  # MCSART_NOALLOC_MAX_VOXELS
     img = dev(torch, volume((13, 567, 568), seed=6))
@@ -58,3 +60,18 @@ def test_copy_without_the_added_slice_projects_to_the_same_bits(ctx, torch_cuda)
         torch.cuda.synchronize()
         assert host(outs[0]).any()
         np.testing.assert_array_equal(host(outs[0]), host(outs[1]))
+
+
+@pytest.mark.parametrize("nz", [63, 65, 128, 129])
+def test_depths_around_the_copy_s_tile_match_the_oracle(ctx, torch_cuda, oracle, nz):
+    """The copy turns 32 columns by 64 slices at a time (1e-5 relative L2: the
+    bound of the parity tests)."""
+    torch = torch_cuda
+    g = geo(nx=33, ny=5, nz=nz, na=20, nb=150, SO=120.0, SD=180.0, da=3.0, db=1.7)
+    img = volume((nz, 5, 33), seed=nz)
+    out = torch.full((g["nb"], g["na"]), 7.0, device="cuda")
+    for a in (0.3, 1.5):
+        ctx.host_projection(out, dev(torch, img), a, *[g[k] for k in ARGS])
+        ctx.synchronize()
+        o = oracle.projection(img, a, g)
+        assert np.linalg.norm(o) > 0 and rel_l2(host(out), o) <= 1e-5, (a, rel_l2(host(out), o))
