@@ -114,6 +114,24 @@ MC_EXPORT int mcsart_projection_views(mcsart_ctx *ctx, float *d_proj, const floa
     return finish(ctx, "mcsart_projection_views");
 }
 
+// Scratch of the slice-lane backprojector, or none where there is no memory for
+// it or the stream is being captured (a graph must not keep an address that a
+// later call may give back): bp_kernel needs none.
+static int bp_cells_workspace(mcsart_ctx *ctx, const Geom &g, float **cells) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    MC_CHECK_CUDA(cudaStreamIsCapturing(ctx->stream, &capture));
+    if (capture != cudaStreamCaptureStatusNone) return MCSART_OK;
+    void *ws = nullptr;
+    const int rc = workspace(ctx, "bp_cells", bp_cells(g.na, g.nb) * sizeof(float), &ws);
+    if (rc == MCSART_ERR_OUT_OF_MEMORY) {
+        (void)cudaGetLastError();
+        clear_error();
+        return MCSART_OK;
+    }
+    *cells = (float *)ws;
+    return rc;
+}
+
 MC_EXPORT int mcsart_backprojection(mcsart_ctx *ctx, float *d_img, const float *d_proj,
                                     float angle, float SO, float SD, float da, int na, float ai,
                                     float db, int nb, float bi, int nx, int ny, int nz) {
@@ -123,10 +141,9 @@ MC_EXPORT int mcsart_backprojection(mcsart_ctx *ctx, float *d_img, const float *
     const Geom g = make_geom(SO, SD, da, na, ai, db, nb, bi, nx, ny, nz);
     MC_TRY(validate_geom(g));
     const bool proven = bp_geom_proven(g);
-    if (nvox(nx, ny, nz) >= BP_SLICE_LANES_MIN) {
-        void *ws;
-        MC_TRY(workspace(ctx, "bp_cells", bp_cells(na, nb) * sizeof(float), &ws));
-        float *cells = (float *)ws;
+    float *cells = nullptr;
+    if (nvox(nx, ny, nz) >= BP_SLICE_LANES_MIN) MC_TRY(bp_cells_workspace(ctx, g, &cells));
+    if (cells != nullptr) {
         MC_LAUNCH(ctx, bp_cells_kernel, dim3(div_up(na, 32), div_up(nb, 32)), dim3(32, 8), 0, cells,
                   d_proj, na, nb);
         // 16 slices per tile where the last 32 would be at most half full

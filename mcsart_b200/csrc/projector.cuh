@@ -128,7 +128,7 @@ enum SumMode { SUM_REF = 0, SUM_PLAIN = 1, SUM_KAHAN = 2 };
 
 // ------------------------------------------------------------------------
 // FP64 geometry (options.geom64, with the split summation modes): the same
-// footprint formulas as ray_geom / ray_slabs (src/cu_projection.cu:23-144),
+// footprint formulas as ray_geom / slab_u (src/cu_projection.cu:23-144),
 // every boundary coordinate and overlap weight in FP64; the volume terms
 // v * w are accumulated in FP32 (plainly or Kahan-compensated), the weight
 // sum (the projection of a ones-volume, the SART row normaliser) in FP64.

@@ -52,3 +52,27 @@ def test_larger_volume_matches_the_oracle(ctx, torch_cuda, oracle):
     proj = np.random.default_rng(3).random((70, 80), dtype=np.float32)
     for a in (0.3, 2.4):
         assert rel_l2(_bp(ctx, torch, proj, a, g), oracle.backprojection(proj, a, g)) <= 1e-4
+
+
+def test_capture_on_a_new_context_needs_no_scratch(torch_cuda):
+    """A captured call takes bp_kernel, which keeps no workspace: the same bits."""
+    import mcsart_b200 as m
+    torch = torch_cuda
+    g = geo(nx=128, ny=128, nz=128, na=80, nb=70, SO=300.0, SD=450.0, da=2.9, db=2.9)
+    proj = dev(torch, np.random.default_rng(4).random((70, 80), dtype=np.float32))
+    eager, captured = (torch.full((128, 128, 128), 7.0, device="cuda") for _ in range(2))
+    s = torch.cuda.Stream()
+    ctx = m.Context(stream=s)
+    # (a smaller volume first, so that the kernel's code is loaded)
+    small = torch.empty((8, 128, 128), device="cuda")
+    torch.cuda.synchronize()
+    ctx.host_backprojection(small, proj, 0.3, *_args(dict(g, nz=8)))
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s):
+        ctx.host_backprojection(captured, proj, 0.3, *_args(g))
+    ctx.host_backprojection(eager, proj, 0.3, *_args(g))
+    ctx.synchronize()
+    graph.replay()
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(host(captured), host(eager))
