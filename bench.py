@@ -183,20 +183,20 @@ def algorithmic_bytes(p) -> dict:
     }
 
 
-# DRAM bytes per launch of the workload's kernels (dram__bytes.sum.per_second
-# x gpu__time_duration.sum), from one ncu capture of each in the benchmark
-# step (cold cache, FP32 storage, built-in launch shapes); summaries with the
+# DRAM bytes per launch of the workload's kernels (dram__bytes_read.sum +
+# dram__bytes_write.sum), from one ncu capture of each in a loop of the same
+# problem over three views (cold cache, FP32 storage, built-in launch shapes); summaries with the
 # commands are kept under profiles/.
 NCU_DRAM_BYTES = {
-    "motion256": {"fp_motion": 132078080, "fp_image": 42956032, "bp_div": 2872064,
-                  "field_update_prep": 613819647, "bp_field_update_prep": 573643608},
+    "motion256": {"fp_motion": 140513792, "fp_image": 42095104, "bp_div": 2864640,
+                  "field_update_prep": 613819647, "bp_field_update_prep": 581573632},
 }
 
 # Issue-slot utilisation (smsp__issue_active) of the projector and
 # backprojector from the same captures: these kernels are bound by issue and
 # latency, not by HBM.
-NCU_ISSUE_ACTIVE = {"motion256": {"fp_image": 0.570, "fp_motion": 0.602, "bp_div": 0.817,
-                                  "bp_field_update_prep": 0.663}}
+NCU_ISSUE_ACTIVE = {"motion256": {"fp_image": 0.729, "fp_motion": 0.692, "bp_div": 0.821,
+                                  "bp_field_update_prep": 0.628}}
 
 # Views per pass of the CPU samples: the engine line's cpu_baseline leg
 # (about 10 s of CPU work) and each step of the reference arm (a few seconds,
