@@ -36,7 +36,17 @@ int validate_ctx(mcsart_ctx *ctx) {
     return MCSART_OK;
 }
 
+static bool capturing(cudaStream_t stream) {
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(stream, &s) != cudaSuccess || s != cudaStreamCaptureStatusNone;
+}
+
 int workspace(mcsart_ctx *ctx, const char *name, size_t bytes, void **out) {
+    if (ctx->scratch_pending && ctx->scratch_stream != ctx->stream && !capturing(ctx->stream)) {
+        MC_CHECK_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->scratch_done, 0));
+        ctx->scratch_stream = ctx->stream;
+    }
+    ctx->scratch_used = true;
     auto &b = ctx->ws[name];
     if (b.bytes < bytes) {
         if (b.ptr) {
@@ -58,6 +68,14 @@ int workspace(mcsart_ctx *ctx, const char *name, size_t bytes, void **out) {
 }
 
 int finish(mcsart_ctx *ctx, const char *what) {
+    if (ctx->scratch_used && !capturing(ctx->stream)) {
+        if (!ctx->scratch_done)
+            MC_CHECK_CUDA(cudaEventCreateWithFlags(&ctx->scratch_done, cudaEventDisableTiming));
+        MC_CHECK_CUDA(cudaEventRecord(ctx->scratch_done, ctx->stream));
+        ctx->scratch_stream = ctx->stream;
+        ctx->scratch_pending = true;
+    }
+    ctx->scratch_used = false;
     if (ctx->synchronous) {
         const cudaError_t e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) {
@@ -194,6 +212,7 @@ mcsart_ctx::~mcsart_ctx() {
     lanes.clear();
     for (auto e : lane_done) cudaEventDestroy(e);
     if (batch_start) cudaEventDestroy(batch_start);
+    if (scratch_done) cudaEventDestroy(scratch_done);
     for (auto &r : prof_pending) {
         cudaEventDestroy(r.e0);
         cudaEventDestroy(r.e1);
