@@ -40,14 +40,30 @@ int launch_fp_plain(mcsart_ctx *ctx, float *d_proj, const float *d_imgZ, float a
     return launch_fp_ref<K, false, float>(ctx, grid, a);
 }
 
-// The z-fastest copy of a volume the projector reads, in a workspace.
+// The z-fastest copy of a volume the projector reads, in a workspace; in a
+// captured call in memory of the graph's own (*owned, given back by zfast_free
+// behind the projector), so that the graph keeps no address that a later call
+// may give back and a first call can be captured.
 template <typename VT>
-int zfast_copy(mcsart_ctx *ctx, const char *name, const VT *src, const Geom &g, const VT **out) {
+int zfast_copy(mcsart_ctx *ctx, const char *name, const VT *src, const Geom &g, const VT **out,
+               void **owned) {
+    const size_t bytes = nvox(g.nx, g.ny, g.nzp) * sizeof(VT);
     void *ws;
-    MC_TRY(workspace(ctx, name, nvox(g.nx, g.ny, g.nzp) * sizeof(VT), &ws));
+    *owned = nullptr;
+    if (capturing(ctx->stream)) {
+        MC_CHECK_CUDA(cudaMallocAsync(&ws, bytes, ctx->stream));
+        *owned = ws;
+    } else {
+        MC_TRY(workspace(ctx, name, bytes, &ws));
+    }
     MC_LAUNCH(ctx, (zfast_kernel<VT, VT>), zfast_grid(g.nx, g.ny, g.nz), dim3(32, 8), 0, (VT *)ws,
               src, g.nx, g.ny, g.nz, g.nzp);
     *out = (const VT *)ws;
+    return MCSART_OK;
+}
+
+int zfast_free(mcsart_ctx *ctx, void *owned) {
+    if (owned) MC_CHECK_CUDA(cudaFreeAsync(owned, ctx->stream));
     return MCSART_OK;
 }
 
@@ -87,8 +103,10 @@ MC_EXPORT int mcsart_projection(mcsart_ctx *ctx, float *d_proj, const float *d_i
     const Geom g = make_geom(SO, SD, da, na, ai, db, nb, bi, nx, ny, nz);
     MC_TRY(validate_geom(g));
     const float *imgZ;
-    MC_TRY(zfast_copy(ctx, "fp_volZ", d_img, g, &imgZ));
+    void *owned;
+    MC_TRY(zfast_copy(ctx, "fp_volZ", d_img, g, &imgZ, &owned));
     MC_TRY(launch_fp_plain<1>(ctx, d_proj, imgZ, angle, nullptr, 1, g));
+    MC_TRY(zfast_free(ctx, owned));
     return finish(ctx, "mcsart_projection");
 }
 
@@ -107,8 +125,10 @@ MC_EXPORT int mcsart_projection_views(mcsart_ctx *ctx, float *d_proj, const floa
     MC_TRY(workspace(ctx, "fp_angles", (size_t)n_views * sizeof(float), &wsA));
     MC_CHECK_CUDA(cudaMemcpyAsync(wsA, h_angles, (size_t)n_views * sizeof(float),
                                   cudaMemcpyHostToDevice, ctx->stream));
-    MC_TRY(zfast_copy(ctx, "fp_volZ", d_img, g, &imgZ));
+    void *owned;
+    MC_TRY(zfast_copy(ctx, "fp_volZ", d_img, g, &imgZ, &owned));
     MC_TRY(launch_fp_plain<1>(ctx, d_proj, imgZ, 0.0f, (const float *)wsA, n_views, g));
+    MC_TRY(zfast_free(ctx, owned));
     // the angle staging buffer must outlive the launch before the host array is reused
     MC_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
     return finish(ctx, "mcsart_projection_views");
@@ -118,9 +138,7 @@ MC_EXPORT int mcsart_projection_views(mcsart_ctx *ctx, float *d_proj, const floa
 // it or the stream is being captured (a graph must not keep an address that a
 // later call may give back): bp_kernel needs none.
 static int bp_cells_workspace(mcsart_ctx *ctx, const Geom &g, float **cells) {
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    MC_CHECK_CUDA(cudaStreamIsCapturing(ctx->stream, &capture));
-    if (capture != cudaStreamCaptureStatusNone) return MCSART_OK;
+    if (capturing(ctx->stream)) return MCSART_OK;
     void *ws = nullptr;
     const int rc = workspace(ctx, "bp_cells", bp_cells(g.na, g.nb) * sizeof(float), &ws);
     if (rc == MCSART_ERR_OUT_OF_MEMORY) {
@@ -417,10 +435,10 @@ MC_EXPORT int mcsart_snrm2(mcsart_ctx *ctx, int n, const float *d_x, float *h_re
 namespace {
 
 template <typename VT>
-int projection_ex_typed(mcsart_ctx *ctx, float *d_proj, const VT *d_img, int fp_sum, int geom64,
-                        float angle, const Geom &g) {
+int projection_ex_launch(mcsart_ctx *ctx, float *d_proj, const VT *zf, int fp_sum, int geom64,
+                         float angle, const Geom &g) {
     FPArgs<VT, 1, VT> a{};
-    MC_TRY(zfast_copy(ctx, "fp_volZ_ex", d_img, g, &a.vol.zf[0]));
+    a.vol.zf[0] = zf;
     a.g = g;
     a.angle = angle;
     a.mode = FP_PLAIN;
@@ -442,6 +460,16 @@ int projection_ex_typed(mcsart_ctx *ctx, float *d_proj, const VT *d_img, int fp_
     else
         MC_LAUNCH(ctx, (fp_kernel<1, false, SUM_KAHAN, VT, VT>), grid, block, smem, a);
     return MCSART_OK;
+}
+
+template <typename VT>
+int projection_ex_typed(mcsart_ctx *ctx, float *d_proj, const VT *d_img, int fp_sum, int geom64,
+                        float angle, const Geom &g) {
+    const VT *zf;
+    void *owned;
+    MC_TRY(zfast_copy(ctx, "fp_volZ_ex", d_img, g, &zf, &owned));
+    MC_TRY(projection_ex_launch(ctx, d_proj, zf, fp_sum, geom64, angle, g));
+    return zfast_free(ctx, owned);
 }
 
 template <typename FT>

@@ -36,7 +36,7 @@ int validate_ctx(mcsart_ctx *ctx) {
     return MCSART_OK;
 }
 
-static bool capturing(cudaStream_t stream) {
+bool capturing(cudaStream_t stream) {
     cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
     return cudaStreamIsCapturing(stream, &s) != cudaSuccess || s != cudaStreamCaptureStatusNone;
 }
