@@ -527,8 +527,13 @@ template <typename VT, bool PAIR> struct FPWindow {
     static constexpr unsigned BYTES = PAIRS + (PAIR ? 2 * FPW * ES + 16 : 0);
 };
 
-// An N-byte asynchronous copy, or N zeros where !in (nothing is read then).
+// An N-byte asynchronous copy, or N zeros where !in (nothing is read then); both
+// addresses on N bytes either way.
+#ifndef MCSART_ON_COPY
+#define MCSART_ON_COPY(dst, src, n)  // a test program's check of the addresses
+#endif
 template <int N> __device__ __forceinline__ void cp_async(unsigned dst, const void *src, bool in) {
+    MCSART_ON_COPY(dst, src, N);
     const int n = in ? N : 0;
     if (N == 16)
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n)
@@ -836,13 +841,17 @@ __global__ void __launch_bounds__(FPC_THREADS, MINB) fp_ref_kernel(const FPArgs<
                         if (lane == 0) sm.mask[(i0 >> 5) & 1] = make_uint4(in, st, slow, 0);
                         __syncwarp();
                     }
-                    const SlabCopy *const c = sm.copy + (i0 & 63);
-                    const unsigned dst = win0 + s % NST * (S * 2 * W::BYTES);
+                    // no window of a warp that is not narrow is read (SC_STAGE), and
+                    // at an odd pitch its copies would not be aligned
+                    if (w_narrow) {
+                        const SlabCopy *const c = sm.copy + (i0 & 63);
+                        const unsigned dst = win0 + s % NST * (S * 2 * W::BYTES);
 #pragma unroll
-                    for (int q = 0; q < S; q++)
-                        window_copy<VT, PAIR>(dst + q * 2 * W::BYTES, base,
-                                              *reinterpret_cast<const int2 *>(c + q), lane, bit,
-                                              lane_off, lane_dst);
+                        for (int q = 0; q < S; q++)
+                            window_copy<VT, PAIR>(dst + q * 2 * W::BYTES, base,
+                                                  *reinterpret_cast<const int2 *>(c + q), lane,
+                                                  bit, lane_off, lane_dst);
+                    }
                 }
                 cp_async_commit();
             };
