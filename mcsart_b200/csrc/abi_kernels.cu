@@ -312,8 +312,13 @@ MC_EXPORT int mcsart_add2(mcsart_ctx *ctx, float *img1, const float *img, int nx
     MC_TRY(validate_dims(nx, ny, nz));
     MC_REQUIRE(img1 && img && img0, "pointers must be non-NULL");
     MC_REQUIRE(ind >= 1 && ind <= 3, "ind must be 1, 2 or 3 (got %d)", ind);
-    MC_LAUNCH(ctx, add2_kernel, stencil_grid(nx, ny, nz), dim3(32, 8), 0, img1, img, nx, ny, nz,
-              img0, weight, ind);
+    const Grid3 g(nx, ny, nz);
+    if (nx >= ADD2_TILE_MIN && ny >= ADD2_TILE_MIN && g.n > ADD2_ROWS_MAX) {
+        MC_LAUNCH(ctx, add2_kernel, add2_grid(nx, ny, nz), dim3(32, 8), 0, img1, img, nx, ny, nz,
+                  img0, weight, ind);
+    } else {
+        MC_TRY(launch_stencil(ctx, "add2_kernel", g, Add2Op{img1, img, img0, weight, ind}));
+    }
     return finish(ctx, "mcsart_add2");
 }
 
@@ -335,8 +340,7 @@ MC_EXPORT int mcsart_initial2(mcsart_ctx *ctx, float *img, int nx, int ny, int n
     MC_TRY(validate_ctx(ctx));
     MC_TRY(validate_dims(nx, ny, nz));
     MC_REQUIRE(img && img0, "pointers must be non-NULL");
-    MC_LAUNCH(ctx, initial2_kernel, stencil_grid(nx, ny, nz), dim3(32, 8), 0, img, nx, ny, nz, img0,
-              volume, flow);
+    MC_TRY(launch_stencil(ctx, "initial2_kernel", Grid3(nx, ny, nz), Initial2Op{img, img0, volume + flow}));
     return finish(ctx, "mcsart_initial2");
 }
 
@@ -360,8 +364,7 @@ MC_EXPORT int mcsart_multiple(mcsart_ctx *ctx, float *img1, int nx, int ny, int 
     MC_TRY(validate_dims(nx, ny, nz));
     MC_REQUIRE(img1 && img0, "pointers must be non-NULL");
     MC_REQUIRE(ind >= 1 && ind <= 3, "ind must be 1, 2 or 3 (got %d)", ind);
-    MC_LAUNCH(ctx, multiple_kernel, stencil_grid(nx, ny, nz), dim3(32, 8), 0, img1, nx, ny, nz,
-              img0, weight, ind);
+    MC_TRY(launch_stencil(ctx, "multiple_kernel", Grid3(nx, ny, nz), MultipleOp{img1, img0, weight, ind}));
     return finish(ctx, "mcsart_multiple");
 }
 
@@ -374,8 +377,9 @@ MC_EXPORT int mcsart_update_udvf(mcsart_ctx *ctx, float *ax, float *ay, float *a
     MC_TRY(validate_ctx(ctx));
     MC_TRY(validate_dims(nx, ny, nz));
     MC_REQUIRE(ax && ay && az && bx && by && bz && img && img0, "pointers must be non-NULL");
-    MC_LAUNCH(ctx, update_udvf_kernel, stencil_grid(nx, ny, nz), dim3(32, 8), 0, ax, ay, az, bx, by,
-              bz, img, img0, volume_diff, flow_diff, nx, ny, nz);
+    const Grid3 g(nx, ny, nz);
+    MC_LAUNCH(ctx, update_udvf_kernel, stream_blocks(g.n), 256, 0, g, ax, ay, az, bx, by, bz, img, img0,
+              volume_diff, flow_diff);
     return finish(ctx, "mcsart_update_udvf");
 }
 
@@ -386,8 +390,7 @@ MC_EXPORT int mcsart_diff(mcsart_ctx *ctx, float *img1, const float *img, int nx
     MC_TRY(validate_dims(nx, ny, nz));
     MC_REQUIRE(img1 && img, "pointers must be non-NULL");
     MC_REQUIRE(ind >= 1 && ind <= 3, "ind must be 1, 2 or 3 (got %d)", ind);
-    MC_LAUNCH(ctx, diff_kernel, stencil_grid(nx, ny, nz), dim3(32, 8), 0, img1, img, nx, ny, nz,
-              ind);
+    MC_TRY(launch_stencil(ctx, "diff_kernel", Grid3(nx, ny, nz), DiffOp{img1, img, ind}));
     return finish(ctx, "mcsart_diff");
 }
 

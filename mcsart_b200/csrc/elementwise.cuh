@@ -54,21 +54,68 @@ __device__ __forceinline__ float fwd_diff(const T *img0, int64_t id, const Vox &
     }
 }
 
-// The stencil kernels (bound by memory): blockDim (32, 8), 32 x 32 (x, y)
-// tiles of one slice, four voxels per thread; the grid (stencil_grid) covers
-// the tiles of a slice and as many slices as a grid may, and a block goes on
-// through the rest.  No voxel's coordinates are divided out of its index, whose
-// 64-bit divisions took much of the time of a one-dimensional grid (at
-// 201x173x97: initial2 21 against 13 us, add2, which also read a field across
-// its rows, 25 against 18.5, event time of a few us included).
-#define MC_STENCIL_TILES(nx, ny, nz)                                                           \
-    for (int iz = blockIdx.z; iz < (nz); iz += gridDim.z)                                      \
-        for (int y0 = blockIdx.y * 32; y0 < (ny); y0 += gridDim.y * 32)
-#define MC_STENCIL_VOXELS(nx, ny)                                                              \
-    _Pragma("unroll") for (int k = 0; k < 4; k++) if (const int iy = y0 + threadIdx.y + 8 * k;  \
-                                                      ix < (nx) && iy < (ny))
-inline dim3 stencil_grid(int nx, int ny, int nz) {
-    return dim3(div_up(nx, 32), std::min(div_up(ny, 32), 65535u), std::min((unsigned)nz, 65535u));
+// Division by one divisor d, 1 <= d < 2^31, of many n < 2^31, as a product and a
+// shift (T. Granlund, P. L. Montgomery, "Division by invariant integers using
+// multiplication", PLDI 1994): with 2^(l-1) < d <= 2^l and m = ceil(2^(31+l) / d),
+// m d exceeds 2^(31+l) by less than 2^l, so floor(n m / 2^(31+l)) = floor(n / d).
+struct FastDiv {
+    unsigned m, shift;
+    explicit FastDiv(int d) {
+        int l = 0;
+        while (((int64_t)1 << l) < d) l++;
+        shift = 31 + l;
+        m = (unsigned)((((uint64_t)1 << shift) + d - 1) / (uint64_t)d);
+    }
+    __host__ __device__ __forceinline__ unsigned div(unsigned n) const {
+        return (unsigned)((uint64_t)n * m >> shift);
+    }
+};
+
+// The stencil kernels (bound by memory) go through the volume's voxels in memory
+// order (fewer than 2^31: the indices are unsigned and do not wrap); the
+// coordinates come from the index by two FastDivs, so that every lane has a voxel
+// whatever the slices' shape.  With 32 x 32 tiles of a slice (event time of a
+// call, tiles against this): diff 21 and 11 us at 1x4096x64, 179 and 140 us at
+// 512x512x256; initial2 24 and 12 us, 181 and 146 us.
+struct Grid3 {
+    unsigned n;
+    int nx, ny, nz;
+    FastDiv by_nx, by_ny;
+    Grid3(int nx_, int ny_, int nz_)
+        : n((unsigned)nx_ * ny_ * nz_), nx(nx_), ny(ny_), nz(nz_), by_nx(nx_), by_ny(ny_) {}
+    __device__ __forceinline__ Vox at(unsigned id) const {
+        const unsigned row = by_nx.div(id), iz = by_ny.div(row);
+        return Vox{(int)(id - row * (unsigned)nx), (int)(row - iz * (unsigned)ny), (int)iz};
+    }
+};
+// A block is 256 threads of N voxels each, 256 apart, all read before the first is
+// stored: N = 4, or 1 where the GPU holds a thread for every voxel (diff in a
+// chain of launches, N = 4 against 1: 2.3 and 1.8 us at 64x64x64, 2.5 and 2.5 us
+// at 100x90x64).
+constexpr unsigned STENCIL_SMALL = 148 * 2048;
+template <unsigned N, typename F> __device__ __forceinline__ void stencil(const Grid3 &g, F f) {
+    for (unsigned b = blockIdx.x * (256 * N) + threadIdx.x; b < g.n; b += gridDim.x * (256 * N)) {
+        float v[N];
+#pragma unroll
+        for (unsigned k = 0; k < N; k++)
+            if (const unsigned id = b + 256 * k; id < g.n) v[k] = f.value(id, g.at(id), g);
+#pragma unroll
+        for (unsigned k = 0; k < N; k++)
+            if (const unsigned id = b + 256 * k; id < g.n) f.store(id, v[k]);
+    }
+}
+template <unsigned N, typename F>
+static __global__ void __launch_bounds__(256) stencil_kernel(const Grid3 g, const F op) {
+    stencil<N>(g, op);
+}
+template <typename F>
+int launch_stencil(mcsart_ctx *ctx, const char *name, const Grid3 &g, const F &op) {
+    ctx->label = name;
+    if (g.n <= STENCIL_SMALL)
+        MC_LAUNCH(ctx, (stencil_kernel<1, F>), div_up(g.n, 256), 256, 0, g, op);
+    else
+        MC_LAUNCH(ctx, (stencil_kernel<4, F>), std::min(div_up(g.n, 1024), 148u * 8), 256, 0, g, op);
+    return MCSART_OK;
 }
 
 // cu_add.cu:9-18
@@ -90,38 +137,64 @@ static __global__ void __launch_bounds__(256) add_kernel(float *img1, const floa
 }
 
 // cu_add.cu:28-59: img1[id] += img[iy + ix*ny + iz*nx*ny] * weight * d_ind img0
-// (img read through a tile, with its memory order along the lanes; the other
-// arrays' values are loaded before the barrier, so that a block waits on
-// memory once)
+struct Add2Op {
+    float *img1;
+    const float *img, *img0;
+    float weight;
+    int ind;
+    __device__ float value(unsigned id, const Vox &v, const Grid3 &g) const {
+        const unsigned plane = (unsigned)g.nx * g.ny;
+        return __fmaf_rn(img[v.iy + (unsigned)v.ix * g.ny + v.iz * plane] * weight,
+                         fwd_diff(img0, id, v, g.nx, g.ny, g.nz, ind), img1[id]);
+    }
+    __device__ void store(unsigned id, float v) const { img1[id] = v; }
+};
+// The same with img read through a 32 x 32 tile of a slice, its memory order along
+// the lanes (blockDim (32, 8), four voxels per thread; the other arrays' values
+// are loaded before the barrier, so that a block waits on memory once).  For
+// slices of ADD2_TILE_MIN and more a side: narrower ones leave the tile's lanes
+// idle (8x8x20000: 38 us, Add2Op in a stencil kernel 13), and volumes of at most
+// ADD2_ROWS_MAX fill too few blocks (in a chain of launches, tiles against rows:
+// 3.1 and 1.9 us at 36x36x100, 2.7 and 2.8 us at 64x64x64).
+constexpr int ADD2_TILE_MIN = 16;
+constexpr unsigned ADD2_ROWS_MAX = 148 * 1024;
+inline dim3 add2_grid(int nx, int ny, int nz) {
+    return dim3(div_up(nx, 32), std::min(div_up(ny, 32), 65535u), std::min((unsigned)nz, 65535u));
+}
 static __global__ void __launch_bounds__(256) add2_kernel(float *img1, const float *img, int nx,
                                                           int ny, int nz, const float *img0,
                                                           float weight, int ind) {
     __shared__ float tile[32][33];
     const int x0 = blockIdx.x * 32, ix = x0 + threadIdx.x;
     const int64_t step = ind == 1 ? 1 : ind == 2 ? nx : (int64_t)nx * ny;
-    MC_STENCIL_TILES(nx, ny, nz) {
-        const int64_t slice = (int64_t)iz * nx * ny;
-        float t[4], df[4], old[4];
+    for (int iz = blockIdx.z; iz < nz; iz += gridDim.z)
+        for (int y0 = blockIdx.y * 32; y0 < ny; y0 += gridDim.y * 32) {
+            const int64_t slice = (int64_t)iz * nx * ny;
+            float t[4], df[4], old[4];
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const int tx = x0 + threadIdx.y + 8 * k, ty = y0 + threadIdx.x;
-            t[k] = tx < nx && ty < ny ? img[ty + (int64_t)tx * ny + slice] : 0.0f;
-        }
-        MC_STENCIL_VOXELS(nx, ny) {
-            const int64_t id = ix + (int64_t)iy * nx + slice;
-            const bool last = ind == 1 ? ix == nx - 1 : ind == 2 ? iy == ny - 1 : iz == nz - 1;
-            df[k] = last ? 0.0f : img0[id + step] - img0[id];  // fwd_diff
-            old[k] = img1[id];
-        }
+            for (int k = 0; k < 4; k++) {
+                const int tx = x0 + threadIdx.y + 8 * k, ty = y0 + threadIdx.x;
+                t[k] = tx < nx && ty < ny ? img[ty + (int64_t)tx * ny + slice] : 0.0f;
+            }
 #pragma unroll
-        for (int k = 0; k < 4; k++) tile[threadIdx.y + 8 * k][threadIdx.x] = t[k];
-        __syncthreads();
-        MC_STENCIL_VOXELS(nx, ny) {
-            const int64_t id = ix + (int64_t)iy * nx + slice;
-            img1[id] = __fmaf_rn(tile[threadIdx.x][iy - y0] * weight, df[k], old[k]);
+            for (int k = 0; k < 4; k++)
+                if (const int iy = y0 + threadIdx.y + 8 * k; ix < nx && iy < ny) {
+                    const int64_t id = ix + (int64_t)iy * nx + slice;
+                    const bool last = ind == 1 ? ix == nx - 1 : ind == 2 ? iy == ny - 1 : iz == nz - 1;
+                    df[k] = last ? 0.0f : img0[id + step] - img0[id];  // fwd_diff
+                    old[k] = img1[id];
+                }
+#pragma unroll
+            for (int k = 0; k < 4; k++) tile[threadIdx.y + 8 * k][threadIdx.x] = t[k];
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (const int iy = y0 + threadIdx.y + 8 * k; ix < nx && iy < ny) {
+                    const int64_t id = ix + (int64_t)iy * nx + slice;
+                    img1[id] = __fmaf_rn(tile[threadIdx.x][iy - y0] * weight, df[k], old[k]);
+                }
+            __syncthreads();
         }
-        __syncthreads();
-    }
 }
 
 // cu_initial.cu:10-17
@@ -137,21 +210,18 @@ static __global__ void __launch_bounds__(256) initial_kernel(float *img, int64_t
 }
 
 // cu_initial.cu:27-49
-static __global__ void __launch_bounds__(256) initial2_kernel(float *img, int nx, int ny, int nz,
-                                                              const float *img0, float volume,
-                                                              float flow) {
-    const int ix = blockIdx.x * 32 + threadIdx.x;
-    MC_STENCIL_TILES(nx, ny, nz) {
-        MC_STENCIL_VOXELS(nx, ny) {
-            const int64_t id = ix + (int64_t)iy * nx + (int64_t)iz * nx * ny;
-            const Vox v{ix, iy, iz};
-            const float dfx = fwd_diff(img0, id, v, nx, ny, nz, 1);
-            const float dfy = fwd_diff(img0, id, v, nx, ny, nz, 2);
-            const float dfz = fwd_diff(img0, id, v, nx, ny, nz, 3);
-            img[id] = (dfx + dfy + dfz) * (volume + flow);
-        }
+struct Initial2Op {
+    float *img;
+    const float *img0;
+    float s;  // volume + flow
+    __device__ float value(unsigned id, const Vox &v, const Grid3 &g) const {
+        const float dfx = fwd_diff(img0, id, v, g.nx, g.ny, g.nz, 1);
+        const float dfy = fwd_diff(img0, id, v, g.nx, g.ny, g.nz, 2);
+        const float dfz = fwd_diff(img0, id, v, g.nx, g.ny, g.nz, 3);
+        return (dfx + dfy + dfz) * s;
     }
-}
+    __device__ void store(unsigned id, float v) const { img[id] = v; }
+};
 
 // cu_division.cu:11-25
 struct DivisionOp {
@@ -174,64 +244,60 @@ static __global__ void __launch_bounds__(256) division_kernel(float *img1, const
 }
 
 // cu_multiple.cu:11-43
-static __global__ void __launch_bounds__(256) multiple_kernel(float *img1, int nx, int ny, int nz,
-                                                              const float *img0, float weight,
-                                                              int ind) {
-    const int ix = blockIdx.x * 32 + threadIdx.x;
-    MC_STENCIL_TILES(nx, ny, nz) {
-        MC_STENCIL_VOXELS(nx, ny) {
-            const int64_t id = ix + (int64_t)iy * nx + (int64_t)iz * nx * ny;
-            img1[id] *= weight * fwd_diff(img0, id, Vox{ix, iy, iz}, nx, ny, nz, ind);
-        }
+struct MultipleOp {
+    float *img1;
+    const float *img0;
+    float weight;
+    int ind;
+    __device__ float value(unsigned id, const Vox &v, const Grid3 &g) const {
+        return img1[id] * (weight * fwd_diff(img0, id, v, g.nx, g.ny, g.nz, ind));
     }
-}
+    __device__ void store(unsigned id, float v) const { img1[id] = v; }
+};
 
 // cu_update_udvf.cu:11-62.  b pairs alpha_y/beta_y with the x gradient and
 // alpha_x/beta_x with the y gradient (:45-50) while the update adds the x
-// component to alpha_x (:55), exactly as the reference does.
+// component to alpha_x (:55), exactly as the reference does.  One voxel at a time:
+// each field is read again behind the stores before it, as there.
 static __global__ void __launch_bounds__(256) update_udvf_kernel(
-    float *ax, float *ay, float *az, float *bx, float *by, float *bz, const float *img,
-    const float *img0, float volume_diff, float flow_diff, int nx, int ny, int nz) {
-    const int ix = blockIdx.x * 32 + threadIdx.x;
-    MC_STENCIL_TILES(nx, ny, nz) {
-        MC_STENCIL_VOXELS(nx, ny) {
-            const int64_t id = ix + (int64_t)iy * nx + (int64_t)iz * nx * ny;
-            const Vox v{ix, iy, iz};
-            const float dfI = img0[id] - img[id];
-            const float dfx = fwd_diff(img, id, v, nx, ny, nz, 1);
-            const float dfy = fwd_diff(img, id, v, nx, ny, nz, 2);
-            const float dfz = fwd_diff(img, id, v, nx, ny, nz, 3);
-            const float cax = dfx * volume_diff, cay = dfy * volume_diff, caz = dfz * volume_diff;
-            const float cbx = dfx * flow_diff, cby = dfy * flow_diff, cbz = dfz * flow_diff;
-            const float w = cax * cax + cay * cay + caz * caz + cbx * cbx + cby * cby + cbz * cbz;
-            const float a_x = ay[id], a_y = ax[id], a_z = az[id];
-            const float b_x = by[id], b_y = bx[id], b_z = bz[id];
-            float b = dfI - cax * a_x - cay * a_y - caz * a_z - cbx * b_x - cby * b_y - cbz * b_z;
-            if (w == 0) continue;
-            b /= w;
-            ax[id] += 1.0f / 6 * b * cax;
-            ay[id] += 1.0f / 6 * b * cay;
-            az[id] += 1.0f / 6 * b * caz;
-            bx[id] += 1.0f / 6 * b * cbx;
-            by[id] += 1.0f / 6 * b * cby;
-            bz[id] += 1.0f / 6 * b * cbz;
-        }
+    const Grid3 g, float *ax, float *ay, float *az, float *bx, float *by, float *bz,
+    const float *img, const float *img0, float volume_diff, float flow_diff) {
+    for (unsigned id = blockIdx.x * 256 + threadIdx.x; id < g.n; id += gridDim.x * 256) {
+        const Vox v = g.at(id);
+        const float dfI = img0[id] - img[id];
+        const float dfx = fwd_diff(img, id, v, g.nx, g.ny, g.nz, 1);
+        const float dfy = fwd_diff(img, id, v, g.nx, g.ny, g.nz, 2);
+        const float dfz = fwd_diff(img, id, v, g.nx, g.ny, g.nz, 3);
+        const float cax = dfx * volume_diff, cay = dfy * volume_diff, caz = dfz * volume_diff;
+        const float cbx = dfx * flow_diff, cby = dfy * flow_diff, cbz = dfz * flow_diff;
+        const float w = cax * cax + cay * cay + caz * caz + cbx * cbx + cby * cby + cbz * cbz;
+        const float a_x = ay[id], a_y = ax[id], a_z = az[id];
+        const float b_x = by[id], b_y = bx[id], b_z = bz[id];
+        float b = dfI - cax * a_x - cay * a_y - caz * a_z - cbx * b_x - cby * b_y - cbz * b_z;
+        if (w == 0) continue;
+        b /= w;
+        ax[id] += 1.0f / 6 * b * cax;
+        ay[id] += 1.0f / 6 * b * cay;
+        az[id] += 1.0f / 6 * b * caz;
+        bx[id] += 1.0f / 6 * b * cbx;
+        by[id] += 1.0f / 6 * b * cby;
+        bz[id] += 1.0f / 6 * b * cbz;
     }
 }
 
 // mex_diff.cu:75-113: backward difference, 0 on both faces.
-static __global__ void __launch_bounds__(256) diff_kernel(float *img1, const float *img, int nx,
-                                                          int ny, int nz, int ind) {
-    const int ix = blockIdx.x * 32 + threadIdx.x;
-    MC_STENCIL_TILES(nx, ny, nz) {
-        MC_STENCIL_VOXELS(nx, ny) {
-            const int64_t id = ix + (int64_t)iy * nx + (int64_t)iz * nx * ny;
-            const int i = ind == 1 ? ix : ind == 2 ? iy : iz, m = ind == 1 ? nx : ind == 2 ? ny : nz;
-            const int64_t step = ind == 1 ? 1 : ind == 2 ? nx : (int64_t)nx * ny;
-            img1[id] = (i == m - 1 || i == 0) ? 0.0f : img[id] - img[id - step];
-        }
+struct DiffOp {
+    float *img1;
+    const float *img;
+    int ind;
+    __device__ float value(unsigned id, const Vox &v, const Grid3 &g) const {
+        const int i = ind == 1 ? v.ix : ind == 2 ? v.iy : v.iz;
+        const int m = ind == 1 ? g.nx : ind == 2 ? g.ny : g.nz;
+        const unsigned step = ind == 1 ? 1 : ind == 2 ? g.nx : (unsigned)g.nx * g.ny;
+        return (i == m - 1 || i == 0) ? 0.0f : img[id] - img[id - step];
     }
-}
+    __device__ void store(unsigned id, float v) const { img1[id] = v; }
+};
 
 // --------------------------------------------------------- fused kernels
 // z-fastest copy of an x-fastest volume: dst[iz + (ix + iy*nx)*nzp] =
