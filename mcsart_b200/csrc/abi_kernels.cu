@@ -191,13 +191,13 @@ MC_EXPORT int mcsart_backprojection(mcsart_ctx *ctx, float *d_img, const float *
 template <typename SRC, typename FT>
 static int launch_deform(mcsart_ctx *ctx, FT *out, const SRC &src, const Fields<FT> &f, int nx,
                          int ny, int nz, float volume, float flow) {
-    if (warp_vec(nx, f, sizeof(FT) == 4 ? (const void *)out : nullptr) &&
-        (uintptr_t)out % (4 * sizeof(FT)) == 0)
-        MC_LAUNCH(ctx, (deform_kernel<4, SRC, FT>), warp_grid<4>(nx, ny, nz), dim3(32, 8), 0, out, src,
-                  f, nx, ny, nz, volume, flow);
+    const Grid3 g(nx, ny, nz);
+    if (warp_vec(nx, f) && (uintptr_t)out % (4 * sizeof(FT)) == 0)
+        MC_LAUNCH(ctx, (deform_kernel<4, SRC, FT>), warp_blocks<4>(g), 256, 0, out, src, f, g, volume,
+                  flow);
     else
-        MC_LAUNCH(ctx, (deform_kernel<1, SRC, FT>), warp_grid<1>(nx, ny, nz), dim3(32, 8), 0, out, src,
-                  f, nx, ny, nz, volume, flow);
+        MC_LAUNCH(ctx, (deform_kernel<1, SRC, FT>), warp_blocks<1>(g), 256, 0, out, src, f, g, volume,
+                  flow);
     return MCSART_OK;
 }
 
@@ -229,8 +229,8 @@ static int deform_common(mcsart_ctx *ctx, bool first_order, float *d_img1, const
         src = (const float *)ws;
     }
     if (first_order) {
-        MC_LAUNCH(ctx, deform2_kernel, warp_grid<1>(nx, ny, nz), dim3(32, 8), 0, d_img1, src, f, nx,
-                  ny, nz, volume, flow);
+        const Grid3 g(nx, ny, nz);
+        MC_LAUNCH(ctx, deform2_kernel, warp_blocks<1>(g), 256, 0, d_img1, src, f, g, volume, flow);
         return MCSART_OK;
     }
     return launch_deform(ctx, d_img1, SrcLinear<float>{src}, f, nx, ny, nz, volume, flow);

@@ -38,10 +38,6 @@ __device__ __forceinline__ void st4(float *p, int64_t i, float4 v) {
     reinterpret_cast<float4 *>(p)[i] = v;
 }
 
-struct Vox {
-    int ix, iy, iz;
-};
-
 // Forward difference along ind, 0 on the last plane (cu_add.cu:37-57).
 template <typename T>
 __device__ __forceinline__ float fwd_diff(const T *img0, int64_t id, const Vox &v, int nx, int ny,
@@ -54,40 +50,10 @@ __device__ __forceinline__ float fwd_diff(const T *img0, int64_t id, const Vox &
     }
 }
 
-// Division by one divisor d, 1 <= d < 2^31, of many n < 2^31, as a product and a
-// shift (T. Granlund, P. L. Montgomery, "Division by invariant integers using
-// multiplication", PLDI 1994): with 2^(l-1) < d <= 2^l and m = ceil(2^(31+l) / d),
-// m d exceeds 2^(31+l) by less than 2^l, so floor(n m / 2^(31+l)) = floor(n / d).
-struct FastDiv {
-    unsigned m, shift;
-    explicit FastDiv(int d) {
-        int l = 0;
-        while (((int64_t)1 << l) < d) l++;
-        shift = 31 + l;
-        m = (unsigned)((((uint64_t)1 << shift) + d - 1) / (uint64_t)d);
-    }
-    __host__ __device__ __forceinline__ unsigned div(unsigned n) const {
-        return (unsigned)((uint64_t)n * m >> shift);
-    }
-};
-
 // The stencil kernels (bound by memory) go through the volume's voxels in memory
-// order (fewer than 2^31: the indices are unsigned and do not wrap); the
-// coordinates come from the index by two FastDivs, so that every lane has a voxel
-// whatever the slices' shape.  With 32 x 32 tiles of a slice (event time of a
+// order (Grid3), so that every lane has a voxel whatever the slices' shape.  With 32 x 32 tiles of a slice (event time of a
 // call, tiles against this): diff 21 and 11 us at 1x4096x64, 179 and 140 us at
 // 512x512x256; initial2 24 and 12 us, 181 and 146 us.
-struct Grid3 {
-    unsigned n;
-    int nx, ny, nz;
-    FastDiv by_nx, by_ny;
-    Grid3(int nx_, int ny_, int nz_)
-        : n((unsigned)nx_ * ny_ * nz_), nx(nx_), ny(ny_), nz(nz_), by_nx(nx_), by_ny(ny_) {}
-    __device__ __forceinline__ Vox at(unsigned id) const {
-        const unsigned row = by_nx.div(id), iz = by_ny.div(row);
-        return Vox{(int)(id - row * (unsigned)nx), (int)(row - iz * (unsigned)ny), (int)iz};
-    }
-};
 // A block is 256 threads of N voxels each, 256 apart, all read before the first is
 // stored: N = 4, or 1 where the GPU holds a thread for every voxel (diff in a
 // chain of launches, N = 4 against 1: 2.3 and 1.8 us at 64x64x64, 2.5 and 2.5 us

@@ -126,27 +126,25 @@ inline bool warp_vec(int nx, const Fields<FT> &f, const void *p0 = nullptr, cons
     return nx % 4 == 0 && (fields & m) == 0 && (((uintptr_t)p0 | (uintptr_t)p1) & 15) == 0;
 }
 
-// blockDim (32, 8); a block covers 32 * N columns of 8 rows and walks the
-// slices gridDim.z apart; grid warp_grid<N>.
-template <int N> inline dim3 warp_grid(int nx, int ny, int nz) {
-    return dim3(div_up(nx, 32 * N), div_up(ny, 8), std::min((unsigned)nz, 65535u));
-}
-
 // Drop-in kernel_deformation.  FT: the fields' and the output's storage type.
+// N neighbouring voxels per thread (4 only where warp_vec holds), in memory order
+// (Grid3): blocks of 32 * N columns of 8 rows left most lanes idle in narrow
+// volumes, and had more blocks along y than a grid takes for ny above 524280.  In a
+// chain of launches, such blocks against this, exact weights: 111 and 8.6 us at
+// 8x8x20000, 4.8 and 3.3 at 64x64x64, 433 and 402 at 512x512x256.  Grid:
+// warp_blocks<N>.
 template <int N, typename SRC, typename FT>
 static __global__ void __launch_bounds__(256) deform_kernel(FT *out, const SRC src, Fields<FT> f,
-                                                            int nx, int ny, int nz, float volume,
+                                                            const Grid3 g, float volume,
                                                             float flow) {
-    const int x = (blockIdx.x * 32 + threadIdx.x) * N;
-    if (x >= nx) return;
-    for (int y = blockIdx.y * 8 + threadIdx.y; y < ny; y += gridDim.y * 8)
-        for (int iz = blockIdx.z; iz < nz; iz += gridDim.z) {
-            const int64_t id = x + (int64_t)y * nx + (int64_t)iz * nx * ny;
-            float v[N];
-            warp_sample_n<N>(src, f, id, x, y, iz, nx, ny, nz, volume, flow, v);
-            stn<N>(out, id, v);
-        }
+    const unsigned id = (blockIdx.x * 256 + threadIdx.x) * N;
+    if (id >= g.n) return;
+    const Vox p = g.at(id);
+    float v[N];
+    warp_sample_n<N>(src, f, id, p.ix, p.iy, p.iz, g.nx, g.ny, g.nz, volume, flow, v);
+    stn<N>(out, id, v);
 }
+template <int N> inline unsigned warp_blocks(const Grid3 &g) { return div_up(g.n, 256 * N); }
 
 // Drop-in kernel_forwardDVF (bound by memory; VEC: four voxels per thread).
 template <bool VEC>
@@ -195,29 +193,25 @@ static __global__ void __launch_bounds__(256) forward_dvf4_kernel(float4 *m, Fie
 // Drop-in host_deform2 (first-order warp).  Neighbour reads that fall past
 // the end of the volume (the +nx neighbour of the last rows of the last slice
 // under the transposed index) read 0; the reference reads out of bounds there.
-// blockDim (32, 8), a row of 32 voxels per warp; grid warp_grid<1>.
+// A voxel per thread, in memory order; grid warp_blocks<1>.
 static __global__ void __launch_bounds__(256) deform2_kernel(float *out, const float *in,
-                                                             Fields<float> f, int nx, int ny,
-                                                             int nz, float volume, float flow) {
-    const int64_t n = nvox(nx, ny, nz), plane = (int64_t)nx * ny;
-    const int x = blockIdx.x * 32 + threadIdx.x;
-    if (x >= nx) return;
-    for (int y = blockIdx.y * 8 + threadIdx.y; y < ny; y += gridDim.y * 8)
-        for (int iz = blockIdx.z; iz < nz; iz += gridDim.z) {
-            const int64_t id = x + (int64_t)y * nx + iz * plane;
-            int ix, iy;
-            warp_coords(x, y, nx, ny, ix, iy);
-            const float mx = f.ax[id] * volume + f.bx[id] * flow;
-            const float my = f.ay[id] * volume + f.by[id] * flow;
-            const float mz = f.az[id] * volume + f.bz[id] * flow;
-            const float c = in[id];
-            auto at = [&](int64_t j) { return j < n ? in[j] : 0.0f; };
-            float dx, dy, dz;
-            if (ix == nx - 1) dx = 0; else dx = at(id + 1) - c;
-            if (iy == ny - 1) dy = 0; else dy = at(id + nx) - c;
-            if (iz == nz - 1) dz = 0; else dz = at(id + plane) - c;
-            out[id] = c + dy * mx + dx * my + dz * mz;  // cu_deform.cu:112
-        }
+                                                             Fields<float> f, const Grid3 g,
+                                                             float volume, float flow) {
+    const unsigned id = blockIdx.x * 256 + threadIdx.x, plane = (unsigned)g.nx * g.ny;
+    if (id >= g.n) return;
+    const Vox p = g.at(id);
+    int ix, iy;
+    warp_coords(p.ix, p.iy, g.nx, g.ny, ix, iy);
+    const float mx = f.ax[id] * volume + f.bx[id] * flow;
+    const float my = f.ay[id] * volume + f.by[id] * flow;
+    const float mz = f.az[id] * volume + f.bz[id] * flow;
+    const float c = in[id];
+    auto at = [&](unsigned j) { return j < g.n ? in[j] : 0.0f; };
+    float dx, dy, dz;
+    if (ix == g.nx - 1) dx = 0; else dx = at(id + 1) - c;
+    if (iy == g.ny - 1) dy = 0; else dy = at(id + g.nx) - c;
+    if (p.iz == g.nz - 1) dz = 0; else dz = at(id + plane) - c;
+    out[id] = c + dy * mx + dx * my + dz * mz;  // cu_deform.cu:112
 }
 
 // The image pass's warps are bound by the latency of each voxel's field loads
