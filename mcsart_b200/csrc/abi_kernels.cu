@@ -216,6 +216,7 @@ static int deform_common(mcsart_ctx *ctx, bool first_order, float *d_img1, const
         // (cu_deform.cu:13-38); here the 3D array persists across calls
         if (!ctx->driver) ctx->driver.reset(new DriverState());
         TexVol &tv = ctx->driver->tv_deform;
+        MC_TRY(scratch_begin(ctx));
         MC_TRY(tv.ensure(nx, ny, nz));
         MC_TRY(tv.upload(d_img, ctx->stream));
         return launch_deform(ctx, d_img1, SrcTex{tv.tex}, f, nx, ny, nz, volume, flow);
@@ -484,6 +485,7 @@ int deform_ex_typed(mcsart_ctx *ctx, FT *d_img1, const float *d_img, int nx, int
     if (interp == MCSART_INTERP_TEXTURE) {
         if (!ctx->driver) ctx->driver.reset(new DriverState());
         TexVol &tv = ctx->driver->tv_deform;
+        MC_TRY(scratch_begin(ctx));
         MC_TRY(tv.ensure(nx, ny, nz));
         MC_TRY(tv.upload(d_img, ctx->stream));
         return launch_deform(ctx, d_img1, SrcTex{tv.tex}, f, nx, ny, nz, volume, flow);

@@ -41,12 +41,17 @@ bool capturing(cudaStream_t stream) {
     return cudaStreamIsCapturing(stream, &s) != cudaSuccess || s != cudaStreamCaptureStatusNone;
 }
 
-int workspace(mcsart_ctx *ctx, const char *name, size_t bytes, void **out) {
+int scratch_begin(mcsart_ctx *ctx) {
     if (ctx->scratch_pending && ctx->scratch_stream != ctx->stream && !capturing(ctx->stream)) {
         MC_CHECK_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->scratch_done, 0));
         ctx->scratch_stream = ctx->stream;
     }
     ctx->scratch_used = true;
+    return MCSART_OK;
+}
+
+int workspace(mcsart_ctx *ctx, const char *name, size_t bytes, void **out) {
+    MC_TRY(scratch_begin(ctx));
     auto &b = ctx->ws[name];
     if (b.bytes < bytes) {
         if (b.ptr) {

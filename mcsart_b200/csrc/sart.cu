@@ -785,6 +785,7 @@ static int prepare_problem(mcsart_ctx *ctx, const mcsart_problem *prob, const mc
     MC_REQUIRE(prob->d_img && prob->d_proj, "d_img and d_proj must be non-NULL");
     MC_REQUIRE(opt.dvf_inverse == 0 || prob->d_fields == nullptr || prob->nx == prob->ny,
                "the true DVF inverse (dvf_inverse > 0) needs square slices (nx == ny)");
+    MC_TRY(scratch_begin(ctx));
     if (!ctx->driver) ctx->driver.reset(new DriverState());
     DriverState &S = *ctx->driver;
     const int64_t V = nvox(g.nx, g.ny, g.nz);
@@ -919,6 +920,7 @@ static int aumisart_host(mcsart_ctx *ctx, float *h_outimg, float *h_outproj, flo
     const bool motion = ax != nullptr;
     MC_REQUIRE(!motion || (ay && az && bx && by && bz),
                "alpha_x given: all six DVF fields must be non-NULL");
+    MC_TRY(scratch_begin(ctx));
     if (!ctx->driver) ctx->driver.reset(new DriverState());
     DriverState &S = *ctx->driver;
     const int64_t V = nvox(nx, ny, nz), NP = (int64_t)na * nb;
