@@ -42,9 +42,9 @@ bool capturing(cudaStream_t stream) {
 }
 
 int scratch_begin(mcsart_ctx *ctx) {
-    if (ctx->scratch_pending && ctx->scratch_stream != ctx->stream && !capturing(ctx->stream)) {
+    if (ctx->scratch_pending && ctx->scratch_moved && !capturing(ctx->stream)) {
         MC_CHECK_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->scratch_done, 0));
-        ctx->scratch_stream = ctx->stream;
+        ctx->scratch_moved = false;
     }
     ctx->scratch_used = true;
     return MCSART_OK;
@@ -77,7 +77,6 @@ int finish(mcsart_ctx *ctx, const char *what) {
         if (!ctx->scratch_done)
             MC_CHECK_CUDA(cudaEventCreateWithFlags(&ctx->scratch_done, cudaEventDisableTiming));
         MC_CHECK_CUDA(cudaEventRecord(ctx->scratch_done, ctx->stream));
-        ctx->scratch_stream = ctx->stream;
         ctx->scratch_pending = true;
     }
     ctx->scratch_used = false;
@@ -273,6 +272,7 @@ MC_EXPORT int mcsart_set_stream(mcsart_ctx *ctx, void *stream) {
     clear_error();
     MC_TRY(validate_ctx(ctx));
     ctx->stream = (cudaStream_t)stream;  // NULL: the legacy default stream
+    ctx->scratch_moved = true;
     if (ctx->driver) ctx->driver->invalidate_graphs();
     return MCSART_OK;
 }
