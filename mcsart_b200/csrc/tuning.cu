@@ -203,7 +203,7 @@ MC_EXPORT int mcsart_tuning_save(mcsart_ctx *ctx, const char *path) {
     MC_REQUIRE(path, "path is NULL");
     FILE *f = fopen(path, "w");
     MC_REQUIRE(f, "cannot open %s for writing", path);
-    fprintf(f, "# mcsart tuning cache v3: key fp1 fp3 bp warp fup\n");
+    fprintf(f, "# mcsart tuning cache v4: key fp1 fp3 bp warp fup\n");
     for (const auto &e : ctx->tuning)
         fprintf(f, "%s %d %d %d %d %d\n", e.first.c_str(), e.second.fp1, e.second.fp3,
                 e.second.bp, e.second.warp, e.second.fup);
@@ -219,8 +219,9 @@ MC_EXPORT int mcsart_tuning_load(mcsart_ctx *ctx, const char *path) {
     FILE *f = fopen(path, "r");
     MC_REQUIRE(f, "cannot open %s", path);
     char line[512];
-    int n = 0, bad = 0;
+    int n = 0, bad = 0, version = 4;
     while (fgets(line, sizeof(line), f)) {
+        sscanf(line, "# mcsart tuning cache v%d", &version);
         if (line[0] == '#' || line[0] == '\n') continue;
         char key[400];
         Tuning t;
@@ -231,6 +232,8 @@ MC_EXPORT int mcsart_tuning_load(mcsart_ctx *ctx, const char *path) {
             bad++;
             continue;
         }
+        // up to version 3 the numbers stood for other shapes of the projectors
+        if (version < 4) t.fp1 = t.fp3 = -1;
         ctx->tuning[key] = t;
         n++;
     }
