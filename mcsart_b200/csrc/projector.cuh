@@ -1009,8 +1009,7 @@ int launch_fp_ref(mcsart_ctx *ctx, dim3 grid, const FPArgs<VT, K, MT> &a) {
 // its ray's axial part.  Each slab's terms are summed first (in-plane voxel,
 // then slice) and the slab sums added, plainly or with Kahan compensation.
 // GEO64: FP64 geometry and weight sum (ray_geom64): every coordinate, box edge
-// and overlap weight in FP64 (an edge's overlap is divided by the footprint's
-// width by way of its reciprocal, one FP64 rounding more), volume terms in FP32.
+// and overlap weight in FP64, the weights summed one by one; volume terms in FP32.
 // Bound by instruction issue: FP64 operations, and divisions in FP32 geometry.
 // 128x128x96, 256x192 detector, Kahan, FP64 geometry: 146 us with a thread
 // computing its ray's footprints by itself, now 65; 256x256x160, 512x384, FP32
@@ -1030,10 +1029,10 @@ __device__ __forceinline__ double overlap(double i, double lo, double hi) {
 __device__ __forceinline__ float overlap(float i, float lo, float hi) {
     return __fsub_rn(fminf(__fadd_rn(i, 1.0f), hi), fmaxf(i, lo));
 }
+// The quotient by the width, correctly rounded in both (inv: SlabSplit's).
 __device__ __forceinline__ double split_weight(double i, double lo, double hi, double inv) {
-    return overlap(i, lo, hi) * inv;
+    return mk_div64(overlap(i, lo, hi), hi - lo, inv);
 }
-// (FP32: the correctly rounded quotient by the width, as the reference order)
 __device__ __forceinline__ float split_weight(float i, float lo, float hi, float width) {
     return __fdiv_rn(overlap(i, lo, hi), width);
 }
@@ -1162,7 +1161,7 @@ __device__ __forceinline__ void split_slabs(const typename SplitReal<GEO64>::Ray
             const R wz0 = split_weight((R)z.z0, z.lo, z.hi, z.inv);  // :86 / :139
             const R wz1 = z.z1 > z.z0 ? split_weight((R)(z.z0 + 1), z.lo, z.hi, z.inv) : (R)0;
             float ss[K];
-            R ssw = 0;
+            R ssw = GEO64 ? accw : (R)0;  // FP64: straight on
 #pragma unroll
             for (int k = 0; k < K; k++) ss[k] = 0.0f;
             for (int i = 0; i < e.n; i++) {
@@ -1177,7 +1176,7 @@ __device__ __forceinline__ void split_slabs(const typename SplitReal<GEO64>::Ray
             for (int k = 0; k < K; k++) split_add<SUM>(acc[k], cmp[k], ss[k]);
             if constexpr (ONES) {
                 if constexpr (GEO64)
-                    accw += ssw;
+                    accw = ssw;
                 else
                     split_add<SUM>(accw, cmpw, ssw);
             }
