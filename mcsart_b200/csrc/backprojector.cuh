@@ -272,15 +272,14 @@ __device__ __forceinline__ void bp_gather_view64(const BPArgs &p, float angle, c
                                                  float *acc0, double *acc1) {
     const Geom &g = p.g;
     const double SO = g.SO, SD = g.SD, cphi = p.cos64, sphi = p.sin64;
-    // (box ends over the pitches by way of their reciprocals)
-    const double ida = 1.0 / (double)g.da, idb = 1.0 / (double)g.db;
+    const double da = g.da, db = g.db, ya = 1.0 / da, yb = 1.0 / db;
     const double xc = (double)ix - g.nx / 2 + 0.5, yc = (double)iy - g.ny / 2 + 0.5;
     const double t = xc * cphi + yc * sphi, u = -xc * sphi + yc * cphi;
     const double rl = SD / (t - 0.5 + SO), rr = SD / (t + 0.5 + SO), r0 = SD / (t + SO);
     const double all = rl * (u - 0.5), alr = rl * (u + 0.5);
     const double arr = rr * (u + 0.5), arl = rr * (u - 0.5), at = r0 * u;
-    const double amax = fmax(fmax(fmax(all, arr), fmax(alr, arl)), at) * ida - g.ai + 0.5;
-    const double amin = fmin(fmin(fmin(all, arr), fmin(alr, arl)), at) * ida - g.ai + 0.5;
+    const double amax = mk_div64(fmax(fmax(fmax(all, arr), fmax(alr, arl)), at), da, ya) - g.ai + 0.5;
+    const double amin = mk_div64(fmin(fmin(fmin(all, arr), fmin(alr, arl)), at), da, ya) - g.ai + 0.5;
     const int ia0 = max(0, (int)floor(fmax(amin, -1.0)));
     const int ia1 = (int)ceil(fmin(amax, (double)g.na));  // columns ia < ia1
 #pragma unroll
@@ -289,8 +288,8 @@ __device__ __forceinline__ void bp_gather_view64(const BPArgs &p, float angle, c
         if (iz >= g.nz) continue;
         const double zc = (double)iz - g.nz / 2 + 0.5;
         const double bl = rl * zc, br = rr * zc, bt = r0 * (zc + 0.5), bb = r0 * (zc - 0.5);
-        const double bmax = fmax(fmax(bl, br), fmax(bt, bb)) * idb - g.bi + 0.5;
-        const double bmin = fmin(fmin(bl, br), fmin(bt, bb)) * idb - g.bi + 0.5;
+        const double bmax = mk_div64(fmax(fmax(bl, br), fmax(bt, bb)), db, yb) - g.bi + 0.5;
+        const double bmin = mk_div64(fmin(fmin(bl, br), fmin(bt, bb)), db, yb) - g.bi + 0.5;
         const int ib0 = max(0, (int)floor(fmax(bmin, -1.0)));
         const int ib1 = (int)ceil(fmin(bmax, (double)g.nb));
         for (int ia = ia0; ia < ia1; ia++) {
