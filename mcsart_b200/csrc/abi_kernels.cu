@@ -452,18 +452,9 @@ int projection_ex_launch(mcsart_ctx *ctx, float *d_proj, const VT *zf, int fp_su
             ctx, dim3(div_up(g.na, FPC_COLS), div_up(g.nb, FPC_ROWS), 1), a);
     a.cos64 = cos((double)angle);
     a.sin64 = sin((double)angle);
-    const int groups = fp_auto_groups((int64_t)g.na * div_up(g.nb, 32), std::max(g.nx, g.ny));
-    const dim3 grid(g.na, div_up(g.nb, 32), 1), block(32, groups);
-    const size_t smem = (size_t)groups * 2 * 32 * sizeof(float);
-    if (fp_sum == SUM_PLAIN && geom64)
-        MC_LAUNCH(ctx, (fp_kernel<1, false, SUM_PLAIN, VT, VT, true>), grid, block, smem, a);
-    else if (fp_sum == SUM_PLAIN)
-        MC_LAUNCH(ctx, (fp_kernel<1, false, SUM_PLAIN, VT, VT>), grid, block, smem, a);
-    else if (geom64)
-        MC_LAUNCH(ctx, (fp_kernel<1, false, SUM_KAHAN, VT, VT, true>), grid, block, smem, a);
-    else
-        MC_LAUNCH(ctx, (fp_kernel<1, false, SUM_KAHAN, VT, VT>), grid, block, smem, a);
-    return MCSART_OK;
+    const int groups = fp_auto_groups((int64_t)div_up(g.na, 32) * g.nb, std::max(g.nx, g.ny));
+    return fp_sum == SUM_PLAIN ? launch_fp_split<1, false, SUM_PLAIN>(ctx, groups, geom64 != 0, a)
+                               : launch_fp_split<1, false, SUM_KAHAN>(ctx, groups, geom64 != 0, a);
 }
 
 template <typename VT>

@@ -1001,19 +1001,36 @@ int launch_fp_ref(mcsart_ctx *ctx, dim3 grid, const FPArgs<VT, K, MT> &a) {
 }
 
 // ------------------------------------------------------------------------
-// Projector of the split summation modes: blockDim (32, groups), the 32 lanes
-// 32 consecutive detector rows of one column, threadIdx.y = slab group of the
-// same 32 rays, gridDim (na, ceil(nb/32), views).  A warp's lanes compute the
-// column's in-plane footprint of 32 slabs at a time, one slab each, into a
-// table of the warp's own, and then walk the slabs together, each lane adding
-// its ray's axial part.  Each slab's terms are summed first (in-plane voxel,
-// then slice) and the slab sums added, plainly or with Kahan compensation.
+// Projector of the split summation modes: blockDim (32, groups), threadIdx.y =
+// slab group of the same 32 rays.  The 32 lanes are 32 consecutive detector rows
+// of one column (gridDim (na, ceil(nb/32), views)): they compute the column's
+// in-plane footprint of 32 slabs at a time, one slab each, into a table of the
+// warp's own, and then walk the slabs together, each lane adding its ray's axial
+// part.  RAYS: 32 consecutive columns of one row (gridDim (ceil(na/32), nb,
+// views)), each lane with its own footprints, for detectors whose rows would not
+// fill the warps (split_rays).  Each slab's terms are summed first (in-plane
+// voxel, then slice) and the slab sums added, plainly or with Kahan compensation.
 // GEO64: FP64 geometry and weight sum (ray_geom64): every coordinate, box edge
 // and overlap weight in FP64, the weights summed one by one; volume terms in FP32.
 // Bound by instruction issue: FP64 operations, and divisions in FP32 geometry.
 // 128x128x96, 256x192 detector, Kahan, FP64 geometry: 146 us with a thread
 // computing its ray's footprints by itself, now 65; 256x256x160, 512x384, FP32
 // geometry: 387, now 338.
+
+// Whether the split-sum projector's lanes are columns: where rows would leave lanes
+// idle and the shared footprints do not make up for it.  A ray with footprints of
+// its own costs 1.3 times one without in FP32 geometry and twice in FP64 (each
+// measured with full warps).  The kernel by events, rows against columns:
+// 512x512x1 with a 1024x1 detector 97 and 42 us, 512x512x4 with 1024x4 130 and 56;
+// a call at 256x256x160 with 512x33 87 and 64 us, and in FP64, which keeps the
+// rows there, 100 against 123.
+inline bool split_rays(const Geom &g, bool geom64) {
+    const int64_t rows = (g.nb + 31) / 32 * 32, cols = (g.na + 31) / 32 * 32;
+    return g.nb * cols * (geom64 ? 20 : 13) < rows * g.na * 10;
+}
+inline dim3 split_grid(const Geom &g, bool rays) {
+    return rays ? dim3(div_up(g.na, 32), g.nb) : dim3(g.na, div_up(g.nb, 32));
+}
 
 // In-plane footprint of one slab: voxels u_lo .. u_lo + n - 1 (in the volume)
 // with the first one's column at element `row`, the edges, the reciprocal width
@@ -1037,7 +1054,8 @@ __device__ __forceinline__ float split_weight(float i, float lo, float hi, float
     return __fdiv_rn(overlap(i, lo, hi), width);
 }
 
-__device__ __forceinline__ SlabSplit<double> slab_split(const RayGeom64 &r, int d, int su, int sd) {
+// (without the weights)
+__device__ __forceinline__ SlabSplit<double> slab_edges(const RayGeom64 &r, int d, int su, int sd) {
     SlabSplit<double> e;
     e.dc = ((double)d + 0.5) - r.d_half - r.src_d;  // :52 / :105
     const double c0 = r.r0 * e.dc + r.u_off + r.u_half, c1 = r.r1 * e.dc + r.u_off + r.u_half;
@@ -1047,12 +1065,10 @@ __device__ __forceinline__ SlabSplit<double> slab_split(const RayGeom64 &r, int 
     e.inv = 1.0 / (e.hi - e.lo);
     e.u_lo = max(0, __double2int_rd(e.lo));
     e.n = max(0, min(r.nu - 1, __double2int_rd(e.hi)) - e.u_lo + 1);
-    e.w0 = split_weight((double)e.u_lo, e.lo, e.hi, e.inv);  // :83 / :136
-    e.w1 = split_weight(e.u_lo + 1.0, e.lo, e.hi, e.inv);
     e.row = e.u_lo * su + d * sd;
     return e;
 }
-__device__ __forceinline__ SlabSplit<float> slab_split(const RayGeom &r, int d, int su, int sd) {
+__device__ __forceinline__ SlabSplit<float> slab_edges(const RayGeom &r, int d, int su, int sd) {
     SlabSplit<float> e;
     e.dc = __fsub_rn(__fsub_rn(__fadd_rn((float)d, 0.5f), r.d_half), r.src_d);  // :52 / :105
     // :54-63 / :107-116
@@ -1065,10 +1081,13 @@ __device__ __forceinline__ SlabSplit<float> slab_split(const RayGeom &r, int d, 
     e.inv = __fsub_rn(e.hi, e.lo);
     e.u_lo = max(0, (int)floorf(e.lo));
     e.n = max(0, min(r.nu - 1, (int)floorf(e.hi)) - e.u_lo + 1);
-    e.w0 = split_weight((float)e.u_lo, e.lo, e.hi, e.inv);  // :83 / :136
-    e.w1 = split_weight((float)(e.u_lo + 1), e.lo, e.hi, e.inv);
     e.row = e.u_lo * su + d * sd;
     return e;
+}
+
+// The weight of the footprint's voxel i (:83 / :136).
+template <typename R> __device__ __forceinline__ R slab_weight(const SlabSplit<R> &e, int i) {
+    return split_weight((R)(e.u_lo + i), e.lo, e.hi, e.inv);
 }
 
 // Axial edges of a slab (:71-77 / :124-130, "ratio * xc + z1 + nz / 2", z1 = 0)
@@ -1131,9 +1150,10 @@ template <int SUM> __device__ __forceinline__ void split_add(float &s, float &c,
 template <bool GEO64> struct SplitReal { using R = float; using Ray = RayGeom; };
 template <> struct SplitReal<true> { using R = double; using Ray = RayGeom64; };
 
-// Slabs [d0, d1) of the warp's rays: s[k], and sw (FP32 slab sums of FP32
-// weights, FP64 sum of FP64 weights); tab: 32 entries of the warp's own.
-template <int K, bool ONES, int SUM, bool GEO64, typename VT>
+// Slabs [d0, d1) of the lane's ray: s[k], and sw (FP32 slab sums of FP32 weights,
+// FP64 sum of FP64 weights); tab (not RAYS): 32 entries of the warp's own, whose
+// rays have the same slabs.
+template <int K, bool ONES, int SUM, bool GEO64, bool RAYS, typename VT>
 __device__ __forceinline__ void split_slabs(const typename SplitReal<GEO64>::Ray &r,
                                             const FPVolumes<VT, K> &v, const Geom &g, int d0, int d1,
                                             SlabSplit<typename SplitReal<GEO64>::R> *tab, float *s,
@@ -1148,14 +1168,24 @@ __device__ __forceinline__ void split_slabs(const typename SplitReal<GEO64>::Ray
     R accw = 0;
 #pragma unroll
     for (int k = 0; k < K; k++) { acc[k] = 0.0f; cmp[k] = 0.0f; }
-    for (int c0 = d0; c0 < d1; c0 += 32) {
-        __syncwarp();
-        if (c0 + lane < d1) tab[lane] = slab_split(r, c0 + lane, su, sd);
-        __syncwarp();
-        const int m = min(32, d1 - c0);
+    for (int c0 = d0; c0 < d1; c0 += RAYS ? 1 : 32) {
+        SlabSplit<R> own;
+        if (RAYS) {
+            own = slab_edges(r, c0, su, sd);
+        } else {
+            __syncwarp();
+            if (c0 + lane < d1) {
+                SlabSplit<R> e = slab_edges(r, c0 + lane, su, sd);
+                e.w0 = slab_weight(e, 0);
+                e.w1 = slab_weight(e, 1);
+                tab[lane] = e;
+            }
+            __syncwarp();
+        }
+        const int m = RAYS ? 1 : min(32, d1 - c0);
         for (int j = 0; j < m; j++) {
-            const SlabSplit<R> &e = tab[j];
-            if (e.n == 0) continue;  // the same for the whole warp
+            const SlabSplit<R> &e = RAYS ? own : tab[j];
+            if (e.n == 0) continue;  // (not RAYS: the same for the whole warp)
             const SplitZ<R> z = split_z(r.rz0, r.rz1, e.dc, z_half, g.nz);
             if (z.z0 > z.z1) continue;
             const R wz0 = split_weight((R)z.z0, z.lo, z.hi, z.inv);  // :86 / :139
@@ -1165,7 +1195,7 @@ __device__ __forceinline__ void split_slabs(const typename SplitReal<GEO64>::Ray
 #pragma unroll
             for (int k = 0; k < K; k++) ss[k] = 0.0f;
             for (int i = 0; i < e.n; i++) {
-                const R wu = i == 0 ? e.w0 : i == 1 ? e.w1 : split_weight((R)(e.u_lo + i), e.lo, e.hi, e.inv);
+                const R wu = !RAYS && i == 0 ? e.w0 : !RAYS && i == 1 ? e.w1 : slab_weight(e, i);
                 const int a = e.row + i * su;
                 split_term<K, ONES>(v.zf, a + z.z0, wu, wz0, ss, ssw);
                 if (z.z1 > z.z0) split_term<K, ONES>(v.zf, a + z.z0 + 1, wu, wz1, ss, ssw);
@@ -1187,31 +1217,34 @@ __device__ __forceinline__ void split_slabs(const typename SplitReal<GEO64>::Ray
     sw = accw;
 }
 
-template <int K, bool ONES, int SUM, typename VT, typename MT = VT, bool GEO64 = false>
+template <int K, bool ONES, int SUM, typename VT, typename MT = VT, bool GEO64 = false,
+          bool RAYS = false>
 __global__ void __launch_bounds__(256) fp_kernel(const FPArgs<VT, K, MT> p) {
     constexpr int NS = K + (ONES ? 1 : 0);
     extern __shared__ float sm_fp[];  // [groups][NS][32]
     __shared__ double sm_w64[GEO64 ? 8 : 1][32];  // GEO64: the groups' FP64 weight sums
-    __shared__ SlabSplit<typename SplitReal<GEO64>::R> sm_tab[8][32];
+    __shared__ SlabSplit<typename SplitReal<GEO64>::R> sm_tab[RAYS ? 1 : 8][32];
     const int lane = threadIdx.x;
     const Geom &g = p.g;
-    const int ia = blockIdx.x, ib = blockIdx.y * 32 + lane;
-    const bool active = ib < g.nb;
+    const int ia = RAYS ? blockIdx.x * 32 + lane : blockIdx.x;
+    const int ib = RAYS ? blockIdx.y : blockIdx.y * 32 + lane;
+    const bool active = ia < g.na && ib < g.nb;
     const int groups = blockDim.y, grp = threadIdx.y;
     float s[K], sw = 0.0f;
     double sw64 = 0.0;
     {
-        // lanes past the last row repeat its ray; nothing of them is stored
-        const int row = min(ib, g.nb - 1);
+        // lanes past the last row or column repeat its ray; nothing of them is stored
+        const int row = min(ib, g.nb - 1), col = min(ia, g.na - 1);
+        auto *const tab = sm_tab[RAYS ? 0 : grp];
         if constexpr (GEO64) {
-            const RayGeom64 r = ray_geom64(p.cos64, p.sin64, ia, row, g);
+            const RayGeom64 r = ray_geom64(p.cos64, p.sin64, col, row, g);
             const int per = (r.nd + groups - 1) / groups, d0 = grp * per, d1 = min(r.nd, d0 + per);
-            split_slabs<K, ONES, SUM, true, VT>(r, p.vol, g, d0, d1, sm_tab[grp], s, sw64);
+            split_slabs<K, ONES, SUM, true, RAYS, VT>(r, p.vol, g, d0, d1, tab, s, sw64);
         } else {
             const float angle = p.angles ? p.angles[blockIdx.z] : p.angle;
-            const RayGeom r = ray_geom(cosf(angle), sinf(angle), ia, row, g);  // :23-24
+            const RayGeom r = ray_geom(cosf(angle), sinf(angle), col, row, g);  // :23-24
             const int per = (r.nd + groups - 1) / groups, d0 = grp * per, d1 = min(r.nd, d0 + per);
-            split_slabs<K, ONES, SUM, false, VT>(r, p.vol, g, d0, d1, sm_tab[grp], s, sw);
+            split_slabs<K, ONES, SUM, false, RAYS, VT>(r, p.vol, g, d0, d1, tab, s, sw);
         }
     }
 #pragma unroll
@@ -1256,6 +1289,24 @@ __global__ void __launch_bounds__(256) fp_kernel(const FPArgs<VT, K, MT> p) {
         nr2 += __shfl_down_sync(0xffffffffu, nr2, off);
     }
     if (lane == 0) p.norm_part[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] = make_double2(nb2, nr2);
+}
+
+// Launch of fp_kernel for one view, in FP32 or FP64 geometry (a: cos64, sin64 set).
+template <int K, bool ONES, int SUM, typename VT, typename MT>
+int launch_fp_split(mcsart_ctx *ctx, int groups, bool geom64, const FPArgs<VT, K, MT> &a) {
+    const bool rays = split_rays(a.g, geom64);
+    const dim3 grid = split_grid(a.g, rays), block(32, groups);
+    const size_t smem = (size_t)groups * (K + 1) * 32 * sizeof(float);
+    if (!ctx->label) ctx->label = "fp_kernel";
+    if (geom64 && rays)
+        MC_LAUNCH(ctx, (fp_kernel<K, ONES, SUM, VT, MT, true, true>), grid, block, smem, a);
+    else if (geom64)
+        MC_LAUNCH(ctx, (fp_kernel<K, ONES, SUM, VT, MT, true, false>), grid, block, smem, a);
+    else if (rays)
+        MC_LAUNCH(ctx, (fp_kernel<K, ONES, SUM, VT, MT, false, true>), grid, block, smem, a);
+    else
+        MC_LAUNCH(ctx, (fp_kernel<K, ONES, SUM, VT, MT, false, false>), grid, block, smem, a);
+    return MCSART_OK;
 }
 
 }  // namespace mcsart

@@ -86,12 +86,14 @@ template <typename ST, int INTERP, int SUM> struct Runner {
         V = nvox(P.g.nx, P.g.ny, P.g.nz);
         VZ = nvox(P.g.nx, P.g.ny, P.g.nzp);
         NP = (int64_t)P.g.na * P.g.nb;
-        fp_bx = SUM == SUM_REF ? (int)div_up(P.g.na, FPC_COLS) : P.g.na;
-        fp_by = (int)div_up(P.g.nb, SUM == SUM_REF ? FPC_ROWS : 32);
+        const dim3 split = split_grid(P.g, split_rays(P.g, opt.geom64));
+        fp_bx = SUM == SUM_REF ? (int)div_up(P.g.na, FPC_COLS) : (int)split.x;
+        fp_by = SUM == SUM_REF ? (int)div_up(P.g.nb, FPC_ROWS) : (int)split.y;
         fp_blocks = fp_bx * fp_by;
         groups = SUM == SUM_REF ? 1
                  : opt.fp_groups > 0 ? std::min(opt.fp_groups, 8)
-                                     : fp_auto_groups(fp_blocks, std::max(P.g.nx, P.g.ny));
+                                     : fp_auto_groups((int64_t)div_up(P.g.na, 32) * P.g.nb,
+                                                      std::max(P.g.nx, P.g.ny));
         subset = std::min(std::max(opt.subset, 1), BP_MAX_VIEWS);
         inv_iters = P.motion_model ? opt.dvf_inverse : 0;
         for (int v = 0; v < P.n_views; v++) views_img.push_back(v);
@@ -186,15 +188,10 @@ template <typename ST, int INTERP, int SUM> struct Runner {
                 case 3: MC_TRY((launch_fp_ref<K, ONES, VT, ST, false, 2, 2, 6, K == 3>(ctx, grid, a))); break;
                 default: MC_TRY((launch_fp_ref<K, ONES, VT, ST, false, 4, 2, 5, K == 3>(ctx, grid, a))); break;
             }
-        } else if (opt.geom64) {
-            const size_t smem = (size_t)groups * (K + 1) * 32 * sizeof(float);
+        } else {
             a.cos64 = cos((double)P.angles[v]);
             a.sin64 = sin((double)P.angles[v]);
-            MC_LAUNCH(ctx, (fp_kernel<K, ONES, SUM == SUM_REF ? SUM_PLAIN : SUM, VT, ST, true>),
-                      grid, dim3(32, groups), smem, a);
-        } else {
-            const size_t smem = (size_t)groups * (K + 1) * 32 * sizeof(float);
-            MC_LAUNCH(ctx, (fp_kernel<K, ONES, SUM, VT, ST>), grid, dim3(32, groups), smem, a);
+            MC_TRY((launch_fp_split<K, ONES, SUM>(ctx, groups, opt.geom64 != 0, a)));
         }
         return MCSART_OK;
     }
