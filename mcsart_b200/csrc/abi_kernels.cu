@@ -56,8 +56,7 @@ int zfast_copy(mcsart_ctx *ctx, const char *name, const VT *src, const Geom &g, 
     } else {
         MC_TRY(workspace(ctx, name, bytes, &ws));
     }
-    MC_LAUNCH(ctx, (zfast_kernel<VT, VT>), zfast_grid(g.nx, g.ny, g.nz), dim3(32, 8), 0, (VT *)ws,
-              src, g.nx, g.ny, g.nz, g.nzp);
+    MC_TRY(zfast(ctx, (VT *)ws, src, g));
     *out = (const VT *)ws;
     return MCSART_OK;
 }

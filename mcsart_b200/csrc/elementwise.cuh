@@ -301,6 +301,42 @@ static __global__ void __launch_bounds__(256) zfast_kernel(DT *dst, const ST *sr
 inline dim3 zfast_grid(int nx, int ny, int nz) {
     return dim3(div_up(nx, 32) * (unsigned)ny, div_up(nz, ZF_Z));
 }
+// The same with a column per thread, for volumes of at most ZF_THIN slices (a
+// multiple of 2), which leave most of a tile's threads idle (512x512x4: 19 us,
+// this 7.  Grid ceil(nx * ny / 256).
+constexpr int ZF_THIN = 8;
+template <typename ST, typename DT>
+static __global__ void __launch_bounds__(256) zfast_thin_kernel(DT *dst, const ST *src, int plane,
+                                                                int nz, int nzp) {
+    const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (c >= plane) return;
+    float v[ZF_THIN];
+#pragma unroll
+    for (int k = 0; k < ZF_THIN; k++) v[k] = k < nz ? ldv(src, c + (int64_t)k * plane) : 0.0f;
+#pragma unroll
+    for (int k = 0; k < ZF_THIN; k++)
+        if (k < nzp) dst[c * nzp + k] = cvt<DT>(v[k]);
+}
+// The launch of either (not a context's: mcsart_projection_noalloc has none).
+template <typename ST, typename DT>
+void zfast_launch(cudaStream_t stream, DT *dst, const ST *src, int nx, int ny, int nz, int nzp) {
+    if (nz <= ZF_THIN)
+        zfast_thin_kernel<ST, DT><<<div_up((int64_t)nx * ny, 256), 256, 0, stream>>>(dst, src, nx * ny,
+                                                                                    nz, nzp);
+    else
+        zfast_kernel<ST, DT><<<zfast_grid(nx, ny, nz), dim3(32, 8), 0, stream>>>(dst, src, nx, ny, nz,
+                                                                                nzp);
+}
+template <typename ST, typename DT>
+int zfast(mcsart_ctx *ctx, DT *dst, const ST *src, const Geom &g) {
+    if (ctx->profiling) MC_TRY(prof_before(ctx, "zfast_kernel"));
+    zfast_launch(ctx->stream, dst, src, g.nx, g.ny, g.nz, g.nzp);
+    ctx->launches++;
+    MC_TRY(check_launch("zfast_kernel"));
+    if (ctx->profiling) MC_TRY(prof_after(ctx));
+    ctx->label = nullptr;
+    return MCSART_OK;
+}
 
 // Loads the 32x32 tile of a field read at the transposed index
 // t = iy + ix*ny + iz*nx*ny for the block's (x, y) tile into tile[lx][ly].

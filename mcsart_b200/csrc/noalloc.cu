@@ -73,7 +73,7 @@ int current_context_id(unsigned long long *id) {
 
 // Set-up on the first call per device and context, with that device
 // current: the scratch's address (cudaGetSymbolAddress, which also makes the
-// runtime's context current), and both kernels loaded so that later calls
+// runtime's context current), and the kernels loaded so that later calls
 // load nothing.  Later calls in the same context only compare the id.
 int scratch_of_current_device(float **out) {
     int dev = -1;
@@ -100,6 +100,7 @@ int scratch_of_current_device(float **out) {
     MC_CHECK_CUDA(cudaGetSymbolAddress(&p, g_noalloc_volZ));
     cudaFuncAttributes fa;
     MC_CHECK_CUDA(cudaFuncGetAttributes(&fa, zfast_kernel<float, float>));
+    MC_CHECK_CUDA(cudaFuncGetAttributes(&fa, zfast_thin_kernel<float, float>));
     MC_CHECK_CUDA(cudaFuncGetAttributes(&fa, fp_ref_kernel<1, false, float>));
     unsigned long long id = 0;
     MC_TRY(current_context_id(&id));
@@ -131,8 +132,7 @@ MC_EXPORT int mcsart_projection_noalloc(void *stream, float *d_proj, const float
     MC_TRY(scratch_of_current_device(&scratch));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
 
-    zfast_kernel<float, float><<<zfast_grid(nx, ny, nz), dim3(32, 8), 0, s>>>(scratch, d_img, nx,
-                                                                              ny, nz, g.nzp);
+    zfast_launch(s, scratch, d_img, nx, ny, nz, g.nzp);
     MC_CHECK_CUDA(cudaGetLastError());
     FPArgs<float, 1> a{};
     a.vol.zf[0] = scratch;

@@ -333,13 +333,6 @@ template <typename ST, int INTERP, int SUM> struct Runner {
         return dim3(div_up(P.g.nx, 32 * N), div_up(P.g.ny, 8 * WR), P.g.nz);
     }
 
-    // A z-fastest copy for the projector.
-    template <typename SRC_T, typename DST_T> int zfast(DST_T *dst, const SRC_T *src) {
-        MC_LAUNCH(ctx, (zfast_kernel<SRC_T, DST_T>), zfast_grid(P.g.nx, P.g.ny, P.g.nz),
-                  dim3(32, 8), 0, dst, src, P.g.nx, P.g.ny, P.g.nz, P.g.nzp);
-        return MCSART_OK;
-    }
-
     // The image pass's forward warp of the volume into a view's phase, in the
     // tuned launch shape (slices per thread).
     template <int WR> int warp_fwd_shape(ST *d, bool hw, float volume, float flow) {
@@ -404,7 +397,7 @@ template <typename ST, int INTERP, int SUM> struct Runner {
     // AUMISART.cu:42-63
     int enqueue_image_static() {
         MC_CHECK_CUDA(cudaMemsetAsync(S.norm_tmp.ptr, 0, P.n_views * sizeof(float), ctx->stream));
-        MC_TRY(zfast(S.imgZ.as<float>(), (const float *)P.img));
+        MC_TRY(zfast(ctx, S.imgZ.as<float>(), (const float *)P.img, P.g));
         FPVolumes<float, 1> vol{};
         vol.zf[0] = S.imgZ.as<float>();
         const int n = (int)views_img.size();
@@ -529,7 +522,7 @@ template <typename ST, int INTERP, int SUM> struct Runner {
         ST *fw = (ST *)P.fields;
         MC_CHECK_CUDA(cudaMemsetAsync(S.norm_tmp.ptr, 0, P.n_views * sizeof(float), ctx->stream));
         FPVolumes<ST, 3> vol{};
-        MC_TRY((zfast<float, ST>(S.imgS.as<ST>(), (const float *)P.img)));
+        MC_TRY(zfast(ctx, S.imgS.as<ST>(), (const float *)P.img, P.g));
         vol.zf[0] = S.imgS.as<ST>();
         // the reference-order projector reads img0 and the initial2 volume
         // as interleaved pairs (one load for both), the split-sum one apart
