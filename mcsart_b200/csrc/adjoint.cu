@@ -33,7 +33,7 @@ struct __align__(16) AdjColumn {
     int axis;  // 1: x-driven
 };
 // d_half and src_d (RayGeom) of each driving axis; general: set where some ray is
-// not narrow (ray_axial), or the depth is 1.
+// not narrow (ray_axial).
 struct AdjAxes {
     float d_half[2], src_d[2];
     int general;
@@ -56,7 +56,7 @@ static __global__ void adj_rays_kernel(RayGeom *cols, AdjColumn *colz, AdjAxes *
         if (ia >= g.na) return;
         const RayGeom r = ray_geom(cphi, sphi, ia, ib, g);
         rows[ib + (int64_t)ia * g.nb] = make_float4(r.rz0, r.rz1, tile[tx][j], 0.0f);
-        if (g.nz < 2 || !ray_axial(r, (float)(g.nz / 2)).narrow) axes->general = 1;
+        if (!ray_axial(r, (float)(g.nz / 2), g.nz).narrow) axes->general = 1;
         if (ib != 0) continue;
         cols[ia] = r;
         const RayGeom l = ray_geom(cphi, sphi, ia, g.nb - 1, g);

@@ -293,15 +293,18 @@ __device__ __forceinline__ SlabU slab_u(const RayGeom &r, int d) {
 //          cz0 and cz1 grow with the detector row (products, quotients and
 //          sums round monotonically) and cz0 <= cz1 are the minimum and the
 //          maximum themselves; and dz is in [2^-19, 0.99], so the footprint
-//          spans at most the two slices Z1 and Z1 + 1.
+//          spans at most the two slices Z1 and Z1 + 1.  With one slice nz/2 is
+//          0, and each edge is 0 or at least 2^-79 in magnitude.
 // On a narrow ray's slabs with 0 <= Z1 every division's operands are in
 // mk_div's checked range: dz is; n0 is dz or (Z1 + 1) - zi1 with
 // 0 <= zi1 < Z1 + 1, at least 2^-24 and positive; n1, used only when
-// Z2 = Z1 + 1, is zi2 - (Z1 + 1), +0 or at least an ulp of 1.
+// Z2 = Z1 + 1, is zi2 - (Z1 + 1), +0 or at least an ulp of 1.  With Z1 = -1, n1 is
+// cz1 itself, a sum with nz/2, so +0 or at least 2^-24 for nz/2 >= 1, and +0 or at
+// least 2^-79 with one slice (a product and a sum with +0, never -0).
 struct RayAxial {
     bool zsafe, narrow;
 };
-__device__ __forceinline__ RayAxial ray_axial(const RayGeom &r, float z_half) {
+__device__ __forceinline__ RayAxial ray_axial(const RayGeom &r, float z_half, int nz) {
     const float dc_lo = __fsub_rn(__fsub_rn(0.5f, r.d_half), r.src_d) - 1.0f;
     const float dc_hi = __fsub_rn(__fsub_rn((float)r.nd - 0.5f, r.d_half), r.src_d) + 1.0f;
     const float dmax = fmaxf(fabsf(dc_lo), fabsf(dc_hi));
@@ -317,6 +320,11 @@ __device__ __forceinline__ RayAxial ray_axial(const RayGeom &r, float z_half) {
     const float dz_min = (drz * dmin - 2.0f * err) * (1.0f - 0x1p-20f);
     const float dz_max = (drz * dmax + 2.0f * err) * (1.0f + 0x1p-20f);
     a.narrow = a.zsafe && ordered && dz_min >= 0x1p-19f && dz_max <= 0.99f;
+    if (nz < 2) {
+        // (a factor of 2 for the rounding of these products)
+        const float e0 = fabsf(r.rz0) * dmin, e1 = fabsf(r.rz1) * dmin;
+        a.narrow = a.narrow && (r.rz0 == 0.0f || e0 >= 0x1p-78f) && (r.rz1 == 0.0f || e1 >= 0x1p-78f);
+    }
     return a;
 }
 
@@ -596,9 +604,8 @@ __device__ __forceinline__ void window_read(const unsigned char *w, int z, float
     }
 }
 
-// Two neighbouring staged slabs (narrow rays, nz >= 2).  The branch-free
-// division is exact wherever its quotient is used (ray_axial; with Z1 = -1, n1
-// is cz1 itself, a sum with nz/2 >= 1, so +0 or at least 2^-24).
+// Two neighbouring staged slabs (narrow rays).  The branch-free division is exact
+// wherever its quotient is used (ray_axial).
 // What the reference's loops do not visit is read as zero, so its terms add a
 // zero to the sums: slices outside the volume and a second in-plane voxel that
 // is not visited are zeros in the window, and slice Z1 + 1 of a ray whose Z2 is
@@ -769,9 +776,9 @@ __global__ void __launch_bounds__(FPC_THREADS, MINB) fp_ref_kernel(const FPArgs<
                 const float cphi = cosf(angle), sphi = sinf(angle);  // :23-24
                 // lanes past the last row repeat its ray; nothing of them is stored
                 const RayGeom r = ray_geom(cphi, sphi, ia, min(ib, g.nb - 1), g);
-                const RayAxial ax = ray_axial(r, z_half);
+                const RayAxial ax = ray_axial(r, z_half, nz);
                 w_safe = __all_sync(0xffffffffu, ax.zsafe);
-                w_narrow = __all_sync(0xffffffffu, ax.narrow) && nz >= 2 && g.nzp % 2 == 0;
+                w_narrow = __all_sync(0xffffffffu, ax.narrow) && g.nzp % 2 == 0;
                 // the warp's slabs: those where some ray meets the volume
                 int lo, hi;
                 ray_zrange(r, z_half, nz, lo, hi);
