@@ -480,8 +480,8 @@ __device__ __forceinline__ void fp_slab_general(const RayGeom &r, const Geom &g,
     }
 }
 
-// One slab of one ray straight from memory, for warps whose rays are not
-// narrow: at most two slices Z1, Z1 + 1, with the operand ranges tested; false,
+// One slab of one ray straight from memory, for slabs of narrow warps that are not
+// staged: at most two slices Z1, Z1 + 1, with the operand ranges tested; false,
 // with nothing added, where a lane's footprint does not fit.
 template <int K, bool ONES, typename VT, bool PAIR>
 __device__ __forceinline__ bool fp_slab_direct(float rz0, float rz1, float dc, float a, float b,
@@ -522,6 +522,84 @@ __device__ __forceinline__ bool fp_slab_direct(float rz0, float rz1, float dc, f
             if (p0) accw = __fmaf_rn(wu, wz0, accw);
             if (p1) accw = __fmaf_rn(wu, wz1, accw);
         }
+    }
+    return true;
+}
+
+// One slab of one ray straight from memory, for warps whose rays are not narrow:
+// axial footprints of at most three slices Z1 .. Z1 + 2, with the operand ranges
+// tested; false, with nothing added, where a lane's does not fit.  The in-plane
+// footprint is the table entry's (fast: voxels at o and, if two_u, o + su with
+// weights a, b) or, of any width, worked out again; either is the same for the
+// whole warp.  All of a slab's loads are issued before its terms.
+template <int K, bool ONES, typename VT, bool PAIR>
+__device__ __forceinline__ bool fp_slab_wide(const RayGeom &r, int d, bool fast, float dc, float a,
+                                               float b, int o, int su, int sd, bool two_u,
+                                               const VT *const *base, int nz, float z_half,
+                                               float *acc, float &accw) {
+    // :71-77 / :124-130 ("ratio * xc + z1 + nz / 2", z1 = 0)
+    const float cz0 = __fadd_rn(__fmul_rn(r.rz0, dc), z_half);
+    const float cz1 = __fadd_rn(__fmul_rn(r.rz1, dc), z_half);
+    const float zi1 = fminf(cz0, cz1), zi2 = fmaxf(cz0, cz1);
+    float fz0;
+    const int Z1 = mk_floor(zi1, fz0);
+    const float fz1 = __fadd_rn(fz0, 1.0f), fz2 = __fadd_rn(fz0, 2.0f), dz = __fsub_rn(zi2, zi1);
+    // Z2 = floor(zi2), compared against the exact floats
+    const bool two = zi2 >= fz1, three = zi2 >= fz2;
+    // :86 / :139, the overlaps of slices Z1 (Z1 <= zi1), Z1 + 1 and Z1 + 2
+    const float n0 = __fsub_rn(fminf(fz1, zi2), zi1);
+    const float n1 = __fsub_rn(fminf(fz2, zi2), fz1);
+    const float n2 = __fsub_rn(zi2, fz2);
+    const bool outside = zi2 < 0.0f || zi1 >= (float)nz;
+    const bool ok = outside || (zi2 < __fadd_rn(fz0, 3.0f) && mk_den_ok(dz) && mk_num_ok(n0) &&
+                                (!two || mk_num_ok(n1)) && (!three || mk_num_ok(n2)));
+    if (!__all_sync(0xffffffffu, ok)) return false;
+    const float y = mk_recip(dz);
+    const float wz0 = mk_div(n0, dz, y), wz1 = mk_div(n1, dz, y), wz2 = mk_div(n2, dz, y);
+    const bool p0 = (unsigned)Z1 < (unsigned)nz, p1 = two && (unsigned)(Z1 + 1) < (unsigned)nz;
+    const bool p2 = three && (unsigned)(Z1 + 2) < (unsigned)nz;
+    // (slices outside the volume read 0, and nothing is added for them)
+    const auto load = [&](int at, float (*v)[K]) {
+#pragma unroll
+        for (int j = 0; j < 3; j++)
+            if (j == 0 ? p0 : j == 1 ? p1 : p2) fp_voxel<K, PAIR>(base, at + Z1 + j, v[j]);
+    };
+    const auto add = [&](const float (*v)[K], float wu) {
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            if (p0) acc[k] = __fmaf_rn(__fmul_rn(v[0][k], wu), wz0, acc[k]);
+            if (p1) acc[k] = __fmaf_rn(__fmul_rn(v[1][k], wu), wz1, acc[k]);
+            if (p2) acc[k] = __fmaf_rn(__fmul_rn(v[2][k], wu), wz2, acc[k]);
+        }
+        if (ONES) {
+            if (p0) accw = __fmaf_rn(wu, wz0, accw);
+            if (p1) accw = __fmaf_rn(wu, wz1, accw);
+            if (p2) accw = __fmaf_rn(wu, wz2, accw);
+        }
+    };
+    float v0[3][K], v1[3][K];
+    if (fast) {
+        load(o, v0);
+        if (two_u) load(o + su, v1);
+        add(v0, a);
+        if (two_u) add(v1, b);
+        return true;
+    }
+    const SlabU e = slab_u(r, d);
+    const bool narrow = e.U2 - e.U1 <= 1;
+    const float du = narrow ? 0.0f : __fsub_rn(e.b, e.a);
+    const int u_lo = max(0, e.U1), u_hi = min(r.nu - 1, e.U2);
+    const auto weight = [&](int u) {  // :83 / :136
+        return narrow ? (u == e.U1 ? e.a : e.b)
+                      : __fdiv_rn(__fsub_rn(fminf(__fadd_rn((float)u, 1.0f), e.b),
+                                            fmaxf((float)u, e.a)), du);
+    };
+    for (int u = u_lo; u <= u_hi; u += 2) {
+        const int at = u * su + d * sd;
+        load(at, v0);
+        if (u < u_hi) load(at + su, v1);
+        add(v0, weight(u));
+        if (u < u_hi) add(v1, weight(u + 1));
     }
     return true;
 }
@@ -719,6 +797,47 @@ template <typename VT, bool PAIR, int S, int NST> struct FPShared {
     __align__(16) unsigned char win[NST * S][2][FPWindow<VT, PAIR>::BYTES];
 };
 
+// Slabs i0 .. i0 + 31 of a warp that is not narrow (slab i is wlo + i, n in all): a
+// table of them, one by each lane, and then one slab after another.
+template <int K, bool ONES, typename VT, bool PAIR, typename Shared>
+__device__ __forceinline__ void fp_slabs_wide(Shared &sm, const Geom &g, int wlo, int i0, int n,
+                                              float rz0, float rz1, bool safe, const VT *const *base,
+                                              int nz, float z_half, float *acc, float &accw) {
+    const int lane = threadIdx.x & 31;
+    RayGeom r = sm.ray;
+    int su, sd;
+    zf_strides(r.xdrive, g, su, sd);
+    {
+        SlabCopy c;
+        SlabPair &y = sm.pairs[lane >> 1];
+        int f;
+        float a, b, dc;
+        int zb;
+        slab_entry(r, wlo + min(i0 + lane, n - 1), su, sd, rz0, rz1, false, z_half, nz, c, f, a, b,
+                   dc, zb);
+        sm.copy[lane] = c;
+        sm.flags[lane] = f;
+        y.a[lane & 1] = a;
+        y.b[lane & 1] = b;
+        y.dc[lane & 1] = dc;
+    }
+    __syncwarp();
+    r.rz0 = rz0;
+    r.rz1 = rz1;
+#pragma unroll 1
+    for (int q = 0; q < min(32, n - i0); q++) {
+        const int f = sm.flags[q];
+        if (!(f & SC_ANY)) continue;
+        const SlabPair &y = sm.pairs[q >> 1];
+        if (safe && fp_slab_wide<K, ONES, VT, PAIR>(r, wlo + i0 + q, (f & SC_FAST) != 0, y.dc[q & 1],
+                                                    y.a[q & 1], y.b[q & 1], sm.copy[q].o, su, sd,
+                                                    (f & SC_TWO) != 0, base, nz, z_half, acc, accw))
+            continue;
+        fp_slab_general<K, ONES, VT, PAIR>(r, g, wlo + i0 + q, base, z_half, acc, accw);
+    }
+    __syncwarp();  // the table may be overwritten now
+}
+
 // Row block i of n in dispatch order, from the middle of the detector
 // outwards (m, m+1, m-1, m+2, ...): central rays cross the whole volume,
 // outer ones fewer slabs (ray_zrange), so the longest blocks start first and
@@ -739,10 +858,16 @@ __device__ __forceinline__ int middle_out(int i, int n) {
 // tuning may choose; every choice gives the same bits).
 // PAIR (three volumes): the second and third volumes interleaved in one
 // array, vol.zf[1] (fp_voxel).
+// WIDE: warps that are not narrow take a loop of their own (fp_slabs_wide): at
+// 256x256x160 with 256x192 cells 1.03 slices high 206 us a call, 354 by the stages'
+// one-by-one form; with cells 1.55 high 250 and 463.  Its code beside the stages
+// costs the narrow warps 0 to 1.5 %, so that the launchers leave it out where cells
+// are low (fp_wide).  The bits are the same.
 template <int K> constexpr int fp_stage() { return K >= 3 ? 4 : 8; }
 template <int K> constexpr int fp_min_blocks() { return K >= 3 ? 5 : 6; }
 template <int K, bool ONES, typename VT, typename MT = VT, bool MULTI = false,
-          int S = fp_stage<K>(), int NST = 2, int MINB = fp_min_blocks<K>(), bool PAIR = false>
+          int S = fp_stage<K>(), int NST = 2, int MINB = fp_min_blocks<K>(), bool PAIR = false,
+          bool WIDE = true>
 __global__ void __launch_bounds__(FPC_THREADS, MINB) fp_ref_kernel(const FPArgs<VT, K, MT> p) {
     static_assert(K == 1 || PAIR, "one volume, or three with the last two paired");
     static_assert(32 % S == 0 && S % 2 == 0 && (NST - 1) * S <= 32, "a table holds whole stages");
@@ -811,7 +936,14 @@ __global__ void __launch_bounds__(FPC_THREADS, MINB) fp_ref_kernel(const FPArgs<
             const int64_t lane_off = (lane >> 4) * (int64_t)su + 2 * (lane & 15);
             const unsigned lane_dst = (lane >> 4) * W::BYTES + 2 * W::ES * (lane & 15);
             const int n = wlo <= whi ? whi - wlo + 1 : 0;  // slab i of the warp is wlo + i
-            const int stages = (n + S - 1) / S;
+            // a warp that is not narrow has no staged slab
+            if (WIDE) {
+#pragma unroll 1
+                for (int i0 = 0; !w_narrow && i0 < n; i0 += 32)
+                    fp_slabs_wide<K, ONES, VT, PAIR>(sm, g, wlo, i0, n, rz0, rz1, w_safe, base, nz,
+                                                     z_half, acc, accw);
+            }
+            const int stages = !WIDE || w_narrow ? (n + S - 1) / S : 0;
 
             // Copies the windows of stage s (slabs s*S ..), filling the table
             // of 32 slabs first where the stage begins one.
@@ -827,8 +959,8 @@ __global__ void __launch_bounds__(FPC_THREADS, MINB) fp_ref_kernel(const FPArgs<
                         int f;
                         float a, b, dc;
                         int zb;
-                        slab_entry(rc, wlo + min(i, n - 1), su, sd, rc.rz0, sm.rz_last, w_narrow,
-                                   z_half, nz, c, f, a, b, dc, zb);
+                        slab_entry(rc, wlo + min(i, n - 1), su, sd, rc.rz0, sm.rz_last,
+                                   WIDE || w_narrow, z_half, nz, c, f, a, b, dc, zb);
                         if (i >= n) {
                             f = 0;
                             c.pairs = 0;
@@ -850,7 +982,7 @@ __global__ void __launch_bounds__(FPC_THREADS, MINB) fp_ref_kernel(const FPArgs<
                     }
                     // no window of a warp that is not narrow is read (SC_STAGE), and
                     // at an odd pitch its copies would not be aligned
-                    if (w_narrow) {
+                    if (WIDE || w_narrow) {
                         const SlabCopy *const c = sm.copy + (i0 & 63);
                         const unsigned dst = win0 + s % NST * (S * 2 * W::BYTES);
 #pragma unroll
@@ -900,7 +1032,7 @@ __global__ void __launch_bounds__(FPC_THREADS, MINB) fp_ref_kernel(const FPArgs<
                         RayGeom rc = sm.ray;
                         rc.rz0 = rz0;
                         rc.rz1 = rz1;
-                        if (w_safe && (f & SC_FAST) &&
+                        if ((WIDE || w_safe) && (f & SC_FAST) &&
                             fp_slab_direct<K, ONES, VT, PAIR>(
                                 rz0, rz1, yq.dc[q & 1], yq.a[q & 1], yq.b[q & 1],
                                 o - (yq.zb[q & 1] - MK_MAGIC_BITS), su, (f & SC_TWO) != 0,
@@ -988,16 +1120,24 @@ __global__ void __launch_bounds__(FPC_THREADS, MINB) fp_ref_kernel(const FPArgs<
     }
 }
 
+// Whether a call gains by the loop for warps that are not narrow: cells higher than
+// ray_axial's bound at the volume's far side.
+inline bool fp_wide(const Geom &g) {
+    const float far = g.SO + 0.5f * (float)(g.nx > g.ny ? g.nx : g.ny);
+    return g.db * far > 0.99f * g.SD;
+}
+
 // Launch of fp_ref_kernel, one block per FPC_COLS x FPC_ROWS detector cells and
 // view.
 template <typename VT, bool PAIR, int S, int NST> constexpr size_t fp_ref_smem() {
     return FPC_COLS * sizeof(FPShared<VT, PAIR, S, NST>);
 }
 template <int K, bool ONES, typename VT, typename MT = VT, bool MULTI = false,
-          int S = fp_stage<K>(), int NST = 2, int MINB = fp_min_blocks<K>(), bool PAIR = false>
+          int S = fp_stage<K>(), int NST = 2, int MINB = fp_min_blocks<K>(), bool PAIR = false,
+          bool WIDE = true>
 int launch_fp_ref(mcsart_ctx *ctx, dim3 grid, const FPArgs<VT, K, MT> &a) {
     constexpr size_t smem = fp_ref_smem<VT, PAIR, S, NST>();
-    const auto kernel = fp_ref_kernel<K, ONES, VT, MT, MULTI, S, NST, MINB, PAIR>;
+    const auto kernel = fp_ref_kernel<K, ONES, VT, MT, MULTI, S, NST, MINB, PAIR, WIDE>;
     // above 48 KB with the kernel's static arrays a launch needs the larger limit
     if (smem > 44 * 1024)
         MC_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -68,7 +68,7 @@ static unsigned bits(float f) { unsigned u; memcpy(&u, &f, 4); return u; }
 
 // (FP_IMAGE and FP_MOTION give the sums as residual and pair of a zero measurement:
 //  one volume with the weights' sum, or three volumes)
-template <int K, typename VT> long long run(const Geom &g, float angle) {
+template <int K, typename VT, bool WIDE = true> long long run(const Geom &g, float angle) {
     constexpr bool ONES = K == 1, PAIR = K == 3;
     const int64_t n = (int64_t)g.nx * g.ny * g.nzp, np = (int64_t)g.na * g.nb;
     VT *v0, *v1, *meas;
@@ -98,7 +98,7 @@ template <int K, typename VT> long long run(const Geom &g, float angle) {
     a.norm_part = part;
     plain_kernel<K, ONES, PAIR, VT><<<div_up(np, 128), 128>>>(a, sums);
     constexpr size_t smem = fp_ref_smem<VT, PAIR, fp_stage<K>(), 2>();
-    fp_ref_kernel<K, ONES, VT, VT, false, fp_stage<K>(), 2, fp_min_blocks<K>(), PAIR>
+    fp_ref_kernel<K, ONES, VT, VT, false, fp_stage<K>(), 2, fp_min_blocks<K>(), PAIR, WIDE>
         <<<grid, FPC_THREADS, smem>>>(a);
     CHECK(cudaDeviceSynchronize());
     std::vector<float> s(np * 4), r(np);
@@ -128,7 +128,7 @@ int main(int argc, char **argv) {
     g.ai = strtof(argv[11], nullptr); g.bi = strtof(argv[12], nullptr);
     const float angle = strtof(argv[13], nullptr);
     const long long bad = run<1, float>(g, angle) + run<3, float>(g, angle) + run<1, __half>(g, angle) +
-                          run<3, __nv_bfloat16>(g, angle);
+                          run<3, __nv_bfloat16>(g, angle) + run<1, float, false>(g, angle);
     unsigned long long mis = 0;
     CHECK(cudaMemcpyFromSymbol(&mis, g_misaligned, sizeof(mis)));
     printf("%llu %lld\n", mis, bad);
