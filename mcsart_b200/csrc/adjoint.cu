@@ -39,39 +39,36 @@ struct AdjAxes {
     int general;
 };
 
-// blockDim (32, 8): 32 x 32 rays, turned through shared memory.
+// blockDim (32, 32): 32 x 32 rays, a thread each (four each in 32 x 8 threads took
+// 4 us more where the blocks are few), turned through shared memory.
 // rows[ib + ia*nb] = (rz0, rz1, value)
-static __global__ void adj_rays_kernel(RayGeom *cols, AdjColumn *colz, AdjAxes *axes, float4 *rows,
-                                       const float *proj, float angle, Geom g) {
+static __global__ void __launch_bounds__(1024) adj_rays_kernel(RayGeom *cols, AdjColumn *colz,
+                                                               AdjAxes *axes, float4 *rows,
+                                                               const float *proj, float angle, Geom g) {
     __shared__ float tile[32][33];
     const int tx = threadIdx.x, ty = threadIdx.y;
-    const int a0 = blockIdx.x * 32, b0 = blockIdx.y * 32, ib = b0 + tx;
-    for (int j = ty; j < 32; j += 8)
-        if (a0 + tx < g.na && b0 + j < g.nb) tile[j][tx] = proj[a0 + tx + (int64_t)(b0 + j) * g.na];
+    const int a0 = blockIdx.x * 32, b0 = blockIdx.y * 32, ib = b0 + tx, ia = a0 + ty;
+    if (a0 + tx < g.na && b0 + ty < g.nb) tile[ty][tx] = proj[a0 + tx + (int64_t)(b0 + ty) * g.na];
     __syncthreads();
+    if (ib >= g.nb || ia >= g.na) return;
     const float cphi = cosf(angle), sphi = sinf(angle);  // as the projector
-    if (ib >= g.nb) return;
-    for (int j = ty; j < 32; j += 8) {
-        const int ia = a0 + j;
-        if (ia >= g.na) return;
-        const RayGeom r = ray_geom(cphi, sphi, ia, ib, g);
-        rows[ib + (int64_t)ia * g.nb] = make_float4(r.rz0, r.rz1, tile[tx][j], 0.0f);
-        if (!ray_axial(r, (float)(g.nz / 2), g.nz).narrow) axes->general = 1;
-        if (ib != 0) continue;
-        cols[ia] = r;
-        const RayGeom l = ray_geom(cphi, sphi, ia, g.nb - 1, g);
-        AdjColumn c;
-        c.q0 = 0.5f * (r.rz0 + r.rz1);
-        c.qs = g.nb > 1 ? (0.5f * (l.rz0 + l.rz1) - c.q0) / (float)(g.nb - 1) : 0.0f;
-        c.half = 0.5f * fabsf(r.rz1 - r.rz0);
-        c.axis = r.xdrive ? 1 : 0;
-        colz[ia] = c;
-        if (ia == 0) {
-            axes->d_half[1] = __fdiv_rn((float)g.nx, 2.0f);
-            axes->d_half[0] = __fdiv_rn((float)g.ny, 2.0f);
-            axes->src_d[1] = -__fmul_rn(g.SO, cphi);
-            axes->src_d[0] = -__fmul_rn(g.SO, sphi);
-        }
+    const RayGeom r = ray_geom(cphi, sphi, ia, ib, g);
+    rows[ib + (int64_t)ia * g.nb] = make_float4(r.rz0, r.rz1, tile[tx][ty], 0.0f);
+    if (!ray_axial(r, (float)(g.nz / 2), g.nz).narrow) axes->general = 1;
+    if (ib != 0) return;
+    cols[ia] = r;
+    const RayGeom l = ray_geom(cphi, sphi, ia, g.nb - 1, g);
+    AdjColumn c;
+    c.q0 = 0.5f * (r.rz0 + r.rz1);
+    c.qs = g.nb > 1 ? (0.5f * (l.rz0 + l.rz1) - c.q0) / (float)(g.nb - 1) : 0.0f;
+    c.half = 0.5f * fabsf(r.rz1 - r.rz0);
+    c.axis = r.xdrive ? 1 : 0;
+    colz[ia] = c;
+    if (ia == 0) {
+        axes->d_half[1] = __fdiv_rn((float)g.nx, 2.0f);
+        axes->d_half[0] = __fdiv_rn((float)g.ny, 2.0f);
+        axes->src_d[1] = -__fmul_rn(g.SO, cphi);
+        axes->src_d[0] = -__fmul_rn(g.SO, sphi);
     }
 }
 
@@ -165,19 +162,22 @@ __device__ __forceinline__ float adj_voxel(const float4 *rows, const AdjColumn *
     return acc;
 }
 
-// A block is 32 voxel columns of one row y and ZL slices of them; the lanes of a
-// warp are the ZL slices of 32 / ZL columns.  The slices of a column share its
+// A block is adj_x<ZL>() voxel columns of one row y and ZL slices of them; the lanes
+// of a warp are the ZL slices of 32 / ZL columns.  The slices of a column share its
 // detector columns and their in-plane weights, and neighbouring slices read
 // neighbouring rows.  Bound by instruction issue.  With a voxel per thread, lanes
 // along x, every lane fetched its own columns and rows: one view of a projector
 // and adjoint pair at 256x256x160, 512x384, 909 us, now 394
 // (the gather 529, now 267; 240 with the branch-free division).
-constexpr int ADJ_X = 32, ADJ_THREADS = 256;
+// Volumes of up to four slices take no more lanes than those along z: 512x512x1
+// with a 1024x1 detector 44-46 us by eight, 16-29 by one.
+constexpr int ADJ_THREADS = 256;
+template <int ZL> constexpr int adj_x() { return ZL >= 8 ? 32 : ADJ_THREADS / ZL; }
 template <int ZL>
 static __global__ void __launch_bounds__(ADJ_THREADS) adj_gather_kernel(
     float *img, const float4 *rows, const AdjColumn *colz, const AdjAxes *axes, const SlabU *slabs,
     const int2 *range, Geom g, int nmax) {
-    constexpr int XL = 32 / ZL;
+    constexpr int XL = 32 / ZL, ADJ_X = adj_x<ZL>();
     __shared__ float tile[ZL][ADJ_X + 1];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const unsigned gx = (g.nx + ADJ_X - 1) / ADJ_X, y = blockIdx.x / gx;
@@ -202,7 +202,7 @@ template <int ZL>
 static int launch_adj_gather(mcsart_ctx *ctx, float *img, const float4 *rows, const AdjColumn *colz,
                              const AdjAxes *axes, const SlabU *slabs, const int2 *range,
                              const Geom &g, int nmax) {
-    MC_LAUNCH(ctx, adj_gather_kernel<ZL>, dim3(div_up(g.nx, ADJ_X) * (unsigned)g.ny, div_up(g.nz, ZL)),
+    MC_LAUNCH(ctx, adj_gather_kernel<ZL>, dim3(div_up(g.nx, adj_x<ZL>()) * (unsigned)g.ny, div_up(g.nz, ZL)),
               ADJ_THREADS, 0, img, rows, colz, axes, slabs, range, g, nmax);
     return MCSART_OK;
 }
@@ -223,28 +223,35 @@ MC_EXPORT int mcsart_backprojection_adjoint(mcsart_ctx *ctx, float *d_img, const
     g.na = na; g.nb = nb; g.nx = nx; g.ny = ny; g.nz = nz;
     MC_TRY(validate_geom(g));
     const int nmax = std::max(nx, ny);
-    void *w_cols, *w_colz, *w_axes, *w_rows, *w_slabs, *w_range;
-    MC_TRY(workspace(ctx, "adj_cols", (size_t)na * sizeof(RayGeom), &w_cols));
-    MC_TRY(workspace(ctx, "adj_colz", (size_t)na * sizeof(AdjColumn), &w_colz));
-    MC_TRY(workspace(ctx, "adj_axes", sizeof(AdjAxes), &w_axes));
+    void *w_cols, *w_rows, *w_slabs, *w_range;
+    // the columns' tables in one workspace
+    MC_TRY(workspace(ctx, "adj_cols",
+                     (size_t)na * (sizeof(AdjColumn) + sizeof(RayGeom)) + sizeof(AdjAxes), &w_cols));
     MC_TRY(workspace(ctx, "adj_rows", (size_t)na * nb * sizeof(float4), &w_rows));
     MC_TRY(workspace(ctx, "adj_slabs", (size_t)na * nmax * sizeof(SlabU), &w_slabs));
     const int64_t n_range = 2LL * nmax * nmax;
     MC_TRY(workspace(ctx, "adj_range", (size_t)n_range * sizeof(int2), &w_range));
-    RayGeom *cols = (RayGeom *)w_cols;
-    AdjColumn *colz = (AdjColumn *)w_colz;
-    AdjAxes *axes = (AdjAxes *)w_axes;
+    AdjColumn *colz = (AdjColumn *)w_cols;
+    RayGeom *cols = (RayGeom *)(colz + na);
+    AdjAxes *axes = (AdjAxes *)(cols + na);
     float4 *rows = (float4 *)w_rows;
     SlabU *slabs = (SlabU *)w_slabs;
     int2 *range = (int2 *)w_range;
     MC_LAUNCH(ctx, adj_range_init_kernel, (unsigned)std::min<int64_t>(div_up(n_range, 256), 4096),
               256, 0, range, n_range, axes);
-    MC_LAUNCH(ctx, adj_rays_kernel, dim3(div_up(na, 32), div_up(nb, 32)), dim3(32, 8), 0, cols, colz,
+    MC_LAUNCH(ctx, adj_rays_kernel, dim3(div_up(na, 32), div_up(nb, 32)), dim3(32, 32), 0, cols, colz,
               axes, rows, d_proj, angle, g);
     MC_LAUNCH(ctx, adj_slabs_kernel, dim3(div_up(na, 128), nmax), 128, 0, cols, slabs, range, g,
               nmax);
-    // 32 slices a warp, 8 where a quarter or more of its lanes would have none
-    if (div_up(nz, 32) * 32 - nz < nz / 4)
+    // 32 slices a warp, 8 where a quarter or more of its lanes would have none, as
+    // many as there are below that
+    if (nz == 1)
+        MC_TRY(launch_adj_gather<1>(ctx, d_img, rows, colz, axes, slabs, range, g, nmax));
+    else if (nz == 2)
+        MC_TRY(launch_adj_gather<2>(ctx, d_img, rows, colz, axes, slabs, range, g, nmax));
+    else if (nz <= 4)
+        MC_TRY(launch_adj_gather<4>(ctx, d_img, rows, colz, axes, slabs, range, g, nmax));
+    else if (div_up(nz, 32) * 32 - nz < nz / 4)
         MC_TRY(launch_adj_gather<32>(ctx, d_img, rows, colz, axes, slabs, range, g, nmax));
     else
         MC_TRY(launch_adj_gather<8>(ctx, d_img, rows, colz, axes, slabs, range, g, nmax));
