@@ -129,11 +129,13 @@ __device__ __forceinline__ float adj_voxel(const float4 *rows, const AdjColumn *
             }
             // rows whose axial footprint can reach z: its centre c0 + s * row is
             // linear in the row; tol (slices) covers the rounding of these
-            // floats and of the ratios, and every candidate is tested exactly
+            // floats and of the ratios (2^-21 of the distance from the centre
+            // plane, at most nz/2 within the volume), and every candidate is
+            // tested exactly
             int ib_lo = 0, ib_hi = nb - 1;
             const float c0 = c.q0 * dc + z_half, s = c.qs * dc;
             if (fabsf(s) > 1e-6f) {
-                const float tol = 1e-3f + 0x1p-18f * (fabsf(c0) + fabsf(s) * (float)nb);
+                const float tol = 1e-3f + 0x1p-18f * (fabsf(c0) + fabsf(s) * (float)nb + z_half);
                 const float h = c.half * fabsf(dc) + 0.5f + tol, m = fz + 0.5f - c0, y = 1.0f / s;
                 const float ta = (m - h) * y, tb = (m + h) * y;
                 const float lo = fminf(ta, tb), hi = fmaxf(ta, tb);
