@@ -108,7 +108,14 @@ MC_EXPORT int mcsart_projection(mcsart_ctx *ctx, float *d_proj, const float *d_i
     MC_TRY(validate_geom(g));
     const float *imgZ;
     void *owned;
-    MC_TRY(zfast_copy(ctx, "fp_volZ", d_img, g, &imgZ, &owned));
+    const int rc = zfast_copy(ctx, "fp_volZ", d_img, g, &imgZ, &owned);
+    if (rc == MCSART_ERR_OUT_OF_MEMORY) {
+        (void)cudaGetLastError();
+        clear_error();
+        MC_LAUNCH(ctx, fp_nocopy_kernel, dim3(div_up(na, 128), nb), 128, 0, d_proj, d_img, angle, g);
+        return finish(ctx, "mcsart_projection");
+    }
+    MC_TRY(rc);
     MC_TRY(launch_fp_plain<1>(ctx, d_proj, imgZ, angle, nullptr, 1, g));
     MC_TRY(zfast_free(ctx, owned));
     return finish(ctx, "mcsart_projection");

@@ -1,0 +1,64 @@
+"""Calls with little device memory left: those that kept a smaller scratch, or none,
+before they took the present forms fall back to forms with as little, with the
+same bits."""
+import numpy as np
+import pytest
+
+from conftest import geo, host
+
+pytestmark = pytest.mark.gpu
+
+ARGS = ("SO", "SD", "da", "na", "ai", "db", "nb", "bi", "nx", "ny", "nz")
+MB = 1 << 20
+
+
+class Full:
+    """Holds device memory so that about `left` MB are free."""
+
+    def __init__(self, torch, left):
+        self.torch, self.left = torch, left
+
+    def __enter__(self):
+        torch = self.torch
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        self.held, step = [], 1 << 36
+        while step >= 2 * MB:
+            spare = torch.cuda.mem_get_info()[0] - self.left * MB
+            n = min(step, spare) // (2 * MB) * (2 * MB)
+            if n <= 0:
+                break
+            try:
+                self.held.append(torch.empty(n, dtype=torch.uint8, device="cuda"))
+            except torch.cuda.OutOfMemoryError:
+                step //= 2
+        free = torch.cuda.mem_get_info()[0]
+        assert (self.left - 8) * MB <= free <= (self.left + 8) * MB, free
+
+    def __exit__(self, *exc):
+        del self.held
+        self.torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("angle", [0.3, 1.5])
+def test_projection_without_room_for_a_copy(torch_cuda, angle):
+    import mcsart_b200 as m
+    torch = torch_cuda
+    g = geo(nx=320, ny=300, nz=301, na=70, nb=61, SO=900.0, SD=1350.0, da=6.5, db=7.2)
+    a = [g[k] for k in ARGS]
+    img = torch.rand((301, 300, 320), device="cuda")  # 115 MB
+    want, got = (torch.full((61, 70), 7.0, device="cuda") for _ in range(2))
+    with m.Context() as c:
+        torch.cuda.synchronize()
+        c.host_projection(want, img, angle, *a)
+        c.synchronize()
+    with m.Context() as c:
+        small = geo()
+        c.host_projection(torch.zeros((28, 40), device="cuda"), torch.zeros((16, 20, 24), device="cuda"),
+                          angle, *[small[k] for k in ARGS])
+        c.synchronize()
+        with Full(torch, 64):
+            c.host_projection(got, img, angle, *a)
+            c.synchronize()
+    np.testing.assert_array_equal(host(got), host(want))
+    assert host(want).any()
