@@ -294,13 +294,26 @@ MC_EXPORT int mcsart_invert_dvf(mcsart_ctx *ctx, float *inv_x, float *inv_y, flo
     MC_REQUIRE(nx == ny, "the warp is a displacement field only for square slices (nx == ny)");
     MC_REQUIRE(n_iter >= 1 && n_iter <= 64, "n_iter must be in [1, 64]");
     const int64_t n = nvox(nx, ny, nz);
-    void *ws;
-    MC_TRY(workspace(ctx, "inv_m", n * sizeof(float4), &ws));
-    float4 *m = (float4 *)ws;
     const Fields<float> f{ax, ay, az, bx, by, bz};
+    const dim3 grid(div_up(nx, 32), div_up(ny, 8), nz), block(32, 8);
+    void *ws;
+    const int rc = workspace(ctx, "inv_m", n * sizeof(float4), &ws);
+    if (rc == MCSART_ERR_OUT_OF_MEMORY) {
+        (void)cudaGetLastError();
+        clear_error();
+        MC_TRY(workspace(ctx, "inv_m", n * 3 * sizeof(float), &ws));
+        float *const m = (float *)ws;
+        MC_LAUNCH(ctx, forward_dvf_kernel<false>, stream_blocks(n), 256, 0, m, m + n, m + 2 * n, f, n,
+                  volume, flow);
+        MC_LAUNCH(ctx, invert_dvf_kernel, grid, block, 0, inv_x, inv_y, inv_z,
+                  (DispPlanes{m, m + n, m + 2 * n}), nx, ny, nz, n_iter);
+        return finish(ctx, "mcsart_invert_dvf");
+    }
+    MC_TRY(rc);
+    float4 *m = (float4 *)ws;
     MC_LAUNCH(ctx, forward_dvf4_kernel, stream_blocks(n), 256, 0, m, f, n, volume, flow);
-    MC_LAUNCH(ctx, invert_dvf_kernel, dim3(div_up(nx, 32), div_up(ny, 8), nz), dim3(32, 8), 0,
-              inv_x, inv_y, inv_z, m, nx, ny, nz, n_iter);
+    MC_LAUNCH(ctx, invert_dvf_kernel, grid, block, 0, inv_x, inv_y, inv_z, DispPacked{m}, nx, ny, nz,
+              n_iter);
     return finish(ctx, "mcsart_invert_dvf");
 }
 

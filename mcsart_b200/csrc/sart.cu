@@ -432,7 +432,7 @@ template <typename ST, int INTERP, int SUM> struct Runner {
             MC_LAUNCH(ctx, forward_dvf4_kernel, stream_blocks(V), 256, 0, m, ff, V, volume, flow);
             ctx->label = "dvf_inverse";
             MC_LAUNCH(ctx, invert_dvf_kernel, dim3(div_up(g.nx, 32), div_up(g.ny, 8), g.nz),
-                      dim3(32, 8), 0, n, n + V, n + 2 * V, m, g.nx, g.ny, g.nz, inv_iters);
+                      dim3(32, 8), 0, n, n + V, n + 2 * V, DispPacked{m}, g.nx, g.ny, g.nz, inv_iters);
             ctx->label = "warp_back_add";
             if (hw) {
                 MC_LAUNCH(ctx, warp_back_add_disp_kernel<SrcTex>, tile_grid(), dim3(32, 8), 0,

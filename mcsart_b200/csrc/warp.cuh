@@ -367,9 +367,20 @@ static __global__ void __launch_bounds__(256) warp_back_add_kernel(
 // returned in the forward layout: ox = N_Y, oy = N_X, oz = N_Z, so that a
 // warp with displacement (ox, oy, oz) undoes the warp with (mx, my, mz).
 // blockDim (32, 8), 32x8 tiles of slice blockIdx.z.
-// m: the displacement as float4 (mx, my, mz, 0) per voxel, so that the three
-// components of a corner are one load (24 loads a step from three arrays took
-// 688 us at 256x256x160 and 8 steps).
+// SRC: the displacement's corners.  DispPacked, as float4 (mx, my, mz, 0) per voxel,
+// so that the three components of a corner are one load; DispPlanes, three arrays,
+// where there is no memory for the fourth component (688 us against 430 at
+// 256x256x160 and 8 steps).
+struct DispPacked {
+    const float4 *m;
+    __device__ __forceinline__ float4 at(int i) const { return __ldg(m + i); }
+};
+struct DispPlanes {
+    const float *x, *y, *z;
+    __device__ __forceinline__ float4 at(int i) const {
+        return make_float4(__ldg(x + i), __ldg(y + i), __ldg(z + i), 0.0f);
+    }
+};
 __device__ __forceinline__ float lerp8(float t000, float t100, float t010, float t110, float t001,
                                        float t101, float t011, float t111, float a, float b,
                                        float c) {
@@ -379,8 +390,9 @@ __device__ __forceinline__ float lerp8(float t000, float t100, float t010, float
     const float c0 = fmaf(b, c10 - c00, c00), c1 = fmaf(b, c11 - c01, c01);
     return fmaf(c, c1 - c0, c0);
 }
+template <typename SRC>
 static __global__ void __launch_bounds__(256) invert_dvf_kernel(float *ox, float *oy, float *oz,
-                                                                const float4 *m, int nx, int ny,
+                                                                const SRC m, int nx, int ny,
                                                                 int nz, int iters) {
     const int X = blockIdx.x * 32 + threadIdx.x, Y = blockIdx.y * 8 + threadIdx.y, Z = blockIdx.z;
     if (X >= nx || Y >= ny) return;
@@ -393,11 +405,11 @@ static __global__ void __launch_bounds__(256) invert_dvf_kernel(float *ox, float
         lin_axis(py, ny, y0, y1, b);
         lin_axis(pz, nz, z0, z1, c);
         const int sz = nx * ny;  // fits: volumes hold fewer than 2^31 voxels
-        const float4 *const r00 = m + (y0 * nx + z0 * sz), *const r10 = m + (y1 * nx + z0 * sz);
-        const float4 *const r01 = m + (y0 * nx + z1 * sz), *const r11 = m + (y1 * nx + z1 * sz);
-        const float4 t000 = __ldg(r00 + x0), t100 = __ldg(r00 + x1), t010 = __ldg(r10 + x0),
-                     t110 = __ldg(r10 + x1), t001 = __ldg(r01 + x0), t101 = __ldg(r01 + x1),
-                     t011 = __ldg(r11 + x0), t111 = __ldg(r11 + x1);
+        const int r00 = y0 * nx + z0 * sz, r10 = y1 * nx + z0 * sz;
+        const int r01 = y0 * nx + z1 * sz, r11 = y1 * nx + z1 * sz;
+        const float4 t000 = m.at(r00 + x0), t100 = m.at(r00 + x1), t010 = m.at(r10 + x0),
+                     t110 = m.at(r10 + x1), t001 = m.at(r01 + x0), t101 = m.at(r01 + x1),
+                     t011 = m.at(r11 + x0), t111 = m.at(r11 + x1);
 #define MC_LERP(q) lerp8(t000.q, t100.q, t010.q, t110.q, t001.q, t101.q, t011.q, t111.q, a, b, c)
         // D = (my, mx, mz): the in-slice transposed index swaps the first two
         const float dX = MC_LERP(y), dY = MC_LERP(x), dZ = MC_LERP(z);

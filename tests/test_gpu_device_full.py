@@ -62,3 +62,23 @@ def test_projection_without_room_for_a_copy(torch_cuda, angle):
             c.synchronize()
     np.testing.assert_array_equal(host(got), host(want))
     assert host(want).any()
+
+
+def test_dvf_inverse_without_room_for_packed_displacements(torch_cuda):
+    import mcsart_b200 as m
+    torch = torch_cuda
+    n = (224, 224, 200)  # 40 MB an array
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    fields = torch.rand((6, n[2], n[1], n[0]), device="cuda", generator=gen) * 2 - 1
+    want, got = (torch.zeros((3, n[2], n[1], n[0]), device="cuda") for _ in range(2))
+    with m.Context() as c:
+        torch.cuda.synchronize()
+        c.invert_dvf(*want, *fields, 0.7, 0.3, *n, 5)
+        c.synchronize()
+    with m.Context() as c:
+        c.invert_dvf(*got[:, :1, :1, :1].contiguous().cuda(), *fields, 0.7, 0.3, 1, 1, 1, 1)
+        c.synchronize()
+        with Full(torch, 136):  # between 3 and 4 arrays
+            c.invert_dvf(*got, *fields, 0.7, 0.3, *n, 5)
+            c.synchronize()
+    np.testing.assert_array_equal(host(got), host(want))
