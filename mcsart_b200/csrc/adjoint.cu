@@ -39,11 +39,34 @@ struct AdjAxes {
     int general;
 };
 
+// A ray for the gather: its axial ratios and its value; RowNarrow, the ratios alone,
+// the value read where the projection is (where there is no memory for RowWide).
+struct __align__(16) RowWide {
+    float rz0, rz1, value, pad;
+    __device__ __forceinline__ void set(float a, float b, float v) {
+        *reinterpret_cast<float4 *>(this) = make_float4(a, b, v, 0.0f);
+    }
+};
+struct __align__(8) RowNarrow {
+    float rz0, rz1;
+    __device__ __forceinline__ void set(float a, float b, float) {
+        *reinterpret_cast<float2 *>(this) = make_float2(a, b);
+    }
+};
+__device__ __forceinline__ float4 adj_row(const RowWide *row, int ib, const float *, int) {
+    return __ldg(reinterpret_cast<const float4 *>(row + ib));
+}
+__device__ __forceinline__ float4 adj_row(const RowNarrow *row, int ib, const float *proj, int na) {
+    const float2 q = __ldg(reinterpret_cast<const float2 *>(row + ib));
+    return make_float4(q.x, q.y, __ldg(proj + (int64_t)ib * na), 0.0f);
+}
+
 // blockDim (32, 32): 32 x 32 rays, a thread each (four each in 32 x 8 threads took
 // 4 us more where the blocks are few), turned through shared memory.
-// rows[ib + ia*nb] = (rz0, rz1, value)
+// rows[ib + ia*nb]
+template <typename ROW>
 static __global__ void __launch_bounds__(1024) adj_rays_kernel(RayGeom *cols, AdjColumn *colz,
-                                                               AdjAxes *axes, float4 *rows,
+                                                               AdjAxes *axes, ROW *rows,
                                                                const float *proj, float angle, Geom g) {
     __shared__ float tile[32][33];
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -53,7 +76,7 @@ static __global__ void __launch_bounds__(1024) adj_rays_kernel(RayGeom *cols, Ad
     if (ib >= g.nb || ia >= g.na) return;
     const float cphi = cosf(angle), sphi = sinf(angle);  // as the projector
     const RayGeom r = ray_geom(cphi, sphi, ia, ib, g);
-    rows[ib + (int64_t)ia * g.nb] = make_float4(r.rz0, r.rz1, tile[tx][ty], 0.0f);
+    rows[ib + (int64_t)ia * g.nb].set(r.rz0, r.rz1, tile[tx][ty]);
     if (!ray_axial(r, (float)(g.nz / 2), g.nz).narrow) axes->general = 1;
     if (ib != 0) return;
     cols[ia] = r;
@@ -100,9 +123,9 @@ static __global__ void adj_slabs_kernel(const RayGeom *cols, SlabU *slabs, int2 
 
 // Voxel (x, y, z) of the gather.  NARROW: every ray is (AdjAxes): the axial edges
 // are in order, and the branch-free division is exact (ray_axial, fp_pair_staged).
-template <bool NARROW>
-__device__ __forceinline__ float adj_voxel(const float4 *rows, const AdjColumn *colz,
-                                           const AdjAxes &axes, const SlabU *slabs,
+template <bool NARROW, typename ROW>
+__device__ __forceinline__ float adj_voxel(const ROW *rows, const float *proj,
+                                           const AdjColumn *colz, const AdjAxes &axes, const SlabU *slabs,
                                            const int2 *range, const Geom &g, int nmax, int x, int y,
                                            int z) {
     const float z_half = (float)(g.nz / 2), fz = (float)z;
@@ -143,9 +166,9 @@ __device__ __forceinline__ float adj_voxel(const float4 *rows, const AdjColumn *
                 ib_lo = max(0, (int)ceilf(fmaxf(lo, 0.0f)));
                 ib_hi = min(nb - 1, (int)floorf(fminf(hi, (float)(nb - 1))));
             }
-            const float4 *const row = rows + (int64_t)ia * nb;
+            const ROW *const row = rows + (int64_t)ia * nb;
             for (int ib = ib_lo; ib <= ib_hi; ib++) {
-                const float4 q = __ldg(row + ib);
+                const float4 q = adj_row(row, ib, proj + ia, g.na);
                 // the projector's axial footprint (fp_slab_general)
                 const float cz0 = __fadd_rn(__fmul_rn(q.x, dc), z_half);
                 const float cz1 = __fadd_rn(__fmul_rn(q.y, dc), z_half);
@@ -175,9 +198,9 @@ __device__ __forceinline__ float adj_voxel(const float4 *rows, const AdjColumn *
 // with a 1024x1 detector 44-46 us by eight, 16-29 by one.
 constexpr int ADJ_THREADS = 256;
 template <int ZL> constexpr int adj_x() { return ZL >= 8 ? 32 : ADJ_THREADS / ZL; }
-template <int ZL>
+template <int ZL, typename ROW>
 static __global__ void __launch_bounds__(ADJ_THREADS) adj_gather_kernel(
-    float *img, const float4 *rows, const AdjColumn *colz, const AdjAxes *axes, const SlabU *slabs,
+    float *img, const ROW *rows, const float *proj, const AdjColumn *colz, const AdjAxes *axes, const SlabU *slabs,
     const int2 *range, Geom g, int nmax) {
     constexpr int XL = 32 / ZL, ADJ_X = adj_x<ZL>();
     __shared__ float tile[ZL][ADJ_X + 1];
@@ -188,9 +211,9 @@ static __global__ void __launch_bounds__(ADJ_THREADS) adj_gather_kernel(
     const AdjAxes ax = *axes;
     for (int cx = warp * XL + lane / ZL; cx < ADJ_X; cx += ADJ_THREADS / ZL)
         if (x0 + cx < g.nx && zb + lz < g.nz)
-            tile[lz][cx] = ax.general ? adj_voxel<false>(rows, colz, ax, slabs, range, g, nmax,
+            tile[lz][cx] = ax.general ? adj_voxel<false>(rows, proj, colz, ax, slabs, range, g, nmax,
                                                          x0 + cx, (int)y, zb + lz)
-                                      : adj_voxel<true>(rows, colz, ax, slabs, range, g, nmax,
+                                      : adj_voxel<true>(rows, proj, colz, ax, slabs, range, g, nmax,
                                                         x0 + cx, (int)y, zb + lz);
     __syncthreads();
     for (int i = t; i < ZL * ADJ_X; i += ADJ_THREADS) {
@@ -200,12 +223,41 @@ static __global__ void __launch_bounds__(ADJ_THREADS) adj_gather_kernel(
     }
 }
 
-template <int ZL>
-static int launch_adj_gather(mcsart_ctx *ctx, float *img, const float4 *rows, const AdjColumn *colz,
+template <int ZL, typename ROW>
+static int launch_adj_gather(mcsart_ctx *ctx, float *img, const ROW *rows, const float *proj,
+                             const AdjColumn *colz,
                              const AdjAxes *axes, const SlabU *slabs, const int2 *range,
                              const Geom &g, int nmax) {
-    MC_LAUNCH(ctx, adj_gather_kernel<ZL>, dim3(div_up(g.nx, adj_x<ZL>()) * (unsigned)g.ny, div_up(g.nz, ZL)),
-              ADJ_THREADS, 0, img, rows, colz, axes, slabs, range, g, nmax);
+    MC_LAUNCH(ctx, (adj_gather_kernel<ZL, ROW>), dim3(div_up(g.nx, adj_x<ZL>()) * (unsigned)g.ny, div_up(g.nz, ZL)),
+              ADJ_THREADS, 0, img, rows, proj, colz, axes, slabs, range, g, nmax);
+    return MCSART_OK;
+}
+
+// The passes of a view, with the scratch laid out.
+template <typename ROW>
+static int launch_adjoint(mcsart_ctx *ctx, float *img, const float *proj, float angle, const Geom &g,
+                          RayGeom *cols, AdjColumn *colz, AdjAxes *axes, ROW *rows, SlabU *slabs,
+                          int2 *range) {
+    const int nx = g.nx, ny = g.ny, nz = g.nz, na = g.na, nb = g.nb, nmax = std::max(nx, ny);
+    const int64_t n_range = 2LL * nmax * nmax;
+    MC_LAUNCH(ctx, adj_range_init_kernel, (unsigned)std::min<int64_t>(div_up(n_range, 256), 4096),
+              256, 0, range, n_range, axes);
+    MC_LAUNCH(ctx, adj_rays_kernel<ROW>, dim3(div_up(na, 32), div_up(nb, 32)), dim3(32, 32), 0, cols, colz,
+              axes, rows, proj, angle, g);
+    MC_LAUNCH(ctx, adj_slabs_kernel, dim3(div_up(na, 128), nmax), 128, 0, cols, slabs, range, g,
+              nmax);
+    // 32 slices a warp, 8 where a quarter or more of its lanes would have none, as
+    // many as there are below that
+    if (nz == 1)
+        MC_TRY(launch_adj_gather<1>(ctx, img, rows, proj, colz, axes, slabs, range, g, nmax));
+    else if (nz == 2)
+        MC_TRY(launch_adj_gather<2>(ctx, img, rows, proj, colz, axes, slabs, range, g, nmax));
+    else if (nz <= 4)
+        MC_TRY(launch_adj_gather<4>(ctx, img, rows, proj, colz, axes, slabs, range, g, nmax));
+    else if (div_up(nz, 32) * 32 - nz < nz / 4)
+        MC_TRY(launch_adj_gather<32>(ctx, img, rows, proj, colz, axes, slabs, range, g, nmax));
+    else
+        MC_TRY(launch_adj_gather<8>(ctx, img, rows, proj, colz, axes, slabs, range, g, nmax));
     return MCSART_OK;
 }
 
@@ -229,33 +281,27 @@ MC_EXPORT int mcsart_backprojection_adjoint(mcsart_ctx *ctx, float *d_img, const
     // the columns' tables in one workspace
     MC_TRY(workspace(ctx, "adj_cols",
                      (size_t)na * (sizeof(AdjColumn) + sizeof(RayGeom)) + sizeof(AdjAxes), &w_cols));
-    MC_TRY(workspace(ctx, "adj_rows", (size_t)na * nb * sizeof(float4), &w_rows));
     MC_TRY(workspace(ctx, "adj_slabs", (size_t)na * nmax * sizeof(SlabU), &w_slabs));
     const int64_t n_range = 2LL * nmax * nmax;
     MC_TRY(workspace(ctx, "adj_range", (size_t)n_range * sizeof(int2), &w_range));
+    int rc = workspace(ctx, "adj_rows", (size_t)na * nb * sizeof(RowWide), &w_rows);
+    const bool narrow = rc == MCSART_ERR_OUT_OF_MEMORY;
+    if (narrow) {
+        (void)cudaGetLastError();
+        clear_error();
+        rc = workspace(ctx, "adj_rows", (size_t)na * nb * sizeof(RowNarrow), &w_rows);
+    }
+    MC_TRY(rc);
     AdjColumn *colz = (AdjColumn *)w_cols;
     RayGeom *cols = (RayGeom *)(colz + na);
     AdjAxes *axes = (AdjAxes *)(cols + na);
-    float4 *rows = (float4 *)w_rows;
     SlabU *slabs = (SlabU *)w_slabs;
     int2 *range = (int2 *)w_range;
-    MC_LAUNCH(ctx, adj_range_init_kernel, (unsigned)std::min<int64_t>(div_up(n_range, 256), 4096),
-              256, 0, range, n_range, axes);
-    MC_LAUNCH(ctx, adj_rays_kernel, dim3(div_up(na, 32), div_up(nb, 32)), dim3(32, 32), 0, cols, colz,
-              axes, rows, d_proj, angle, g);
-    MC_LAUNCH(ctx, adj_slabs_kernel, dim3(div_up(na, 128), nmax), 128, 0, cols, slabs, range, g,
-              nmax);
-    // 32 slices a warp, 8 where a quarter or more of its lanes would have none, as
-    // many as there are below that
-    if (nz == 1)
-        MC_TRY(launch_adj_gather<1>(ctx, d_img, rows, colz, axes, slabs, range, g, nmax));
-    else if (nz == 2)
-        MC_TRY(launch_adj_gather<2>(ctx, d_img, rows, colz, axes, slabs, range, g, nmax));
-    else if (nz <= 4)
-        MC_TRY(launch_adj_gather<4>(ctx, d_img, rows, colz, axes, slabs, range, g, nmax));
-    else if (div_up(nz, 32) * 32 - nz < nz / 4)
-        MC_TRY(launch_adj_gather<32>(ctx, d_img, rows, colz, axes, slabs, range, g, nmax));
+    if (narrow)
+        MC_TRY(launch_adjoint(ctx, d_img, d_proj, angle, g, cols, colz, axes, (RowNarrow *)w_rows, slabs,
+                              range));
     else
-        MC_TRY(launch_adj_gather<8>(ctx, d_img, rows, colz, axes, slabs, range, g, nmax));
+        MC_TRY(launch_adjoint(ctx, d_img, d_proj, angle, g, cols, colz, axes, (RowWide *)w_rows, slabs,
+                              range));
     return finish(ctx, "mcsart_backprojection_adjoint");
 }

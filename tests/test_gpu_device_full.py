@@ -82,3 +82,27 @@ def test_dvf_inverse_without_room_for_packed_displacements(torch_cuda):
             c.invert_dvf(*got, *fields, 0.7, 0.3, *n, 5)
             c.synchronize()
     np.testing.assert_array_equal(host(got), host(want))
+
+
+def test_adjoint_without_room_for_the_rays_values(torch_cuda):
+    import mcsart_b200 as m
+    torch = torch_cuda
+    # 64 MB of ray values and ratios, 32 MB of ratios; a few MB of tables
+    g = geo(nx=40, ny=36, nz=33, na=2048, nb=2048, SO=120.0, SD=180.0, da=0.05, db=0.05)
+    a = [g[k] for k in ARGS]
+    proj = torch.rand((2048, 2048), device="cuda", generator=torch.Generator(device="cuda").manual_seed(2))
+    want, got = (torch.zeros((33, 36, 40), device="cuda") for _ in range(2))
+    small = geo()
+    with m.Context() as c:
+        torch.cuda.synchronize()
+        c.host_backprojection_adjoint(want, proj, 0.3, *a)
+        c.synchronize()
+    with m.Context() as c:
+        c.host_backprojection_adjoint(torch.zeros((16, 20, 24), device="cuda"),
+                                      torch.zeros((28, 40), device="cuda"), 0.3, *[small[k] for k in ARGS])
+        c.synchronize()
+        with Full(torch, 56):
+            c.host_backprojection_adjoint(got, proj, 0.3, *a)
+            c.synchronize()
+    np.testing.assert_array_equal(host(got), host(want))
+    assert host(want).any()
