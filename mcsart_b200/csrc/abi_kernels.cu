@@ -276,7 +276,10 @@ MC_EXPORT int mcsart_forward_dvf(mcsart_ctx *ctx, float *mx, float *my, float *m
     MC_REQUIRE(mx && my && mz && ax && ay && az && bx && by && bz, "pointers must be non-NULL");
     const int64_t n = nvox(nx, ny, nz);
     const Fields<float> f{ax, ay, az, bx, by, bz};
-    const bool vec = aligned16({mx, my, mz, ax, ay, az, bx, by, bz});
+    // (a component computed in place of a later one's field is read back there, as
+    // the reference's kernel does, voxel by voxel)
+    const bool shared = mx == ay || mx == by || mx == az || mx == bz || my == az || my == bz;
+    const bool vec = !shared && aligned16({mx, my, mz, ax, ay, az, bx, by, bz});
     MC_LAUNCH(ctx, (vec ? &forward_dvf_kernel<true> : &forward_dvf_kernel<false>),
               pointwise_blocks(n, vec), 256, 0, mx, my, mz, f, n, volume, flow);
     return finish(ctx, "mcsart_forward_dvf");

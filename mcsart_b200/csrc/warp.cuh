@@ -146,7 +146,8 @@ static __global__ void __launch_bounds__(256) deform_kernel(FT *out, const SRC s
 }
 template <int N> inline unsigned warp_blocks(const Grid3 &g) { return div_up(g.n, 256 * N); }
 
-// Drop-in kernel_forwardDVF (bound by memory; VEC: four voxels per thread).
+// Drop-in kernel_forwardDVF (bound by memory; VEC: four voxels per thread, all fields
+// read before the first component is stored).
 template <bool VEC>
 static __global__ void __launch_bounds__(256) forward_dvf_kernel(float *mx, float *my, float *mz,
                                                                  Fields<float> f, int64_t n,
