@@ -35,14 +35,9 @@ int launch_fp_plain(mcsart_ctx *ctx, float *d_proj, const float *d_imgZ, float a
     a.out = d_proj;
     // the reference's summation order: bitwise the reference kernel's output
     const dim3 grid(div_up(g.na, FPC_COLS), div_up(g.nb, FPC_ROWS), n_views);
-    constexpr int S = fp_stage<K>(), MINB = fp_min_blocks<K>();
-    const bool wide = fp_wide(g);
     // several views (mcsart_projection_views): the multi-view instantiation
-    if (n_views > 1 && wide) return launch_fp_ref<K, false, float, float, true>(ctx, grid, a);
-    if (n_views > 1)
-        return launch_fp_ref<K, false, float, float, true, S, 2, MINB, false, false>(ctx, grid, a);
-    if (wide) return launch_fp_ref<K, false, float>(ctx, grid, a);
-    return launch_fp_ref<K, false, float, float, false, S, 2, MINB, false, false>(ctx, grid, a);
+    if (n_views > 1) return launch_fp_ref<K, false, float, float, true>(ctx, grid, a);
+    return launch_fp_ref<K, false, float>(ctx, grid, a);
 }
 
 // The z-fastest copy of a volume the projector reads, in a workspace; in a

@@ -21,6 +21,9 @@ static __device__ __align__(256) float g_noalloc_volZ[MCSART_NOALLOC_MAX_VOXELS]
 
 namespace {
 
+constexpr auto WideKernel = fp_ref_kernel<1, false, float, float, false, fp_stage<1>(), 2,
+                                          fp_min_blocks<1>(), false, true>;
+
 constexpr int kMaxDevices = 64;
 std::mutex g_setup_mu;
 
@@ -102,6 +105,7 @@ int scratch_of_current_device(float **out) {
     MC_CHECK_CUDA(cudaFuncGetAttributes(&fa, zfast_kernel<float, float>));
     MC_CHECK_CUDA(cudaFuncGetAttributes(&fa, zfast_thin_kernel<float, float>));
     MC_CHECK_CUDA(cudaFuncGetAttributes(&fa, fp_ref_kernel<1, false, float>));
+    MC_CHECK_CUDA(cudaFuncGetAttributes(&fa, WideKernel));
     unsigned long long id = 0;
     MC_TRY(current_context_id(&id));
     s.ctx_id = id;
@@ -143,7 +147,10 @@ MC_EXPORT int mcsart_projection_noalloc(void *stream, float *d_proj, const float
     a.out = d_proj;
     const dim3 grid(div_up(na, FPC_COLS), div_up(nb, FPC_ROWS), 1);
     constexpr size_t smem = fp_ref_smem<float, false, fp_stage<1>(), 2>();
-    fp_ref_kernel<1, false, float><<<grid, dim3(FPC_THREADS), smem, s>>>(a);
+    if (fp_wide(g))
+        WideKernel<<<grid, dim3(FPC_THREADS), smem, s>>>(a);
+    else
+        fp_ref_kernel<1, false, float><<<grid, dim3(FPC_THREADS), smem, s>>>(a);
     MC_CHECK_CUDA(cudaGetLastError());
     return MCSART_OK;
 }

@@ -624,6 +624,9 @@ template <typename VT, bool PAIR> struct FPWindow {
 #ifndef MCSART_ON_COPY
 #define MCSART_ON_COPY(dst, src, n)  // a test program's check of the addresses
 #endif
+#ifndef MCSART_ON_FORM
+#define MCSART_ON_FORM(form)  // and its count of the forms that warps take
+#endif
 template <int N> __device__ __forceinline__ void cp_async(unsigned dst, const void *src, bool in) {
     MCSART_ON_COPY(dst, src, N);
     const int n = in ? N : 0;
@@ -837,8 +840,11 @@ __device__ __forceinline__ void fp_slabs_wide(Shared &sm, const Geom &g, int wlo
         const SlabPair &y = sm.pairs[q >> 1];
         if (safe && fp_slab_wide<K, ONES, VT, PAIR>(r, wlo + i0 + q, (f & SC_FAST) != 0, y.dc[q & 1],
                                                     y.a[q & 1], y.b[q & 1], sm.copy[q].o, su, sd,
-                                                    (f & SC_TWO) != 0, base, nz, z_half, acc, accw))
+                                                    (f & SC_TWO) != 0, base, nz, z_half, acc, accw)) {
+            MCSART_ON_FORM(4);
             continue;
+        }
+        MCSART_ON_FORM(5);
         fp_slab_general<K, ONES, VT, PAIR>(r, g, wlo + i0 + q, base, z_half, acc, accw);
     }
     __syncwarp();  // the table may be overwritten now
@@ -867,13 +873,13 @@ __device__ __forceinline__ int middle_out(int i, int n) {
 // WIDE: warps that are not narrow take a loop of their own (fp_slabs_wide): at
 // 256x256x160 with 256x192 cells 1.03 slices high 206 us a call, 354 by the stages'
 // one-by-one form; with cells 1.55 high 250 and 463.  Its code beside the stages
-// costs the narrow warps 0 to 1.5 %, so that the launchers leave it out where cells
-// are low (fp_wide).  The bits are the same.
+// costs the narrow warps 0 to 1.5 %, so that launches leave it out where cells are
+// low (fp_wide).  The bits are the same.
 template <int K> constexpr int fp_stage() { return K >= 3 ? 4 : 8; }
 template <int K> constexpr int fp_min_blocks() { return K >= 3 ? 5 : 6; }
 template <int K, bool ONES, typename VT, typename MT = VT, bool MULTI = false,
           int S = fp_stage<K>(), int NST = 2, int MINB = fp_min_blocks<K>(), bool PAIR = false,
-          bool WIDE = true>
+          bool WIDE = false>
 __global__ void __launch_bounds__(FPC_THREADS, MINB) fp_ref_kernel(const FPArgs<VT, K, MT> p) {
     static_assert(K == 1 || PAIR, "one volume, or three with the last two paired");
     static_assert(32 % S == 0 && S % 2 == 0 && (NST - 1) * S <= 32, "a table holds whole stages");
@@ -1018,12 +1024,14 @@ __global__ void __launch_bounds__(FPC_THREADS, MINB) fp_ref_kernel(const FPArgs<
                 m.y = m.y >> (i0 & 31) & ALL;
                 m.z = m.z >> (i0 & 31) & ALL;
                 if (m.x == ALL) {
+                    MCSART_ON_FORM(0);
 #pragma unroll
                     for (int q = 0; q < S; q += 2)
                         fp_pair_staged<K, ONES, true, VT, PAIR>(rz0, rz1, y[q / 2], true, true,
                                                                 w[q][0], nz, z_half, acc, accw);
                 } else if (m.z == 0) {
                     if (m.y == 0) continue;  // no staged slab: no ray meets the volume
+                    MCSART_ON_FORM(1);
 #pragma unroll
                     for (int q = 0; q < S; q += 2)
                         fp_pair_staged<K, ONES, false, VT, PAIR>(rz0, rz1, y[q / 2], m.y >> q & 1u,
@@ -1042,8 +1050,11 @@ __global__ void __launch_bounds__(FPC_THREADS, MINB) fp_ref_kernel(const FPArgs<
                             fp_slab_direct<K, ONES, VT, PAIR>(
                                 rz0, rz1, yq.dc[q & 1], yq.a[q & 1], yq.b[q & 1],
                                 o - (yq.zb[q & 1] - MK_MAGIC_BITS), su, (f & SC_TWO) != 0,
-                                base, nz, z_half, acc, accw))
+                                base, nz, z_half, acc, accw)) {
+                            MCSART_ON_FORM(2);
                             continue;
+                        }
+                        MCSART_ON_FORM(3);
                         fp_slab_general<K, ONES, VT, PAIR>(rc, g, wlo + i0 + q, base, z_half, acc,
                                                            accw);
                     }
@@ -1138,21 +1149,28 @@ inline bool fp_wide(const Geom &g) {
 template <typename VT, bool PAIR, int S, int NST> constexpr size_t fp_ref_smem() {
     return FPC_COLS * sizeof(FPShared<VT, PAIR, S, NST>);
 }
-template <int K, bool ONES, typename VT, typename MT = VT, bool MULTI = false,
-          int S = fp_stage<K>(), int NST = 2, int MINB = fp_min_blocks<K>(), bool PAIR = false,
-          bool WIDE = true>
-int launch_fp_ref(mcsart_ctx *ctx, dim3 grid, const FPArgs<VT, K, MT> &a) {
+template <int K, bool ONES, typename VT, typename MT, bool MULTI, int S, int NST, int MINB, bool PAIR,
+          bool WIDE>
+int launch_fp_form(mcsart_ctx *ctx, dim3 grid, const FPArgs<VT, K, MT> &a) {
     constexpr size_t smem = fp_ref_smem<VT, PAIR, S, NST>();
     const auto kernel = fp_ref_kernel<K, ONES, VT, MT, MULTI, S, NST, MINB, PAIR, WIDE>;
-    // above 48 KB with the kernel's static arrays a launch needs the larger limit
-    if (smem > 44 * 1024)
-        MC_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem));
+    // with the kernel's static arrays within the 48 KB of any launch
+    static_assert(smem <= 44 * 1024, "a shape of more shared memory needs the limit raised");
     if (!ctx->label) ctx->label = "fp_ref_kernel";
     MC_LAUNCH(ctx, kernel, grid, dim3(FPC_THREADS), smem, a);
     return MCSART_OK;
 }
+// (the wide form in the built-in shape: its loop has no stages)
+template <int K, bool ONES, typename VT, typename MT = VT, bool MULTI = false,
+          int S = fp_stage<K>(), int NST = 2, int MINB = fp_min_blocks<K>(), bool PAIR = false>
+int launch_fp_ref(mcsart_ctx *ctx, dim3 grid, const FPArgs<VT, K, MT> &a) {
+    if (fp_wide(a.g))
+        return launch_fp_form<K, ONES, VT, MT, MULTI, fp_stage<K>(), 2, fp_min_blocks<K>(), PAIR, true>(
+            ctx, grid, a);
+    return launch_fp_form<K, ONES, VT, MT, MULTI, S, NST, MINB, PAIR, false>(ctx, grid, a);
+}
 
+// ------------------------------------------------------------------------
 // The projector from the x-fastest volume itself, a ray per thread, where there is
 // no memory for the z-fastest copy: the plain loops, so the same bits (256x256x160,
 // 512x384: 370-380 us against 113-119).  Grid (ceil(na / 128), nb).

@@ -1,11 +1,15 @@
-// Checks fp_ref_kernel (mcsart_b200/csrc/projector.cuh) on one geometry, in each
+// Checks fp_ref_kernel (mcsart_b200/csrc/projector.cuh) on the geometries read, in each
 // storage type, at the volume pitch given (Geom::nzp): every asynchronous copy's
 // addresses are aligned to its size, and every ray's sum has the bits of the
 // reference's plain loops (fp_slab_general on every slab, a thread per ray).
-// Arguments: nx ny nz nzp na nb SO SD da db ai bi angle.  Prints two counts:
-// misaligned copies, rays that differ.
+// A geometry is a line nx ny nz nzp na nb SO SD da db ai bi angle.  Prints for each two
+// counts, misaligned copies and rays that differ, and how often a warp took each of
+// the forms: stages inside the volume, stages at its edge, slabs of narrow warps by at
+// most two slices, by the general loops, slabs of other warps by at most three
+// slices, by the general loops.
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -15,6 +19,11 @@ __device__ unsigned long long g_misaligned;
     do {                                                                  \
         if ((((unsigned long long)(src)) | (dst)) & ((n) - 1))            \
             atomicAdd(&g_misaligned, 1ull);                               \
+    } while (0)
+__device__ unsigned long long g_forms[6];
+#define MCSART_ON_FORM(form)                                              \
+    do {                                                                  \
+        if (threadIdx.x % 32 == 0) atomicAdd(&g_forms[form], 1ull);       \
     } while (0)
 #include "projector.cuh"
 
@@ -118,19 +127,20 @@ template <int K, typename VT, bool WIDE = true> long long run(const Geom &g, flo
     return bad;
 }
 
-int main(int argc, char **argv) {
-    if (argc != 14) return 2;
+int main() {
     Geom g;
-    g.nx = atoi(argv[1]); g.ny = atoi(argv[2]); g.nz = atoi(argv[3]); g.nzp = atoi(argv[4]);
-    g.na = atoi(argv[5]); g.nb = atoi(argv[6]);
-    g.SO = strtof(argv[7], nullptr); g.SD = strtof(argv[8], nullptr);
-    g.da = strtof(argv[9], nullptr); g.db = strtof(argv[10], nullptr);
-    g.ai = strtof(argv[11], nullptr); g.bi = strtof(argv[12], nullptr);
-    const float angle = strtof(argv[13], nullptr);
-    const long long bad = run<1, float>(g, angle) + run<3, float>(g, angle) + run<1, __half>(g, angle) +
-                          run<3, __nv_bfloat16>(g, angle) + run<1, float, false>(g, angle);
-    unsigned long long mis = 0;
-    CHECK(cudaMemcpyFromSymbol(&mis, g_misaligned, sizeof(mis)));
-    printf("%llu %lld\n", mis, bad);
+    float angle;
+    while (scanf("%d %d %d %d %d %d %f %f %f %f %f %f %f", &g.nx, &g.ny, &g.nz, &g.nzp, &g.na, &g.nb,
+                 &g.SO, &g.SD, &g.da, &g.db, &g.ai, &g.bi, &angle) == 13) {
+        unsigned long long mis = 0, f[6] = {};
+        CHECK(cudaMemcpyToSymbol(g_misaligned, &mis, sizeof(mis)));
+        CHECK(cudaMemcpyToSymbol(g_forms, f, sizeof(f)));
+        const long long bad = run<1, float>(g, angle) + run<3, float>(g, angle) +
+                              run<1, __half>(g, angle) + run<3, __nv_bfloat16>(g, angle) +
+                              run<1, float, false>(g, angle);
+        CHECK(cudaMemcpyFromSymbol(&mis, g_misaligned, sizeof(mis)));
+        CHECK(cudaMemcpyFromSymbol(f, g_forms, sizeof(f)));
+        printf("%llu %lld %llu %llu %llu %llu %llu %llu\n", mis, bad, f[0], f[1], f[2], f[3], f[4], f[5]);
+    }
     return 0;
 }
