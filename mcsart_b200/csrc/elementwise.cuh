@@ -51,9 +51,10 @@ __device__ __forceinline__ float fwd_diff(const T *img0, int64_t id, const Vox &
 }
 
 // The stencil kernels (bound by memory) go through the volume's voxels in memory
-// order (Grid3), so that every lane has a voxel whatever the slices' shape.  With 32 x 32 tiles of a slice (event time of a
-// call, tiles against this): diff 21 and 11 us at 1x4096x64, 179 and 140 us at
-// 512x512x256; initial2 24 and 12 us, 181 and 146 us.
+// order (Grid3), so that every lane has a voxel whatever the slices' shape.  With
+// 32 x 32 tiles of a slice (event time of a call, tiles against this): diff 21 and
+// 11 us at 1x4096x64, 179 and 140 us at 512x512x256; initial2 24 and 12 us, 181 and
+// 146 us.
 // A block is 256 threads of N voxels each, 256 apart, all read before the first is
 // stored: N = 4, or 1 where the GPU holds a thread for every voxel (diff in a
 // chain of launches, N = 4 against 1: 2.3 and 1.8 us at 64x64x64, 2.5 and 2.5 us
