@@ -187,7 +187,7 @@ __device__ __forceinline__ float adj_voxel(const ROW *rows, const float *proj,
     return acc;
 }
 
-// A block is adj_x<ZL>() voxel columns of one row y and ZL slices of them; the lanes
+// A block is adj_x<ZL>() (or fewer, X) voxel columns of one row y and ZL slices of them; the lanes
 // of a warp are the ZL slices of 32 / ZL columns.  The slices of a column share its
 // detector columns and their in-plane weights, and neighbouring slices read
 // neighbouring rows.  Bound by instruction issue.  With a voxel per thread, lanes
@@ -198,11 +198,13 @@ __device__ __forceinline__ float adj_voxel(const ROW *rows, const float *proj,
 // with a 1024x1 detector 44-46 us by eight, 16-29 by one.
 constexpr int ADJ_THREADS = 256;
 template <int ZL> constexpr int adj_x() { return ZL >= 8 ? 32 : ADJ_THREADS / ZL; }
-template <int ZL, typename ROW>
+// X: the block's columns; with 32 a warp goes through one after another, with 8 (small
+// volumes, which do not fill the GPU with such blocks) it has one or two.
+template <int ZL, typename ROW, int X>
 static __global__ void __launch_bounds__(ADJ_THREADS) adj_gather_kernel(
     float *img, const ROW *rows, const float *proj, const AdjColumn *colz, const AdjAxes *axes, const SlabU *slabs,
     const int2 *range, Geom g, int nmax) {
-    constexpr int XL = 32 / ZL, ADJ_X = adj_x<ZL>();
+    constexpr int XL = 32 / ZL, ADJ_X = X;
     __shared__ float tile[ZL][ADJ_X + 1];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const unsigned gx = (g.nx + ADJ_X - 1) / ADJ_X, y = blockIdx.x / gx;
@@ -223,13 +225,18 @@ static __global__ void __launch_bounds__(ADJ_THREADS) adj_gather_kernel(
     }
 }
 
-template <int ZL, typename ROW>
+// Blocks of 32 columns below which 8 are taken: two an SM (32x32x32: 17-19 and 11 us).
+constexpr int ADJ_FEW_BLOCKS = 148 * 2;
+template <int ZL, typename ROW, int X = adj_x<ZL>()>
 static int launch_adj_gather(mcsart_ctx *ctx, float *img, const ROW *rows, const float *proj,
-                             const AdjColumn *colz,
-                             const AdjAxes *axes, const SlabU *slabs, const int2 *range,
-                             const Geom &g, int nmax) {
-    MC_LAUNCH(ctx, (adj_gather_kernel<ZL, ROW>), dim3(div_up(g.nx, adj_x<ZL>()) * (unsigned)g.ny, div_up(g.nz, ZL)),
-              ADJ_THREADS, 0, img, rows, proj, colz, axes, slabs, range, g, nmax);
+                             const AdjColumn *colz, const AdjAxes *axes, const SlabU *slabs,
+                             const int2 *range, const Geom &g, int nmax) {
+    const dim3 grid(div_up(g.nx, X) * (unsigned)g.ny, div_up(g.nz, ZL));
+    if constexpr (X == 32)
+        if ((int64_t)grid.x * grid.y < ADJ_FEW_BLOCKS)
+            return launch_adj_gather<ZL, ROW, 8>(ctx, img, rows, proj, colz, axes, slabs, range, g, nmax);
+    MC_LAUNCH(ctx, (adj_gather_kernel<ZL, ROW, X>), grid, ADJ_THREADS, 0, img, rows, proj, colz, axes,
+              slabs, range, g, nmax);
     return MCSART_OK;
 }
 
