@@ -22,6 +22,14 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU; calls the engine's C ABI")
 
 
+def pytest_collection_modifyitems(items):
+    """Where the rebuilt reference is missing, the tests that need it fail in the
+    ``ref`` fixture; they come last, so that ``-x`` runs all others first."""
+    from oracle import ref_runner
+    if not ref_runner.available():
+        items.sort(key=lambda it: "ref" in getattr(it, "fixturenames", ()))
+
+
 def rel_l2(a, b) -> float:
     """||a - b|| / ||b|| in float64."""
     a = np.asarray(a, np.float64)
