@@ -5,6 +5,7 @@ everything else runs on CPU (oracle, host logic, library loading, gloo ranks).
 """
 from __future__ import annotations
 
+import inspect
 import os
 import sys
 
@@ -23,11 +24,16 @@ def pytest_configure(config):
 
 
 def pytest_collection_modifyitems(items):
-    """Where the rebuilt reference is missing, the tests that need it fail in the
-    ``ref`` fixture; they come last, so that ``-x`` runs all others first."""
+    """Where the rebuilt reference is missing, the tests that call it fail; they
+    come last, so that ``-x`` runs all others first."""
     from oracle import ref_runner
+
+    def calls_reference(item):
+        return ("ref" in getattr(item, "fixturenames", ())
+                or "ref_runner" in inspect.unwrap(item.function).__code__.co_varnames)
+
     if not ref_runner.available():
-        items.sort(key=lambda it: "ref" in getattr(it, "fixturenames", ()))
+        items.sort(key=calls_reference)
 
 
 def rel_l2(a, b) -> float:
